@@ -156,6 +156,11 @@ _SIGNATURES = {
                     _c_int, _c_int, _c_p, _c_int, _c_p],
     "mu_moe_gemm_mma": [_c_p, _c_ll, _c_p, _c_int, _c_p, _c_p, _c_ll, _c_ll, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_p,
                         _c_ll, _c_int, _c_p, _c_int, _c_p],
+    "mu_moe_gather": [_c_p, _c_ll, _c_p, _c_int, _c_int, _c_int, _c_p, _c_p],
+    "mu_moe_gemm_tc": [_c_p, _c_ll, _c_ll, _c_p, _c_p, _c_p, _c_int, _c_p, _c_p, _c_int, _c_int, _c_int, _c_p, _c_ll, _c_int,
+                       _c_int, _c_p, _c_p, _c_p],
+    "mu_heads_gemm_tc": [_c_p, _c_int, _c_ll, _c_ll, _c_p, _c_int, _c_int, _c_int, _c_int, _c_p, _c_ll, _c_ll, _c_int, _c_p,
+                         _c_ll, _c_p, _c_p],
     "mu_heads_gemm": [_c_p, _c_ll, _c_ll, _c_p, _c_ll, _c_ll, _c_int, _c_int, _c_int, _c_int, _c_p, _c_ll, _c_ll, _c_int,
                       _c_p, _c_ll, _c_p],
     "mu_moe_combine": [_c_p, _c_ll, _c_p, _c_p, _c_int, _c_int, _c_int, _c_p, _c_ll, _c_p, _c_p, _c_ll, _c_int, _c_p,
@@ -1119,9 +1124,25 @@ def moe_route(h: torch.Tensor, router: torch.Tensor, correction: Optional[torch.
            ("moe_route(experts={}, top={})", n_experts, top))
 
 
+MOE_TC_ROWS = 128                # tile_rows of the tcgen05 experts' product
+
+
 def moe_tc_ok(x_dtype: torch.dtype, k1: int, k2: int) -> bool:
     """Whether the experts' products of a bfloat16 layer go to the tensor cores (both inner sizes multiples of 8)."""
     return LATENT_TC and x_dtype == torch.bfloat16 and k1 % 8 == 0 and k2 % 8 == 0
+
+
+def moe_gather(x: torch.Tensor, slot_of: torch.Tensor, top: int, out: torch.Tensor) -> torch.Tensor:
+    """out[slot] = x[pair // top] for every (token, expert) pair that has a slot: the rows of the tcgen05 experts' product
+    in the order of its tiles.  bfloat16, rows in whole 16-byte pieces."""
+    _need_cuda(x, slot_of, out)
+    _i32(slot_of, "slot_of")
+    if (x.dtype != torch.bfloat16 or out.dtype != torch.bfloat16 or x.stride(1) != 1 or not out.is_contiguous()
+            or out.shape[0] < slot_of.numel() or out.shape[1] != x.shape[1] or x.shape[0] * top != slot_of.numel()):
+        raise KernelError("moe_gather takes bfloat16 rows, a slot per pair and a contiguous output row per slot")
+    _check(library().mu_moe_gather(_ptr(x), x.stride(0), _ptr(slot_of), slot_of.numel(), int(top), x.shape[1], _ptr(out),
+                                   _stream()), "moe_gather")
+    return out
 
 
 def moe_group(expert_of: torch.Tensor, n_experts: int, slot_of: torch.Tensor, pair_of: torch.Tensor,
@@ -1147,7 +1168,8 @@ def moe_gemm(x: torch.Tensor, pair_of: Optional[torch.Tensor], top: int, w1: tor
     (``act``: None or ``relu2``);
     ``w1``/``w2`` [experts, n, k]; rows of ``x`` by the slot's token (``pair_of``) or by slot.  bfloat16 operands
     with 16-byte aligned rows go to the tensor cores unless ``tensor_cores`` is false.  ``tile_rows``: what
-    ``moe_group`` was given (the CUDA-core product takes its own tile only).  ``row_weight`` (float32, one per pair, or
+    ``moe_group`` was given (the CUDA-core product takes its own tile only; ``MOE_TC_ROWS`` is the tcgen05 product, whose
+    rows of ``x`` are by slot, ``pair_of`` telling only whose row weight a slot has).  ``row_weight`` (float32, one per pair, or
     per slot without ``pair_of``): the row of x is taken times it (the products are, before the activation)."""
     _need_cuda(x, pair_of, w1, w2, tile_info, n_tiles, out, row_weight)
     if row_weight is not None and (row_weight.dtype != torch.float32 or not row_weight.is_contiguous()):
@@ -1164,6 +1186,16 @@ def moe_gemm(x: torch.Tensor, pair_of: Optional[torch.Tensor], top: int, w1: tor
         raise KernelError(f"moe_gemm: activation '{act}' is not taken (relu2 without a second weight stack, or none)")
     code = ACT_CODES[act]
     tile_rows = int(tile_rows) or moe_tile_rows()
+    if tile_rows == MOE_TC_ROWS:
+        # rows by slot (``moe_gather``), tiles of up to 128 of them: the tcgen05 product
+        if not tensor_cores or x.dtype != torch.bfloat16:
+            raise KernelError(f"tiles of {MOE_TC_ROWS} slots are the tensor cores', for bfloat16 rows")
+        _check(library().mu_moe_gemm_tc(_ptr(x), x.shape[0], x.stride(0), _ptr(pair_of), _ptr(w1), _ptr(w2), w1.shape[0],
+                                        _ptr(tile_info), _ptr(n_tiles), int(max_tiles), w1.shape[1], w1.shape[2], _ptr(out),
+                                        out.stride(0), _is_bf16(out), code, _ptr(row_weight),
+                                        status_word(x.device).data_ptr(), _stream()),
+               ("moe_gemm_tc(n={}, k={})", w1.shape[1], w1.shape[2]))
+        return out
     if (tensor_cores and x.dtype == torch.bfloat16 and w1.shape[2] % 8 == 0 and x.stride(0) % 8 == 0
             and x.data_ptr() % 16 == 0 and w1.data_ptr() % 16 == 0 and (w2 is None or w2.data_ptr() % 16 == 0)):
         _check(library().mu_moe_gemm_mma(_ptr(x), x.stride(0), _ptr(pair_of), int(top), _ptr(w1), _ptr(w2),
@@ -1180,6 +1212,9 @@ def moe_gemm(x: torch.Tensor, pair_of: Optional[torch.Tensor], top: int, w1: tor
     return out
 
 
+HEADS_TC_ROWS = 64               # more rows than this a head, and the per-head products go to the tcgen05 kernel
+
+
 def heads_gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, x_head_stride: int, out_head_stride: int,
                gate: Optional[torch.Tensor] = None) -> torch.Tensor:
     """out[t, h, :] = W[h] x[t, h, :] for every row t and head h: ``w`` [heads, n, k]; ``x`` / ``out`` views whose first
@@ -1193,6 +1228,15 @@ def heads_gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, x_head_strid
             and x.stride(0) % 8 == 0 and x_head_stride % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
             and x.stride(1) == 1 and out.stride(1) == 1):
         fused = gate is not None and gate.dtype == torch.bfloat16 and gate.stride(1) == 1 and gate.shape == out.shape
+        if x.shape[0] > HEADS_TC_ROWS and k % 64 == 0 and x.shape[1] >= (heads - 1) * x_head_stride + k:
+            _check(library().mu_heads_gemm_tc(_ptr(x), x.shape[1], x.stride(0), int(x_head_stride), _ptr(w), x.shape[0], heads,
+                                              n, k, _ptr(out), out.stride(0), int(out_head_stride), _is_bf16(out),
+                                              _ptr(gate) if fused else None, gate.stride(0) if fused else 0,
+                                              status_word(x.device).data_ptr(), _stream()),
+                   ("heads_gemm_tc(heads={}, n={}, k={})", heads, n, k))
+            if gate is not None and not fused:
+                sigmoid_gate(out, gate)
+            return out
         _check(library().mu_heads_gemm(_ptr(x), x.stride(0), int(x_head_stride), _ptr(w), w.stride(0), w.stride(1),
                                        x.shape[0], heads, n, k, _ptr(out), out.stride(0), int(out_head_stride),
                                        _is_bf16(out), _ptr(gate) if fused else None, gate.stride(0) if fused else 0,

@@ -111,10 +111,10 @@ class RoutedExperts(FeedForward):
         P = T * top
         gated = self.form == "gated_silu"
         gate_of = ctx.buffer("moe.shared_gate", (T,), torch.float32) if self.shared_gate is not None else None
-        # tiles of 64 slots where the tensor cores take the products and an expert has the rows to fill them
+        # tiles of 128 slots where the tensor cores take the products, their rows gathered first
         tile_rows = self.tile_rows
         if ops.moe_tc_ok(dt, self.hidden_size, self.inner_size) and h.stride(0) % 8 == 0 and h.data_ptr() % 16 == 0:
-            tile_rows = 64 if P >= 48 * E else 32
+            tile_rows = ops.MOE_TC_ROWS
         max_tiles = P // tile_rows + E                     # every grouping of P pairs into E experts fits
         index = ctx.buffer("moe.index", (3 * P + 3 * max_tiles + 4,), torch.int32)
         expert_of, slot_of, pair_of = index[:P], index[P:2 * P], index[2 * P:3 * P]
@@ -126,15 +126,18 @@ class RoutedExperts(FeedForward):
         ops.moe_group(expert_of, self.n_outputs, slot_of, pair_of, tile_info, n_tiles, tile_rows,
                       n_real=E if self.identity else 0)
         ctx.note("route", weight_of)
+        rows = h
+        if tile_rows == ops.MOE_TC_ROWS:
+            rows = ops.moe_gather(h, slot_of, top, ctx.buffer("moe.rows", (P, self.hidden_size), dt))
         hidden = ctx.buffer("moe.hidden", (P, self.inner_size), dt)
         row_weight = None
         if self.weight_on == "input":
             row_weight, weight_of = weight_of, None              # the first product takes the weights, the sum none
         if gated:
-            ops.moe_gemm(h, pair_of, top, self.w_gate, self.w_up, tile_info, n_tiles, max_tiles, hidden, tile_rows=tile_rows,
+            ops.moe_gemm(rows, pair_of, top, self.w_gate, self.w_up, tile_info, n_tiles, max_tiles, hidden, tile_rows=tile_rows,
                          row_weight=row_weight)
         else:
-            ops.moe_gemm(h, pair_of, top, self.w_up, None, tile_info, n_tiles, max_tiles, hidden, tile_rows=tile_rows,
+            ops.moe_gemm(rows, pair_of, top, self.w_up, None, tile_info, n_tiles, max_tiles, hidden, tile_rows=tile_rows,
                          act="relu2", row_weight=row_weight)
         ctx.note("act", hidden)
         y = ctx.buffer("moe.out", (P, self.hidden_size), torch.float32)

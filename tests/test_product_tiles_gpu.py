@@ -37,3 +37,79 @@ def test_float32_tiles(m, n, k):
     assert float((odd[:, 1:n + 1].double() - plain).abs().max() / plain.square().mean().sqrt().clamp_min(1e-30)) < 1e-5
     assert not odd[:, 0].any() and not odd[:, n + 1:].any()
     assert torch.equal(ops.linear(a[m // 2:m // 2 + 1], w, bias), ops.linear(a, w, bias)[m // 2:m // 2 + 1])
+
+
+# tiles of 128 slots: an expert without rows, with one, with exactly a tile and one more; few and many experts; columns and
+# k past a box; identity experts (no slots) and weights on the input
+@pytest.mark.parametrize("form,experts,identity,top,tokens,D,F", [
+    ("gated", 3, 0, 1, 1, 64, 64), ("gated", 5, 0, 2, 300, 200, 136), ("gated", 40, 0, 4, 70, 72, 264),
+    ("relu2", 4, 0, 4, 128, 128, 128), ("relu2", 6, 3, 3, 129, 136, 72), ("relu2", 2, 0, 1, 700, 328, 520),
+    ("relu2", 64, 8, 6, 8, 256, 704)])
+def test_experts_over_tiles_of_128_slots(form, experts, identity, top, tokens, D, F):
+    """bfloat16 operands, float32 sums: the float32 result within 1e-5 of its rms per term's root, the hidden rows within
+    their rounding (2^-8 of a value, and as much of the rms for values near zero)."""
+    ops = _ops()
+    rng = np.random.default_rng(tokens)
+    dt = torch.bfloat16
+    h, gate, up = _rand((tokens, D), 1, dt), _rand((experts, F, D), 2, dt, D ** -0.5), _rand((experts, F, D), 3, dt, D ** -0.5)
+    down = _rand((experts, D, F), 4, dt, F ** -0.5)
+    chosen = np.stack([rng.permutation(experts + identity)[:top] for _ in range(tokens)]).astype(np.int32)
+    if experts > 3:
+        chosen[chosen == 1] = 0                                        # an expert that nobody chose
+    P, rows = tokens * top, ops.MOE_TC_ROWS
+    expert_of = torch.as_tensor(chosen.reshape(-1)).cuda()
+    slot_of, pair_of = (torch.zeros(P, dtype=torch.int32, device="cuda") for _ in range(2))
+    most = P // rows + experts
+    info, n = torch.zeros(3 * most, dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    ops.moe_group(expert_of, experts + identity, slot_of, pair_of, info, n, rows, n_real=experts if identity else 0)
+    xs = ops.moe_gather(h, slot_of, top, torch.zeros((P, D), dtype=dt, device="cuda"))
+    hidden, y = torch.zeros((P, F), dtype=dt, device="cuda"), torch.zeros((P, D), device="cuda")
+    weight = _rand((P,), 5).abs()
+    if form == "gated":
+        ops.moe_gemm(xs, pair_of, top, gate, up, info, n, most, hidden, tile_rows=rows, row_weight=weight)
+    else:
+        ops.moe_gemm(xs, pair_of, top, up, None, info, n, most, hidden, tile_rows=rows, act="relu2")
+    ops.moe_gemm(hidden, None, top, down, None, info, n, most, y, tile_rows=rows)
+    ops.check_status()
+    slots = slot_of.cpu().numpy()
+    assert sorted(s for s in slots if s >= 0) == list(range(int((chosen < experts).sum())))
+    for p in range(P):
+        e = int(chosen.reshape(-1)[p])
+        if e >= experts:
+            assert slots[p] == -1
+    real = torch.as_tensor(np.nonzero(slots >= 0)[0]).cuda()
+    at, e = slot_of[real].long(), expert_of[real].long()
+    x = h[real // top].double()
+    z = torch.einsum("pd,pfd->pf", x, up.double()[e])
+    if form == "gated":
+        z, g = z * weight[real].double()[:, None], torch.einsum("pd,pfd->pf", x, gate.double()[e]) * weight[real].double()[:, None]
+        want = g * torch.sigmoid(g) * z
+    else:
+        want = torch.relu(z) ** 2
+    got = hidden[at].double()
+    rms = want.square().mean().sqrt()
+    assert float(((got - want).abs() / (want.abs() + rms)).max()) < 2.0 ** -8
+    want = torch.einsum("pf,pdf->pd", got, down.double()[e])
+    assert float((y[at].double() - want).abs().max() / want.square().mean().sqrt()) < 1e-5 * max(1.0, math.sqrt(F / 512))
+
+
+# more rows than the small kernel takes, a row past a tile, output columns past a tile, slices with gaps between them
+@pytest.mark.parametrize("rows,heads,n,k,lead", [(65, 3, 128, 64, 32), (129, 2, 40, 128, 0), (300, 5, 264, 64, 8), (128, 1, 512, 192, 0)])
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+def test_products_per_head_on_tcgen05(rows, heads, n, k, lead, out_dtype):
+    ops = _ops()
+    xs, os_ = k + lead, n + 8
+    x, w = _rand((rows, heads * xs), 1, torch.bfloat16), _rand((heads, n, k), 2, torch.bfloat16, k ** -0.5)
+    gate = _rand((rows, heads * os_), 3, torch.bfloat16)
+    for g in (None, gate):
+        out = torch.zeros((rows, heads * os_), device="cuda", dtype=out_dtype)
+        ops.heads_gemm(x, w, out, xs, os_, gate=g)
+        ops.check_status()
+        want = torch.einsum("thk,hnk->thn", x.double().reshape(rows, heads, xs)[:, :, :k], w.double())
+        if g is not None:
+            want = want * torch.sigmoid(g.double().reshape(rows, heads, os_)[:, :, :n])
+        got = out.reshape(rows, heads, os_)
+        if g is None:
+            assert not got[:, :, n:].any()                             # nothing written between the slices
+        bound = 1e-5 if out_dtype == torch.float32 else 2.0 ** -8
+        assert float(((got[:, :, :n].double() - want).abs() / (want.abs() + want.square().mean().sqrt())).max()) < bound
