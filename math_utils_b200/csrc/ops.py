@@ -156,6 +156,12 @@ _SIGNATURES = {
                     _c_int, _c_int, _c_p, _c_int, _c_p],
     "mu_moe_gemm_mma": [_c_p, _c_ll, _c_p, _c_int, _c_p, _c_p, _c_ll, _c_ll, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_p,
                         _c_ll, _c_int, _c_p, _c_int, _c_p],
+    "mu_chunk_scan_fits": [_c_int, _c_int],
+    "mu_chunk_scan_scratch": [_c_int] * 5,
+    "mu_linear_scan_chunks": [_c_p, _c_p, _c_p, _c_ll, _c_p, _c_p, _c_int, _c_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_f,
+                              _c_p, _c_p, _c_p, _c_p, _c_ll, _c_ll, _c_p, _c_ll, _c_p, _c_p],
+    "mu_ssd_scan_chunks": [_c_p, _c_int, _c_p, _c_ll, _c_int, _c_p, _c_p, _c_p, _c_p, _c_int, _c_p, _c_int, _c_int, _c_int,
+                           _c_int, _c_int, _c_int, _c_p, _c_p, _c_p, _c_p, _c_ll, _c_ll, _c_p, _c_p],
     "mu_moe_gather": [_c_p, _c_ll, _c_p, _c_int, _c_int, _c_int, _c_p, _c_p],
     "mu_moe_gemm_tc": [_c_p, _c_ll, _c_ll, _c_p, _c_p, _c_p, _c_int, _c_p, _c_p, _c_int, _c_int, _c_int, _c_p, _c_ll, _c_int,
                        _c_int, _c_p, _c_p, _c_p],
@@ -652,6 +658,44 @@ def ssd_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias, a_log, skip, n_he
     return out
 
 
+def chunk_scan_ok(dk: int, dv: int) -> bool:
+    """Whether ``linear_scan_chunks`` and ``ssd_scan_chunks`` take keys and values of these sizes."""
+    return bool(library().mu_chunk_scan_fits(int(dk), int(dv)))
+
+
+def _chunk_scratch(device, n_tokens: int, n_seqs: int, n_heads: int, dk: int, dv: int) -> torch.Tensor:
+    lib = library()
+    lib.mu_chunk_scan_scratch.restype = _c_ll
+    return scratch("chunk_scan", device, int(lib.mu_chunk_scan_scratch(n_tokens, n_seqs, n_heads, dk, dv)), torch.float32)
+
+
+def ssd_scan_chunks(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias, a_log, skip, n_heads: int, head_dim: int, n_state: int,
+                    groups: int, tiles: torch.Tensor, tok_seq, seq_first, seq_slots, state: torch.Tensor, state_offset: int,
+                    out: torch.Tensor) -> torch.Tensor:
+    """``ssd_scan`` for steps of many tokens, chunk by chunk on tensor cores; ``tiles``: the step's query tiles (int32
+    [n, 2])."""
+    _need_cuda(xbc, dt_raw, dt_bias, a_log, skip, tiles, tok_seq, seq_first, seq_slots, state, out)
+    for t, name in ((tiles, "tiles"), (tok_seq, "tok_seq"), (seq_first, "seq_first"), (seq_slots, "seq_slots")):
+        _i32(t, name)
+    inner, T, n_seqs = n_heads * head_dim, xbc.shape[0], seq_slots.numel()
+    if (xbc.dtype != torch.float32 or not xbc.is_contiguous() or xbc.shape[1] != inner + 2 * groups * n_state
+            or dt_raw.stride(1) != 1 or tuple(dt_raw.shape) != (T, n_heads) or out.dtype != torch.float32
+            or not out.is_contiguous() or out.shape != (T, inner) or state.dtype != torch.float32 or state.stride(1) != 1
+            or state.shape[1] < state_offset + inner * n_state):
+        raise KernelError("ssd_scan_chunks: inputs, state or output do not fit")
+    for t in (dt_bias, a_log, skip):
+        if t.dtype != torch.float32 or t.numel() != n_heads or not t.is_contiguous():
+            raise KernelError("ssd_scan_chunks: one float32 per head for dt_bias, A_log and D")
+    room = _chunk_scratch(xbc.device, T, n_seqs, n_heads, n_state, head_dim)
+    _check(library().mu_ssd_scan_chunks(_ptr(xbc), xbc.shape[1], _ptr(dt_raw), dt_raw.stride(0), _is_bf16(dt_raw), _ptr(dt_bias),
+                                        _ptr(a_log), _ptr(skip), _ptr(tiles), tiles.shape[0], _ptr(tok_seq), T, n_seqs,
+                                        int(n_heads), int(head_dim), int(n_state), int(groups), _ptr(seq_first),
+                                        _ptr(seq_slots), _ptr(room), _ptr(state), state.stride(0), int(state_offset), _ptr(out),
+                                        _stream()), ("ssd_scan_chunks(heads={}, P={}, N={})", n_heads, head_dim, n_state),
+           launches=3)
+    return out
+
+
 def selective_scan_max_state() -> int:
     return int(library().mu_selective_scan_max_state())
 
@@ -875,6 +919,35 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.
                                     out.stride(0), _ptr(norm_out), int(T > 4 * seq_slots.numel()), _stream(),
                                     0 if constant else 4 * n_heads, int(silu_rows)),
            ("linear_scan(heads={}, dk={}, dv={})", n_heads, dk, dv))
+    return out
+
+
+def linear_scan_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, gates: torch.Tensor, n_heads: int, dk: int, dv: int,
+                       scale: float, tiles: torch.Tensor, tok_seq, seq_first, seq_slots, state: torch.Tensor,
+                       state_offset: int, out: torch.Tensor, norm_out: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """``linear_scan`` with gates [T, heads, 4] for steps of many tokens, chunk by chunk on tensor cores; ``tiles``: the
+    step's query tiles (int32 [n, 2])."""
+    _need_cuda(q, k, v, gates, tiles, tok_seq, seq_first, seq_slots, state, out, norm_out)
+    for t, name in ((tiles, "tiles"), (tok_seq, "tok_seq"), (seq_first, "seq_first"), (seq_slots, "seq_slots")):
+        _i32(t, name)
+    T, n_seqs = q.shape[0], seq_slots.numel()
+    for t, n in ((q, n_heads * dk), (k, n_heads * dk), (v, n_heads * dv)):
+        if t.dtype != torch.float32 or tuple(t.shape) != (T, n) or t.stride(1) != 1 or t.stride(0) != q.stride(0):
+            raise KernelError("linear_scan_chunks: queries, keys and values are float32 column blocks of one buffer")
+    values = n_heads * dk * (dv + (1 if norm_out is not None else 0))
+    if (tuple(gates.shape) != (T, n_heads, 4) or gates.dtype != torch.float32 or not gates.is_contiguous()
+            or out.dtype != torch.float32 or out.stride(1) != 1 or tuple(out.shape) != (T, n_heads * dv)
+            or state.dtype != torch.float32 or state.stride(1) != 1 or state.shape[1] < state_offset + values):
+        raise KernelError("linear_scan_chunks: gates, state or output do not fit")
+    if norm_out is not None and (norm_out.dtype != torch.float32 or not norm_out.is_contiguous()
+                                 or tuple(norm_out.shape) != (T, n_heads)):
+        raise KernelError("linear_scan_chunks: the normalizer's read-out is contiguous float32 [T, heads]")
+    room = _chunk_scratch(q.device, T, n_seqs, n_heads, dk, dv)
+    _check(library().mu_linear_scan_chunks(_ptr(q), _ptr(k), _ptr(v), q.stride(0), _ptr(gates), _ptr(tiles), tiles.shape[0],
+                                           _ptr(tok_seq), T, n_seqs, int(n_heads), int(dk), int(dv), float(scale),
+                                           _ptr(seq_first), _ptr(seq_slots), _ptr(room), _ptr(state), state.stride(0),
+                                           int(state_offset), _ptr(out), out.stride(0), _ptr(norm_out), _stream()),
+           ("linear_scan_chunks(heads={}, dk={}, dv={})", n_heads, dk, dv), launches=3)
     return out
 
 

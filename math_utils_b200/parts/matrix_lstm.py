@@ -12,7 +12,9 @@ With a running maximum m that starts at zero, m <- max(f + m, i), the state is k
     o = S^T q / (max(|n . q|, exp(-m)) + 1e-6).
 Each head's o is brought to unit rms over vdim; the heads side by side are multiplied by a weight of all heads' size
 and by sigmoid(G x), and go through the output matrix.  S, n and m are float32 and live in the sequence's cache slot;
-gates and recurrence are float32, and so are the rows the projections leave for them.
+gates and recurrence are float32, and so are the rows the projections leave for them.  In bfloat16 models the recurrence
+of prompt steps goes chunk by chunk over tensor cores (``ops.linear_scan_chunks``), every operand at 22 bits; single tokens,
+short runs and the 32-bit path go token by token (``ops.linear_scan``).
 """
 from __future__ import annotations
 
@@ -61,7 +63,11 @@ class MatrixLstm(Mixer):
         self.columns = tuple(m.shape[0] for m in mats)
         self.proj = Linear(torch.cat(mats, dim=0).contiguous(), None, runtime)
         self.out = Linear(t("out"), None, runtime)
+        # 16-byte pieces everywhere: rows of the stacked product, a slot's state (both padded to them), keys and values
+        self.chunked = runtime.dtype == torch.bfloat16 and runtime.ops.chunk_scan_ok(self.dim, self.vdim)
         self.i_bias, self.f_bias, self.norm_weight = t("i_bias"), t("f_bias"), t("norm")
+
+    CHUNKED_TOKENS = 32              # tokens a sequence brings on average from which on the chunked form pays
 
     def forward(self, h, residual, ctx, cache, owns_cache: bool, accumulate: bool = True) -> None:
         ops, T, H = self.runtime.ops, ctx.n_tokens, self.n_heads
@@ -75,8 +81,12 @@ class MatrixLstm(Mixer):
                       self.m_offset, gates)
         o = ctx.buffer("mlstm.o", (T, self.inner), torch.float32)
         read = ctx.buffer("mlstm.normalizer", (T, H), torch.float32)
-        ops.linear_scan(q, k, v, gates, H, self.dim, self.vdim, self.dim ** -0.5, ctx.seq_first, ctx.seq_slots, cache.values,
-                        0, o, norm_out=read)
+        if self.chunked and ctx.q_tiles is not None and T >= self.CHUNKED_TOKENS * ctx.n_seqs:
+            ops.linear_scan_chunks(q, k, v, gates, H, self.dim, self.vdim, self.dim ** -0.5, ctx.q_tiles, ctx.tok_seq,
+                                   ctx.seq_first, ctx.seq_slots, cache.values, 0, o, norm_out=read)
+        else:
+            ops.linear_scan(q, k, v, gates, H, self.dim, self.vdim, self.dim ** -0.5, ctx.seq_first, ctx.seq_slots,
+                            cache.values, 0, o, norm_out=read)
         ctx.note("scan", o)
         gated = ctx.buffer("mlstm.gated", (T, self.inner), self.runtime.dtype)
         ops.gated_group_norm(o, gate, self.norm_weight, H, self.eps, gated, gate_after=True, sigmoid=True, den=read,

@@ -10,7 +10,9 @@ tap is the current token's) and silu.  dt = softplus(dt + dt_bias).  Per head, w
 The heads' y, side by side, is multiplied by silu(z), brought to unit rms in ``norm_groups`` equal parts, multiplied
 by a weight, and goes through the output matrix.  A sequence's state (the convolution's last taps - 1 inputs and
 every head's S) is float32 and lives in the sequence's cache slot; decays, step sizes and the recurrence are
-float32 whatever the compute dtype.
+float32 whatever the compute dtype.  In bfloat16 models the recurrence of prompt steps goes chunk by chunk over tensor
+cores (``ops.ssd_scan_chunks``), every operand at 22 bits; single tokens, short runs and the 32-bit path go token by token
+(``ops.ssd_scan``).
 """
 from __future__ import annotations
 
@@ -58,7 +60,12 @@ class StateSpaceMixer(Mixer):
         self.proj = Linear(t("in"), None, runtime)
         self.out = Linear(t("out"), None, runtime)
         self.conv_weight, self.conv_bias = t("conv"), t("conv_bias")
+        # the chunked form stages 16-byte pieces: of the convolved rows, of a slot's state and of its offset
+        self.chunked = (runtime.dtype == torch.bfloat16 and runtime.ops.chunk_scan_ok(self.state, self.head_dim)
+                        and self.channels % 4 == 0 and self.inner % 4 == 0)
         self.dt_bias, self.a_log, self.skip, self.norm_weight = t("dt_bias"), t("A_log"), t("D"), t("norm")
+
+    CHUNKED_TOKENS = 32              # tokens a sequence brings on average from which on the chunked form pays
 
     def forward(self, h, residual, ctx, cache, owns_cache: bool, accumulate: bool = True) -> None:
         ops, dt = self.runtime.ops, self.runtime.dtype
@@ -72,8 +79,12 @@ class StateSpaceMixer(Mixer):
         ops.ssd_conv(conv_in, self.conv_weight, self.conv_bias, ctx.tok_seq, ctx.seq_first, ctx.seq_slots, cache.values,
                      ctx.is_decode, xbc)
         y = ctx.buffer("ssd.y", (T, inner), torch.float32)
-        ops.ssd_scan(xbc, dt_raw, self.dt_bias, self.a_log, self.skip, self.n_heads, self.head_dim, self.state,
-                     self.groups, ctx.seq_first, ctx.seq_slots, cache.values, self.tail_values, y)
+        recurrence = (xbc, dt_raw, self.dt_bias, self.a_log, self.skip, self.n_heads, self.head_dim, self.state, self.groups)
+        if self.chunked and ctx.q_tiles is not None and T >= self.CHUNKED_TOKENS * ctx.n_seqs:
+            ops.ssd_scan_chunks(*recurrence, ctx.q_tiles, ctx.tok_seq, ctx.seq_first, ctx.seq_slots, cache.values,
+                                self.tail_values, y)
+        else:
+            ops.ssd_scan(*recurrence, ctx.seq_first, ctx.seq_slots, cache.values, self.tail_values, y)
         ctx.note("scan", y)
         gated = ctx.buffer("ssd.gated", (T, inner), dt)
         ops.gated_group_norm(y, z, self.norm_weight, self.norm_groups, self.eps, gated)

@@ -1,0 +1,116 @@
+"""The recurrences taken chunk by chunk against float64 and against their token-by-token kernels, at the edges of the chunks."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+LENS = [(64,), (1, 130), (63, 65, 200), (700,), (129, 2, 64, 31)]
+
+
+def _ops():
+    from math_utils_b200.csrc import ops
+    return ops
+
+
+def _ints(x):
+    return torch.as_tensor(np.asarray(x, dtype=np.int32)).cuda()
+
+
+def _step(lens):
+    first = np.concatenate([[0], np.cumsum(lens)])
+    tiles = [(first[s] + o, min(64, n - o)) for s, n in enumerate(lens) for o in range(0, n, 64)]
+    return _ints(tiles[::-1]), _ints(np.repeat(np.arange(len(lens)), lens)), _ints(first), first
+
+
+def _rand(shape, seed, scale=1.0):
+    return torch.randn(shape, generator=torch.Generator(device="cuda").manual_seed(seed), device="cuda") * scale
+
+
+def _rel(got, want):
+    return float((got.double() - want).norm() / want.norm())
+
+
+def _no_further_off(chunks, token_by_token, want):
+    """Operands at 22 bits: a term is off by some 2^-22 of itself, no more than a running sum of hundreds of float32 terms;
+    held to 1e-6 and to twice what the token-by-token kernel shows."""
+    assert _rel(chunks, want) < max(1e-6, 2.0 * _rel(token_by_token, want))
+
+
+@pytest.mark.parametrize("lens", LENS)
+@pytest.mark.parametrize("H,dk,dv,norm", [(2, 128, 128, True), (3, 16, 4, True), (1, 48, 100, False), (2, 96, 200, True)])
+def test_linear_scan_in_chunks(lens, H, dk, dv, norm):
+    ops = _ops()
+    tiles, tok_seq, seq_first, first = _step(lens)
+    T, slots = sum(lens), list(range(len(lens)))[::-1]
+    u = _rand((T, H * (2 * dk + dv) + 4), 1)
+    q, k, v = u[:, :H * dk], u[:, H * dk:2 * H * dk], u[:, 2 * H * dk:2 * H * dk + H * dv]
+    decay = torch.rand((T, H), generator=torch.Generator(device="cuda").manual_seed(2), device="cuda")
+    decay = 1.0 - 0.1 * decay ** 3                               # memories of ten tokens to thousands
+    decay[T // 2] = 0.0                                          # all that was is forgotten
+    gates = torch.zeros((T, H, 4), device="cuda")
+    gates[..., 0], gates[..., 1] = decay, _rand((T, H), 3).abs()
+    values = H * dk * (dv + (1 if norm else 0))
+    start = _rand((len(lens), values + -values % 4), 4, 0.3)
+    scale = dk ** -0.5
+    got = {}
+    for name in ("chunks", "tokens"):
+        state, out = start.clone(), torch.zeros((T, H * dv), device="cuda")
+        read = torch.zeros((T, H), device="cuda") if norm else None
+        if name == "chunks":
+            ops.linear_scan_chunks(q, k, v, gates, H, dk, dv, scale, tiles, tok_seq, seq_first, _ints(slots), state, 0, out, read)
+        else:
+            ops.linear_scan(q, k, v, gates, H, dk, dv, scale, seq_first, _ints(slots), state, 0, out, norm_out=read)
+        got[name] = (out, state[:, :values], read)
+    want_out = torch.zeros((T, H, dv + 1), dtype=torch.float64, device="cuda")
+    want_state = start[:, :values].double().clone()
+    for s, slot in enumerate(slots):
+        held = start[slot, :values].double()
+        S = held[:H * dk * dv].reshape(H, dv, dk)
+        n = held[H * dk * dv:].reshape(H, 1, dk) if norm else torch.zeros((H, 1, dk), dtype=torch.float64, device="cuda")
+        S = torch.cat([S, n], 1)
+        for t in range(first[s], first[s + 1]):
+            vt = torch.cat([v[t].double().reshape(H, dv), torch.ones((H, 1), dtype=torch.float64, device="cuda")], 1)
+            S = S * gates[t, :, 0].double()[:, None, None] + (gates[t, :, 1].double()[:, None] * vt)[:, :, None] * k[t].double().reshape(H, 1, dk)
+            want_out[t] = scale * torch.einsum("hvd,hd->hv", S, q[t].double().reshape(H, dk))
+        want_state[slot] = torch.cat([S[:, :dv].reshape(-1)] + ([S[:, dv].reshape(-1)] if norm else []))
+    _no_further_off(got["chunks"][0], got["tokens"][0], want_out[..., :dv].reshape(T, H * dv))
+    _no_further_off(got["chunks"][1], got["tokens"][1], want_state)
+    if norm:
+        _no_further_off(got["chunks"][2], got["tokens"][2], want_out[..., dv])
+
+
+@pytest.mark.parametrize("lens", LENS)
+@pytest.mark.parametrize("H,P,N,G,dtype", [(4, 64, 128, 1, torch.bfloat16), (2, 4, 16, 2, torch.float32), (6, 100, 48, 2, torch.bfloat16)])
+def test_state_space_scan_in_chunks(lens, H, P, N, G, dtype):
+    ops = _ops()
+    tiles, tok_seq, seq_first, first = _step(lens)
+    T, slots, inner = sum(lens), list(range(len(lens)))[::-1], H * P
+    xbc = _rand((T, inner + 2 * G * N), 1)
+    dt_raw = _rand((T, H + 3), 2).to(dtype)[:, :H]
+    dt_bias, skip = _rand((H,), 3) - 3.0, _rand((H,), 4)
+    a_log = torch.log(1.0 + 7.0 * torch.rand((H,), generator=torch.Generator(device="cuda").manual_seed(5), device="cuda"))
+    offset = 8
+    start = _rand((len(lens), offset + H * N * P), 6, 0.3)
+    got = {}
+    for name in ("chunks", "tokens"):
+        state, y = start.clone(), torch.zeros((T, inner), device="cuda")
+        if name == "chunks":
+            ops.ssd_scan_chunks(xbc, dt_raw, dt_bias, a_log, skip, H, P, N, G, tiles, tok_seq, seq_first, _ints(slots), state, offset, y)
+        else:
+            ops.ssd_scan(xbc, dt_raw, dt_bias, a_log, skip, H, P, N, G, seq_first, _ints(slots), state, offset, y)
+        got[name] = (y, state)
+    want_state, want = start.double().clone(), torch.zeros((T, inner), dtype=torch.float64, device="cuda")
+    dt = torch.nn.functional.softplus(dt_raw.double() + dt_bias.double(), threshold=200.0)
+    decay = torch.exp(-torch.exp(a_log.double()) * dt)
+    x = xbc.double()
+    for s, slot in enumerate(slots):
+        S = start[slot, offset:].double().reshape(H, N, P)
+        for t in range(first[s], first[s + 1]):
+            B, C = (x[t, a:a + G * N].reshape(G, N).repeat_interleave(H // G, 0) for a in (inner, inner + G * N))
+            xt = x[t, :inner].reshape(H, P)
+            S = S * decay[t][:, None, None] + (dt[t][:, None] * B)[:, :, None] * xt[:, None, :]
+            want[t] = (torch.einsum("hnp,hn->hp", S, C) + skip.double()[:, None] * xt).reshape(-1)
+        want_state[slot, offset:] = S.reshape(-1)
+    _no_further_off(got["chunks"][0], got["tokens"][0], want)
+    _no_further_off(got["chunks"][1], got["tokens"][1], want_state)
