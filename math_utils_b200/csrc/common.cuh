@@ -137,6 +137,15 @@ template <int N> __device__ __forceinline__ void copy_async_wait() { asm volatil
 
 __device__ __forceinline__ float softplus(float z) { return fmaxf(z, 0.0f) + log1pf(expf(-fabsf(z))); }
 
+// cap * tanh(s / cap): the series near zero (five terms, to 0.3, where the next one is 5e-8 of the sum), beyond it
+// 1 - 2 / (e^(2y) + 1) with the fast exponential, where the result is no smaller than 0.29.
+__device__ __forceinline__ float softcap_fast(float s, float cap, float inv_cap) {
+    const float y = s * inv_cap, a = fabsf(y), y2 = y * y;
+    const float near = y * fmaf(y2, fmaf(y2, fmaf(y2, fmaf(y2, 62.0f / 2835.0f, -17.0f / 315.0f), 2.0f / 15.0f), -1.0f / 3.0f), 1.0f);
+    const float far = copysignf(1.0f - __fdividef(2.0f, __expf(2.0f * fminf(a, 40.0f)) + 1.0f), y);
+    return cap * (a < 0.3f ? near : far);
+}
+
 // --- programmatic dependent launch -------------------------------------------------------
 // Kernels of the single-token step are launched so that the next one may start while the
 // previous one drains: it runs its prologue (index arithmetic, prefetch of weights, which

@@ -20,15 +20,6 @@ namespace mu {
 constexpr int MM_TILE = 64;       // queries per block, keys per page
 constexpr int MM_PAD = 8;         // entries between rows in shared memory: ldmatrix without bank conflicts
 
-// cap * tanh(s / cap): the series near zero (five terms, to 0.3, where the next one is 5e-8 of the sum), beyond it
-// 1 - 2 / (e^(2y) + 1) with the fast exponential, where the result is no smaller than 0.29.
-__device__ __forceinline__ float softcap_fast(float s, float cap, float inv_cap) {
-    const float y = s * inv_cap, a = fabsf(y), y2 = y * y;
-    const float near = y * fmaf(y2, fmaf(y2, fmaf(y2, fmaf(y2, 62.0f / 2835.0f, -17.0f / 315.0f), 2.0f / 15.0f), -1.0f / 3.0f), 1.0f);
-    const float far = copysignf(1.0f - __fdividef(2.0f, __expf(2.0f * fminf(a, 40.0f)) + 1.0f), y);
-    return cap * (a < 0.3f ? near : far);
-}
-
 // VD: the head's value entries rounded up to 32, 64 or 128 (columns past vdim are zeros in shared memory).
 template <int MAPS, int VD>
 __global__ void __launch_bounds__(128, 1)

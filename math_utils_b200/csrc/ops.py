@@ -156,6 +156,10 @@ _SIGNATURES = {
                     _c_int, _c_int, _c_p, _c_int, _c_p],
     "mu_moe_gemm_mma": [_c_p, _c_ll, _c_p, _c_int, _c_p, _c_p, _c_ll, _c_ll, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_p,
                         _c_ll, _c_int, _c_p, _c_int, _c_p],
+    "mu_mapped_attention_tc_fits": [_c_int] * 6,
+    "mu_mapped_attention_tc": [_c_p, _c_ll, _c_int, _c_p, _c_ll, _c_p, _c_int, _c_int, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int,
+                               _c_int, _c_int, _c_int, _c_f, _c_int, _c_f, _c_f, _c_f, _c_int, _c_p, _c_ll, _c_p, _c_p,
+                               _c_p, _c_int, _c_p, _c_ll, _c_int, _c_p, _c_int, _c_f, _c_int, _c_int, _c_p, _c_int],
     "mu_chunk_scan_fits": [_c_int, _c_int],
     "mu_chunk_scan_scratch": [_c_int] * 5,
     "mu_linear_scan_chunks": [_c_p, _c_p, _c_p, _c_ll, _c_p, _c_p, _c_int, _c_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_f,
@@ -534,6 +538,15 @@ def qk_prepare(q: torch.Tensor, k: Optional[torch.Tensor], v: Optional[torch.Ten
            ("qk_prepare(dim={}, maps={})", dim, maps))
 
 
+def mapped_tc_ok(q: torch.Tensor, out: torch.Tensor, n_kv_heads: int, maps: int, dim: int, vdim: int, page_tokens: int,
+                 shared: bool = False) -> bool:
+    """Whether ``mapped_attention`` takes the tcgen05 kernel for these queries (bfloat16 rows given wide tiles)."""
+    return (MAPPED_TC and q.dtype == torch.bfloat16 and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0
+            and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0
+            and bool(library().mu_mapped_attention_tc_fits(int(n_kv_heads), int(maps), int(dim), int(vdim), int(page_tokens),
+                                                           int(shared))))
+
+
 def mapped_attention(q: torch.Tensor, rows: torch.Tensor, block_table: torch.Tensor, page_tokens: int, tok_pos, tok_seq,
                      n_heads: int, n_kv_heads: int, maps: int, dim: int, vdim: int, scale: float, window: int,
                      out: torch.Tensor, lam: float = 0.0, out_scale: float = 1.0, eps: float = 0.0,
@@ -541,7 +554,8 @@ def mapped_attention(q: torch.Tensor, rows: torch.Tensor, block_table: torch.Ten
                      tensor_cores: Optional[bool] = None, single_tokens: bool = False,
                      head_scale: Optional[torch.Tensor] = None, sink: bool = False,
                      gate: Optional[torch.Tensor] = None, chunk: int = 0, slopes: Optional[torch.Tensor] = None,
-                     keep: int = 0, softcap: float = 0.0, shared: bool = False) -> torch.Tensor:
+                     keep: int = 0, softcap: float = 0.0, shared: bool = False,
+                     tiles_wide: Optional[torch.Tensor] = None, head_sink: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Softmax attention of every (token, head) over the cached rows it sees (``window`` 0: all up to its own
     position), one result per score map over the same values; with two maps a1 - lam * a2.  ``unit_rms`` brings
     each head's result to unit rms (eps inside the root); ``out_scale`` multiplies it.
@@ -556,7 +570,10 @@ def mapped_attention(q: torch.Tensor, rows: torch.Tensor, block_table: torch.Ten
     multiplies each head's result by sigmoid(gate[t, h]), or as [T, heads * vdim] entry by entry; ``chunk`` c > 0 replaces the window: position p sees
     p - p % c .. p; ``slopes`` (float32, one per head): a key at distance n loses slopes[h] * n of its score;
     ``keep`` (with a window): the sequence's first ``keep`` positions stay in sight; ``softcap`` c > 0 makes a scaled score s
-    c * tanh(s / c) before anything is taken off it; ``shared``: the rows hold keys alone, which are the values too."""
+    c * tanh(s / c) before anything is taken off it; ``shared``: the rows hold keys alone, which are the values too.
+
+    ``tiles_wide`` (as ``tiles``, in runs of up to 128 tokens) lets the step take the tcgen05 kernel where it fits
+    (``mapped_tc_ok``); ``head_sink`` (float32, one per head; that kernel only): the sink's score, not scaled."""
     _need_cuda(q, rows, block_table, tok_pos, tok_seq, out, head_scale, gate, slopes)
     if slopes is not None and (slopes.dtype != torch.float32 or slopes.numel() != n_heads or not slopes.is_contiguous()):
         raise KernelError("mapped_attention: slopes are one contiguous float32 per head")
@@ -594,6 +611,22 @@ def mapped_attention(q: torch.Tensor, rows: torch.Tensor, block_table: torch.Ten
         return out
     if tensor_cores is None:
         tensor_cores = MAPPED_TC
+    if head_sink is not None and (head_sink.dtype != torch.float32 or head_sink.numel() != n_heads or not head_sink.is_contiguous()):
+        raise KernelError("mapped_attention: head_sink is one contiguous float32 per head")
+    if (tensor_cores and tiles_wide is not None and rows.dtype == torch.bfloat16
+            and mapped_tc_ok(q, out, n_kv_heads, maps, dim, vdim, page_tokens, shared)
+            and not (gate_each and (gate.stride(0) % 2 or gate.data_ptr() % 4))):
+        _need_cuda(tiles_wide, head_sink)
+        _i32(tiles_wide, "tiles_wide")
+        _check(library().mu_mapped_attention_tc(
+            _ptr(q), q.stride(0), q.shape[0], _ptr(rows), rows.shape[0], _ptr(block_table), block_table.shape[1],
+            int(page_tokens), _ptr(tok_pos), _ptr(tok_seq), _ptr(tiles_wide), tiles_wide.shape[0], int(n_heads), int(n_kv_heads),
+            int(maps), int(dim), int(vdim), float(scale), int(window), float(lam), float(out_scale), float(eps), int(unit_rms),
+            _ptr(out), out.stride(0), status_word(q.device).data_ptr(), _stream(), *extras, _ptr(head_sink), 0),
+            ("mapped_attention_tc(heads={}/{}, maps={}, dim={}, vdim={})", n_heads, n_kv_heads, maps, dim, vdim))
+        return out
+    if head_sink is not None:
+        raise KernelError("mapped_attention: sinks with a score per head need the tcgen05 kernel")
     if (tensor_cores and tiles is not None and rows.dtype == torch.bfloat16 and q.stride(0) % 8 == 0
             and out.stride(0) % 2 == 0 and q.data_ptr() % 16 == 0 and out.data_ptr() % 4 == 0
             and not (gate_each and (gate.stride(0) % 2 or gate.data_ptr() % 4))

@@ -187,6 +187,7 @@ class MappedAttention(Mixer):
                              self.n_kv_heads, self.maps, self.dim, self.vdim, self.scale, self.window, heads,
                              lam=self.lam, out_scale=self.out_scale, eps=self.eps, unit_rms=self.maps == 2,
                              tiles=None if ctx.is_decode else ctx.q_tiles, single_tokens=ctx.is_decode,
+                             tiles_wide=None if ctx.is_decode else ctx.q_tiles_wide,
                              gate=gate, chunk=self.chunk, slopes=self.slope_table, keep=self.keep,
                              sink=self.sink, softcap=self.softcap, shared=self.shared_rows)
         ctx.note("attn", heads)

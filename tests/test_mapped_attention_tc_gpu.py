@@ -1,0 +1,113 @@
+"""Prompt attention with score maps on tcgen05 against float64: tiles of 128 queries whose last is short, steps that bring only
+a sequence's last tokens, edges of windows, chunks and kept positions, every option of the kernel."""
+import math
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+LENS, NEW = [130, 1, 64, 129, 7, 500, 257], [130, 1, 64, 3, 7, 270, 257]
+
+
+def _rand(shape, seed, scale=1.0):
+    return (torch.randn(shape, generator=torch.Generator(device="cuda").manual_seed(seed), device="cuda") * scale).to(torch.bfloat16)
+
+
+def _ints(x):
+    return torch.as_tensor(np.asarray(x, dtype=np.int32)).cuda()
+
+
+def _case(H, G, maps, dim, vdim, window=0, chunk=0, keep=0, shared=False, softcap=0.0, sink=False, slopes=False, gate=None,
+          head_scale=False, head_sink=False, unit=False):
+    return locals()
+
+
+CASES = [
+    _case(2, 1, 2, 64, 128, window=100, unit=True),
+    _case(3, 3, 2, 16, 48, unit=True, window=300),
+    _case(2, 2, 2, 128, 128),                                   # 256 key entries a head: two stages of pages
+    _case(4, 2, 1, 128, 128, sink=True, gate="head", head_scale=True),
+    _case(2, 2, 1, 192, 128, head_sink=True),
+    _case(4, 1, 1, 16, 16, window=7),
+    _case(2, 1, 1, 96, 96, chunk=64, gate="head"),
+    _case(2, 1, 1, 80, 112, chunk=150, sink=True),
+    _case(2, 2, 1, 64, 64, window=70, keep=5, slopes=True),
+    _case(3, 1, 1, 32, 80, window=90, keep=130, slopes=True),
+    _case(2, 1, 1, 48, 64, window=130, softcap=3.0, gate="entry"),
+    _case(4, 2, 1, 64, 64, chunk=100, shared=True, sink=True),
+    _case(1, 1, 1, 128, 128, shared=True),
+]
+
+
+@pytest.mark.parametrize("c", CASES, ids=lambda c: "-".join(f"{k}{v}" for k, v in c.items() if v))
+def test_mapped_attention_on_tcgen05(c):
+    """The result is rounded to bfloat16 (2^-9 of a value); weights act with 16 bits, scores are float32 sums of bfloat16
+    products, and the fast exponential is off by 2^-22 of its argument's size: 2^-8 of a value plus 2^-9 of the row's rms."""
+    from math_utils_b200.csrc import ops
+    H, G, maps, dim, vdim, shared = (c[k] for k in ("H", "G", "maps", "dim", "vdim", "shared"))
+    scale, lam, out_scale, eps = 2.0 * dim ** -0.5, 0.45 if maps == 2 else 0.0, 0.8, 1e-3
+    width = G * (maps * dim + (0 if shared else vdim))
+    n_pages = [-(-n // 64) for n in LENS]
+    order = np.random.default_rng(1).permutation(sum(n_pages) + 2)
+    table, at = np.zeros((len(LENS), max(n_pages)), dtype=np.int32), 0
+    for s, n in enumerate(n_pages):
+        table[s, :n] = order[at:at + n]
+        at += n
+    rows = _rand((sum(n_pages) + 2, 64, width), 2)
+    tok_seq = np.repeat(np.arange(len(LENS)), NEW)
+    tok_pos = np.concatenate([np.arange(n - k, n) for n, k in zip(LENS, NEW)])
+    T, tiles, at = len(tok_seq), [], 0
+    for k in NEW:
+        tiles += [(at + o, min(128, k - o)) for o in range(0, k, 128)]
+        at += k
+    padded = _rand((T, H * maps * dim + 8), 3)
+    q = padded[:, :H * maps * dim]
+    heads = torch.arange(H, device="cuda")
+    slopes = 2.0 ** (-8.0 * (heads + 1).float() / H) if c["slopes"] else None
+    head_scale = 0.5 + heads.float() / H if c["head_scale"] else None
+    head_sink = heads.float() - 0.5 if c["head_sink"] else None
+    gate = _rand((T, H * (vdim if c["gate"] == "entry" else 1)), 4) if c["gate"] else None
+    out = torch.zeros((T, H * vdim), device="cuda", dtype=torch.bfloat16)
+    ops.mapped_attention(q, rows, _ints(table), 64, _ints(tok_pos), _ints(tok_seq), H, G, maps, dim, vdim, scale, c["window"], out,
+                         lam=lam, out_scale=out_scale, eps=eps, unit_rms=c["unit"], chunk=c["chunk"], keep=c["keep"],
+                         slopes=slopes, softcap=c["softcap"], sink=c["sink"], shared=shared, gate=gate, head_scale=head_scale,
+                         head_sink=head_sink, tiles_wide=_ints(tiles))
+    ops.check_status()
+    want = torch.zeros((T, H, vdim), dtype=torch.float64, device="cuda")
+    for s, (n, k) in enumerate(zip(LENS, NEW)):
+        held = rows[torch.as_tensor(table[s, :n_pages[s]].astype(np.int64)).cuda()].double().reshape(-1, width)[:n]
+        mine = torch.as_tensor(np.nonzero(tok_seq == s)[0]).cuda()
+        keys = held[:, :G * maps * dim].reshape(n, G, maps, dim).repeat_interleave(H // G, 1)
+        values = (keys[:, :, 0] if shared else held[:, G * maps * dim:].reshape(n, G, vdim).repeat_interleave(H // G, 1))
+        p = torch.arange(n - k, n, device="cuda")[:, None]
+        j = torch.arange(n, device="cuda")[None, :]
+        lo = p - p % c["chunk"] if c["chunk"] else p - c["window"] + 1 if c["window"] else 0 * p
+        seen = (j <= p) & ((j >= lo) | (j < c["keep"]))
+        parts = []
+        for m in range(maps):
+            x = torch.einsum("ihd,jhd->hij", q[mine].double().reshape(k, H, maps, dim)[:, :, m], keys[:, :, m]) * scale
+            if head_scale is not None:
+                x = x * head_scale.double()[:, None, None]
+            if c["softcap"]:
+                x = c["softcap"] * torch.tanh(x / c["softcap"])
+            if slopes is not None:
+                x = x - slopes.double()[:, None, None] * (p - j)
+            x = x.masked_fill(~seen, -math.inf)
+            extra = torch.zeros(H, dtype=torch.float64, device="cuda") if c["sink"] else head_sink.double() if c["head_sink"] else None
+            if extra is not None:
+                x = torch.cat([x, extra[:, None, None].expand(H, k, 1)], -1)
+            parts.append(torch.einsum("hij,jhd->ihd", torch.softmax(x, -1)[..., :n], values))
+        o = parts[0] - (lam * parts[1] if maps == 2 else 0.0)
+        if c["unit"]:
+            o = o / torch.sqrt((o * o).mean(-1, keepdim=True) + eps)
+        o = o * out_scale
+        if gate is not None:
+            o = o * torch.sigmoid(gate[mine].double()).reshape(k, H, -1)
+        want[mine] = o
+    err = (out.double().reshape(T, H, vdim) - want).abs()
+    bound = 2.0 ** -8 * want.abs() + 2.0 ** -9 * want.square().mean(-1, keepdim=True).sqrt() + 1e-6
+    worst = (err / bound).amax((1, 2))
+    bad = int(worst.argmax())
+    assert float(worst[bad]) < 1.0, f"{float(worst[bad]):.2f} of the bound at token {bad} (sequence {tok_seq[bad]}, position {tok_pos[bad]})"
