@@ -22,6 +22,15 @@
 //                    The order of every sum is fixed by the column alone: a token's result does not depend on how
 //                    the sequence was cut into steps or on the batch.
 //
+// Long steps with one decay per head take four tokens between two exchanges (BLOCKED).  With S the state before them,
+// d_j their decays, D_j = d_0 .. d_j and c_ij = d_(i+1) .. d_j,
+//     u_j = beta_j (v_j - D_j S^T k_j - sum_{i<j} c_ij (k_i . k_j) u_i),   o_j = D_j S^T q_j + sum_{i<=j} c_ij (k_i . q_j) u_i,
+//     S  <- D_3 S + sum_i c_i3 k_i u_i:
+// the same recurrence with its sums in another order, all float32.  The four S^T k_j go round the lanes together, the products
+// of keys and queries within a block of four are made once a chunk (a warp a block), and the state is multiplied by a decay
+// once in four tokens.  What bounds the token-by-token form is its chain (347 cycles a token at one warp a scheduler, of which
+// the exchange is a third).
+//
 // Option: a decay per head and key channel instead of one per head (the rows of S decay each by its own number).  The
 // decays are then made by mu_low_rank (linear_scan.cu) and staged beside the keys; S decays before the two sums, which
 // are S^T k and S^T q of the decayed state, and the read-out is S^T q + u (k . q): one exchange a token again.
@@ -82,6 +91,9 @@ __host__ __device__ constexpr int dl_columns(int lanes) { return DL_PER * DL_THR
 __host__ __device__ constexpr int dl_chunk_floats(int dkp, int cols, bool per_channel) {
     return DL_CHUNK * ((per_channel ? 3 : 2) * dkp + cols + 4);
 }
+// What a block of four tokens needs besides, made from a staged chunk: [0..3] beta; [4..7] D_j; [8..11] c_i3;
+// [12..17] c_ij (k_i . k_j) for ij = 01 02 12 03 13 23; [18..23] c_ij (k_i . q_j) likewise; [24..27] k_j . q_j.
+constexpr int DL_BLOCK = 4, DL_COEF = 28;
 
 // LANES lanes hold two columns of S, R entries of each a lane (a multiple of 4; dk <= LANES R).  The columns are dealt
 // to the lanes four entries at a time: lane l holds entries 4 (l + LANES i) .. 4 (l + LANES i) + 3, i < R / 4, so that
@@ -89,8 +101,8 @@ __host__ __device__ constexpr int dl_chunk_floats(int dkp, int cols, bool per_ch
 // and R follow from dk alone, so the order of the sums does too.
 // VEC: dk, dv, the row length and the state's offset and stride are all multiples of 4, so keys, queries, values and
 // the state move 16 bytes at a time.  PER_CHANNEL: `decay` is [T][n_heads * dk] (else [T][n_heads]).
-template <int R, int LANES, bool VEC, bool PER_CHANNEL>
-__global__ void __launch_bounds__(DL_THREADS, R > 8 ? 2 : 4)
+template <int R, int LANES, bool VEC, bool PER_CHANNEL, bool BLOCKED>
+__global__ void __launch_bounds__(DL_THREADS, R > 8 || BLOCKED ? 2 : 4)
 delta_scan_kernel(const float* __restrict__ qkv, int channels, const float* __restrict__ kq,
                   const float* __restrict__ beta, const float* __restrict__ decay, int n_heads, int n_kv_heads, int dk,
                   int dv, const int* __restrict__ seq_first, const int* __restrict__ seq_slots,
@@ -98,6 +110,8 @@ delta_scan_kernel(const float* __restrict__ qkv, int channels, const float* __re
     constexpr int DKP = LANES * R, Q = R / 4, COLS = dl_columns(LANES), BUF = dl_chunk_floats(DKP, COLS, PER_CHANNEL);
     constexpr int GROUP = LANES / DL_PER;                    // tokens whose read-outs are summed together
     extern __shared__ __align__(16) float dl_smem[];
+    __shared__ __align__(16) float dl_coef[BLOCKED ? DL_CHUNK / DL_BLOCK : 1][DL_COEF];
+    __shared__ float dl_dots[BLOCKED ? DL_CHUNK / DL_BLOCK : 1][16];
     const int s = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * COLS;
     const int tid = threadIdx.x, c0 = DL_PER * (tid / LANES), l = tid % LANES;
     const int g = h / (n_heads / n_kv_heads);
@@ -242,10 +256,149 @@ delta_scan_kernel(const float* __restrict__ qkv, int channels, const float* __re
                 sum[c] = l == 0 ? fmaf(u, par.z, share) : share;
             }
         };
+        if constexpr (BLOCKED) {
+            const int warp = tid >> 5, lane = tid & 31, b0 = warp * DL_BLOCK;
+            if (b0 + DL_BLOCK <= n) {                        // this warp's block: 12 products of keys and queries
+                float dots[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) dots[i] = 0.0f;
+                for (int d = 4 * lane; d < DKP; d += 128) {
+                    float4 kx[4], qx[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        kx[j] = *reinterpret_cast<const float4*>(ks + (b0 + j) * DKP + d);
+                        qx[j] = *reinterpret_cast<const float4*>(qs + (b0 + j) * DKP + d);
+                    }
+#pragma unroll
+                    for (int j = 1, at = 0; j < 4; ++j)
+#pragma unroll
+                        for (int i = 0; i < j; ++i, ++at) {
+                            dots[at] += (kx[i].x * kx[j].x + kx[i].y * kx[j].y) + (kx[i].z * kx[j].z + kx[i].w * kx[j].w);
+                            dots[6 + at] += (kx[i].x * qx[j].x + kx[i].y * qx[j].y) + (kx[i].z * qx[j].z + kx[i].w * qx[j].w);
+                        }
+                }
+#pragma unroll
+                for (int i = 0; i < 12; ++i) dots[i] += __shfl_xor_sync(0xffffffffu, dots[i], 16);
+#pragma unroll
+                for (int width = 8; width >= 1; width >>= 1)
+#pragma unroll
+                    for (int i = 0; i < width; ++i) {
+                        const bool upper = (lane & width) != 0;
+                        const float send = upper ? dots[i] : dots[i + width];
+                        const float keep = upper ? dots[i + width] : dots[i];
+                        dots[i] = keep + __shfl_xor_sync(0xffffffffu, send, width);
+                    }
+                if (lane < 16) dl_dots[warp][lane] = dots[0];
+                __syncwarp();
+                if (lane < DL_COEF) {
+                    const float* par = sc + b0 * 4;
+                    const float d1 = par[5], d2 = par[9], d3 = par[13];
+                    float x;
+                    if (lane < 4) {
+                        x = par[4 * lane];
+                    } else if (lane < 8) {
+                        x = par[1] * (lane > 4 ? d1 : 1.0f) * (lane > 5 ? d2 : 1.0f) * (lane > 6 ? d3 : 1.0f);
+                    } else if (lane < 12) {
+                        x = (lane < 9 ? d1 : 1.0f) * (lane < 10 ? d2 : 1.0f) * (lane < 11 ? d3 : 1.0f);
+                    } else if (lane < 24) {
+                        const int at = (lane - 12) % 6;      // 01 02 12 03 13 23
+                        const int i = at == 0 || at == 1 || at == 3 ? 0 : at == 5 ? 2 : 1, j = at == 0 ? 1 : at < 3 ? 2 : 3;
+                        x = dl_dots[warp][lane - 12] * (i < 1 ? d1 : 1.0f) * (i < 2 && j >= 2 ? d2 : 1.0f) * (j >= 3 ? d3 : 1.0f);
+                    } else {
+                        x = par[4 * (lane - 24) + 2];
+                    }
+                    dl_coef[warp][lane] = x;
+                }
+            }
+            __syncthreads();
+        }
+        // Four tokens; their read-outs' shares go to sum[2 j + c].
+        auto block = [&](int tok, float* sum) {
+            const float4* cf = reinterpret_cast<const float4*>(dl_coef[BLOCKED ? tok / DL_BLOCK : 0]);
+            ulonglong2 kr[DL_BLOCK][Q];
+            float2x a[DL_BLOCK][DL_PER], o[DL_BLOCK][DL_PER];
+#pragma unroll
+            for (int j = 0; j < DL_BLOCK; ++j) {
+#pragma unroll
+                for (int c = 0; c < DL_PER; ++c) a[j][c] = o[j][c] = 0;
+#pragma unroll
+                for (int i = 0; i < Q; ++i) kr[j][i] = *reinterpret_cast<const ulonglong2*>(ks + (tok + j) * DKP + 4 * (l + LANES * i));
+            }
+#pragma unroll
+            for (int i = 0; i < Q; ++i)
+#pragma unroll
+                for (int j = 0; j < DL_BLOCK; ++j)
+#pragma unroll
+                    for (int c = 0; c < DL_PER; ++c) {
+                        a[j][c] = pair_fma(S[c][2 * i], kr[j][i].x, a[j][c]);
+                        a[j][c] = pair_fma(S[c][2 * i + 1], kr[j][i].y, a[j][c]);
+                    }
+            float sk[DL_BLOCK][DL_PER];
+#pragma unroll
+            for (int j = 0; j < DL_BLOCK; ++j)
+#pragma unroll
+                for (int c = 0; c < DL_PER; ++c) {
+                    const float2 x = floats_of_pair(a[j][c]);
+                    sk[j][c] = x.x + x.y;
+                }
+#pragma unroll
+            for (int w = LANES / 2; w > 0; w >>= 1)
+#pragma unroll
+                for (int j = 0; j < DL_BLOCK; ++j)
+#pragma unroll
+                    for (int c = 0; c < DL_PER; ++c) sk[j][c] += __shfl_xor_sync(0xffffffffu, sk[j][c], w);
+            // (the read-outs' products while the exchange is under way)
+#pragma unroll
+            for (int j = 0; j < DL_BLOCK; ++j)
+#pragma unroll
+                for (int i = 0; i < Q; ++i) {
+                    const ulonglong2 qr = *reinterpret_cast<const ulonglong2*>(qs + (tok + j) * DKP + 4 * (l + LANES * i));
+#pragma unroll
+                    for (int c = 0; c < DL_PER; ++c) {
+                        o[j][c] = pair_fma(S[c][2 * i], qr.x, o[j][c]);
+                        o[j][c] = pair_fma(S[c][2 * i + 1], qr.y, o[j][c]);
+                    }
+                }
+            const float4 be = cf[0], D = cf[1], E = cf[2], ka = cf[3], kb = cf[4], qa = cf[5], dq = cf[6];
+            // ka, kb, qa: kk01 kk02 kk12 kk03 | kk13 kk23 qk01 qk02 | qk12 qk03 qk13 qk23
+            const float2x whole = pair_of_floats(D.w, D.w);
+#pragma unroll
+            for (int c = 0; c < DL_PER; ++c) {
+                auto value = [&](int j) {
+                    const float2 v = *reinterpret_cast<const float2*>(vs + (tok + j) * COLS + c0);
+                    return c ? v.y : v.x;
+                };
+                const float u0 = be.x * (value(0) - D.x * sk[0][c]);
+                const float u1 = be.y * (value(1) - D.y * sk[1][c] - ka.x * u0);
+                const float u2 = be.z * (value(2) - D.z * sk[2][c] - ka.y * u0 - ka.z * u1);
+                const float u3 = be.w * (value(3) - D.w * sk[3][c] - ka.w * u0 - kb.x * u1 - kb.y * u2);
+                const float2x w0 = pair_of_floats(E.x * u0, E.x * u0), w1 = pair_of_floats(E.y * u1, E.y * u1);
+                const float2x w2 = pair_of_floats(E.z * u2, E.z * u2), w3 = pair_of_floats(u3, u3);
+#pragma unroll
+                for (int i = 0; i < Q; ++i) {
+                    S[c][2 * i] = pair_fma(kr[3][i].x, w3, pair_fma(kr[2][i].x, w2, pair_fma(kr[1][i].x, w1,
+                                           pair_fma(kr[0][i].x, w0, pair_mul(whole, S[c][2 * i])))));
+                    S[c][2 * i + 1] = pair_fma(kr[3][i].y, w3, pair_fma(kr[2][i].y, w2, pair_fma(kr[1][i].y, w1,
+                                               pair_fma(kr[0][i].y, w0, pair_mul(whole, S[c][2 * i + 1])))));
+                }
+                const float own[DL_BLOCK] = {dq.x * u0, dq.y * u1 + kb.z * u0, dq.z * u2 + kb.w * u0 + qa.x * u1,
+                                             dq.w * u3 + qa.y * u0 + qa.z * u1 + qa.w * u2};
+                const float Dj[DL_BLOCK] = {D.x, D.y, D.z, D.w};
+#pragma unroll
+                for (int j = 0; j < DL_BLOCK; ++j) {
+                    const float2 x = floats_of_pair(o[j][c]);
+                    const float share = Dj[j] * (x.x + x.y);
+                    sum[DL_PER * j + c] = l == 0 ? share + own[j] : share;
+                }
+            }
+        };
         for (int t0 = 0; t0 < n; t0 += GROUP) {
             float acc[LANES];                                // token t0 + i, column c at [2 i + c]
             const int left = n - t0;
-            if (left >= GROUP) {                             // a whole group: no branch between the tokens
+            if (BLOCKED && left >= GROUP) {
+#pragma unroll
+                for (int i = 0; i < GROUP; i += DL_BLOCK) block(t0 + i, acc + DL_PER * i);
+            } else if (left >= GROUP) {                             // a whole group: no branch between the tokens
 #pragma unroll
                 for (int i = 0; i < GROUP; ++i) step(t0 + i, acc + DL_PER * i);
             } else {
@@ -338,11 +491,11 @@ MU_EXPORT int mu_delta_scan(const float* qkv, int channels, const float* kq, con
     // scheduler; they start in plain stream order, on an empty device.
     // the two staging buffers of a block are most of what it needs of an SM: with the largest share of the on-chip
     // memory as shared memory several blocks fit, and the state is read once, so the L1 is no loss
-#define MU_DELTA_SCAN_V(R, LANES, V, PC)                                                                              \
+#define MU_DELTA_SCAN_V(R, LANES, V, PC, BL)                                                                            \
     do {                                                                                                              \
         const size_t smem = 2 * sizeof(float) * mu::dl_chunk_floats(LANES * R, mu::dl_columns(LANES), PC);            \
         const dim3 grid(n_seqs, n_heads, (dv + mu::dl_columns(LANES) - 1) / mu::dl_columns(LANES));                   \
-        auto kernel = mu::delta_scan_kernel<R, LANES, V, PC>;                                                         \
+        auto kernel = mu::delta_scan_kernel<R, LANES, V, PC, BL>;                                                        \
         if (!mu::allow_shared((const void*)kernel, smem)) return MU_ERR_LAUNCH;                                       \
         mu::prefer_shared_memory((const void*)kernel);                                                                \
         const dim3 block(mu::DL_THREADS);                                                                             \
@@ -354,10 +507,11 @@ MU_EXPORT int mu_delta_scan(const float* qkv, int channels, const float* kq, con
     } while (0)
 #define MU_DELTA_SCAN(R, LANES)                                                                                       \
     do {                                                                                                              \
-        if (vec && per_channel) MU_DELTA_SCAN_V(R, LANES, true, true);                                                \
-        if (per_channel) MU_DELTA_SCAN_V(R, LANES, false, true);                                                      \
-        if (vec) MU_DELTA_SCAN_V(R, LANES, true, false);                                                              \
-        MU_DELTA_SCAN_V(R, LANES, false, false);                                                                      \
+        if (vec && per_channel) MU_DELTA_SCAN_V(R, LANES, true, true, false);                                         \
+        if (per_channel) MU_DELTA_SCAN_V(R, LANES, false, true, false);                                               \
+        if (vec && long_steps) MU_DELTA_SCAN_V(R, LANES, true, false, true);                                          \
+        if (vec) MU_DELTA_SCAN_V(R, LANES, true, false, false);                                                       \
+        MU_DELTA_SCAN_V(R, LANES, false, false, false);                                                                    \
     } while (0)
     if (dk <= 32) MU_DELTA_SCAN(4, 8);
     if (dk <= 64) MU_DELTA_SCAN(4, 16);
