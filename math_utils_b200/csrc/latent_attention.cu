@@ -58,38 +58,45 @@ __global__ void rotary_kernel(const TI* __restrict__ x, long long ldx, int x_hea
 // With q (and qa): the same block also rotates the token's queries (every head's rot_dim entries at q + h *
 // q_head_stride) into qa + h * qa_head_stride as float32, so that a step needs one launch for both.  With dkv
 // null only the queries are rotated (a layer that reads another layer's cache).
-template <typename T>
+constexpr int LA_TURNS = 768;     // rotated pairs at most (a cached row has 1,536 values at most)
+
+template <typename T, typename TQ>
 __global__ void latent_append_kernel(const T* __restrict__ dkv, long long ld, const float* __restrict__ norm_w, float eps,
                                      const float* __restrict__ freqs, float mag, int rot_dims, int kv_rank, int rot_dim,
                                      const int* __restrict__ tok_pos, const int* __restrict__ tok_seq,
                                      const int* __restrict__ block_table, int max_pages, int page_tokens,
-                                     T* __restrict__ rows, const T* __restrict__ q, long long ldq, int q_head_stride,
-                                     float* __restrict__ qa, long long ldqa, int qa_head_stride, int n_heads,
+                                     T* __restrict__ rows, const T* q, long long ldq, int q_head_stride,
+                                     TQ* qa, long long ldqa, int qa_head_stride, int n_heads,
                                      int pairs) {
     __shared__ float scratch[32];
     pdl_trigger();
     pdl_wait();
     const int t = blockIdx.x;
     const int p = tok_pos[t];
+    // the angles of a token are the same for every head: made once
+    __shared__ float2 turns[LA_TURNS];
+    for (int e = threadIdx.x; e < rot_dims / 2; e += blockDim.x) {
+        float sn, cs;
+        sincosf((float)p * freqs[e], &sn, &cs);
+        turns[e] = make_float2(sn * mag, cs * mag);
+    }
+    __syncthreads();
     if (q) {
         const int half = rot_dims / 2, per_head = rot_dim - half;
-        const float pos = (float)p;
         const T* src = q + (long long)t * ldq;
-        float* dst = qa + (long long)t * ldqa;
+        TQ* dst = qa + (long long)t * ldqa;                  // (may be the queries' own place)
         for (int i = threadIdx.x; i < n_heads * per_head; i += blockDim.x) {
             const int h = i / per_head, e = i % per_head;
             const T* s = src + (long long)h * q_head_stride;
-            float* d = dst + (long long)h * qa_head_stride;
+            TQ* d = dst + (long long)h * qa_head_stride;
             if (e < half) {
-                float sn, cs;
-                sincosf(pos * freqs[e], &sn, &cs);
-                sn *= mag; cs *= mag;
+                const float sn = turns[e].x, cs = turns[e].y;
                 const int lo = pairs ? 2 * e : e, hi = pairs ? 2 * e + 1 : e + half;
                 const float u = to_float(s[lo]), v = to_float(s[hi]);
-                d[lo] = u * cs - v * sn;
-                d[hi] = v * cs + u * sn;
+                d[lo] = from_float<TQ>(u * cs - v * sn);
+                d[hi] = from_float<TQ>(v * cs + u * sn);
             } else {
-                d[e + half] = to_float(s[e + half]);
+                d[e + half] = from_float<TQ>(to_float(s[e + half]));
             }
         }
     }
@@ -106,14 +113,11 @@ __global__ void latent_append_kernel(const T* __restrict__ dkv, long long ld, co
     const float inv = 1.0f / sqrtf(block_sum(s, scratch) / (float)kv_rank + eps);
     for (int d = threadIdx.x; d < kv_rank; d += blockDim.x) dst[d] = from_float<T>(to_float(src[d]) * inv * norm_w[d]);
     const int half = rot_dims / 2;
-    const float pos = (float)p;
     src += kv_rank;
     dst += kv_rank;
     for (int e = threadIdx.x; e < rot_dim - half; e += blockDim.x) {
         if (e < half) {
-            float sn, cs;
-            sincosf(pos * freqs[e], &sn, &cs);
-            sn *= mag; cs *= mag;
+            const float sn = turns[e].x, cs = turns[e].y;
             const int lo = pairs ? 2 * e : e, hi = pairs ? 2 * e + 1 : e + half;
             const float u = to_float(src[lo]), v = to_float(src[hi]);
             dst[lo] = from_float<T>(u * cs - v * sn);
@@ -283,6 +287,49 @@ int latent_attention_any(const float* q, const T* rows, const int* block_table, 
     return MU_ERR_UNSUPPORTED_SIZE;
 }
 
+// A block a page of the expanded rows; sizes in pieces of eight bfloat16 entries.
+__global__ void __launch_bounds__(256)
+latent_rows_kernel(const uint4* __restrict__ cache, const int* __restrict__ block_table, int max_pages,
+                   const int* __restrict__ tok_pos, const int* __restrict__ seq_first, int n_seqs, int rank, int rot,
+                   uint4* __restrict__ latents, uint4* __restrict__ rows, int width, int rot_at, int* __restrict__ table,
+                   int max_pages_out) {
+    __shared__ int found[3];                                 // sequence, page within it, its length
+    pdl_trigger();
+    pdl_wait();
+    const int page = blockIdx.x, tid = threadIdx.x;
+    if (tid < 32) {                                          // 32 sequences at a time: their pages, summed up
+        if (tid == 0) found[0] = -1;
+        __syncwarp();
+        int before = 0;
+        for (int s0 = 0; s0 < n_seqs && before <= page; s0 += 32) {
+            const int s = s0 + tid;
+            const int len = s < n_seqs ? tok_pos[seq_first[s + 1] - 1] + 1 : 0, mine = (len + 63) / 64;
+            int upto = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int other = __shfl_up_sync(0xffffffffu, upto, o);
+                if (tid >= o) upto += other;
+            }
+            const int at = page - before - (upto - mine);
+            if (at >= 0 && at < mine) found[0] = s, found[1] = at, found[2] = len;
+            before += __shfl_sync(0xffffffffu, upto, 31);
+        }
+    }
+    __syncthreads();
+    const int s = found[0], at = found[1];
+    if (s < 0) return;
+    const int left = found[2] - 64 * at;                     // positions of the page that exist
+    if (tid == 0 && at < max_pages_out) table[(long long)s * max_pages_out + at] = page;
+    const uint4* src = cache + (long long)block_table[(long long)s * max_pages + at] * 64 * (rank + rot);
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    for (int i = tid; i < 64 * (rank + rot); i += 256) {
+        const int r = i / (rank + rot), c = i - r * (rank + rot);
+        const uint4 v = r < left ? src[i] : zero;
+        if (c < rank) latents[((long long)page * 64 + r) * rank + c] = v;
+        else rows[((long long)page * 64 + r) * width + rot_at + c - rank] = v;
+    }
+}
+
 }  // namespace mu
 
 MU_EXPORT int mu_rotary(const void* x, long long ldx, int x_head_stride, int x_bf16, void* y, long long ldy,
@@ -304,25 +351,47 @@ MU_EXPORT int mu_rotary(const void* x, long long ldx, int x_head_stride, int x_b
 }
 
 // dkv may be null (no cache row is written) if q is given; q may be null (no queries are rotated).
+// qa: float32, or with qa_bf16 (bfloat16 caches) bfloat16, where it may be q's own place.
 MU_EXPORT int mu_latent_append(const void* dkv, long long ld, const float* norm_w, float eps, const float* freqs,
                                float mag, int rot_dims, int kv_rank, int rot_dim, const int* tok_pos,
                                const int* tok_seq, const int* block_table, int max_pages, int page_tokens,
                                int n_tokens, void* rows, int is_bf16, const void* q, long long ldq, int q_head_stride,
-                               float* qa, long long ldqa, int qa_head_stride, int n_heads, void* stream, int pairs) {
+                               void* qa, long long ldqa, int qa_head_stride, int n_heads, void* stream, int pairs, int qa_bf16) {
     if (n_tokens <= 0) return MU_OK;
     if ((!dkv && !q) || !freqs || !tok_pos || kv_rank <= 0 || rot_dim < 0 || rot_dims % 2 || rot_dims > rot_dim ||
-        (dkv && (!norm_w || !tok_seq || !block_table || !rows || page_tokens <= 0)) || (q && (!qa || n_heads <= 0)))
+        (dkv && (!norm_w || !tok_seq || !block_table || !rows || page_tokens <= 0)) || (q && (!qa || n_heads <= 0)) ||
+        (qa_bf16 && !is_bf16))
         return MU_ERR_BAD_ARGUMENT;
+    if (rot_dims / 2 > mu::LA_TURNS) return MU_ERR_UNSUPPORTED_SIZE;
     cudaStream_t s = (cudaStream_t)stream;
     const dim3 grid(n_tokens), block(kv_rank >= 512 ? 256 : 128);
-    if (is_bf16)
-        return mu::launch_pdl(mu::latent_append_kernel<__nv_bfloat16>, grid, block, 0, s, 1, (const __nv_bfloat16*)dkv,
-                              ld, norm_w, eps, freqs, mag, rot_dims, kv_rank, rot_dim, tok_pos, tok_seq, block_table,
-                              max_pages, page_tokens, (__nv_bfloat16*)rows, (const __nv_bfloat16*)q, ldq, q_head_stride,
-                              qa, ldqa, qa_head_stride, n_heads, pairs);
-    return mu::launch_pdl(mu::latent_append_kernel<float>, grid, block, 0, s, 1, (const float*)dkv, ld, norm_w, eps,
-                          freqs, mag, rot_dims, kv_rank, rot_dim, tok_pos, tok_seq, block_table, max_pages, page_tokens,
-                          (float*)rows, (const float*)q, ldq, q_head_stride, qa, ldqa, qa_head_stride, n_heads, pairs);
+    typedef __nv_bfloat16 bf;
+#define MU_APPEND(T, TQ)                                                                                                \
+    return mu::launch_pdl(mu::latent_append_kernel<T, TQ>, grid, block, 0, s, 1, (const T*)dkv, ld, norm_w, eps, freqs, mag, \
+                          rot_dims, kv_rank, rot_dim, tok_pos, tok_seq, block_table, max_pages, page_tokens, (T*)rows,   \
+                          (const T*)q, ldq, q_head_stride, (TQ*)qa, ldqa, qa_head_stride, n_heads, pairs)
+    if (is_bf16 && qa_bf16) MU_APPEND(bf, bf);
+    if (is_bf16) MU_APPEND(bf, float);
+    MU_APPEND(float, float);
+#undef MU_APPEND
+}
+
+// For prompt steps whose keys and values are expanded (every position that the step's sequences hold, their pages one after
+// another, a sequence's on a page of its own): latents [n_pages * 64][kv_rank] receives the cached latents, rows
+// [n_pages * 64][width] the shared rotated part at column rot_at, both zeros past a sequence's end, and table [n_seqs]
+// [max_pages_out] the pages' numbers.  seq_first: the step's flat tokens per sequence, the last of each at its sequence's end.
+MU_EXPORT int mu_latent_rows(const void* cache, const int* block_table, int max_pages, const int* tok_pos, const int* seq_first,
+                             int n_seqs, int n_pages, int kv_rank, int rot_dim, void* latents, void* rows, int width, int rot_at,
+                             int* table, int max_pages_out, void* stream) {
+    if (n_pages <= 0 || n_seqs <= 0) return MU_OK;
+    if (!cache || !block_table || !tok_pos || !seq_first || !latents || !rows || !table || kv_rank <= 0 || rot_dim < 0 ||
+        rot_at + rot_dim > width)
+        return MU_ERR_BAD_ARGUMENT;
+    if (kv_rank % 8 || rot_dim % 8 || width % 8 || rot_at % 8 || (((uintptr_t)cache | (uintptr_t)latents | (uintptr_t)rows) & 15))
+        return MU_ERR_ALIGNMENT;
+    return mu::launch_pdl(mu::latent_rows_kernel, dim3(n_pages), dim3(256), 0, (cudaStream_t)stream, 1, (const uint4*)cache,
+                          block_table, max_pages, tok_pos, seq_first, n_seqs, kv_rank / 8, rot_dim / 8, (uint4*)latents,
+                          (uint4*)rows, width / 8, rot_at / 8, table, max_pages_out);
 }
 
 // q: float32 [n_tokens, n_heads, width]; out: [n_tokens, ldo] with head h at columns h * kv_rank.

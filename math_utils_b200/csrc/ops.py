@@ -141,7 +141,7 @@ _SIGNATURES = {
     "mu_rotary": [_c_p, _c_ll, _c_int, _c_int, _c_p, _c_ll, _c_int, _c_int, _c_p, _c_p, _c_f, _c_int, _c_int, _c_int,
                   _c_int, _c_p],
     "mu_latent_append": [_c_p, _c_ll, _c_p, _c_f, _c_p, _c_f, _c_int, _c_int, _c_int, _c_p, _c_p, _c_p, _c_int, _c_int,
-                         _c_int, _c_p, _c_int, _c_p, _c_ll, _c_int, _c_p, _c_ll, _c_int, _c_int, _c_p, _c_int],
+                         _c_int, _c_p, _c_int, _c_p, _c_ll, _c_int, _c_p, _c_ll, _c_int, _c_int, _c_p, _c_int, _c_int],
     "mu_moe_combine_tanh": [_c_p, _c_ll, _c_p, _c_p, _c_int, _c_int, _c_int, _c_p, _c_p, _c_p, _c_p, _c_ll, _c_p],
     "mu_latent_attention": [_c_p, _c_p, _c_p, _c_int, _c_int, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_f, _c_int,
                             _c_p, _c_ll, _c_p, _c_p, _c_int, _c_p, _c_p],
@@ -156,6 +156,8 @@ _SIGNATURES = {
                     _c_int, _c_int, _c_p, _c_int, _c_p],
     "mu_moe_gemm_mma": [_c_p, _c_ll, _c_p, _c_int, _c_p, _c_p, _c_ll, _c_ll, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_p,
                         _c_ll, _c_int, _c_p, _c_int, _c_p],
+    "mu_latent_rows": [_c_p, _c_p, _c_int, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_p, _c_p, _c_int, _c_int, _c_p, _c_int,
+                       _c_p],
     "mu_mapped_attention_tc_fits": [_c_int] * 6,
     "mu_mapped_attention_tc": [_c_p, _c_ll, _c_int, _c_p, _c_ll, _c_p, _c_int, _c_int, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int,
                                _c_int, _c_int, _c_int, _c_f, _c_int, _c_f, _c_f, _c_f, _c_int, _c_p, _c_ll, _c_p, _c_p,
@@ -1109,7 +1111,8 @@ def latent_append(dkv: Optional[torch.Tensor], norm_weight: Optional[torch.Tenso
     go to the token's row of the latent cache ``rows`` [pages, page_tokens, kv_rank + rot_dim].
 
     ``queries`` = (q, q_head_stride, qa, qa_head_stride, n_heads): the same launch rotates every head's ``rot_dim``
-    entries (views whose first element is head 0's first rotated entry) from ``q`` into the float32 ``qa``.  With
+    entries (views whose first element is head 0's first rotated entry) from ``q`` into ``qa``, float32 or in ``q``'s dtype
+    (which may be ``q`` itself).  With
     ``dkv`` None only that is done (a layer that reads another layer's cache).  ``pairs``: entry 2i turns with
     entry 2i + 1 instead of entry i with entry i + rot_dims / 2."""
     _need_cuda(dkv, norm_weight, freqs, tok_pos, tok_seq, block_table, rows)
@@ -1125,8 +1128,8 @@ def latent_append(dkv: Optional[torch.Tensor], norm_weight: Optional[torch.Tenso
     if queries is not None:
         q, qs, qa, qas, heads = queries
         _need_cuda(q, qa)
-        if q.dtype != rows.dtype or qa.dtype != torch.float32 or q.stride(1) != 1 or qa.stride(1) != 1:
-            raise KernelError("latent_append: queries in the cache's dtype, rotated queries as float32")
+        if q.dtype != rows.dtype or qa.dtype not in (torch.float32, rows.dtype) or q.stride(1) != 1 or qa.stride(1) != 1:
+            raise KernelError("latent_append: queries in the cache's dtype, rotated queries as float32 or likewise")
     elif dkv is None:
         raise KernelError("latent_append: nothing to do")
     n_tokens = dkv.shape[0] if dkv is not None else q.shape[0]
@@ -1136,8 +1139,61 @@ def latent_append(dkv: Optional[torch.Tensor], norm_weight: Optional[torch.Tenso
                                       int(page_tokens), n_tokens, _ptr(rows), _is_bf16(rows), _ptr(q),
                                       q.stride(0) if q is not None else 0, int(qs), _ptr(qa),
                                       qa.stride(0) if qa is not None else 0, int(qas), int(heads), _stream(),
-                                      int(pairs)),
+                                      int(pairs), int(qa is not None and qa.dtype == torch.bfloat16)),
            "latent_append")
+
+
+def latent_rows(cache: torch.Tensor, block_table: torch.Tensor, tok_pos, seq_first, n_pages: int, kv_rank: int,
+                latents: torch.Tensor, rows: torch.Tensor, rot_at: int, table: torch.Tensor) -> None:
+    """Every position that a prompt step's sequences hold, their pages of 64 one after another (``n_pages`` in all): the
+    cached latents to ``latents`` [n_pages * 64, kv_rank], the rotated part that all heads share to the columns from
+    ``rot_at`` on of ``rows`` [n_pages, 64, width], and the pages' numbers to ``table`` [sequences, *].  Zeros past a
+    sequence's end."""
+    _need_cuda(cache, block_table, tok_pos, seq_first, latents, rows, table)
+    for t, name in ((block_table, "block_table"), (tok_pos, "tok_pos"), (seq_first, "seq_first"), (table, "table")):
+        _i32(t, name)
+    n_seqs, rot_dim = table.shape[0], cache.shape[2] - kv_rank
+    if (cache.dtype != torch.bfloat16 or not cache.is_contiguous() or cache.shape[1] != 64 or latents.dtype != cache.dtype
+            or rows.dtype != cache.dtype or not latents.is_contiguous() or not rows.is_contiguous() or not table.is_contiguous()
+            or tuple(latents.shape) != (n_pages * 64, kv_rank) or rows.dim() != 3 or rows.shape[0] < n_pages or rows.shape[1] != 64
+            or block_table.shape[0] != n_seqs or seq_first.numel() != n_seqs + 1):
+        raise KernelError("latent_rows: the cache, its table and the outputs do not fit")
+    _check(library().mu_latent_rows(_ptr(cache), _ptr(block_table), block_table.shape[1], _ptr(tok_pos), _ptr(seq_first), n_seqs,
+                                    int(n_pages), int(kv_rank), int(rot_dim), _ptr(latents), _ptr(rows), rows.shape[2],
+                                    int(rot_at), _ptr(table), table.shape[1], _stream()), "latent_rows")
+
+
+def latent_prompt_ok(dim: int, rot_dim: int, vdim: int, kv_rank: int) -> bool:
+    """Whether prompt steps of latent attention may expand their keys and values for ``latent_prompt``."""
+    return (LATENT_TC and MAPPED_TC and dim % 64 == 0 and dim > 0 and rot_dim % 16 == 0 and rot_dim > 0 and vdim % 16 == 0
+            and 0 < vdim <= 128 and kv_rank % 8 == 0 and dim + rot_dim <= 256)
+
+
+def latent_prompt(q: torch.Tensor, rows: torch.Tensor, table: torch.Tensor, tok_pos, tok_seq, tiles_wide: torch.Tensor,
+                  n_heads: int, dim: int, rot_dim: int, vdim: int, scale: float, out: torch.Tensor,
+                  sink: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """Causal attention of [T, heads * (dim + rot_dim)] bfloat16 queries over expanded rows [pages, 64, width] = the heads'
+    keys (dim each), their values (vdim each), and the rot_dim key entries that all heads share; ``sink`` and ``gate``
+    ([T, heads * vdim]) as for ``latent_attention`` and its output gate."""
+    _need_cuda(q, rows, table, tok_pos, tok_seq, tiles_wide, out, sink, gate)
+    for t, name in ((table, "table"), (tok_pos, "tok_pos"), (tok_seq, "tok_seq"), (tiles_wide, "tiles_wide")):
+        _i32(t, name)
+    kw = dim + rot_dim
+    if (q.dtype != torch.bfloat16 or rows.dtype != q.dtype or out.dtype != q.dtype or q.stride(1) != 1 or out.stride(1) != 1
+            or q.shape[1] != n_heads * kw or tuple(out.shape) != (q.shape[0], n_heads * vdim) or not rows.is_contiguous()
+            or rows.shape[1] != 64 or rows.shape[2] != n_heads * (dim + vdim) + rot_dim or table.stride(1) != 1):
+        raise KernelError("latent_prompt: queries, rows and output do not fit")
+    if sink is not None and (sink.dtype != torch.float32 or sink.numel() != n_heads or not sink.is_contiguous()):
+        raise KernelError("latent_prompt: the sink is one contiguous float32 per head")
+    if gate is not None and (gate.dtype != q.dtype or tuple(gate.shape) != tuple(out.shape) or gate.stride(1) != 1):
+        raise KernelError("latent_prompt: the gate is laid out as the output")
+    _check(library().mu_mapped_attention_tc(
+        _ptr(q), q.stride(0), q.shape[0], _ptr(rows), rows.shape[0], _ptr(table), table.shape[1], 64, _ptr(tok_pos), _ptr(tok_seq),
+        _ptr(tiles_wide), tiles_wide.shape[0], int(n_heads), int(n_heads), 1, kw, int(vdim), float(scale), 0, 0.0, 1.0, 0.0, 0,
+        _ptr(out), out.stride(0), status_word(q.device).data_ptr(), _stream(), None, 0, _ptr(gate),
+        gate.stride(0) if gate is not None else 0, 0, None, 0, 0.0, int(gate is not None), 0, _ptr(sink), int(dim)),
+        ("latent_prompt(heads={}, dim={}+{}, vdim={})", n_heads, dim, rot_dim, vdim))
+    return out
 
 
 def latent_attention(q: torch.Tensor, rows: torch.Tensor, block_table: torch.Tensor, page_tokens: int, tok_pos, tok_seq,

@@ -106,6 +106,11 @@ class LatentAttention(Mixer):
         self.q_up = t("uk").reshape(H, self.dim, self.kv_rank).transpose(1, 2).contiguous()      # [H, kv_rank, dim]
         self.v_up = t("uv").reshape(H, self.vdim, self.kv_rank).contiguous()                     # [H, vdim, kv_rank]
         self.out = Linear(t("out"), None, runtime)
+        # one product for all heads' keys and values, where prompt steps expand them
+        self.expand = None
+        if runtime.dtype == torch.bfloat16 and not self.window and runtime.ops.latent_prompt_ok(self.dim, self.rot_dim,
+                                                                                                self.vdim, self.kv_rank):
+            self.expand = Linear(torch.cat([t("uk"), t("uv")], dim=0).contiguous(), None, runtime)
         # (one entry at least, so that the kernels always get a table)
         self.freq_table = torch.tensor(self.freqs or [0.0], dtype=torch.float64).to(torch.float32).to(runtime.device)
 
@@ -128,6 +133,9 @@ class LatentAttention(Mixer):
         table = ctx.block_tables[cache.group]
         if owns_cache and not self.own_kv:
             raise ConfigError("a latent-attention layer without a down-projection cannot own a cache")
+        if self._expands(ctx, q, cache):
+            self._prompt(q, views, gate, residual, ctx, cache, owns_cache, accumulate, table)
+            return
         # queries in latent space, float32: [T, H, kv_rank | rot_dim]
         qa = ctx.buffer("latent.q", (T, H * self.row), torch.float32)
         # one launch: this step's cache rows (norm, rotation) and the rotated part of the queries
@@ -146,6 +154,37 @@ class LatentAttention(Mixer):
         ctx.note("mixed", mixed)
         heads = ctx.buffer("latent.heads", (T, H * self.vdim), dt)
         ops.heads_gemm(mixed, self.v_up, heads, r, self.vdim, gate=gate)
+        ctx.note("attn", heads)
+        self.out(heads, residual=residual if accumulate else None, out=residual)
+
+    # A prompt step expands its sequences' positions where they are no more than this many times its own tokens: each costs
+    # 2 r H (d + d_v) operations whoever sees it.
+    EXPANDED_PER_TOKEN = 4
+
+    def _expands(self, ctx, q, cache) -> bool:
+        if (self.expand is None or ctx.is_decode or ctx.q_tiles_wide is None or ctx.n_tokens <= 64 or cache.page_tokens != 64
+                or q.stride(0) % 8 or q.data_ptr() % 16):
+            return False
+        held = sum(start + n for start, n in zip(ctx.starts, ctx.q_lens))
+        return held <= self.EXPANDED_PER_TOKEN * ctx.n_tokens
+
+    def _prompt(self, q, views, gate, residual, ctx, cache, owns_cache, accumulate, table) -> None:
+        ops, dt = self.runtime.ops, self.runtime.dtype
+        T, H, r = ctx.n_tokens, self.n_heads, self.kv_rank
+        rotated = (q[:, self.dim:], self.q_head, q[:, self.dim:], self.q_head, H)
+        ops.latent_append(views[self.at["dkv"]] if owns_cache else None, self.norm_weight, self.eps, self.freq_table,
+                          self.magnitude, self.rot_dims, r, self.rot_dim, ctx.tok_pos, ctx.tok_seq, table, cache.page_tokens,
+                          cache.pages, queries=rotated, pairs=self.rot_layout == "pairs")
+        pages = [-(-(start + n) // 64) for start, n in zip(ctx.starts, ctx.q_lens)]
+        n_pages, both = sum(pages), H * (self.dim + self.vdim)
+        latents = ctx.buffer("latent.held", (n_pages * 64, r), dt)
+        rows = ctx.buffer("latent.rows", (n_pages, 64, both + self.rot_dim), dt)
+        page_list = ctx.buffer("latent.pages", (ctx.n_seqs, max(pages)), torch.int32)
+        ops.latent_rows(cache.pages, table, ctx.tok_pos, ctx.seq_first, n_pages, r, latents, rows, both, page_list)
+        self.expand(latents, out=rows.view(n_pages * 64, both + self.rot_dim)[:, :both])
+        heads = ctx.buffer("latent.heads", (T, H * self.vdim), dt)
+        ops.latent_prompt(q, rows, page_list, ctx.tok_pos, ctx.tok_seq, ctx.q_tiles_wide, H, self.dim, self.rot_dim, self.vdim,
+                          self.scale, heads, sink=self.sink, gate=gate)
         ctx.note("attn", heads)
         self.out(heads, residual=residual if accumulate else None, out=residual)
 
