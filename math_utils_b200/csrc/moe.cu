@@ -31,6 +31,7 @@ namespace mu {
 constexpr int MOE_TM = 32, MOE_TN = 64, MOE_TK = 32;
 
 constexpr int ROUTE_WARPS = 16;
+constexpr size_t ROUTE_SMEM = 100 * 1024;
 
 // A block takes TOK consecutive tokens: their rows are staged in shared memory as float32, the warps share the
 // experts (each logit one warp's sum over the row, lanes striding along it; a router row is read once for the
@@ -75,42 +76,69 @@ moe_route_kernel(const T* __restrict__ h, long long ldh, const float* __restrict
     const bool wide = hidden % 4 == 0 && ((uintptr_t)router & 15) == 0 &&
                       ((uintptr_t)gate_w & 15) == 0;                          // rows of the router in 16-byte pieces
     // (with gate_w: one more sum, over the shared expert's gate row, by the warp whose turn it is)
-    for (int e = warp; e < n_experts + (gate_w ? 1 : 0); e += ROUTE_WARPS) {
-        const float* w = e < n_experts ? router + (long long)e * hidden : gate_w;
-        float z[TOK];
-        if (wide) {
-            const float4* w4 = reinterpret_cast<const float4*>(w);
-            const float4* h4 = reinterpret_cast<const float4*>(hrow);
-            const int n4 = hidden / 4;
-            float z0[TOK], z1[TOK], z2[TOK], z3[TOK];                        // a lane's sum in four parts, then in order
-#pragma unroll
-            for (int i = 0; i < TOK; ++i) z0[i] = z1[i] = z2[i] = z3[i] = 0.0f;
-#pragma unroll 8
-            for (int d = lane; d < n4; d += 32) {                            // (unrolled: the row's loads go out together)
-                const float4 b = w4[d];
-#pragma unroll
-                for (int i = 0; i < TOK; ++i) {
-                    const float4 a = h4[i * n4 + d];
-                    z0[i] += a.x * b.x; z1[i] += a.y * b.y; z2[i] += a.z * b.z; z3[i] += a.w * b.w;
-                }
-            }
-#pragma unroll
-            for (int i = 0; i < TOK; ++i) z[i] = (z0[i] + z1[i]) + (z2[i] + z3[i]);
-        } else {
-#pragma unroll
-            for (int i = 0; i < TOK; ++i) z[i] = 0.0f;
-            for (int d = lane; d < hidden; d += 32) {
-                const float b = w[d];
-#pragma unroll
-                for (int i = 0; i < TOK; ++i) z[i] += hrow[i * hidden + d] * b;
-            }
-        }
+    const int rows = n_experts + (gate_w ? 1 : 0);
+    auto row_of = [&](int e) { return e < n_experts ? router + (long long)e * hidden : gate_w; };
+    auto put = [&](int e, const float (&z)[TOK]) {
 #pragma unroll
         for (int i = 0; i < TOK; ++i) {
             const float zi = warp_sum(z[i]);
             if (lane == 0 && i < nt) {
                 if (e < n_experts) score_all[i * n_experts + e] = zi;
                 else gate_out[t0 + i] = 1.0f / (1.0f + expf(-zi));
+            }
+        }
+    };
+    // NE router rows a pass: a staged row's piece, read from shared memory once, serves them all (with one row a pass the
+    // kernel waits for those reads: four multiply-adds each)
+    constexpr int NE = TOK >= 4 ? 2 : 1, AHEAD = TOK == 8 ? 1 : TOK == 4 ? 4 : 8;
+    for (int e0 = warp; e0 < rows; e0 += NE * ROUTE_WARPS) {
+        if (wide) {
+            const float4* w4[NE];
+#pragma unroll
+            for (int n = 0; n < NE; ++n) w4[n] = reinterpret_cast<const float4*>(row_of(min(e0 + n * ROUTE_WARPS, rows - 1)));
+            const float4* h4 = reinterpret_cast<const float4*>(hrow);
+            const int n4 = hidden / 4;
+            float z0[NE][TOK], z1[NE][TOK], z2[NE][TOK], z3[NE][TOK];        // a lane's sum in four parts, then in order
+#pragma unroll
+            for (int n = 0; n < NE; ++n)
+#pragma unroll
+                for (int i = 0; i < TOK; ++i) z0[n][i] = z1[n][i] = z2[n][i] = z3[n][i] = 0.0f;
+#pragma unroll AHEAD
+            for (int d = lane; d < n4; d += 32) {                            // (unrolled: the rows' loads go out together)
+                float4 b[NE];
+#pragma unroll
+                for (int n = 0; n < NE; ++n) b[n] = w4[n][d];
+#pragma unroll
+                for (int i = 0; i < TOK; ++i) {
+                    const float4 a = h4[i * n4 + d];
+#pragma unroll
+                    for (int n = 0; n < NE; ++n) {
+                        z0[n][i] += a.x * b[n].x; z1[n][i] += a.y * b[n].y; z2[n][i] += a.z * b[n].z; z3[n][i] += a.w * b[n].w;
+                    }
+                }
+            }
+#pragma unroll
+            for (int n = 0; n < NE; ++n) {
+                float z[TOK];
+#pragma unroll
+                for (int i = 0; i < TOK; ++i) z[i] = (z0[n][i] + z1[n][i]) + (z2[n][i] + z3[n][i]);
+                if (e0 + n * ROUTE_WARPS < rows) put(e0 + n * ROUTE_WARPS, z);
+            }
+        } else {
+#pragma unroll
+            for (int n = 0; n < NE; ++n) {
+                const int e = e0 + n * ROUTE_WARPS;
+                if (e >= rows) break;
+                const float* w = row_of(e);
+                float z[TOK];
+#pragma unroll
+                for (int i = 0; i < TOK; ++i) z[i] = 0.0f;
+                for (int d = lane; d < hidden; d += 32) {
+                    const float b = w[d];
+#pragma unroll
+                    for (int i = 0; i < TOK; ++i) z[i] += hrow[i * hidden + d] * b;
+                }
+                put(e, z);
             }
         }
     }
@@ -157,34 +185,64 @@ moe_route_kernel(const T* __restrict__ h, long long ldh, const float* __restrict
 }
 
 // One block.  slot_of[pair], pair_of[slot], and the tile list: tile_info[3 i] = expert, [3 i + 1] = first slot,
-// [3 i + 2] = rows; n_tiles[0] = how many.
-__global__ void moe_group_kernel(const int* __restrict__ expert_of, int n_pairs, int n_experts, int* __restrict__ slot_of,
-                                 int* __restrict__ pair_of, int* __restrict__ tile_info, int* __restrict__ n_tiles,
-                                 int tile_rows, int n_real) {
+// [3 i + 2] = rows; n_tiles[0] = how many.  It is a chain of latencies (read, count, sum up, write), so each is gone through
+// once: a thread's pairs are read together and stay in registers (GROUP_KEPT a thread; what is beyond is read again), the
+// count of a pair's expert hands it its place within the expert, and a warp sums the counts up.  (Which pair of an expert
+// gets which slot changes no result: every row is computed by itself.)
+constexpr int GROUP_KEPT = 16;
+
+__global__ void __launch_bounds__(1024)
+moe_group_kernel(const int* __restrict__ expert_of, int n_pairs, int n_experts, int* __restrict__ slot_of,
+                 int* __restrict__ pair_of, int* __restrict__ tile_info, int* __restrict__ n_tiles, int tile_rows, int n_real) {
     extern __shared__ int smi[];                       // count [n_experts], first [n_experts + 1], tile0 [n_experts + 1]
     int* count = smi;
     int* first = smi + n_experts;
     int* tile0 = first + n_experts + 1;
+    for (int e = threadIdx.x; e < n_experts; e += blockDim.x) count[e] = 0;
     pdl_trigger();
     pdl_wait();
-    for (int e = threadIdx.x; e < n_experts; e += blockDim.x) count[e] = 0;
     __syncthreads();
-    for (int p = threadIdx.x; p < n_pairs; p += blockDim.x)
-        if (expert_of[p] < n_real) atomicAdd(&count[expert_of[p]], 1);
+    const int kept = GROUP_KEPT * blockDim.x;
+    int expert[GROUP_KEPT], place[GROUP_KEPT];
+#pragma unroll
+    for (int i = 0; i < GROUP_KEPT; ++i) {
+        const int p = threadIdx.x + i * blockDim.x;
+        expert[i] = p < n_pairs ? expert_of[p] : n_real;
+    }
+#pragma unroll
+    for (int i = 0; i < GROUP_KEPT; ++i) place[i] = expert[i] < n_real ? atomicAdd(&count[expert[i]], 1) : -1;
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (n_pairs > kept) {                              // (these take places from the end of their experts' slots, below)
+        for (int p = kept + threadIdx.x; p < n_pairs; p += blockDim.x)
+            if (expert_of[p] < n_real) atomicAdd(&count[expert_of[p]], 1);
+        __syncthreads();
+    }
+    if (threadIdx.x < 32) {
         int at = 0, tiles = 0;
-        for (int e = 0; e < n_experts; ++e) {
-            first[e] = at;
-            tile0[e] = tiles;
-            at += count[e];
-            tiles += (count[e] + tile_rows - 1) / tile_rows;
+        for (int e0 = 0; e0 < n_experts; e0 += 32) {
+            const int e = e0 + threadIdx.x, n = e < n_experts ? count[e] : 0, t = (n + tile_rows - 1) / tile_rows;
+            int upto_n = n, upto_t = t;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int on = __shfl_up_sync(0xffffffffu, upto_n, o), ot = __shfl_up_sync(0xffffffffu, upto_t, o);
+                if ((int)threadIdx.x >= o) upto_n += on, upto_t += ot;
+            }
+            if (e < n_experts) first[e] = at + upto_n - n, tile0[e] = tiles + upto_t - t;
+            at += __shfl_sync(0xffffffffu, upto_n, 31);
+            tiles += __shfl_sync(0xffffffffu, upto_t, 31);
         }
-        first[n_experts] = at;
-        tile0[n_experts] = tiles;
-        n_tiles[0] = tiles;
+        if (threadIdx.x == 0) n_tiles[0] = tiles;
     }
     __syncthreads();
+#pragma unroll
+    for (int i = 0; i < GROUP_KEPT; ++i) {
+        const int p = threadIdx.x + i * blockDim.x;
+        if (p < n_pairs) {
+            const int slot = place[i] < 0 ? -1 : first[expert[i]] + place[i];   // (-1: an identity expert, nothing to compute)
+            slot_of[p] = slot;
+            if (slot >= 0) pair_of[slot] = p;
+        }
+    }
     for (int e = threadIdx.x; e < n_experts; e += blockDim.x) {
         const int n = count[e];
         for (int i = 0, k = tile0[e]; i < n; i += tile_rows, ++k) {
@@ -192,21 +250,17 @@ __global__ void moe_group_kernel(const int* __restrict__ expert_of, int n_pairs,
             tile_info[3 * k + 1] = first[e] + i;
             tile_info[3 * k + 2] = min(tile_rows, n - i);
         }
-        count[e] = 0;                                  // now the cursor within the expert's slots
     }
+    if (n_pairs <= kept) return;
     __syncthreads();
-    // slots in the order of the pairs within each expert: a thread takes a run of pairs, runs in thread order
-    // would need a scan per expert; the order within an expert changes no result (every row is computed by
-    // itself), so the slots are simply drawn
-    for (int p = threadIdx.x; p < n_pairs; p += blockDim.x) {
+    for (int p = kept + threadIdx.x; p < n_pairs; p += blockDim.x) {
         const int e = expert_of[p];
-        if (e >= n_real) {                             // an identity expert: nothing to compute
-            slot_of[p] = -1;
-            continue;
+        int slot = -1;
+        if (e < n_real) {
+            slot = first[e] + atomicSub(&count[e], 1) - 1;
+            pair_of[slot] = p;
         }
-        const int slot = first[e] + atomicAdd(&count[e], 1);
         slot_of[p] = slot;
-        pair_of[slot] = p;
     }
 }
 
@@ -412,24 +466,27 @@ MU_EXPORT int mu_moe_route(const void* h, long long ldh, int h_bf16, const float
     // prompt steps: several tokens a block, so that the router's rows are read once for all of them (with a block a
     // token the router came out of the L2 once per token); few tokens: a block each, spread over the SMs
     int tok = n_tokens >= 4 * mu::sm_count() ? 8 : 1;
-    while (tok > 1 && (size_t)tok * (hidden + 2 * n_experts) * sizeof(float) > 48 * 1024) tok /= 2;
+    // (as many as leave room for two blocks an SM; one token takes no more than 48 KB, as it always did)
+    while (tok > 1 && (size_t)tok * (hidden + 2 * n_experts) * sizeof(float) > mu::ROUTE_SMEM) tok /= 2;
     const size_t smem = (size_t)tok * (hidden + 2 * n_experts) * sizeof(float);
-    if (smem > 48 * 1024) return MU_ERR_UNSUPPORTED_SIZE;
+    if (tok == 1 && smem > 48 * 1024) return MU_ERR_UNSUPPORTED_SIZE;
     cudaStream_t s = (cudaStream_t)stream;
     const dim3 grid((n_tokens + tok - 1) / tok), block(mu::ROUTE_WARPS * 32);
 #define MU_ROUTE(T, TOK)                                                                                               \
+    if (!mu::allow_shared(reinterpret_cast<const void*>(mu::moe_route_kernel<T, TOK>), TOK > 1 ? mu::ROUTE_SMEM : 0))  \
+        return MU_ERR_LAUNCH;                                                                                          \
     return mu::launch_pdl(mu::moe_route_kernel<T, TOK>, grid, block, smem, s, 1, (const T*)h, ldh, router, correction, \
                           n_tokens, hidden, n_experts, top, scale, softmax, renormalize, expert_of, weight_of,         \
                           renorm_eps, gate_w, gate_out)
     if (h_bf16) {
-        if (tok == 8) MU_ROUTE(__nv_bfloat16, 8);
-        if (tok == 4) MU_ROUTE(__nv_bfloat16, 4);
-        if (tok == 2) MU_ROUTE(__nv_bfloat16, 2);
+        if (tok == 8) { MU_ROUTE(__nv_bfloat16, 8); }
+        if (tok == 4) { MU_ROUTE(__nv_bfloat16, 4); }
+        if (tok == 2) { MU_ROUTE(__nv_bfloat16, 2); }
         MU_ROUTE(__nv_bfloat16, 1);
     }
-    if (tok == 8) MU_ROUTE(float, 8);
-    if (tok == 4) MU_ROUTE(float, 4);
-    if (tok == 2) MU_ROUTE(float, 2);
+    if (tok == 8) { MU_ROUTE(float, 8); }
+    if (tok == 4) { MU_ROUTE(float, 4); }
+    if (tok == 2) { MU_ROUTE(float, 2); }
     MU_ROUTE(float, 1);
 #undef MU_ROUTE
 }
@@ -445,7 +502,7 @@ MU_EXPORT int mu_moe_group(const int* expert_of, int n_pairs, int n_experts, int
     const size_t smem = (size_t)(3 * n_experts + 2) * sizeof(int);
     if (smem > 48 * 1024) return MU_ERR_UNSUPPORTED_SIZE;
     if (n_real < 0 || n_real > n_experts) return MU_ERR_BAD_ARGUMENT;
-    return mu::launch_pdl(mu::moe_group_kernel, dim3(1), dim3(1024), smem, (cudaStream_t)stream, 1, expert_of, n_pairs,
+    return mu::launch_pdl(mu::moe_group_kernel, dim3(1), dim3(n_pairs > 256 ? 1024 : 128), smem, (cudaStream_t)stream, 1, expert_of, n_pairs,
                           n_experts, slot_of, pair_of, tile_info, n_tiles, tile_rows, n_real > 0 ? n_real : n_experts);
 }
 

@@ -113,3 +113,54 @@ def test_products_per_head_on_tcgen05(rows, heads, n, k, lead, out_dtype):
             assert not got[:, :, n:].any()                             # nothing written between the slices
         bound = 1e-5 if out_dtype == torch.float32 else 2.0 ** -8
         assert float(((got[:, :, :n].double() - want).abs() / (want.abs() + want.square().mean().sqrt())).max()) < bound
+
+
+# one block of 128 threads, of 1024, pairs beyond those it keeps in registers; identity experts; more experts than a warp
+@pytest.mark.parametrize("P,experts,real", [(1, 4, 4), (48, 72, 64), (256, 33, 33), (257, 5, 4), (12288, 64, 64), (20001, 70, 64)])
+@pytest.mark.parametrize("rows", [32, 128])
+def test_grouping_of_pairs(P, experts, real, rows):
+    """Every pair of a real expert has a slot of its own among its expert's, which lie together; the tiles cover them."""
+    ops = _ops()
+    rng = np.random.default_rng(P)
+    expert = rng.integers(0, experts, P).astype(np.int32)
+    expert[expert == 1] = 0
+    slot, pair = (torch.full((P,), -7, dtype=torch.int32, device="cuda") for _ in range(2))
+    most = P // rows + experts
+    info, n = torch.full((3 * most,), -7, dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    ops.moe_group(torch.as_tensor(expert).cuda(), experts, slot, pair, info, n, rows, n_real=real)
+    slot, pair, info, n = slot.cpu().numpy(), pair.cpu().numpy(), info.cpu().numpy().reshape(-1, 3), int(n)
+    chosen = np.nonzero(expert < real)[0]
+    assert (slot[expert >= real] == -1).all()
+    assert sorted(slot[chosen]) == list(range(len(chosen))) and (pair[slot[chosen]] == chosen).all()
+    by_slot = expert[pair[:len(chosen)]]
+    assert (np.diff(by_slot) >= 0).all()
+    want = [(e, a + i, min(rows, c - i)) for e in range(real) for a, c in [(int((expert[chosen] < e).sum()), int((expert == e).sum()))]
+            for i in range(0, c, rows)]
+    assert n == len(want) and [tuple(t) for t in info[:n]] == want
+
+
+# eight, four and two tokens a block (what the staged rows leave room for), a block's tokens cut off, an odd number of rows
+@pytest.mark.parametrize("tokens,hidden,experts,gate", [(601, 256, 64, True), (700, 2048, 17, False), (650, 4096, 16, True),
+                                                        (593, 6200, 5, True)])
+def test_router_of_several_tokens_a_block(tokens, hidden, experts, gate):
+    """Each logit a float32 sum of `hidden` terms in 128 parts: scores within 1e-5; and the bits that a token alone gives."""
+    ops = _ops()
+    h = _rand((tokens, hidden), 1, torch.bfloat16)
+    router, g = _rand((experts, hidden), 2, scale=hidden ** -0.5), _rand((hidden,), 3, scale=hidden ** -0.5) if gate else None
+    top = 3
+
+    def route(x):
+        expert = torch.zeros(x.shape[0] * top, dtype=torch.int32, device="cuda")
+        weight, out = torch.zeros(x.shape[0] * top, device="cuda"), torch.zeros(x.shape[0], device="cuda") if gate else None
+        ops.moe_route(x, router, None, top, 1.0, expert, weight, gate_weight=g, gate_out=out)
+        return expert.reshape(-1, top), weight.reshape(-1, top), out
+
+    expert, weight, out = route(h)
+    s = torch.sigmoid(h.double() @ router.double().T)
+    assert float((weight.double() - torch.gather(s, 1, expert.long())).abs().max()) < 1e-5
+    assert float((s.sort(dim=1, descending=True)[0][:, :top] - weight.double()).abs().max()) < 1e-5
+    if gate:
+        assert float((out.double() - torch.sigmoid(h.double() @ g.double())).abs().max()) < 1e-5
+    for t in (0, 7, tokens - 1):
+        e1, w1, g1 = route(h[t:t + 1])
+        assert torch.equal(e1[0], expert[t]) and torch.equal(w1[0], weight[t]) and (not gate or torch.equal(g1[0], out[t]))
