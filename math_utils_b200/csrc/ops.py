@@ -130,8 +130,11 @@ _SIGNATURES = {
     "mu_ssd_conv": [_c_p, _c_ll, _c_int, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_p, _c_p, _c_p, _c_p, _c_ll,
                     _c_int, _c_p, _c_p, _c_int],
     "mu_selective_scan_max_state": [],
+    "mu_selective_scan_segment": [],
+    "mu_selective_scan_scratch": [_c_int] * 4,
+    "mu_selective_scan_splits": [_c_int] * 3,
     "mu_selective_scan": [_c_p, _c_ll, _c_p, _c_ll, _c_p, _c_ll, _c_p, _c_ll, _c_int, _c_int, _c_p, _c_p, _c_int, _c_int, _c_int,
-                          _c_p, _c_p, _c_p, _c_ll, _c_ll, _c_p, _c_ll, _c_int, _c_int, _c_p],
+                          _c_p, _c_p, _c_p, _c_ll, _c_ll, _c_p, _c_ll, _c_int, _c_int, _c_p, _c_int, _c_p],
     "mu_ssd_scan": [_c_p, _c_int, _c_p, _c_ll, _c_int, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_p,
                     _c_p, _c_p, _c_ll, _c_ll, _c_p, _c_int, _c_p],
     "mu_gated_group_norm": [_c_p, _c_ll, _c_p, _c_ll, _c_p, _c_int, _c_int, _c_int, _c_f, _c_p, _c_ll, _c_int, _c_p, _c_int, _c_int, _c_p, _c_p, _c_int],
@@ -737,11 +740,12 @@ def selective_scan_max_state() -> int:
 
 def selective_scan(x: torch.Tensor, z: torch.Tensor, dt: torch.Tensor, bc: torch.Tensor, b_at: int, c_at: int,
                    rates: torch.Tensor, skip: torch.Tensor, seq_first, seq_slots, state: torch.Tensor, state_offset: int,
-                   out: torch.Tensor) -> torch.Tensor:
+                   out: torch.Tensor, max_len: int = 0) -> torch.Tensor:
     """The recurrence S[c, n] = 2^(dt_c rates[c, n]) S[c, n] + dt_c x_c B_n, out_c = (sum_n S[c, n] C_n + skip_c x_c) silu(z_c)
     over the step's tokens of each sequence, from and to ``state[slot][state_offset:]`` (channels x N float32).  ``x``, ``z``
     and ``out`` [T, channels] in the compute dtype, ``dt`` float32; B and C are the columns of the float32 rows ``bc`` from
-    ``b_at`` and ``c_at`` on, each followed by filling up to a multiple of four."""
+    ``b_at`` and ``c_at`` on, each followed by filling up to a multiple of four.  ``max_len``: the tokens that the longest
+    sequence brings, if the caller knows; few long sequences then go in segments that work at once."""
     _need_cuda(x, z, dt, bc, rates, skip, seq_first, seq_slots, state, out)
     _i32(seq_first, "seq_first"); _i32(seq_slots, "seq_slots")
     T, inner = x.shape
@@ -756,11 +760,20 @@ def selective_scan(x: torch.Tensor, z: torch.Tensor, dt: torch.Tensor, bc: torch
             or not skip.is_contiguous() or state.dtype != torch.float32 or state.stride(1) != 1
             or state.shape[1] < state_offset + inner * N):
         raise KernelError("selective_scan: step sizes, B and C, rates or state do not fit")
-    _check(library().mu_selective_scan(_ptr(x), x.stride(0), _ptr(z), z.stride(0), _ptr(dt), dt.stride(0), _ptr(bc), bc.stride(0),
+    lib, n_seqs = library(), seq_slots.numel()
+    long_steps = T > 4 * n_seqs
+    segments = -(-int(max_len) // lib.mu_selective_scan_segment()) if long_steps else 1
+    room = None
+    if segments > 1 and lib.mu_selective_scan_splits(n_seqs, inner, N):
+        lib.mu_selective_scan_scratch.restype = _c_ll
+        room = scratch("selective_scan", x.device, int(lib.mu_selective_scan_scratch(n_seqs, segments, inner, N)), torch.float32)
+    else:
+        segments = 1
+    _check(lib.mu_selective_scan(_ptr(x), x.stride(0), _ptr(z), z.stride(0), _ptr(dt), dt.stride(0), _ptr(bc), bc.stride(0),
                                        int(b_at), int(c_at), _ptr(rates), _ptr(skip), seq_slots.numel(), inner, N,
                                        _ptr(seq_first), _ptr(seq_slots), _ptr(state), state.stride(0), int(state_offset),
-                                       _ptr(out), out.stride(0), _is_bf16(out), int(T > 4 * seq_slots.numel()), _stream()),
-           ("selective_scan(channels={}, N={})", inner, N))
+                                       _ptr(out), out.stride(0), _is_bf16(out), int(long_steps), _stream(), segments, _ptr(room)),
+           ("selective_scan(channels={}, N={})", inner, N), launches=2 if segments > 1 else 1)
     return out
 
 

@@ -11,7 +11,13 @@
 // large states 8) at a time: B and C by asynchronous copies in two stages, x, dt and z through registers (read ahead while
 // the ones before are worked on), which also carry x and z to the gate.  Tokens past a sequence's end are staged with
 // dt = 0, which leaves the state as it is.  The order of every sum is fixed by N alone: a token's result does not depend on
-// how the sequence was cut into steps or on the batch.
+// how the sequence was cut into steps or on the batch, but for what follows.
+//
+// Long steps of few sequences leave the device with fewer than two warps a scheduler, each waiting for its own exponentials.
+// They go in segments of SS_SEGMENT tokens that work at once: a first launch takes every segment but a sequence's last from
+// a zero state (the first from the slot's) and leaves where it ends and the sum of its dt; the second puts a segment's
+// starting state together from those before it, S <- 2^(A sum dt) S + end, and runs as above.  The exponentials are made
+// almost twice for four times the warps.
 #include "common.cuh"
 
 #include <math.h>
@@ -32,14 +38,24 @@ template <> __device__ __forceinline__ float gated<__nv_bfloat16>(float v, float
     return __fdividef(v * z, 1.0f + __expf(-z));
 }
 
-// SS_CHUNK: tokens staged at a time.  VEC: every pair of a channel's state starts on an 8-byte boundary.
-template <typename TE, int LPC, int NS, bool VEC, int SS_CHUNK>
+constexpr int SS_SEGMENT = 256;
+
+// What the segmented form keeps in scratch; place: sequence * most + segment.
+struct SsSegments {
+    int most;                    // segments of the longest sequence (1: not segmented)
+    float* ends;                 // [places][inner][N padded to pairs]; a sequence's last place: the slot's state before the step
+    float* sums;                 // [places][inner]: sum of dt
+};
+
+// SS_CHUNK: tokens staged at a time.  VEC: every pair of a channel's state starts on an 8-byte boundary.  MODE 0: whole
+// sequences; 1: segments' ends; 2: segments' outputs.
+template <typename TE, int LPC, int NS, bool VEC, int SS_CHUNK, int MODE>
 __global__ void __launch_bounds__(SS_THREADS)
 selective_scan_kernel(const TE* __restrict__ x, long long ldx, const TE* __restrict__ z, long long ldz,
                       const float* __restrict__ dt, long long lddt, const float* __restrict__ bc, long long ldbc, int b_at,
                       int c_at, const float* __restrict__ rates, const float* __restrict__ skip, int inner, int N,
                       const int* __restrict__ seq_first, const int* __restrict__ seq_slots, float* __restrict__ state,
-                      long long state_stride, long long state_offset, TE* __restrict__ y, long long ldy) {
+                      long long state_stride, long long state_offset, TE* __restrict__ y, long long ldy, SsSegments seg) {
     constexpr int NPAD = LPC * NS, Q = NS / 2, COLS = ss_channels(LPC), GROUP = LPC < SS_CHUNK ? LPC : SS_CHUNK;
     constexpr int ROWS = SS_THREADS / COLS;                  // tokens of a chunk that are staged at once, a channel a thread
     constexpr int PER = (SS_CHUNK + ROWS - 1) / ROWS;
@@ -69,13 +85,31 @@ selective_scan_kernel(const TE* __restrict__ x, long long ldx, const TE* __restr
     const bool real = col < inner;
     const float d_skip = real ? skip[col] : 0.0f;
     pdl_wait();
-    const int first = seq_first[s], count = seq_first[s + 1] - first;
+    int first = seq_first[s], count = seq_first[s + 1] - first;
+    const int segment = MODE ? blockIdx.z : 0, segments = MODE ? (count + SS_SEGMENT - 1) / SS_SEGMENT : 1;
+    if (MODE && (segment >= segments || (MODE == 1 && segments == 1))) return;
+    if (MODE == 1 && segment == segments - 1) return;        // (nothing starts from where the last one ends)
+    const int np = (N + 1) & ~1;
+    // the scratch of (this sequence's segment i, this channel)
+    auto end_of = [&](int i) { return seg.ends + (((long long)s * seg.most + i) * inner + c) * np; };
     float* const mine = state + (long long)seq_slots[s] * state_stride + state_offset + (long long)c * N;
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
         const int n = 2 * (l + LPC * q);
         float2 v = make_float2(0.0f, 0.0f);
-        if (live) {
+        if (MODE == 2 && segments > 1) {
+            // (the slot's state is moved on by the last segment's block while others may not have begun: it was copied)
+            if (live && n < N) {
+                v = *reinterpret_cast<const float2*>(end_of(segment ? 0 : segments - 1) + n);
+                const float2 a = floats_of_pair(A[q]);
+                for (int i = 1; i < segment; ++i) {
+                    const float step = seg.sums[((long long)s * seg.most + i) * inner + c];
+                    const float2 e = *reinterpret_cast<const float2*>(end_of(i) + n);
+                    v.x = fmaf(exp2_fast(step * a.x), v.x, e.x);
+                    v.y = fmaf(exp2_fast(step * a.y), v.y, e.y);
+                }
+            }
+        } else if (live && (MODE != 1 || segment == 0)) {
             if (VEC) {
                 if (n < N) v = *reinterpret_cast<const float2*>(mine + n);
             } else {
@@ -84,7 +118,13 @@ selective_scan_kernel(const TE* __restrict__ x, long long ldx, const TE* __restr
             }
         }
         S[q] = pair_of_floats(v.x, v.y);
+        if (MODE == 1 && segment == 0 && live && n < N) *reinterpret_cast<float2*>(end_of(segments - 1) + n) = v;
     }
+    if (MODE) {
+        first += segment * SS_SEGMENT;
+        count = min(SS_SEGMENT, count - segment * SS_SEGMENT);
+    }
+    float total = 0.0f;                                      // MODE 1: the sum of the channel's dt
     const long long at = first + row, place = real ? col : inner - 1;
     const TE* xp = x + at * ldx + place;
     const TE* zp = z + at * ldz + place;
@@ -147,6 +187,7 @@ selective_scan_kernel(const TE* __restrict__ x, long long ldx, const TE* __restr
 #pragma unroll
             for (int i = 0; i < GROUP; ++i) {
                 const float2 d = ds[b][t0 + i][ch];
+                if (MODE == 1) total += d.x;
                 const float2x d2 = pair_of_floats(d.x, d.x), x2 = pair_of_floats(d.y, d.y);
                 float2x a = 0;                               // (two zeros)
 #pragma unroll
@@ -155,11 +196,12 @@ selective_scan_kernel(const TE* __restrict__ x, long long ldx, const TE* __restr
                     const float2x cc = *reinterpret_cast<const float2x*>(&Cs[b][t0 + i][2 * (l + LPC * q)]);
                     const float2 e = floats_of_pair(pair_mul(d2, A[q]));
                     S[q] = pair_fma(pair_of_floats(exp2_fast(e.x), exp2_fast(e.y)), S[q], pair_mul(x2, bb));
-                    a = pair_fma(S[q], cc, a);
+                    if (MODE != 1) a = pair_fma(S[q], cc, a);
                 }
                 const float2 sum = floats_of_pair(a);
                 acc[i] = sum.x + sum.y;
             }
+            if (MODE == 1) continue;
 #pragma unroll
             for (int width = LPC / 2; width >= GROUP; width >>= 1) {
 #pragma unroll
@@ -181,13 +223,22 @@ selective_scan_kernel(const TE* __restrict__ x, long long ldx, const TE* __restr
 #pragma unroll
         for (int k = 0; k < PER; ++k) {
             const int tok = row + ROWS * k;
-            if (tok < n && real)
+            if (MODE != 1 && tok < n && real)
                 yp[(li0 + ROWS * k) * ldy] = from_float<TE>(gated<TE>(fmaf(d_skip, gate_x[k], ys[tok][tid % COLS]), gate_z[k]));
         }
         if (more) stage_rows(li0 + SS_CHUNK, b ^ 1);
     }
     pdl_trigger();
-    if (!live) return;
+    if (!live || (MODE == 2 && segment < segments - 1)) return;
+    if (MODE == 1) {
+        if (l == 0) seg.sums[((long long)s * seg.most + segment) * inner + c] = total;
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            const int n = 2 * (l + LPC * q);
+            if (n < N) *reinterpret_cast<float2*>(end_of(segment) + n) = floats_of_pair(S[q]);
+        }
+        return;
+    }
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
         const int n = 2 * (l + LPC * q);
@@ -208,13 +259,28 @@ MU_EXPORT int mu_selective_scan_max_state() { return 256; }
 
 // x, z, y [T][inner] views (compute dtype), dt [T][inner] float32; bc float32 rows with B from column b_at and C from
 // c_at on (N rounded up to four entries each, 16-byte aligned); rates [inner][N] = A log2(e).  State of a slot from
-// state_offset on: [inner][N].  long_steps: many tokens a sequence; the launch then waits for an empty device.
+// state_offset on: [inner][N].  long_steps: many tokens a sequence; the launch then waits for an empty device.  segments > 1
+// (with long_steps): the longest sequence's tokens over mu_selective_scan_segment, rounded up; scratch then holds
+// mu_selective_scan_scratch floats, 8-byte aligned.
+MU_EXPORT int mu_selective_scan_segment() { return mu::SS_SEGMENT; }
+
+MU_EXPORT long long mu_selective_scan_scratch(int n_seqs, int segments, int inner, int N) {
+    return (long long)n_seqs * segments * inner * (((N + 1) & ~1) + 1);
+}
+
+// Segments are worth their second launch where the scan alone would leave SMs with fewer than four blocks (16 warps).
+MU_EXPORT int mu_selective_scan_splits(int n_seqs, int inner, int N) {
+    const int lanes = N <= 8 ? 4 : N <= 16 ? 8 : N <= 32 ? 16 : 32;
+    return (long long)n_seqs * ((inner + mu::ss_channels(lanes) - 1) / mu::ss_channels(lanes)) < 4ll * mu::sm_count();
+}
+
 MU_EXPORT int mu_selective_scan(const void* x, long long ldx, const void* z, long long ldz, const float* dt, long long lddt,
                                 const float* bc, long long ldbc, int b_at, int c_at, const float* rates, const float* skip,
                                 int n_seqs, int inner, int N, const int* seq_first, const int* seq_slots, float* state,
                                 long long state_stride, long long state_offset, void* y, long long ldy, int is_bf16,
-                                int long_steps, void* stream) {
+                                int long_steps, void* stream, int segments, float* scratch) {
     if (n_seqs <= 0) return MU_OK;
+    if (segments > 1 && (!long_steps || !scratch || ((uintptr_t)scratch & 7) || segments > 65535)) return MU_ERR_BAD_ARGUMENT;
     if (!x || !z || !dt || !bc || !rates || !skip || !seq_first || !seq_slots || !state || !y || inner <= 0 || N <= 0 ||
         b_at < 0 || c_at < 0)
         return MU_ERR_BAD_ARGUMENT;
@@ -223,17 +289,30 @@ MU_EXPORT int mu_selective_scan(const void* x, long long ldx, const void* z, lon
     cudaStream_t s = (cudaStream_t)stream;
     typedef __nv_bfloat16 bf;
     const bool vec = N % 2 == 0 && state_stride % 2 == 0 && state_offset % 2 == 0 && ((uintptr_t)state & 7) == 0;
+    const mu::SsSegments seg = {segments, scratch, scratch + (long long)n_seqs * segments * inner * ((N + 1) & ~1)};
 #define MU_SELECTIVE_V(TE, LPC, NS, V)                                                                                 \
     do {                                                                                                               \
         const dim3 grid(n_seqs, (inner + mu::ss_channels(LPC) - 1) / mu::ss_channels(LPC)), block(mu::SS_THREADS);     \
-        auto kernel = mu::selective_scan_kernel<TE, LPC, NS, V, NS <= 4 ? 16 : 8>;                                                       \
+        constexpr int CHUNK = NS <= 4 ? 16 : 8;                                                                        \
+        auto kernel = mu::selective_scan_kernel<TE, LPC, NS, V, CHUNK, 0>;                                             \
+        if (segments > 1) {                                                                                            \
+            const dim3 cut(grid.x, grid.y, segments);                                                                  \
+            if (int e = mu::launch_pdl(mu::selective_scan_kernel<TE, LPC, NS, V, CHUNK, 1>, cut, block, 0, s, 1,       \
+                                       (const TE*)x, ldx, (const TE*)z, ldz, dt, lddt, bc, ldbc, b_at, c_at, rates,    \
+                                       skip, inner, N, seq_first, seq_slots, state, state_stride, state_offset,        \
+                                       (TE*)y, ldy, seg))                                                              \
+                return e;                                                                                              \
+            return mu::launch_pdl(mu::selective_scan_kernel<TE, LPC, NS, V, CHUNK, 2>, cut, block, 0, s, 1,            \
+                                  (const TE*)x, ldx, (const TE*)z, ldz, dt, lddt, bc, ldbc, b_at, c_at, rates, skip,   \
+                                  inner, N, seq_first, seq_slots, state, state_stride, state_offset, (TE*)y, ldy, seg); \
+        }                                                                                                              \
         if (long_steps)                                                                                                \
             return mu::launch_after(kernel, grid, block, 0, s, (const TE*)x, ldx, (const TE*)z, ldz, dt, lddt, bc,     \
                                     ldbc, b_at, c_at, rates, skip, inner, N, seq_first, seq_slots, state,              \
-                                    state_stride, state_offset, (TE*)y, ldy);                                          \
+                                    state_stride, state_offset, (TE*)y, ldy, seg);                                     \
         return mu::launch_pdl(kernel, grid, block, 0, s, 1, (const TE*)x, ldx, (const TE*)z, ldz, dt, lddt, bc, ldbc,  \
                               b_at, c_at, rates, skip, inner, N, seq_first, seq_slots, state, state_stride,            \
-                              state_offset, (TE*)y, ldy);                                                              \
+                              state_offset, (TE*)y, ldy, seg);                                                         \
     } while (0)
 #define MU_SELECTIVE(LPC, NS)                                                                                          \
     do {                                                                                                               \

@@ -114,3 +114,31 @@ def test_state_space_scan_in_chunks(lens, H, P, N, G, dtype):
         want_state[slot, offset:] = S.reshape(-1)
     _no_further_off(got["chunks"][0], got["tokens"][0], want)
     _no_further_off(got["chunks"][1], got["tokens"][1], want_state)
+
+
+@pytest.mark.parametrize("lens", [(256,), (257, 1), (600, 255, 3), (40, 1025)])
+@pytest.mark.parametrize("C,N,dtype", [(40, 16, torch.bfloat16), (17, 5, torch.float32), (24, 40, torch.float32), (16, 130, torch.bfloat16)])
+def test_selective_scan_in_segments(lens, C, N, dtype):
+    """Segments put together against the whole sequences' scan: the same sums but for the starting states of segments, which
+    a product of 256 decays reaches in one exponential, off by 2^-22 of its argument's size."""
+    ops = _ops()
+    T, slots = sum(lens), list(range(len(lens)))[::-1]
+    first = _ints(np.concatenate([[0], np.cumsum(lens)]))
+    x, z = _rand((T, C), 1).to(dtype), _rand((T, C), 2).to(dtype)
+    dt = torch.nn.functional.softplus(_rand((T, C), 3) - 3.0)
+    n4 = -(-N // 4) * 4
+    bc = _rand((T, 2 * n4), 4)
+    rates = -torch.exp(_rand((C, N), 5)).contiguous() * 1.4427
+    skip = _rand((C,), 6)
+    values = 6 + C * N
+    start = _rand((len(lens), values + -values % 4), 7)
+    got = []
+    for most in (0, max(lens)):
+        state, out = start.clone(), torch.zeros((T, C), dtype=dtype, device="cuda")
+        ops.selective_scan(x, z, dt, bc, 0, n4, rates, skip, first, _ints(slots), state, 6, out, max_len=most)
+        got.append((out, state))
+    assert torch.equal(got[0][1][:, :6], start[:, :6]) and torch.equal(got[1][1][:, :6], start[:, :6])
+    assert _rel(got[1][1], got[0][1].double()) < 2e-6
+    assert _rel(got[1][0], got[0][0].double()) < (2e-6 if dtype == torch.float32 else 2e-3)
+    worst = (got[1][0].double() - got[0][0].double()).abs() / (got[0][0].double().abs() + got[0][0].double().square().mean().sqrt())
+    assert float(worst.max()) < (1e-5 if dtype == torch.float32 else 2.0 ** -7)
