@@ -36,6 +36,8 @@
 
 #include <math.h>
 
+#include <type_traits>
+
 namespace mu {
 
 constexpr int MA_WARPS = 4;
@@ -291,11 +293,53 @@ mapped_attention_kernel(const TE* __restrict__ q, long long ldq, const TE* __res
 
 // Single-token steps.  A block takes one (token, kv head) and every MD_SPLITS-th page of what the token sees
 // (page index modulo MD_SPLITS = blockIdx.z, so the share does not depend on the batch): the page's keys and values
-// of that kv head are staged in shared memory once and serve all query heads of the group, a warp a head, a lane a
-// key for the scores and a lane a value entry for the sums.  Each (token, head, map, share) leaves a maximum, a sum
-// and unnormalised values; mapped_merge_kernel puts the shares together in their order and finishes the head.
-constexpr int MD_SPLITS = 16;
+// of that kv head are staged in shared memory once and serve all query heads of the group, two warps a head (half of the
+// page's keys each), a lane a key for the scores and up to four neighbouring value entries a lane for the sums.  Each
+// (token, head, map, share) leaves a maximum, a sum and unnormalised values; mapped_merge_kernel puts the shares together,
+// a lane a share, and finishes the head.  A share is a chain of latencies (page, scores, sums), so shares are many and short.
+constexpr int MD_SPLITS = 32;
 constexpr int MD_KEYS = 64;         // keys staged at a time: one page
+
+// The product of a staged query (16-byte aligned where vec) and a staged key.
+__device__ __forceinline__ float dot_staged(const float* qs, const float* key, int dim, bool vec) {
+    return dot_key<float>(qs, key, dim, vec);
+}
+__device__ __forceinline__ float dot_staged(const float* qs, const __nv_bfloat16* key, int dim, bool vec) {
+    if (!vec) return dot_key<__nv_bfloat16>(qs, key, dim, false);
+    float s0 = 0.0f, s1 = 0.0f;
+    for (int d = 0; d < dim; d += 8) {
+        const uint4 raw = *reinterpret_cast<const uint4*>(key + d);
+        const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&raw);
+        const float4 qa = *reinterpret_cast<const float4*>(qs + d), qb = *reinterpret_cast<const float4*>(qs + d + 4);
+        const float2 f0 = __bfloat1622float2(p[0]), f1 = __bfloat1622float2(p[1]);
+        const float2 f2 = __bfloat1622float2(p[2]), f3 = __bfloat1622float2(p[3]);
+        s0 = fmaf(qa.x, f0.x, s0); s1 = fmaf(qa.y, f0.y, s1); s0 = fmaf(qa.z, f1.x, s0); s1 = fmaf(qa.w, f1.y, s1);
+        s0 = fmaf(qb.x, f2.x, s0); s1 = fmaf(qb.y, f2.y, s1); s0 = fmaf(qb.z, f3.x, s0); s1 = fmaf(qb.w, f3.y, s1);
+    }
+    return s0 + s1;
+}
+// W neighbouring value entries (aligned to their own size where W > 1).
+template <int W> __device__ __forceinline__ void read_values(float (&x)[W], const float* p) {
+#pragma unroll
+    for (int e = 0; e < W; ++e) x[e] = p[e];
+}
+template <int W> __device__ __forceinline__ void read_values(float (&x)[W], const __nv_bfloat16* p) {
+    if constexpr (W == 1) {
+        x[0] = __bfloat162float(*p);
+    } else {
+        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(p);
+        uint2 raw;
+        if constexpr (W == 4) {
+            raw = *reinterpret_cast<const uint2*>(p);
+            h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+        }
+#pragma unroll
+        for (int e = 0; e < W; e += 2) {
+            const float2 f = __bfloat1622float2(h[e / 2]);
+            x[e] = f.x, x[e + 1] = f.y;
+        }
+    }
+}
 
 template <typename TE, int MAPS>
 __global__ void __launch_bounds__(128)
@@ -314,7 +358,9 @@ mapped_decode_kernel(const TE* __restrict__ q, long long ldq, const TE* __restri
     pdl_trigger();
     pdl_wait();
     const int t = blockIdx.x, g = blockIdx.y, share = blockIdx.z;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, warps = blockDim.x >> 5;
+    // two sets of warps: set 0 takes a page's first 32 keys, set 1 its last; within a set a warp a head, in turns
+    const int tid = threadIdx.x, lane = tid & 31, warps = blockDim.x >> 6;
+    const int half = (tid >> 5) >= warps, warp = (tid >> 5) - half * warps;
     const int group = n_heads / n_kv_heads;
     const int pos = tok_pos[t];
     const int first = chunk > 0 ? pos - pos % chunk : window > 0 ? max(0, pos - window + 1) : 0;
@@ -324,6 +370,9 @@ mapped_decode_kernel(const TE* __restrict__ q, long long ldq, const TE* __restri
     const long long key_off = (long long)g * kw, val_off = (long long)n_kv_heads * kw + (long long)g * vw;
     for (int i = tid; i < group * kw; i += blockDim.x)
         qs[i] = to_float(q[(long long)t * ldq + (long long)g * group * kw + i]);
+    // value entries that lie side by side in a lane, and the place of the lane's i-th
+    const int side = vec && vdim % 128 == 0 ? 4 : vec && vdim % 64 == 0 ? 2 : 1;
+    auto entry = [&](int i) { return side * (lane + 32 * (i / side)) + i % side; };
     // heads of the group this warp takes: warp, warp + warps, ... (at most MD_HEADS of them)
     constexpr int MD_HEADS = 4;
     float m_run[MD_HEADS][MAPS], l_run[MD_HEADS][MAPS], acc[MD_HEADS][MAPS][MA_VPL];
@@ -350,8 +399,10 @@ mapped_decode_kernel(const TE* __restrict__ q, long long ldq, const TE* __restri
             for (int i = tid; i < MD_KEYS * (kc + vc); i += blockDim.x) {
                 const int r = i / (kc + vc), c = i % (kc + vc);
                 const TE* from = c < kc ? src + r * width + key_off + c * E : src + r * width + val_off + (c - kc) * E;
-                *reinterpret_cast<uint4*>(tile + r * pitch + c * E) = *reinterpret_cast<const uint4*>(from);
+                copy_async16(reinterpret_cast<float*>(tile + r * pitch + c * E), reinterpret_cast<const float*>(from));
             }
+            copy_async_commit();
+            copy_async_wait<0>();
         } else {
             for (int i = tid; i < MD_KEYS * rw; i += blockDim.x) {
                 const int r = i / rw, c = i % rw;
@@ -366,44 +417,74 @@ mapped_decode_kernel(const TE* __restrict__ q, long long ldq, const TE* __restri
             if (hg >= group) break;
             const float scale_h = head_scale ? scale * head_scale[g * group + hg] : scale;
             const float slope = slopes ? slopes[g * group + hg] : 0.0f;
+            const int jl = half * 32 + lane, j = key0 + jl;
+            const bool live = (j >= first || j < keep) && j <= pos;
+            if (__ballot_sync(0xffffffffu, live) == 0u) continue;
+            float p[MAPS];
 #pragma unroll
-            for (int half = 0; half < MD_KEYS / 32; ++half) {
-                const int jl = half * 32 + lane, j = key0 + jl;
-                const bool live = (j >= first || j < keep) && j <= pos;
-                if (__ballot_sync(0xffffffffu, live) == 0u) continue;
-                float p[MAPS];
+            for (int a = 0; a < MAPS; ++a) {
+                const float sc = live ? capped_score(dot_staged(qs + hg * kw + a * dim, tile + jl * pitch + a * dim, dim,
+                                                                vec != 0) * scale_h, softcap) -
+                                            slope * (float)(pos - j)
+                                      : -INFINITY;
+                const float m_new = fmaxf(m_run[u][a], warp_max(sc));
+                const float corr = expf(m_run[u][a] - m_new);
+                p[a] = live ? expf(sc - m_new) : 0.0f;
+                l_run[u][a] = l_run[u][a] * corr + warp_sum(p[a]);
+                m_run[u][a] = m_new;
 #pragma unroll
-                for (int a = 0; a < MAPS; ++a) {
-                    const float sc = live ? capped_score(dot_key<TE>(qs + hg * kw + a * dim, tile + jl * pitch + a * dim, dim,
-                                                                     vec != 0) * scale_h, softcap) -
-                                                slope * (float)(pos - j)
-                                          : -INFINITY;
-                    const float m_new = fmaxf(m_run[u][a], warp_max(sc));
-                    const float corr = expf(m_run[u][a] - m_new);
-                    p[a] = live ? expf(sc - m_new) : 0.0f;
-                    l_run[u][a] = l_run[u][a] * corr + warp_sum(p[a]);
-                    m_run[u][a] = m_new;
-#pragma unroll
-                    for (int i = 0; i < MA_VPL; ++i) acc[u][a][i] *= corr;
-                }
+                for (int i = 0; i < MA_VPL; ++i) acc[u][a][i] *= corr;
+            }
+            // a lane's value entries: W neighbours of every 32 W
+            auto add_values = [&](auto w) {
+                constexpr int W = decltype(w)::value;
+#pragma unroll 8
                 for (int jj = 0; jj < 32; ++jj) {
                     float pj[MAPS];
 #pragma unroll
                     for (int a = 0; a < MAPS; ++a) pj[a] = __shfl_sync(0xffffffffu, p[a], jj);
                     const TE* vrow = tile + (half * 32 + jj) * pitch + val_at;
 #pragma unroll
-                    for (int i = 0; i < MA_VPL; ++i) {
-                        const int d = lane + 32 * i;
+                    for (int i = 0; i < MA_VPL; i += W) {
+                        const int d = W * (lane + 32 * (i / W));
                         if (d < vdim) {
-                            const float x = to_float(vrow[d]);
+                            float x[W];
+                            read_values<W>(x, vrow + d);
 #pragma unroll
-                            for (int a = 0; a < MAPS; ++a) acc[u][a][i] = fmaf(pj[a], x, acc[u][a][i]);
+                            for (int e = 0; e < W; ++e)
+#pragma unroll
+                                for (int a = 0; a < MAPS; ++a) acc[u][a][i + e] = fmaf(pj[a], x[e], acc[u][a][i + e]);
                         }
                     }
+                }
+            };
+            if (side == 4) add_values(std::integral_constant<int, 4>());
+            else if (side == 2) add_values(std::integral_constant<int, 2>());
+            else add_values(std::integral_constant<int, 1>());
+        }
+    }
+    // the second set hands its sums over through the page's place
+    __syncthreads();
+    float* hand = reinterpret_cast<float*>(md_raw);            // [group][MAPS][vdim + 2]
+    if (half) {
+#pragma unroll
+        for (int u = 0; u < MD_HEADS; ++u) {
+            const int hg = warp + u * warps;
+            if (hg >= group) break;
+#pragma unroll
+            for (int a = 0; a < MAPS; ++a) {
+                float* to = hand + (hg * MAPS + a) * (vdim + 2);
+                if (lane == 0) to[vdim] = m_run[u][a], to[vdim + 1] = l_run[u][a];
+#pragma unroll
+                for (int i = 0; i < MA_VPL; ++i) {
+                    const int d = entry(i);
+                    if (d < vdim) to[d] = acc[u][a][i];
                 }
             }
         }
     }
+    __syncthreads();
+    if (half) return;
 #pragma unroll
     for (int u = 0; u < MD_HEADS; ++u) {
         const int hg = warp + u * warps;
@@ -412,14 +493,17 @@ mapped_decode_kernel(const TE* __restrict__ q, long long ldq, const TE* __restri
 #pragma unroll
         for (int a = 0; a < MAPS; ++a) {
             const long long item = (((long long)t * n_heads + h) * MAPS + a) * MD_SPLITS + share;
+            const float* from = hand + (hg * MAPS + a) * (vdim + 2);
+            const float m1 = from[vdim], m = fmaxf(m_run[u][a], m1);
+            const float f0 = m_run[u][a] == -INFINITY ? 0.0f : expf(m_run[u][a] - m), f1 = m1 == -INFINITY ? 0.0f : expf(m1 - m);
             if (lane == 0) {
-                part_ml[item * 2] = m_run[u][a];
-                part_ml[item * 2 + 1] = l_run[u][a];
+                part_ml[item * 2] = m;
+                part_ml[item * 2 + 1] = l_run[u][a] * f0 + from[vdim + 1] * f1;
             }
 #pragma unroll
             for (int i = 0; i < MA_VPL; ++i) {
-                const int d = lane + 32 * i;
-                if (d < vdim) part_acc[item * vdim + d] = acc[u][a][i];
+                const int d = entry(i);
+                if (d < vdim) part_acc[item * vdim + d] = acc[u][a][i] * f0 + from[d] * f1;
             }
         }
     }
@@ -437,18 +521,14 @@ mapped_merge_kernel(const float* __restrict__ part_acc, const float* __restrict_
     pdl_wait();
     const int t = blockIdx.x, h = blockIdx.y;
     const long long item0 = ((long long)t * n_heads + h) * MAPS * MD_SPLITS;
-    if (threadIdx.x < MAPS) {
-        const int a = threadIdx.x;
-        float top = sink ? 0.0f : -INFINITY, den = 0.0f;
-        for (int s = 0; s < MD_SPLITS; ++s) top = fmaxf(top, part_ml[(item0 + a * MD_SPLITS + s) * 2]);
-        if (sink) den = expf(-top);
-        for (int s = 0; s < MD_SPLITS; ++s) {
-            const float m = part_ml[(item0 + a * MD_SPLITS + s) * 2];
-            const float f = m == -INFINITY ? 0.0f : expf(m - top);
-            factor[a][s] = f;
-            den += part_ml[(item0 + a * MD_SPLITS + s) * 2 + 1] * f;
-        }
-        for (int s = 0; s < MD_SPLITS; ++s) factor[a][s] /= den;
+    if (threadIdx.x < 32 * MAPS) {                           // a warp a map, a lane a share
+        static_assert(MD_SPLITS == 32, "a lane a share");
+        const int a = threadIdx.x >> 5, s = threadIdx.x & 31;
+        const float2 ml = *reinterpret_cast<const float2*>(part_ml + (item0 + a * MD_SPLITS + s) * 2);
+        const float top = fmaxf(sink ? 0.0f : -INFINITY, warp_max(ml.x));
+        const float f = ml.x == -INFINITY ? 0.0f : expf(ml.x - top);
+        const float den = warp_sum(ml.y * f) + (sink ? expf(-top) : 0.0f);
+        factor[a][s] = f / den;
     }
     __syncthreads();
     float sq = 0.0f;
@@ -456,10 +536,11 @@ mapped_merge_kernel(const float* __restrict__ part_acc, const float* __restrict_
         float o[MAPS];
 #pragma unroll
         for (int a = 0; a < MAPS; ++a) {
-            float num = 0.0f;
+            float num[4] = {0.0f, 0.0f, 0.0f, 0.0f};         // (every share has been written, if with zeros: no load waits)
+#pragma unroll
             for (int s = 0; s < MD_SPLITS; ++s)
-                if (factor[a][s] != 0.0f) num += part_acc[(item0 + a * MD_SPLITS + s) * vdim + d] * factor[a][s];
-            o[a] = num;
+                num[s & 3] = fmaf(part_acc[(item0 + a * MD_SPLITS + s) * vdim + d], factor[a][s], num[s & 3]);
+            o[a] = (num[0] + num[1]) + (num[2] + num[3]);
         }
         const float r = MAPS == 2 ? o[0] - lambda * o[MAPS - 1] : o[0];
         merged[d] = r;
@@ -580,13 +661,15 @@ MU_EXPORT int mu_mapped_attention_decode(const void* q, long long ldq, const voi
     const int esize = is_bf16 ? 2 : 4, per = 16 / esize;
     const int vec = dim % per == 0 && vdim % per == 0 && ((uintptr_t)rows & 15) == 0;
     const int rw = maps * dim + (shared ? 0 : vdim), pitch = rw + (vec ? per : 1);
-    const size_t smem = (((size_t)mu::MD_KEYS * pitch * esize + 15) / 16) * 16 + (size_t)group * maps * dim * sizeof(float);
+    size_t smem = (((size_t)mu::MD_KEYS * pitch * esize + 15) / 16) * 16 + (size_t)group * maps * dim * sizeof(float);
+    const size_t hand = (size_t)group * maps * (vdim + 2) * sizeof(float);
+    if (smem < hand) smem = hand;
     if (smem > 200 * 1024) return MU_ERR_UNSUPPORTED_SIZE;
     cudaStream_t s = (cudaStream_t)stream;
     float* part_acc = scratch;
     float* part_ml = scratch + (long long)n_tokens * n_heads * maps * mu::MD_SPLITS * vdim;
-    const int warps = group >= 4 ? 4 : group;                // a warp a head; more than four heads: in turns
-    const dim3 grid(n_tokens, n_kv_heads, mu::MD_SPLITS), block(32 * warps);
+    const int warps = group >= 4 ? 4 : group;                // a warp a head and half page; more than four heads: in turns
+    const dim3 grid(n_tokens, n_kv_heads, mu::MD_SPLITS), block(64 * warps);
     const dim3 mgrid(n_tokens, n_heads), mblock(vdim > 64 ? 128 : 64);
     typedef __nv_bfloat16 bf;
 #define MU_MAPPED_DECODE(TE, M)                                                                                        \
