@@ -342,7 +342,7 @@ template <int W> __device__ __forceinline__ void read_values(float (&x)[W], cons
 }
 
 template <typename TE, int MAPS>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(256)
 mapped_decode_kernel(const TE* __restrict__ q, long long ldq, const TE* __restrict__ rows,
                      const int* __restrict__ block_table, int max_pages, const int* __restrict__ tok_pos,
                      const int* __restrict__ tok_seq, int n_heads, int n_kv_heads, int dim, int vdim, float scale,

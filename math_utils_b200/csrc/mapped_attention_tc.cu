@@ -18,7 +18,9 @@
 // Sizes: pages of 64; maps * dim a multiple of 16 up to 256, vdim a multiple of 16 up to 128, rows in steps of 8 entries.
 // What bounds it: the softmax's chain per page and stream (64 columns a thread); the products take a fraction of it.
 // Measured (B200, 2 x 1,024 tokens, 8 heads): two maps of 64, values of 128, window 512: 91 -> 33 us beside the mma.sync
-// kernel (64 queries a block, four warps that multiply and exponentiate in turn); the layer around it 136 -> 79 us.
+// kernel (64 queries a block, four warps that multiply and exponentiate in turn); the layer around it 136 -> 79 us.  Latent
+// attention's prompts over expanded rows (2,048 tokens of three sequences, 16 heads of 128 + 64, values of 128): 41 us, and
+// 20 for the product that expands them, where the kernel in latent space took 295; the layer 443 -> 147 us.
 #include "tcgen05.cuh"
 
 #include <math.h>
