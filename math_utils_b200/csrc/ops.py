@@ -701,17 +701,22 @@ def chunk_scan_ok(dk: int, dv: int) -> bool:
     return bool(library().mu_chunk_scan_fits(int(dk), int(dv)))
 
 
-def _chunk_scratch(device, n_tokens: int, n_seqs: int, n_heads: int, dk: int, dv: int) -> torch.Tensor:
+def _room(workspace, name: str, device, numel: int) -> torch.Tensor:
+    """``numel`` floats from the caller's ``workspace(name, numel)``, or of this call alone."""
+    return workspace(name, numel) if workspace is not None else torch.empty(numel, dtype=torch.float32, device=device)
+
+
+def _chunk_scratch(workspace, device, n_tokens: int, n_seqs: int, n_heads: int, dk: int, dv: int) -> torch.Tensor:
     lib = library()
     lib.mu_chunk_scan_scratch.restype = _c_ll
-    return scratch("chunk_scan", device, int(lib.mu_chunk_scan_scratch(n_tokens, n_seqs, n_heads, dk, dv)), torch.float32)
+    return _room(workspace, "chunk_scan", device, int(lib.mu_chunk_scan_scratch(n_tokens, n_seqs, n_heads, dk, dv)))
 
 
 def ssd_scan_chunks(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias, a_log, skip, n_heads: int, head_dim: int, n_state: int,
                     groups: int, tiles: torch.Tensor, tok_seq, seq_first, seq_slots, state: torch.Tensor, state_offset: int,
-                    out: torch.Tensor) -> torch.Tensor:
+                    out: torch.Tensor, workspace=None) -> torch.Tensor:
     """``ssd_scan`` for steps of many tokens, chunk by chunk on tensor cores; ``tiles``: the step's query tiles (int32
-    [n, 2])."""
+    [n, 2]); ``workspace(name, n)``: n floats that stay this caller's while the step runs (allocated if None)."""
     _need_cuda(xbc, dt_raw, dt_bias, a_log, skip, tiles, tok_seq, seq_first, seq_slots, state, out)
     for t, name in ((tiles, "tiles"), (tok_seq, "tok_seq"), (seq_first, "seq_first"), (seq_slots, "seq_slots")):
         _i32(t, name)
@@ -724,7 +729,7 @@ def ssd_scan_chunks(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias, a_log, ski
     for t in (dt_bias, a_log, skip):
         if t.dtype != torch.float32 or t.numel() != n_heads or not t.is_contiguous():
             raise KernelError("ssd_scan_chunks: one float32 per head for dt_bias, A_log and D")
-    room = _chunk_scratch(xbc.device, T, n_seqs, n_heads, n_state, head_dim)
+    room = _chunk_scratch(workspace, xbc.device, T, n_seqs, n_heads, n_state, head_dim)
     _check(library().mu_ssd_scan_chunks(_ptr(xbc), xbc.shape[1], _ptr(dt_raw), dt_raw.stride(0), _is_bf16(dt_raw), _ptr(dt_bias),
                                         _ptr(a_log), _ptr(skip), _ptr(tiles), tiles.shape[0], _ptr(tok_seq), T, n_seqs,
                                         int(n_heads), int(head_dim), int(n_state), int(groups), _ptr(seq_first),
@@ -740,12 +745,13 @@ def selective_scan_max_state() -> int:
 
 def selective_scan(x: torch.Tensor, z: torch.Tensor, dt: torch.Tensor, bc: torch.Tensor, b_at: int, c_at: int,
                    rates: torch.Tensor, skip: torch.Tensor, seq_first, seq_slots, state: torch.Tensor, state_offset: int,
-                   out: torch.Tensor, max_len: int = 0) -> torch.Tensor:
+                   out: torch.Tensor, max_len: int = 0, workspace=None) -> torch.Tensor:
     """The recurrence S[c, n] = 2^(dt_c rates[c, n]) S[c, n] + dt_c x_c B_n, out_c = (sum_n S[c, n] C_n + skip_c x_c) silu(z_c)
     over the step's tokens of each sequence, from and to ``state[slot][state_offset:]`` (channels x N float32).  ``x``, ``z``
     and ``out`` [T, channels] in the compute dtype, ``dt`` float32; B and C are the columns of the float32 rows ``bc`` from
     ``b_at`` and ``c_at`` on, each followed by filling up to a multiple of four.  ``max_len``: the tokens that the longest
-    sequence brings, if the caller knows; few long sequences then go in segments that work at once."""
+    sequence brings, if the caller knows; few long sequences then go in segments that work at once, which need room
+    (``workspace`` as for ``ssd_scan_chunks``)."""
     _need_cuda(x, z, dt, bc, rates, skip, seq_first, seq_slots, state, out)
     _i32(seq_first, "seq_first"); _i32(seq_slots, "seq_slots")
     T, inner = x.shape
@@ -766,7 +772,7 @@ def selective_scan(x: torch.Tensor, z: torch.Tensor, dt: torch.Tensor, bc: torch
     room = None
     if segments > 1 and lib.mu_selective_scan_splits(n_seqs, inner, N):
         lib.mu_selective_scan_scratch.restype = _c_ll
-        room = scratch("selective_scan", x.device, int(lib.mu_selective_scan_scratch(n_seqs, segments, inner, N)), torch.float32)
+        room = _room(workspace, "selective_scan", x.device, int(lib.mu_selective_scan_scratch(n_seqs, segments, inner, N)))
     else:
         segments = 1
     _check(lib.mu_selective_scan(_ptr(x), x.stride(0), _ptr(z), z.stride(0), _ptr(dt), dt.stride(0), _ptr(bc), bc.stride(0),
@@ -972,9 +978,10 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.
 
 def linear_scan_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, gates: torch.Tensor, n_heads: int, dk: int, dv: int,
                        scale: float, tiles: torch.Tensor, tok_seq, seq_first, seq_slots, state: torch.Tensor,
-                       state_offset: int, out: torch.Tensor, norm_out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """``linear_scan`` with gates [T, heads, 4] for steps of many tokens, chunk by chunk on tensor cores; ``tiles``: the
-    step's query tiles (int32 [n, 2])."""
+                       state_offset: int, out: torch.Tensor, norm_out: Optional[torch.Tensor] = None,
+                       workspace=None) -> torch.Tensor:
+    """``linear_scan`` with gates [T, heads, 4] for steps of many tokens, chunk by chunk on tensor cores; ``tiles`` and
+    ``workspace`` as for ``ssd_scan_chunks``."""
     _need_cuda(q, k, v, gates, tiles, tok_seq, seq_first, seq_slots, state, out, norm_out)
     for t, name in ((tiles, "tiles"), (tok_seq, "tok_seq"), (seq_first, "seq_first"), (seq_slots, "seq_slots")):
         _i32(t, name)
@@ -990,7 +997,7 @@ def linear_scan_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, gates:
     if norm_out is not None and (norm_out.dtype != torch.float32 or not norm_out.is_contiguous()
                                  or tuple(norm_out.shape) != (T, n_heads)):
         raise KernelError("linear_scan_chunks: the normalizer's read-out is contiguous float32 [T, heads]")
-    room = _chunk_scratch(q.device, T, n_seqs, n_heads, dk, dv)
+    room = _chunk_scratch(workspace, q.device, T, n_seqs, n_heads, dk, dv)
     _check(library().mu_linear_scan_chunks(_ptr(q), _ptr(k), _ptr(v), q.stride(0), _ptr(gates), _ptr(tiles), tiles.shape[0],
                                            _ptr(tok_seq), T, n_seqs, int(n_heads), int(dk), int(dv), float(scale),
                                            _ptr(seq_first), _ptr(seq_slots), _ptr(room), _ptr(state), state.stride(0),

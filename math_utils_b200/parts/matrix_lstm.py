@@ -83,7 +83,7 @@ class MatrixLstm(Mixer):
         read = ctx.buffer("mlstm.normalizer", (T, H), torch.float32)
         if self.chunked and ctx.q_tiles is not None and T >= self.CHUNKED_TOKENS * ctx.n_seqs:
             ops.linear_scan_chunks(q, k, v, gates, H, self.dim, self.vdim, self.dim ** -0.5, ctx.q_tiles, ctx.tok_seq,
-                                   ctx.seq_first, ctx.seq_slots, cache.values, 0, o, norm_out=read)
+                                   ctx.seq_first, ctx.seq_slots, cache.values, 0, o, norm_out=read, workspace=ctx.scratch)
         else:
             ops.linear_scan(q, k, v, gates, H, self.dim, self.vdim, self.dim ** -0.5, ctx.seq_first, ctx.seq_slots,
                             cache.values, 0, o, norm_out=read)

@@ -82,7 +82,7 @@ class StateSpaceMixer(Mixer):
         recurrence = (xbc, dt_raw, self.dt_bias, self.a_log, self.skip, self.n_heads, self.head_dim, self.state, self.groups)
         if self.chunked and ctx.q_tiles is not None and T >= self.CHUNKED_TOKENS * ctx.n_seqs:
             ops.ssd_scan_chunks(*recurrence, ctx.q_tiles, ctx.tok_seq, ctx.seq_first, ctx.seq_slots, cache.values,
-                                self.tail_values, y)
+                                self.tail_values, y, workspace=ctx.scratch)
         else:
             ops.ssd_scan(*recurrence, ctx.seq_first, ctx.seq_slots, cache.values, self.tail_values, y)
         ctx.note("scan", y)

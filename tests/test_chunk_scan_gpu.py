@@ -128,6 +128,7 @@ def test_selective_scan_in_segments(lens, C, N, dtype):
     dt = torch.nn.functional.softplus(_rand((T, C), 3) - 3.0)
     n4 = -(-N // 4) * 4
     bc = _rand((T, 2 * n4), 4)
+    bc[:, N:n4] = bc[:, n4 + N:] = 0        # as the product leaves the columns that only pad a row
     rates = -torch.exp(_rand((C, N), 5)).contiguous() * 1.4427
     skip = _rand((C,), 6)
     values = 6 + C * N
@@ -142,3 +143,38 @@ def test_selective_scan_in_segments(lens, C, N, dtype):
     assert _rel(got[1][0], got[0][0].double()) < (2e-6 if dtype == torch.float32 else 2e-3)
     worst = (got[1][0].double() - got[0][0].double()).abs() / (got[0][0].double().abs() + got[0][0].double().square().mean().sqrt())
     assert float(worst.max()) < (1e-5 if dtype == torch.float32 else 2.0 ** -7)
+
+
+@pytest.mark.parametrize("lens", [(5,), (16, 7), (35, 2, 49), (150,)])
+@pytest.mark.parametrize("H,G,dk,dv", [(2, 1, 128, 20), (2, 2, 20, 132), (4, 2, 64, 16), (1, 1, 256, 12)])
+def test_delta_scan_in_blocks_of_four(lens, H, G, dk, dv):
+    """Blocks of four tokens and what is left of a step against float64; the steps of one token show what float32 gives."""
+    ops = _ops()
+    T, slots = sum(lens), list(range(len(lens)))[::-1]
+    first = np.concatenate([[0], np.cumsum(lens)])
+    q, k = (torch.nn.functional.normalize(_rand((T, G, dk), s), dim=-1) for s in (1, 2))
+    q = q * dk ** -0.5
+    v = _rand((T, H * dv), 3)
+    qkv = torch.cat([q.reshape(T, -1), k.reshape(T, -1), v], 1).contiguous()
+    kq = (q.double() * k.double()).sum(-1).float().contiguous()
+    beta, decay = torch.sigmoid(_rand((T, H), 4)), 1.0 - 0.2 * torch.sigmoid(_rand((T, H), 5)) ** 2
+    decay[T // 2] = 0.0                                          # all that was is forgotten
+    start = _rand((len(lens), 4 + H * dv * dk), 6, 0.3)
+    block_out, block_state = torch.zeros((T, H * dv), device="cuda"), start.clone()
+    ops.delta_scan(qkv, kq, beta, decay, H, G, dk, dv, _ints(first), _ints(slots), block_state, 4, block_out)
+    token_out, token_state = torch.zeros((T, H * dv), device="cuda"), start.clone()
+    want, want_state = torch.zeros((T, H * dv), dtype=torch.float64, device="cuda"), start.double()
+    for s, slot in enumerate(slots):
+        S = start[slot, 4:].double().reshape(H, dv, dk)
+        for t in range(first[s], first[s + 1]):
+            row = slice(t, t + 1)
+            ops.delta_scan(qkv[row], kq[row], beta[row], decay[row], H, G, dk, dv, _ints([0, 1]), _ints([slot]), token_state, 4,
+                           token_out[row])
+            kt, qt = (x[t].double().repeat_interleave(H // G, 0) for x in (k, q))
+            S = S * decay[t].double()[:, None, None]
+            u = beta[t].double()[:, None] * (v[t].double().reshape(H, dv) - torch.einsum("hvd,hd->hv", S, kt))
+            S = S + u[:, :, None] * kt[:, None, :]
+            want[t] = torch.einsum("hvd,hd->hv", S, qt).reshape(-1)
+        want_state[slot, 4:] = S.reshape(-1)
+    _no_further_off(block_out, token_out, want)
+    _no_further_off(block_state, token_state, want_state)
