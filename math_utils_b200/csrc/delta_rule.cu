@@ -11,7 +11,7 @@
 //                    decay = exp(-exp(A_log) * softplus(a_raw + dt_bias)).  Everything float32.
 // mu_delta_scan      per (sequence, head, a few columns of S), the step's tokens in order:
 //                        S <- decay S;  u = beta (v - S^T k);  S <- S + k u^T;  o = S^T q
-//                    Two columns of S (two value entries) live in the registers of up to 16 lanes, two entries to a
+//                    Two columns of S (two value entries; PER) live in the registers of up to 16 lanes, two entries to a
 //                    64-bit register; a key and a query read from shared memory serve both columns.  A token waits for
 //                    one exchange between the lanes only, that of S^T k, made of the state as the token found it:
 //                    (decay S)^T k = decay (S^T k).  The read-out of the written state is decay (S^T q) + u (k . q);
@@ -20,16 +20,17 @@
 //                    q, k, v, beta, decay and k . q of 16 tokens at a time are copied to shared memory
 //                    asynchronously, the next 16 while these are worked on.
 //                    The order of every sum is fixed by the column alone: a token's result does not depend on how
-//                    the sequence was cut into steps or on the batch.
+//                    the sequence was cut into steps or on the batch, but for the blocks of four below.
 //
-// Long steps with one decay per head take four tokens between two exchanges (BLOCKED).  With S the state before them,
-// d_j their decays, D_j = d_0 .. d_j and c_ij = d_(i+1) .. d_j,
+// Long steps of few sequences with one decay per head take four tokens between two exchanges (BLOCKED).  With S the state
+// before them, d_j their decays, D_j = d_0 .. d_j and c_ij = d_(i+1) .. d_j,
 //     u_j = beta_j (v_j - D_j S^T k_j - sum_{i<j} c_ij (k_i . k_j) u_i),   o_j = D_j S^T q_j + sum_{i<=j} c_ij (k_i . q_j) u_i,
 //     S  <- D_3 S + sum_i c_i3 k_i u_i:
 // the same recurrence with its sums in another order, all float32.  The four S^T k_j go round the lanes together, the products
 // of keys and queries within a block of four are made once a chunk (a warp a block), and the state is multiplied by a decay
-// once in four tokens.  What bounds the token-by-token form is its chain (347 cycles a token at one warp a scheduler, of which
-// the exchange is a third).
+// once in four tokens.  What bounds both forms there is the chain of one warp a scheduler (347 cycles a token, 333 in blocks;
+// 117 instructions, the rest waits for results); 1 x 1,024 tokens of 8 heads of 128 x 128: 181 us, 142 in blocks with one
+// column a lane.
 //
 // Option: a decay per head and key channel instead of one per head (the rows of S decay each by its own number).  The
 // decays are then made by mu_low_rank (linear_scan.cu) and staged beside the keys; S decays before the two sums, which
@@ -80,12 +81,11 @@ delta_prepare_kernel(float* __restrict__ qkv, int channels, const TE* __restrict
 }
 
 constexpr int DL_THREADS = 128;
-constexpr int DL_PER = 2;         // columns of S whose entries a lane holds
 constexpr int DL_CHUNK = 16;      // tokens staged at a time
 constexpr int DL_MAX_DK = 256;    // the longest column
 
-// Columns a block takes: LANES lanes share two columns.
-__host__ __device__ constexpr int dl_columns(int lanes) { return DL_PER * DL_THREADS / lanes; }
+// Columns a block takes: LANES lanes share PER columns.
+__host__ __device__ constexpr int dl_columns(int lanes, int per) { return per * DL_THREADS / lanes; }
 // Floats of one staged chunk: keys, queries (and the channels' decays) padded to DKP entries, the block's values,
 // (beta, decay, k . q, -).
 __host__ __device__ constexpr int dl_chunk_floats(int dkp, int cols, bool per_channel) {
@@ -101,28 +101,28 @@ constexpr int DL_BLOCK = 4, DL_COEF = 28;
 // and R follow from dk alone, so the order of the sums does too.
 // VEC: dk, dv, the row length and the state's offset and stride are all multiples of 4, so keys, queries, values and
 // the state move 16 bytes at a time.  PER_CHANNEL: `decay` is [T][n_heads * dk] (else [T][n_heads]).
-template <int R, int LANES, bool VEC, bool PER_CHANNEL, bool BLOCKED>
-__global__ void __launch_bounds__(DL_THREADS, R > 8 || BLOCKED ? 2 : 4)
+template <int R, int LANES, int PER, bool VEC, bool PER_CHANNEL, bool BLOCKED>
+__global__ void __launch_bounds__(DL_THREADS, R > 8 ? 2 : BLOCKED ? 3 : 4)
 delta_scan_kernel(const float* __restrict__ qkv, int channels, const float* __restrict__ kq,
                   const float* __restrict__ beta, const float* __restrict__ decay, int n_heads, int n_kv_heads, int dk,
                   int dv, const int* __restrict__ seq_first, const int* __restrict__ seq_slots,
                   float* __restrict__ state, long long state_stride, long long state_offset, float* __restrict__ out) {
-    constexpr int DKP = LANES * R, Q = R / 4, COLS = dl_columns(LANES), BUF = dl_chunk_floats(DKP, COLS, PER_CHANNEL);
-    constexpr int GROUP = LANES / DL_PER;                    // tokens whose read-outs are summed together
+    constexpr int DKP = LANES * R, Q = R / 4, COLS = dl_columns(LANES, PER), BUF = dl_chunk_floats(DKP, COLS, PER_CHANNEL);
+    constexpr int GROUP = LANES / PER;                       // tokens whose read-outs are summed together
     extern __shared__ __align__(16) float dl_smem[];
     __shared__ __align__(16) float dl_coef[BLOCKED ? DL_CHUNK / DL_BLOCK : 1][DL_COEF];
     __shared__ float dl_dots[BLOCKED ? DL_CHUNK / DL_BLOCK : 1][16];
     const int s = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * COLS;
-    const int tid = threadIdx.x, c0 = DL_PER * (tid / LANES), l = tid % LANES;
+    const int tid = threadIdx.x, c0 = PER * (tid / LANES), l = tid % LANES;
     const int g = h / (n_heads / n_kv_heads);
-    const int n_live = min(DL_PER, dv - col0 - c0);          // (may be negative)
+    const int n_live = min(PER, dv - col0 - c0);          // (may be negative)
     for (int i = tid; i < 2 * BUF; i += DL_THREADS) dl_smem[i] = 0.0f;   // the padding past dk and dv stays zero
     pdl_wait();
     const int first = seq_first[s], count = seq_first[s + 1] - first;
     float* const mine = state + (long long)seq_slots[s] * state_stride + state_offset + ((long long)h * dv + col0 + c0) * dk;
-    float2x S[DL_PER][2 * Q];                                // the lane's entries in pairs
+    float2x S[PER][2 * Q];                                // the lane's entries in pairs
 #pragma unroll
-    for (int c = 0; c < DL_PER; ++c)
+    for (int c = 0; c < PER; ++c)
 #pragma unroll
         for (int i = 0; i < Q; ++i) {
             const int d = 4 * (l + LANES * i);
@@ -208,9 +208,11 @@ delta_scan_kernel(const float* __restrict__ qkv, int channels, const float* __re
         // share of it goes to `sum`, u (k . q) into lane 0's.
         auto step = [&](int tok, float* sum) {
             const float4 par = *reinterpret_cast<const float4*>(sc + tok * 4);           // beta, decay, k . q
-            const float2 v = *reinterpret_cast<const float2*>(vs + tok * COLS + c0);
+            float2 v = make_float2(0.0f, 0.0f);
+            if constexpr (PER == 2) v = *reinterpret_cast<const float2*>(vs + tok * COLS + c0);
+            else v.x = vs[tok * COLS + c0];
             ulonglong2 kr[Q];
-            float2x a[DL_PER] = {0, 0}, o[DL_PER] = {0, 0};                              // (two zeros each)
+            float2x a[PER] = {}, o[PER] = {};                // (two zeros each)
 #pragma unroll
             for (int i = 0; i < Q; ++i) {
                 const int at = tok * DKP + 4 * (l + LANES * i);
@@ -219,7 +221,7 @@ delta_scan_kernel(const float* __restrict__ qkv, int channels, const float* __re
                 ulonglong2 gr = make_ulonglong2(0, 0);
                 if (PER_CHANNEL) gr = *reinterpret_cast<const ulonglong2*>(gs + at);
 #pragma unroll
-                for (int c = 0; c < DL_PER; ++c) {
+                for (int c = 0; c < PER; ++c) {
                     if (PER_CHANNEL) {
                         S[c][2 * i] = pair_mul(gr.x, S[c][2 * i]);
                         S[c][2 * i + 1] = pair_mul(gr.y, S[c][2 * i + 1]);
@@ -230,19 +232,19 @@ delta_scan_kernel(const float* __restrict__ qkv, int channels, const float* __re
                     o[c] = pair_fma(S[c][2 * i + 1], qr.y, o[c]);
                 }
             }
-            float sk[DL_PER];
+            float sk[PER];
 #pragma unroll
-            for (int c = 0; c < DL_PER; ++c) {
+            for (int c = 0; c < PER; ++c) {
                 const float2 x = floats_of_pair(a[c]);
                 sk[c] = x.x + x.y;
             }
 #pragma unroll
             for (int w = LANES / 2; w > 0; w >>= 1)
 #pragma unroll
-                for (int c = 0; c < DL_PER; ++c) sk[c] += __shfl_xor_sync(0xffffffffu, sk[c], w);
+                for (int c = 0; c < PER; ++c) sk[c] += __shfl_xor_sync(0xffffffffu, sk[c], w);
             const float2x dec2 = pair_of_floats(par.y, par.y);
 #pragma unroll
-            for (int c = 0; c < DL_PER; ++c) {
+            for (int c = 0; c < PER; ++c) {
                 // (one decay for the head: the sums are of the state before it, (decay S)^T k = decay (S^T k))
                 const float u = par.x * ((c ? v.y : v.x) - (PER_CHANNEL ? sk[c] : par.y * sk[c]));
                 const float2x u2 = pair_of_floats(u, u);
@@ -312,15 +314,15 @@ delta_scan_kernel(const float* __restrict__ qkv, int channels, const float* __re
             }
             __syncthreads();
         }
-        // Four tokens; their read-outs' shares go to sum[2 j + c].
+        // Four tokens; their read-outs' shares go to sum[PER j + c].
         auto block = [&](int tok, float* sum) {
             const float4* cf = reinterpret_cast<const float4*>(dl_coef[BLOCKED ? tok / DL_BLOCK : 0]);
             ulonglong2 kr[DL_BLOCK][Q];
-            float2x a[DL_BLOCK][DL_PER], o[DL_BLOCK][DL_PER];
+            float2x a[DL_BLOCK][PER], o[DL_BLOCK][PER];
 #pragma unroll
             for (int j = 0; j < DL_BLOCK; ++j) {
 #pragma unroll
-                for (int c = 0; c < DL_PER; ++c) a[j][c] = o[j][c] = 0;
+                for (int c = 0; c < PER; ++c) a[j][c] = o[j][c] = 0;
 #pragma unroll
                 for (int i = 0; i < Q; ++i) kr[j][i] = *reinterpret_cast<const ulonglong2*>(ks + (tok + j) * DKP + 4 * (l + LANES * i));
             }
@@ -329,15 +331,15 @@ delta_scan_kernel(const float* __restrict__ qkv, int channels, const float* __re
 #pragma unroll
                 for (int j = 0; j < DL_BLOCK; ++j)
 #pragma unroll
-                    for (int c = 0; c < DL_PER; ++c) {
+                    for (int c = 0; c < PER; ++c) {
                         a[j][c] = pair_fma(S[c][2 * i], kr[j][i].x, a[j][c]);
                         a[j][c] = pair_fma(S[c][2 * i + 1], kr[j][i].y, a[j][c]);
                     }
-            float sk[DL_BLOCK][DL_PER];
+            float sk[DL_BLOCK][PER];
 #pragma unroll
             for (int j = 0; j < DL_BLOCK; ++j)
 #pragma unroll
-                for (int c = 0; c < DL_PER; ++c) {
+                for (int c = 0; c < PER; ++c) {
                     const float2 x = floats_of_pair(a[j][c]);
                     sk[j][c] = x.x + x.y;
                 }
@@ -346,7 +348,7 @@ delta_scan_kernel(const float* __restrict__ qkv, int channels, const float* __re
 #pragma unroll
                 for (int j = 0; j < DL_BLOCK; ++j)
 #pragma unroll
-                    for (int c = 0; c < DL_PER; ++c) sk[j][c] += __shfl_xor_sync(0xffffffffu, sk[j][c], w);
+                    for (int c = 0; c < PER; ++c) sk[j][c] += __shfl_xor_sync(0xffffffffu, sk[j][c], w);
             // (the read-outs' products while the exchange is under way)
 #pragma unroll
             for (int j = 0; j < DL_BLOCK; ++j)
@@ -354,7 +356,7 @@ delta_scan_kernel(const float* __restrict__ qkv, int channels, const float* __re
                 for (int i = 0; i < Q; ++i) {
                     const ulonglong2 qr = *reinterpret_cast<const ulonglong2*>(qs + (tok + j) * DKP + 4 * (l + LANES * i));
 #pragma unroll
-                    for (int c = 0; c < DL_PER; ++c) {
+                    for (int c = 0; c < PER; ++c) {
                         o[j][c] = pair_fma(S[c][2 * i], qr.x, o[j][c]);
                         o[j][c] = pair_fma(S[c][2 * i + 1], qr.y, o[j][c]);
                     }
@@ -363,11 +365,8 @@ delta_scan_kernel(const float* __restrict__ qkv, int channels, const float* __re
             // ka, kb, qa: kk01 kk02 kk12 kk03 | kk13 kk23 qk01 qk02 | qk12 qk03 qk13 qk23
             const float2x whole = pair_of_floats(D.w, D.w);
 #pragma unroll
-            for (int c = 0; c < DL_PER; ++c) {
-                auto value = [&](int j) {
-                    const float2 v = *reinterpret_cast<const float2*>(vs + (tok + j) * COLS + c0);
-                    return c ? v.y : v.x;
-                };
+            for (int c = 0; c < PER; ++c) {
+                auto value = [&](int j) { return vs[(tok + j) * COLS + c0 + c]; };
                 const float u0 = be.x * (value(0) - D.x * sk[0][c]);
                 const float u1 = be.y * (value(1) - D.y * sk[1][c] - ka.x * u0);
                 const float u2 = be.z * (value(2) - D.z * sk[2][c] - ka.y * u0 - ka.z * u1);
@@ -388,25 +387,29 @@ delta_scan_kernel(const float* __restrict__ qkv, int channels, const float* __re
                 for (int j = 0; j < DL_BLOCK; ++j) {
                     const float2 x = floats_of_pair(o[j][c]);
                     const float share = Dj[j] * (x.x + x.y);
-                    sum[DL_PER * j + c] = l == 0 ? share + own[j] : share;
+                    sum[PER * j + c] = l == 0 ? share + own[j] : share;
                 }
             }
         };
         for (int t0 = 0; t0 < n; t0 += GROUP) {
-            float acc[LANES];                                // token t0 + i, column c at [2 i + c]
+            float acc[LANES];                                // token t0 + i, column c at [PER i + c]
             const int left = n - t0;
             if (BLOCKED && left >= GROUP) {
 #pragma unroll
-                for (int i = 0; i < GROUP; i += DL_BLOCK) block(t0 + i, acc + DL_PER * i);
+                for (int i = 0; i < GROUP; i += DL_BLOCK) block(t0 + i, acc + PER * i);
             } else if (left >= GROUP) {                             // a whole group: no branch between the tokens
 #pragma unroll
-                for (int i = 0; i < GROUP; ++i) step(t0 + i, acc + DL_PER * i);
+                for (int i = 0; i < GROUP; ++i) step(t0 + i, acc + PER * i);
             } else {
 #pragma unroll
                 for (int i = 0; i < GROUP; ++i) {
+                    if (BLOCKED && i % DL_BLOCK == 0 && i + DL_BLOCK <= left) {
+                        block(t0 + i, acc + PER * i);
+                    } else if (!BLOCKED || i / DL_BLOCK * DL_BLOCK + DL_BLOCK > left) {
 #pragma unroll
-                    for (int c = 0; c < DL_PER; ++c) acc[DL_PER * i + c] = 0.0f;
-                    if (i < left) step(t0 + i, acc + DL_PER * i);
+                        for (int c = 0; c < PER; ++c) acc[PER * i + c] = 0.0f;
+                        if (i < left) step(t0 + i, acc + PER * i);
+                    }
                 }
             }
 #pragma unroll
@@ -419,7 +422,7 @@ delta_scan_kernel(const float* __restrict__ qkv, int channels, const float* __re
                     acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, width);
                 }
             }
-            const int tok = l / DL_PER, c = l % DL_PER;      // what this lane's sum is of
+            const int tok = l / PER, c = l % PER;      // what this lane's sum is of
             if (tok < left && c < n_live)
                 out[((long long)(first + li0 + t0 + tok) * n_heads + h) * dv + col0 + c0 + c] = acc[0];
         }
@@ -429,7 +432,7 @@ delta_scan_kernel(const float* __restrict__ qkv, int channels, const float* __re
     // here has one warp a scheduler, which every waiting warp there slows down.
     pdl_trigger();
 #pragma unroll
-    for (int c = 0; c < DL_PER; ++c)
+    for (int c = 0; c < PER; ++c)
 #pragma unroll
         for (int i = 0; i < Q; ++i) {
             const int d = 4 * (l + LANES * i);
@@ -484,6 +487,11 @@ MU_EXPORT int mu_delta_scan(const float* qkv, int channels, const float* kq, con
         return MU_ERR_BAD_ARGUMENT;
     if (dk > mu::DL_MAX_DK) return MU_ERR_UNSUPPORTED_SIZE;
     cudaStream_t s = (cudaStream_t)stream;
+    // A long step's blocks of four tokens need more instructions than its single tokens and pay while a scheduler has one
+    // warp: 8 heads of 128 x 128, 2 x 1,024 tokens 180.6 us -> 174.5, but 8 x 512 tokens 187 -> 232.  One column a lane
+    // makes twice the blocks and pays while they fit one an SM as well: 1 x 1,024 tokens 174.4 us -> 141.7, 2 x 1,024
+    // 174.5 -> 201.
+    auto blocks = [&](int cols) { return (long long)n_seqs * n_heads * ((dv + cols - 1) / cols); };
     const bool vec = dk % 4 == 0 && dv % 4 == 0 && channels % 4 == 0 && state_stride % 4 == 0 && state_offset % 4 == 0 &&
                      (reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(state) |
                       (per_channel ? reinterpret_cast<uintptr_t>(decay) : 0)) % 16 == 0;
@@ -491,11 +499,12 @@ MU_EXPORT int mu_delta_scan(const float* qkv, int channels, const float* kq, con
     // scheduler; they start in plain stream order, on an empty device.
     // the two staging buffers of a block are most of what it needs of an SM: with the largest share of the on-chip
     // memory as shared memory several blocks fit, and the state is read once, so the L1 is no loss
-#define MU_DELTA_SCAN_V(R, LANES, V, PC, BL)                                                                            \
+#define MU_DELTA_SCAN_V(R, LANES, PER, V, PC, BL)                                                                     \
     do {                                                                                                              \
-        const size_t smem = 2 * sizeof(float) * mu::dl_chunk_floats(LANES * R, mu::dl_columns(LANES), PC);            \
-        const dim3 grid(n_seqs, n_heads, (dv + mu::dl_columns(LANES) - 1) / mu::dl_columns(LANES));                   \
-        auto kernel = mu::delta_scan_kernel<R, LANES, V, PC, BL>;                                                        \
+        constexpr int cols = mu::dl_columns(LANES, PER);                                                              \
+        const size_t smem = 2 * sizeof(float) * mu::dl_chunk_floats(LANES * R, cols, PC);                             \
+        const dim3 grid(n_seqs, n_heads, (dv + cols - 1) / cols);                                                     \
+        auto kernel = mu::delta_scan_kernel<R, LANES, PER, V, PC, BL>;                                                \
         if (!mu::allow_shared((const void*)kernel, smem)) return MU_ERR_LAUNCH;                                       \
         mu::prefer_shared_memory((const void*)kernel);                                                                \
         const dim3 block(mu::DL_THREADS);                                                                             \
@@ -507,11 +516,14 @@ MU_EXPORT int mu_delta_scan(const float* qkv, int channels, const float* kq, con
     } while (0)
 #define MU_DELTA_SCAN(R, LANES)                                                                                       \
     do {                                                                                                              \
-        if (vec && per_channel) MU_DELTA_SCAN_V(R, LANES, true, true, false);                                         \
-        if (per_channel) MU_DELTA_SCAN_V(R, LANES, false, true, false);                                               \
-        if (vec && long_steps) MU_DELTA_SCAN_V(R, LANES, true, false, true);                                          \
-        if (vec) MU_DELTA_SCAN_V(R, LANES, true, false, false);                                                       \
-        MU_DELTA_SCAN_V(R, LANES, false, false, false);                                                                    \
+        if (vec && per_channel) MU_DELTA_SCAN_V(R, LANES, 2, true, true, false);                                      \
+        if (per_channel) MU_DELTA_SCAN_V(R, LANES, 2, false, true, false);                                            \
+        if (vec && long_steps && blocks(mu::dl_columns(LANES, 1)) <= mu::sm_count())                                  \
+            MU_DELTA_SCAN_V(R, LANES, 1, true, false, true);                                                          \
+        if (vec && long_steps && blocks(mu::dl_columns(LANES, 2)) <= mu::sm_count())                                  \
+            MU_DELTA_SCAN_V(R, LANES, 2, true, false, true);                                                          \
+        if (vec) MU_DELTA_SCAN_V(R, LANES, 2, true, false, false);                                                    \
+        MU_DELTA_SCAN_V(R, LANES, 2, false, false, false);                                                            \
     } while (0)
     if (dk <= 32) MU_DELTA_SCAN(4, 8);
     if (dk <= 64) MU_DELTA_SCAN(4, 16);

@@ -296,7 +296,9 @@ mapped_attention_kernel(const TE* __restrict__ q, long long ldq, const TE* __res
 // of that kv head are staged in shared memory once and serve all query heads of the group, two warps a head (half of the
 // page's keys each), a lane a key for the scores and up to four neighbouring value entries a lane for the sums.  Each
 // (token, head, map, share) leaves a maximum, a sum and unnormalised values; mapped_merge_kernel puts the shares together,
-// a lane a share, and finishes the head.  A share is a chain of latencies (page, scores, sums), so shares are many and short.
+// a lane a share, and finishes the head.  A share is a chain of latencies (page, scores, sums), so shares are many and short
+// (8 tokens, 8 heads over 2 kv heads of 128 entries, 1,500 positions, the layer: 43.0 us with 16 shares and a warp a head, 28.7
+// so); one without keys leaves at once and is not read again (64 tokens at 16 positions: 51.7 us where it wrote zeros).
 constexpr int MD_SPLITS = 32;
 constexpr int MD_KEYS = 64;         // keys staged at a time: one page
 
@@ -368,6 +370,16 @@ mapped_decode_kernel(const TE* __restrict__ q, long long ldq, const TE* __restri
     const int* pages = block_table + (long long)tok_seq[t] * max_pages;
     const long long width = (long long)n_kv_heads * rw;
     const long long key_off = (long long)g * kw, val_off = (long long)n_kv_heads * kw + (long long)g * vw;
+    const int kept_pages = min((keep + MD_KEYS - 1) / MD_KEYS, page_lo);            // pages before the window's that hold kept positions
+    auto page_from = [&](int pg) {                             // the share's first page that holds something, from pg on
+        return pg >= kept_pages && pg < page_lo ? pg + (page_lo - pg + MD_SPLITS - 1) / MD_SPLITS * MD_SPLITS : pg;
+    };
+    if (page_from(share) > page_hi) {                          // an empty share leaves no values
+        for (int i = tid; i < group * MAPS; i += blockDim.x)
+            *reinterpret_cast<float2*>(part_ml + ((((long long)t * n_heads + g * group) * MAPS + i) * MD_SPLITS + share) * 2) =
+                make_float2(-INFINITY, 0.0f);
+        return;
+    }
     for (int i = tid; i < group * kw; i += blockDim.x)
         qs[i] = to_float(q[(long long)t * ldq + (long long)g * group * kw + i]);
     // value entries that lie side by side in a lane, and the place of the lane's i-th
@@ -385,12 +397,7 @@ mapped_decode_kernel(const TE* __restrict__ q, long long ldq, const TE* __restri
 #pragma unroll
             for (int i = 0; i < MA_VPL; ++i) acc[u][a][i] = 0.0f;
         }
-    const int kept_pages = min((keep + MD_KEYS - 1) / MD_KEYS, page_lo);            // pages before the window's that hold kept positions
-    for (int pg = share; pg <= page_hi; pg += MD_SPLITS) {
-        if (pg >= kept_pages && pg < page_lo) {                // between the two runs of pages: on to the share's first of the second
-            pg += (page_lo - pg + MD_SPLITS - 1) / MD_SPLITS * MD_SPLITS;
-            if (pg > page_hi) break;
-        }
+    for (int pg = page_from(share); pg <= page_hi; pg = page_from(pg + MD_SPLITS)) {
         __syncthreads();                                       // the page before is done with (and qs is written)
         const TE* src = rows + (long long)pages[pg] * MD_KEYS * width;
         if (vec) {
@@ -513,10 +520,11 @@ template <typename TE, int MAPS>
 __global__ void __launch_bounds__(128)
 mapped_merge_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml, int n_heads, int vdim,
                     float lambda, float out_scale, float eps, int unit_rms, TE* __restrict__ out, long long ldo,
-                    int sink, const TE* __restrict__ gate, long long ldg, int gate_each) {
+                    int sink, const TE* __restrict__ gate, long long ldg, int gate_each, int shares) {
     extern __shared__ float merged[];                        // [vdim]
     __shared__ float scratch[32];
     __shared__ float factor[MAPS][MD_SPLITS];
+    __shared__ unsigned filled[MAPS];                        // shares that hold keys: only their values have been written
     pdl_trigger();
     pdl_wait();
     const int t = blockIdx.x, h = blockIdx.y;
@@ -524,11 +532,14 @@ mapped_merge_kernel(const float* __restrict__ part_acc, const float* __restrict_
     if (threadIdx.x < 32 * MAPS) {                           // a warp a map, a lane a share
         static_assert(MD_SPLITS == 32, "a lane a share");
         const int a = threadIdx.x >> 5, s = threadIdx.x & 31;
-        const float2 ml = *reinterpret_cast<const float2*>(part_ml + (item0 + a * MD_SPLITS + s) * 2);
+        const float2 ml = s < shares ? *reinterpret_cast<const float2*>(part_ml + (item0 + a * MD_SPLITS + s) * 2)
+                                     : make_float2(-INFINITY, 0.0f);
         const float top = fmaxf(sink ? 0.0f : -INFINITY, warp_max(ml.x));
         const float f = ml.x == -INFINITY ? 0.0f : expf(ml.x - top);
         const float den = warp_sum(ml.y * f) + (sink ? expf(-top) : 0.0f);
         factor[a][s] = f / den;
+        const unsigned some = __ballot_sync(0xffffffffu, ml.x != -INFINITY || ml.y != 0.0f);
+        if (s == 0) filled[a] = some;
     }
     __syncthreads();
     float sq = 0.0f;
@@ -536,10 +547,18 @@ mapped_merge_kernel(const float* __restrict__ part_acc, const float* __restrict_
         float o[MAPS];
 #pragma unroll
         for (int a = 0; a < MAPS; ++a) {
-            float num[4] = {0.0f, 0.0f, 0.0f, 0.0f};         // (every share has been written, if with zeros: no load waits)
+            float num[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            const unsigned some = filled[a];
+            const float* from = part_acc + (item0 + a * MD_SPLITS) * vdim + d;
 #pragma unroll
-            for (int s = 0; s < MD_SPLITS; ++s)
-                num[s & 3] = fmaf(part_acc[(item0 + a * MD_SPLITS + s) * vdim + d], factor[a][s], num[s & 3]);
+            for (int s0 = 0; s0 < MD_SPLITS; s0 += 8) {      // eight shares' loads on their way together
+                if ((some >> s0 & 255u) == 0u) continue;
+                float x[8];
+#pragma unroll
+                for (int s = 0; s < 8; ++s) x[s] = some >> (s0 + s) & 1u ? from[(s0 + s) * vdim] : 0.0f;
+#pragma unroll
+                for (int s = 0; s < 8; ++s) num[s & 3] = fmaf(x[s], factor[a][s0 + s], num[s & 3]);
+            }
             o[a] = (num[0] + num[1]) + (num[2] + num[3]);
         }
         const float r = MAPS == 2 ? o[0] - lambda * o[MAPS - 1] : o[0];
@@ -669,7 +688,9 @@ MU_EXPORT int mu_mapped_attention_decode(const void* q, long long ldq, const voi
     float* part_acc = scratch;
     float* part_ml = scratch + (long long)n_tokens * n_heads * maps * mu::MD_SPLITS * vdim;
     const int warps = group >= 4 ? 4 : group;                // a warp a head and half page; more than four heads: in turns
-    const dim3 grid(n_tokens, n_kv_heads, mu::MD_SPLITS), block(64 * warps);
+    const int shares = max_pages < mu::MD_SPLITS ? max_pages : mu::MD_SPLITS;
+    if (shares <= 0) return MU_ERR_BAD_ARGUMENT;
+    const dim3 grid(n_tokens, n_kv_heads, shares), block(64 * warps);
     const dim3 mgrid(n_tokens, n_heads), mblock(vdim > 64 ? 128 : 64);
     typedef __nv_bfloat16 bf;
 #define MU_MAPPED_DECODE(TE, M)                                                                                        \
@@ -685,7 +706,7 @@ MU_EXPORT int mu_mapped_attention_decode(const void* q, long long ldq, const voi
         if (code != MU_OK) return code;                                                                                \
         return mu::launch_pdl(mu::mapped_merge_kernel<TE, M>, mgrid, mblock, (size_t)vdim * sizeof(float), s, 1,       \
                               (const float*)part_acc, (const float*)part_ml, n_heads, vdim, lambda, out_scale, eps,    \
-                              unit_rms, (TE*)out, ldo, sink, (const TE*)gate, ldg, gate_each);                         \
+                              unit_rms, (TE*)out, ldo, sink, (const TE*)gate, ldg, gate_each, shares);                 \
     } while (0)
     if (is_bf16) {
         if (maps == 2) MU_MAPPED_DECODE(bf, 2);

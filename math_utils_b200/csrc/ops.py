@@ -8,6 +8,7 @@ be built or loaded, or a tensor is not on a CUDA device, they raise.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 import threading
 from typing import Optional
@@ -548,8 +549,12 @@ def mapped_tc_ok(q: torch.Tensor, out: torch.Tensor, n_kv_heads: int, maps: int,
     """Whether ``mapped_attention`` takes the tcgen05 kernel for these queries (bfloat16 rows given wide tiles)."""
     return (MAPPED_TC and q.dtype == torch.bfloat16 and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0
             and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0
-            and bool(library().mu_mapped_attention_tc_fits(int(n_kv_heads), int(maps), int(dim), int(vdim), int(page_tokens),
-                                                           int(shared))))
+            and _mapped_tc_fits(int(n_kv_heads), int(maps), int(dim), int(vdim), int(page_tokens), int(shared)))
+
+
+@functools.lru_cache(maxsize=None)
+def _mapped_tc_fits(*sizes) -> bool:
+    return bool(library().mu_mapped_attention_tc_fits(*sizes))
 
 
 def mapped_attention(q: torch.Tensor, rows: torch.Tensor, block_table: torch.Tensor, page_tokens: int, tok_pos, tok_seq,
@@ -743,6 +748,11 @@ def selective_scan_max_state() -> int:
     return int(library().mu_selective_scan_max_state())
 
 
+# Tokens of the longest sequence from which on the scan goes in segments of 256, which make the exponentials almost twice: of
+# 2,048 channels (the mixer around it) 2 x 257 tokens 80 us whole, 111 in segments; 2,000 tokens 226 us and 161.
+SELECTIVE_SEGMENTED = 800
+
+
 def selective_scan(x: torch.Tensor, z: torch.Tensor, dt: torch.Tensor, bc: torch.Tensor, b_at: int, c_at: int,
                    rates: torch.Tensor, skip: torch.Tensor, seq_first, seq_slots, state: torch.Tensor, state_offset: int,
                    out: torch.Tensor, max_len: int = 0, workspace=None) -> torch.Tensor:
@@ -767,14 +777,11 @@ def selective_scan(x: torch.Tensor, z: torch.Tensor, dt: torch.Tensor, bc: torch
             or state.shape[1] < state_offset + inner * N):
         raise KernelError("selective_scan: step sizes, B and C, rates or state do not fit")
     lib, n_seqs = library(), seq_slots.numel()
-    long_steps = T > 4 * n_seqs
-    segments = -(-int(max_len) // lib.mu_selective_scan_segment()) if long_steps else 1
-    room = None
-    if segments > 1 and lib.mu_selective_scan_splits(n_seqs, inner, N):
+    long_steps, segments, room = T > 4 * n_seqs, 1, None
+    if max_len >= SELECTIVE_SEGMENTED and long_steps and lib.mu_selective_scan_splits(n_seqs, inner, N):
+        segments = -(-int(max_len) // lib.mu_selective_scan_segment())
         lib.mu_selective_scan_scratch.restype = _c_ll
         room = _room(workspace, "selective_scan", x.device, int(lib.mu_selective_scan_scratch(n_seqs, segments, inner, N)))
-    else:
-        segments = 1
     _check(lib.mu_selective_scan(_ptr(x), x.stride(0), _ptr(z), z.stride(0), _ptr(dt), dt.stride(0), _ptr(bc), bc.stride(0),
                                        int(b_at), int(c_at), _ptr(rates), _ptr(skip), seq_slots.numel(), inner, N,
                                        _ptr(seq_first), _ptr(seq_slots), _ptr(state), state.stride(0), int(state_offset),

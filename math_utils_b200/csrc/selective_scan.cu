@@ -268,10 +268,11 @@ MU_EXPORT long long mu_selective_scan_scratch(int n_seqs, int segments, int inne
     return (long long)n_seqs * segments * inner * (((N + 1) & ~1) + 1);
 }
 
-// Segments are worth their second launch where the scan alone would leave SMs with fewer than four blocks (16 warps).
+// Segments are worth their second launch where the scan alone leaves SMs with fewer than three blocks (12 warps): 2,048
+// channels, 3 sequences of up to 1,000 tokens 169 us -> 160; of 4 x 500 tokens (3.5 blocks an SM) 134 us -> 154.
 MU_EXPORT int mu_selective_scan_splits(int n_seqs, int inner, int N) {
     const int lanes = N <= 8 ? 4 : N <= 16 ? 8 : N <= 32 ? 16 : 32;
-    return (long long)n_seqs * ((inner + mu::ss_channels(lanes) - 1) / mu::ss_channels(lanes)) < 4ll * mu::sm_count();
+    return (long long)n_seqs * ((inner + mu::ss_channels(lanes) - 1) / mu::ss_channels(lanes)) < 3ll * mu::sm_count();
 }
 
 MU_EXPORT int mu_selective_scan(const void* x, long long ldx, const void* z, long long ldz, const float* dt, long long lddt,

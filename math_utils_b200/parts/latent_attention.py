@@ -160,13 +160,20 @@ class LatentAttention(Mixer):
     # A prompt step expands its sequences' positions where they are no more than this many times its own tokens: each costs
     # 2 r H (d + d_v) operations whoever sees it.
     EXPANDED_PER_TOKEN = 4
+    # ... and where attention over the latents themselves is more work than the launches that expand them: 4 heads of r = 256,
+    # 4 x 500 tokens (2.2 GFLOP) 100 us against 98, 2,000 tokens (8.7 GFLOP) 207 against 98; shorter steps wait for the host.
+    EXPANDED_FLOP = 2.5e9
 
     def _expands(self, ctx, q, cache) -> bool:
         if (self.expand is None or ctx.is_decode or ctx.q_tiles_wide is None or ctx.n_tokens <= 64 or cache.page_tokens != 64
                 or q.stride(0) % 8 or q.data_ptr() % 16):
             return False
-        held = sum(start + n for start, n in zip(ctx.starts, ctx.q_lens))
-        return held <= self.EXPANDED_PER_TOKEN * ctx.n_tokens
+        held = met = 0
+        for start, n in zip(ctx.starts, ctx.q_lens):
+            held += start + n
+            met += n * (2 * start + n)                       # (twice the pairs of tokens and keys)
+        return (held <= self.EXPANDED_PER_TOKEN * ctx.n_tokens
+                and met * self.n_heads * (2 * self.kv_rank + self.rot_dim) >= self.EXPANDED_FLOP)
 
     def _prompt(self, q, views, gate, residual, ctx, cache, owns_cache, accumulate, table) -> None:
         ops, dt = self.runtime.ops, self.runtime.dtype

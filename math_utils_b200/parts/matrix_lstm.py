@@ -67,7 +67,10 @@ class MatrixLstm(Mixer):
         self.chunked = runtime.dtype == torch.bfloat16 and runtime.ops.chunk_scan_ok(self.dim, self.vdim)
         self.i_bias, self.f_bias, self.norm_weight = t("i_bias"), t("f_bias"), t("norm")
 
-    CHUNKED_TOKENS = 32              # tokens a sequence brings on average from which on the chunked form pays
+    # Tokens of the longest sequence from which on the chunked form pays: token by token a step takes as long as its longest
+    # sequence, in chunks two launches more (4 x 64 tokens: 58 us against 66, the host's time either way).
+    # 8 heads of 128 x 128: 2,000 tokens of one sequence 340 us token by token, 163 in chunks; 4 x 500 147 both.
+    CHUNKED_TOKENS = 192
 
     def forward(self, h, residual, ctx, cache, owns_cache: bool, accumulate: bool = True) -> None:
         ops, T, H = self.runtime.ops, ctx.n_tokens, self.n_heads
@@ -81,7 +84,7 @@ class MatrixLstm(Mixer):
                       self.m_offset, gates)
         o = ctx.buffer("mlstm.o", (T, self.inner), torch.float32)
         read = ctx.buffer("mlstm.normalizer", (T, H), torch.float32)
-        if self.chunked and ctx.q_tiles is not None and T >= self.CHUNKED_TOKENS * ctx.n_seqs:
+        if self.chunked and ctx.q_tiles is not None and ctx.max_q_len >= self.CHUNKED_TOKENS:
             ops.linear_scan_chunks(q, k, v, gates, H, self.dim, self.vdim, self.dim ** -0.5, ctx.q_tiles, ctx.tok_seq,
                                    ctx.seq_first, ctx.seq_slots, cache.values, 0, o, norm_out=read, workspace=ctx.scratch)
         else:

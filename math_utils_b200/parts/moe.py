@@ -103,6 +103,15 @@ class RoutedExperts(FeedForward):
             if self.shared_gated:
                 self.shared_gate = tensors[name("shared_gate")].reshape(-1).contiguous()
 
+    # The gathered rows' product costs a launch more.  It pays from some 3 GFLOP on (16 experts of 1,024 x 704 x 3: 512 pairs
+    # 57 us either way, 4,000 pairs 122 us against 95) or with 400 MB of weights to read (48 pairs over 64 experts of 2,048 x
+    # 1,408 x 2: 136 us against 93; over 48 of 1,024 x 704 x 3: 71 against 78).
+    GATHERED_FLOP, GATHERED_BYTES = 3e9, 4e8
+
+    def _gathers(self, pairs: int) -> bool:
+        weights = (3 if self.form == "gated_silu" else 2) * self.hidden_size * self.inner_size
+        return 2 * pairs * weights >= self.GATHERED_FLOP or 2 * min(pairs, self.n_experts) * weights >= self.GATHERED_BYTES
+
     fuses_output_norm = True           # forward(..., output_norm=): the norm of the result, added into the stream
 
     def forward(self, h, residual, ctx, accumulate: bool = True, output_norm=None) -> None:
@@ -111,10 +120,10 @@ class RoutedExperts(FeedForward):
         P = T * top
         gated = self.form == "gated_silu"
         gate_of = ctx.buffer("moe.shared_gate", (T,), torch.float32) if self.shared_gate is not None else None
-        # tiles of 128 slots where the tensor cores take the products, their rows gathered first
         tile_rows = self.tile_rows
         if ops.moe_tc_ok(dt, self.hidden_size, self.inner_size) and h.stride(0) % 8 == 0 and h.data_ptr() % 16 == 0:
-            tile_rows = ops.MOE_TC_ROWS
+            # tiles of 64 slots where an expert has the rows to fill them; where it pays tiles of 128, their rows gathered first
+            tile_rows = ops.MOE_TC_ROWS if self._gathers(P) else 64 if P >= 48 * E else 32
         max_tiles = P // tile_rows + E                     # every grouping of P pairs into E experts fits
         index = ctx.buffer("moe.index", (3 * P + 3 * max_tiles + 4,), torch.int32)
         expert_of, slot_of, pair_of = index[:P], index[P:2 * P], index[2 * P:3 * P]

@@ -65,7 +65,10 @@ class StateSpaceMixer(Mixer):
                         and self.channels % 4 == 0 and self.inner % 4 == 0)
         self.dt_bias, self.a_log, self.skip, self.norm_weight = t("dt_bias"), t("A_log"), t("D"), t("norm")
 
-    CHUNKED_TOKENS = 32              # tokens a sequence brings on average from which on the chunked form pays
+    # Tokens of the longest sequence from which on the chunked form pays: token by token a step takes as long as its longest
+    # sequence, in chunks two launches more (4 x 64 tokens: 58 us against 66, the host's time either way).
+    # 16 heads of 64 x 64: 2,000 tokens of one sequence 524 us token by token, 114 in chunks; 4 x 500 211 and 111.
+    CHUNKED_TOKENS = 192
 
     def forward(self, h, residual, ctx, cache, owns_cache: bool, accumulate: bool = True) -> None:
         ops, dt = self.runtime.ops, self.runtime.dtype
@@ -80,7 +83,7 @@ class StateSpaceMixer(Mixer):
                      ctx.is_decode, xbc)
         y = ctx.buffer("ssd.y", (T, inner), torch.float32)
         recurrence = (xbc, dt_raw, self.dt_bias, self.a_log, self.skip, self.n_heads, self.head_dim, self.state, self.groups)
-        if self.chunked and ctx.q_tiles is not None and T >= self.CHUNKED_TOKENS * ctx.n_seqs:
+        if self.chunked and ctx.q_tiles is not None and ctx.max_q_len >= self.CHUNKED_TOKENS:
             ops.ssd_scan_chunks(*recurrence, ctx.q_tiles, ctx.tok_seq, ctx.seq_first, ctx.seq_slots, cache.values,
                                 self.tail_values, y, workspace=ctx.scratch)
         else:

@@ -116,7 +116,7 @@ def test_state_space_scan_in_chunks(lens, H, P, N, G, dtype):
     _no_further_off(got["chunks"][1], got["tokens"][1], want_state)
 
 
-@pytest.mark.parametrize("lens", [(256,), (257, 1), (600, 255, 3), (40, 1025)])
+@pytest.mark.parametrize("lens", [(800,), (1025, 1), (1000, 255, 3), (40, 1281)])
 @pytest.mark.parametrize("C,N,dtype", [(40, 16, torch.bfloat16), (17, 5, torch.float32), (24, 40, torch.float32), (16, 130, torch.bfloat16)])
 def test_selective_scan_in_segments(lens, C, N, dtype):
     """Segments put together against the whole sequences' scan: the same sums but for the starting states of segments, which
@@ -146,7 +146,8 @@ def test_selective_scan_in_segments(lens, C, N, dtype):
 
 
 @pytest.mark.parametrize("lens", [(5,), (16, 7), (35, 2, 49), (150,)])
-@pytest.mark.parametrize("H,G,dk,dv", [(2, 1, 128, 20), (2, 2, 20, 132), (4, 2, 64, 16), (1, 1, 256, 12)])
+@pytest.mark.parametrize("H,G,dk,dv", [(2, 1, 128, 20), (2, 2, 20, 132), (4, 2, 64, 16), (1, 1, 256, 12),
+                                       (8, 4, 128, 132)])        # one column a lane, two, and single tokens as the sequences grow
 def test_delta_scan_in_blocks_of_four(lens, H, G, dk, dv):
     """Blocks of four tokens and what is left of a step against float64; the steps of one token show what float32 gives."""
     ops = _ops()
