@@ -131,9 +131,8 @@ _SIGNATURES = {
     "mu_ssd_conv": [_c_p, _c_ll, _c_int, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_p, _c_p, _c_p, _c_p, _c_ll,
                     _c_int, _c_p, _c_p, _c_int],
     "mu_selective_scan_max_state": [],
-    "mu_selective_scan_segment": [],
     "mu_selective_scan_scratch": [_c_int] * 4,
-    "mu_selective_scan_splits": [_c_int] * 3,
+    "mu_selective_scan_segments": [_c_int] * 4,
     "mu_selective_scan": [_c_p, _c_ll, _c_p, _c_ll, _c_p, _c_ll, _c_p, _c_ll, _c_int, _c_int, _c_p, _c_p, _c_int, _c_int, _c_int,
                           _c_p, _c_p, _c_p, _c_ll, _c_ll, _c_p, _c_ll, _c_int, _c_int, _c_p, _c_int, _c_p],
     "mu_ssd_scan": [_c_p, _c_int, _c_p, _c_ll, _c_int, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_p,
@@ -748,11 +747,6 @@ def selective_scan_max_state() -> int:
     return int(library().mu_selective_scan_max_state())
 
 
-# Tokens of the longest sequence from which on the scan goes in segments of 256, which make the exponentials almost twice: of
-# 2,048 channels (the mixer around it) 2 x 257 tokens 80 us whole, 111 in segments; 2,000 tokens 226 us and 161.
-SELECTIVE_SEGMENTED = 800
-
-
 def selective_scan(x: torch.Tensor, z: torch.Tensor, dt: torch.Tensor, bc: torch.Tensor, b_at: int, c_at: int,
                    rates: torch.Tensor, skip: torch.Tensor, seq_first, seq_slots, state: torch.Tensor, state_offset: int,
                    out: torch.Tensor, max_len: int = 0, workspace=None) -> torch.Tensor:
@@ -778,8 +772,9 @@ def selective_scan(x: torch.Tensor, z: torch.Tensor, dt: torch.Tensor, bc: torch
         raise KernelError("selective_scan: step sizes, B and C, rates or state do not fit")
     lib, n_seqs = library(), seq_slots.numel()
     long_steps, segments, room = T > 4 * n_seqs, 1, None
-    if max_len >= SELECTIVE_SEGMENTED and long_steps and lib.mu_selective_scan_splits(n_seqs, inner, N):
-        segments = -(-int(max_len) // lib.mu_selective_scan_segment())
+    if long_steps and max_len > 0:
+        segments = lib.mu_selective_scan_segments(n_seqs, inner, N, int(max_len))
+    if segments > 1:
         lib.mu_selective_scan_scratch.restype = _c_ll
         room = _room(workspace, "selective_scan", x.device, int(lib.mu_selective_scan_scratch(n_seqs, segments, inner, N)))
     _check(lib.mu_selective_scan(_ptr(x), x.stride(0), _ptr(z), z.stride(0), _ptr(dt), dt.stride(0), _ptr(bc), bc.stride(0),
@@ -1401,7 +1396,9 @@ def moe_gemm(x: torch.Tensor, pair_of: Optional[torch.Tensor], top: int, w1: tor
     return out
 
 
-HEADS_TC_ROWS = 64               # more rows than this a head, and the per-head products go to the tcgen05 kernel
+# Per-head products of at least so much work go to the tcgen05 kernel: 4 heads of 256 x 32, 256 rows, twice a layer: 81 us with
+# `mma.sync`, 87 so (the host's time); 16 heads of 512 x 128, 2,048 rows (4.3 GFLOP): 440 us and 416.
+HEADS_TC_FLOP = 1e9
 
 
 def heads_gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, x_head_stride: int, out_head_stride: int,
@@ -1417,7 +1414,7 @@ def heads_gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, x_head_strid
             and x.stride(0) % 8 == 0 and x_head_stride % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
             and x.stride(1) == 1 and out.stride(1) == 1):
         fused = gate is not None and gate.dtype == torch.bfloat16 and gate.stride(1) == 1 and gate.shape == out.shape
-        if x.shape[0] > HEADS_TC_ROWS and k % 64 == 0 and x.shape[1] >= (heads - 1) * x_head_stride + k:
+        if 2 * x.shape[0] * heads * n * k >= HEADS_TC_FLOP and x.shape[0] > 64 and k % 64 == 0 and x.shape[1] >= (heads - 1) * x_head_stride + k:
             _check(library().mu_heads_gemm_tc(_ptr(x), x.shape[1], x.stride(0), int(x_head_stride), _ptr(w), x.shape[0], heads,
                                               n, k, _ptr(out), out.stride(0), int(out_head_stride), _is_bf16(out),
                                               _ptr(gate) if fused else None, gate.stride(0) if fused else 0,

@@ -260,19 +260,22 @@ MU_EXPORT int mu_selective_scan_max_state() { return 256; }
 // x, z, y [T][inner] views (compute dtype), dt [T][inner] float32; bc float32 rows with B from column b_at and C from
 // c_at on (N rounded up to four entries each, 16-byte aligned); rates [inner][N] = A log2(e).  State of a slot from
 // state_offset on: [inner][N].  long_steps: many tokens a sequence; the launch then waits for an empty device.  segments > 1
-// (with long_steps): the longest sequence's tokens over mu_selective_scan_segment, rounded up; scratch then holds
+// (with long_steps): what mu_selective_scan_segments says; scratch then holds
 // mu_selective_scan_scratch floats, 8-byte aligned.
-MU_EXPORT int mu_selective_scan_segment() { return mu::SS_SEGMENT; }
-
 MU_EXPORT long long mu_selective_scan_scratch(int n_seqs, int segments, int inner, int N) {
     return (long long)n_seqs * segments * inner * (((N + 1) & ~1) + 1);
 }
 
-// Segments are worth their second launch where the scan alone leaves SMs with fewer than three blocks (12 warps): 2,048
-// channels, 3 sequences of up to 1,000 tokens 169 us -> 160; of 4 x 500 tokens (3.5 blocks an SM) 134 us -> 154.
-MU_EXPORT int mu_selective_scan_splits(int n_seqs, int inner, int N) {
+// Segments of a long step's longest sequence, 1 where the scan goes whole.  They make the exponentials almost twice and pay
+// where the scan alone leaves the SMs with little to do for long.  The mixer around it, 2,048 channels: one sequence (fewer
+// blocks than SMs) of 900 tokens 126 us whole, 108 in segments, of 300 tokens 79 and 95; 2 x 900 tokens 150 and 155, up to
+// 1,000 tokens of 3 sequences 169 and 160; 4 x 500 tokens (3.5 blocks an SM) 134 and 154.
+MU_EXPORT int mu_selective_scan_segments(int n_seqs, int inner, int N, int max_len) {
     const int lanes = N <= 8 ? 4 : N <= 16 ? 8 : N <= 32 ? 16 : 32;
-    return (long long)n_seqs * ((inner + mu::ss_channels(lanes) - 1) / mu::ss_channels(lanes)) < 3ll * mu::sm_count();
+    const long long blocks = (long long)n_seqs * ((inner + mu::ss_channels(lanes) - 1) / mu::ss_channels(lanes));
+    const int sms = mu::sm_count();
+    if (blocks >= 3ll * sms || max_len < (blocks <= sms ? 640 : 960)) return 1;
+    return (max_len + mu::SS_SEGMENT - 1) / mu::SS_SEGMENT;
 }
 
 MU_EXPORT int mu_selective_scan(const void* x, long long ldx, const void* z, long long ldz, const float* dt, long long lddt,

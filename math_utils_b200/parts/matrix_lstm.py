@@ -69,8 +69,8 @@ class MatrixLstm(Mixer):
 
     # Tokens of the longest sequence from which on the chunked form pays: token by token a step takes as long as its longest
     # sequence, in chunks two launches more (4 x 64 tokens: 58 us against 66, the host's time either way).
-    # 8 heads of 128 x 128: 2,000 tokens of one sequence 340 us token by token, 163 in chunks; 4 x 500 147 both.
-    CHUNKED_TOKENS = 192
+    # 8 heads of 128 x 128: 2,000 tokens of one sequence 340 us token by token, 163 in chunks; 1 x 400 81 and 84, 4 x 500 147 both.
+    CHUNKED_TOKENS = 448
 
     def forward(self, h, residual, ctx, cache, owns_cache: bool, accumulate: bool = True) -> None:
         ops, T, H = self.runtime.ops, ctx.n_tokens, self.n_heads

@@ -67,7 +67,8 @@ class StateSpaceMixer(Mixer):
 
     # Tokens of the longest sequence from which on the chunked form pays: token by token a step takes as long as its longest
     # sequence, in chunks two launches more (4 x 64 tokens: 58 us against 66, the host's time either way).
-    # 16 heads of 64 x 64: 2,000 tokens of one sequence 524 us token by token, 114 in chunks; 4 x 500 211 and 111.
+    # 16 heads of 64 x 64: 2,000 tokens of one sequence 524 us token by token, 114 in chunks; 4 x 500 211 and 111;
+    # 4 heads of 64 x 64, 200 tokens 75 and 66.
     CHUNKED_TOKENS = 192
 
     def forward(self, h, residual, ctx, cache, owns_cache: bool, accumulate: bool = True) -> None:
