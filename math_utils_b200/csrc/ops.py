@@ -772,7 +772,7 @@ def selective_scan(x: torch.Tensor, z: torch.Tensor, dt: torch.Tensor, bc: torch
         raise KernelError("selective_scan: step sizes, B and C, rates or state do not fit")
     lib, n_seqs = library(), seq_slots.numel()
     long_steps, segments, room = T > 4 * n_seqs, 1, None
-    if long_steps and max_len > 0:
+    if long_steps and max_len > 512:                         # (two segments never pay)
         segments = lib.mu_selective_scan_segments(n_seqs, inner, N, int(max_len))
     if segments > 1:
         lib.mu_selective_scan_scratch.restype = _c_ll

@@ -165,15 +165,17 @@ class LatentAttention(Mixer):
     EXPANDED_FLOP = 2.5e9
 
     def _expands(self, ctx, q, cache) -> bool:
-        if (self.expand is None or ctx.is_decode or ctx.q_tiles_wide is None or ctx.n_tokens <= 64 or cache.page_tokens != 64
-                or q.stride(0) % 8 or q.data_ptr() % 16):
+        each = self.n_heads * (2 * self.kv_rank + self.rot_dim)
+        if self.expand is None or ctx.is_decode or 2 * ctx.n_tokens * ctx.max_kv_len * each < self.EXPANDED_FLOP:
+            return False
+        if (ctx.q_tiles_wide is None or ctx.n_tokens <= 64 or cache.page_tokens != 64 or q.stride(0) % 8
+                or q.data_ptr() % 16):
             return False
         held = met = 0
         for start, n in zip(ctx.starts, ctx.q_lens):
             held += start + n
             met += n * (2 * start + n)                       # (twice the pairs of tokens and keys)
-        return (held <= self.EXPANDED_PER_TOKEN * ctx.n_tokens
-                and met * self.n_heads * (2 * self.kv_rank + self.rot_dim) >= self.EXPANDED_FLOP)
+        return held <= self.EXPANDED_PER_TOKEN * ctx.n_tokens and met * each >= self.EXPANDED_FLOP
 
     def _prompt(self, q, views, gate, residual, ctx, cache, owns_cache, accumulate, table) -> None:
         ops, dt = self.runtime.ops, self.runtime.dtype

@@ -92,6 +92,10 @@ class RoutedExperts(FeedForward):
         self.w_gate = stack("gate") if gated else None
         self.w_up, self.w_down = stack("up"), stack("down")
         self.tile_rows = runtime.ops.moe_tile_rows()
+        weights = (3 if gated else 2) * self.hidden_size * self.inner_size     # of an expert
+        self.gathered_pairs = -(-self.GATHERED_FLOP // (2 * weights))
+        if 2 * weights * self.n_experts >= self.GATHERED_BYTES:                # (pairs meet as many experts at most)
+            self.gathered_pairs = min(self.gathered_pairs, -(-self.GATHERED_BYTES // (2 * weights)))
         self.shared_up = self.shared_down = self.shared_gate = None
         if self.shared_inner:
             from .linear import Linear
@@ -108,10 +112,6 @@ class RoutedExperts(FeedForward):
     # 1,408 x 2: 136 us against 93; over 48 of 1,024 x 704 x 3: 71 against 78).
     GATHERED_FLOP, GATHERED_BYTES = 3e9, 4e8
 
-    def _gathers(self, pairs: int) -> bool:
-        weights = (3 if self.form == "gated_silu" else 2) * self.hidden_size * self.inner_size
-        return 2 * pairs * weights >= self.GATHERED_FLOP or 2 * min(pairs, self.n_experts) * weights >= self.GATHERED_BYTES
-
     fuses_output_norm = True           # forward(..., output_norm=): the norm of the result, added into the stream
 
     def forward(self, h, residual, ctx, accumulate: bool = True, output_norm=None) -> None:
@@ -123,7 +123,7 @@ class RoutedExperts(FeedForward):
         tile_rows = self.tile_rows
         if ops.moe_tc_ok(dt, self.hidden_size, self.inner_size) and h.stride(0) % 8 == 0 and h.data_ptr() % 16 == 0:
             # tiles of 64 slots where an expert has the rows to fill them; where it pays tiles of 128, their rows gathered first
-            tile_rows = ops.MOE_TC_ROWS if self._gathers(P) else 64 if P >= 48 * E else 32
+            tile_rows = ops.MOE_TC_ROWS if P >= self.gathered_pairs else 64 if P >= 48 * E else 32
         max_tiles = P // tile_rows + E                     # every grouping of P pairs into E experts fits
         index = ctx.buffer("moe.index", (3 * P + 3 * max_tiles + 4,), torch.int32)
         expert_of, slot_of, pair_of = index[:P], index[P:2 * P], index[2 * P:3 * P]
