@@ -39,8 +39,11 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     extern __shared__ unsigned char tc_raw[];
     Smem& sm = *reinterpret_cast<Smem*>(((uintptr_t)tc_raw + 1023) & ~(uintptr_t)1023);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int num_kb = (k + KSUB * TC_BK - 1) / (KSUB * TC_BK);          // a sub-tile past k is zero-filled
-    constexpr uint32_t STAGE_BYTES = KSUB * (TC_BM + BN) * TC_BK * sizeof(__nv_bfloat16);
+    // (a sub-tile that would begin past k is neither fetched nor multiplied: by head there lies the gap after the slice, or the
+    // next head's slice, and zeros of the weights do not make a product with an infinity or a NaN zero)
+    const int num_kb = (k + KSUB * TC_BK - 1) / (KSUB * TC_BK);
+    auto sub_tiles = [&](int kb) { return min(KSUB, (k + TC_BK - 1) / TC_BK - kb * KSUB); };
+    constexpr uint32_t SUB_BYTES = (TC_BM + BN) * TC_BK * sizeof(__nv_bfloat16);
     constexpr uint32_t TMEM_COLS = 2 * BN;
     bool ok = true;
     if (threadIdx.x == 0) {
@@ -94,9 +97,11 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                     const int s = (int)(it % STAGES);
                     ok = mbar_wait(&sm.empty[s], (uint32_t)(((it / STAGES) & 1) ^ 1));
                     if (!ok) break;
-                    mbar_expect_tx(&sm.full[s], STAGE_BYTES);
+                    const int subs = sub_tiles(kb);
+                    mbar_expect_tx(&sm.full[s], subs * SUB_BYTES);
 #pragma unroll
                     for (int u = 0; u < KSUB; ++u) {
+                        if (u >= subs) break;
                         const int x = (kb * KSUB + u) * TC_BK;
                         tma_load_2d(sm.a[s][u], &map_a, ax + x, w.row0, &sm.full[s]);
                         tma_load_2d(sm.b[s][u], &map_w1, x, wy, &sm.full[s]);
@@ -136,12 +141,14 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint64_t a_stage = a_desc0 + (uint64_t)((uint32_t)s * (KSUB * A_SUB));
                     const uint64_t b_stage = b_desc0 + (uint64_t)((uint32_t)s * (KSUB * B_SUB));
+                    const int subs = sub_tiles(kb);
 #pragma unroll
                     for (int u = 0; u < KSUB; ++u)
 #pragma unroll
                         for (int kk = 0; kk < TC_BK / 16; ++kk)
-                            umma_bf16(tmem_d, a_stage + (uint64_t)(u * A_SUB + 2 * kk), b_stage + (uint64_t)(u * B_SUB + 2 * kk),
-                                      idesc, (kb > 0 || u > 0 || kk > 0) ? 1u : 0u);
+                            if (u < subs)
+                                umma_bf16(tmem_d, a_stage + (uint64_t)(u * A_SUB + 2 * kk), b_stage + (uint64_t)(u * B_SUB + 2 * kk),
+                                          idesc, (kb > 0 || u > 0 || kk > 0) ? 1u : 0u);
                     umma_commit(&sm.empty[s]);
                 }
                 if (ok) umma_commit(&sm.acc_full[buf]);

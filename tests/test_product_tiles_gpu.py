@@ -116,6 +116,27 @@ def test_products_per_head_on_tcgen05(rows, heads, n, k, lead, out_dtype, monkey
         assert float(((got[:, :, :n].double() - want).abs() / (want.abs() + want.square().mean().sqrt())).max()) < bound
 
 
+# one stage of 128 and half of the next (k past a whole number of 128), columns of one box and less
+@pytest.mark.parametrize("n,k,lead", [(128, 64, 32), (40, 192, 0), (128, 320, 64), (264, 64, 8)])
+def test_products_per_head_see_their_own_slice_alone(n, k, lead, monkeypatch):
+    """Whatever lies between the slices or in another head's: the same bits as with zeros there."""
+    ops = _ops()
+    monkeypatch.setattr(ops, "HEADS_TC_FLOP", 0.0)
+    rows, heads, xs = 130, 3, k + lead
+    x, w = _rand((rows, heads * xs), 1, torch.bfloat16), _rand((heads, n, k), 2, torch.bfloat16, k ** -0.5)
+    slices = x.reshape(rows, heads, xs)
+    slices[:, :, k:] = 0.0
+    outs = []
+    for _ in range(2):
+        out = torch.zeros((rows, heads * n), device="cuda")
+        ops.heads_gemm(x, w, out, xs, n)
+        ops.check_status()
+        outs.append(out.reshape(rows, heads, n))
+        slices[:, :, k:] = float("nan")
+        slices[:, 1] = float("inf")
+    assert torch.equal(outs[0][:, 0], outs[1][:, 0]) and torch.equal(outs[0][:, 2], outs[1][:, 2])
+
+
 # one block of 128 threads, of 1024, pairs beyond those it keeps in registers; identity experts; more experts than a warp
 @pytest.mark.parametrize("P,experts,real", [(1, 4, 4), (48, 72, 64), (256, 33, 33), (257, 5, 4), (12288, 64, 64), (20001, 70, 64)])
 @pytest.mark.parametrize("rows", [32, 128])
