@@ -50,6 +50,9 @@ struct MtArgs {
     long long ldg, ldo;
     __nv_bfloat16* out;
     int* status;
+    const __nv_bfloat16 *q, *rows;                     // what the maps stand for (mt_row_alone)
+    long long ldq;
+    int row_width;
 };
 
 __device__ __forceinline__ float mt_exp2(float x) {
@@ -77,6 +80,108 @@ __device__ __forceinline__ void mt_tmem_st_32x32(uint32_t taddr, const uint32_t 
           "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]),
           "r"(r[30]), "r"(r[31])
         : "memory");
+}
+
+// What a row's two accumulators are multiplied by, out = w0 O0 + w1 O1, from their references (in units of log2) and sums: the
+// maps' difference, or (one map) both streams under a common maximum; with a sink's share in the sums.
+__device__ __forceinline__ float2 mt_join(const MtArgs& a, int h, float ref0, float sum0, float ref1, float sum1) {
+    constexpr float LOG2E = 1.4426950408889634f;
+    const bool sinks = a.sink || a.head_sink;
+    const float sink = a.head_sink ? a.head_sink[h] * LOG2E : a.sink ? 0.0f : -INFINITY;
+    float2 w;
+    if (a.maps == 2) {
+        const float t0 = fmaxf(ref0, sink), t1 = fmaxf(ref1, sink);
+        const float f0 = ref0 == -INFINITY ? 0.0f : mt_exp2(ref0 - t0), f1 = ref1 == -INFINITY ? 0.0f : mt_exp2(ref1 - t1);
+        const float l0 = sum0 * f0 + (sinks ? mt_exp2(sink - t0) : 0.0f), l1 = sum1 * f1 + (sinks ? mt_exp2(sink - t1) : 0.0f);
+        w.x = l0 > 0.0f ? f0 / l0 : 0.0f;
+        w.y = l1 > 0.0f ? -a.lambda * (f1 / l1) : 0.0f;
+    } else {
+        const float t = fmaxf(fmaxf(ref0, ref1), sink);
+        const float f0 = ref0 == -INFINITY ? 0.0f : mt_exp2(ref0 - t), f1 = ref1 == -INFINITY ? 0.0f : mt_exp2(ref1 - t);
+        const float l = sum0 * f0 + sum1 * f1 + (sinks ? mt_exp2(sink - t) : 0.0f);
+        w.x = l > 0.0f ? f0 / l : 0.0f;
+        w.y = l > 0.0f ? f1 / l : 0.0f;
+    }
+    return w;
+}
+
+// One query's result over exactly the keys that it sees, by a warp: for rows that came out infinite or NaN.  A weight of
+// zero does not keep an infinite or NaN value out of a product, and a tile's rows meet all pages of the tile: those with later
+// tokens, and what lies in the last page behind the sequence's end.  Finite rows pay one multiply-add a value for the check.
+// A row whose scores hold a NaN is NaN throughout and stops there.
+__device__ __noinline__ void mt_row_alone(const MtArgs& a, const int* pages, int page_lo, int kept_pages, int n_pages, int h, int g,
+                                          int flat, int pos) {
+    constexpr float LOG2E = 1.4426950408889634f;
+    const int lane = threadIdx.x & 31, kw = a.maps * a.dim;
+    const int lo = a.chunk > 0 ? pos - pos % a.chunk : a.window > 0 ? pos - a.window + 1 : 0;
+    const float scale = a.head_scale ? a.scale * a.head_scale[h] : a.scale;
+    const float inv_cap = a.softcap > 0.0f ? 1.0f / a.softcap : 0.0f, slope = a.slopes ? a.slopes[h] * LOG2E : 0.0f;
+    float acc[2][4] = {}, ref[2] = {-INFINITY, -INFINITY}, sum[2] = {0.0f, 0.0f};      // columns lane + 32 c
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+        if (m == a.maps) break;
+        const __nv_bfloat16* q = a.q + (long long)flat * a.ldq + (long long)h * kw + m * a.dim;
+        for (int i = 0; i < 2 * n_pages; ++i) {                                         // 32 keys at a time
+            const int page = i / 2 < kept_pages ? i / 2 : page_lo + i / 2 - kept_pages, key = page * MT_K + (i & 1) * 32 + lane;
+            const bool seen = key <= pos && (key >= lo || key < a.keep);
+            const unsigned some = __ballot_sync(0xffffffffu, seen);
+            if (!some) continue;
+            const __nv_bfloat16* rows = a.rows + ((long long)pages[page] * MT_K + (i & 1) * 32) * a.row_width;
+            float x = -INFINITY;
+            if (seen) {
+                const __nv_bfloat16* row = rows + (long long)lane * a.row_width;
+                x = 0.0f;
+                for (int e = 0; e < a.dim; e += 2) {
+                    const int col = m * a.dim + e, far = col - 64 * a.key_split;
+                    const float2 k = __bfloat1622float2(
+                        *reinterpret_cast<const __nv_bfloat162*>(row + (far < 0 ? g * a.key_step + col : a.split_at + far)));
+                    const float2 y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(q + e));
+                    x = fmaf(k.y, y.y, fmaf(k.x, y.x, x));
+                }
+                x *= scale;
+                if (a.softcap > 0.0f) x = softcap_fast(x, a.softcap, inv_cap);
+                x = x * LOG2E - slope * (float)(pos - key);
+            }
+            const float top = fmaxf(ref[m], warp_max(x)), from = top == -INFINITY ? 0.0f : top, f = mt_exp2(ref[m] - from);
+            const float p = seen ? mt_exp2(x - from) : 0.0f;
+            ref[m] = top;
+            sum[m] = sum[m] * f + warp_sum(p);
+            if (isnan(sum[m])) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) acc[m][c] = NAN;
+                break;
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c) acc[m][c] *= f;
+            for (int j = 0; j < 32; ++j) {
+                const float pj = __shfl_sync(0xffffffffu, p, j);
+                if (!(some >> j & 1u)) continue;
+                const __nv_bfloat16* value = rows + (long long)j * a.row_width + a.val_at + g * a.val_step;
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    if (lane + 32 * c < a.vdim) acc[m][c] = fmaf(pj, __bfloat162float(value[lane + 32 * c]), acc[m][c]);
+            }
+        }
+    }
+    const float2 w = mt_join(a, h, ref[0], sum[0], ref[1], sum[1]);
+    float v[4], sq = 0.0f, times = a.out_scale;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        v[c] = acc[0][c] * w.x;
+        if (a.maps == 2) v[c] += acc[1][c] * w.y;
+        if (lane + 32 * c < a.vdim) sq = fmaf(v[c], v[c], sq);
+    }
+    if (a.unit_rms) times *= 1.0f / sqrtf(warp_sum(sq) / (float)a.vdim + a.eps);
+    const __nv_bfloat16* gate = a.gate ? a.gate + (long long)flat * a.ldg : nullptr;
+    if (gate && !a.gate_each) times *= 1.0f / (1.0f + expf(-__bfloat162float(gate[h])));
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const int d = lane + 32 * c;
+        if (d >= a.vdim) break;
+        float y = v[c] * times;
+        if (a.gate_each) y = __fdividef(y, 1.0f + __expf(-__bfloat162float(gate[(long long)h * a.vdim + d])));
+        a.out[(long long)flat * a.ldo + (long long)h * a.vdim + d] = __float2bfloat16_rn(y);
+    }
 }
 
 __global__ void __launch_bounds__(MT_THREADS)
@@ -340,25 +445,9 @@ mapped_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
         } else {
             if (ok) ok = mbar_wait(&sm.x_full, 0);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (ok && !sm.failed) {
-                // what the two accumulators are multiplied by: out = w0 O0 + w1 O1
-                const float ref1 = sm.hand_ml[row][0], sum1 = sm.hand_ml[row][1];
-                const bool sinks = a.sink || a.head_sink;
-                const float sink = a.head_sink ? a.head_sink[h] * LOG2E : a.sink ? 0.0f : -INFINITY;
-                float w0, w1;
-                if (a.maps == 2) {
-                    const float t0 = fmaxf(ref, sink), t1 = fmaxf(ref1, sink);
-                    const float f0 = ref == -INFINITY ? 0.0f : mt_exp2(ref - t0), f1 = ref1 == -INFINITY ? 0.0f : mt_exp2(ref1 - t1);
-                    const float l0 = sum * f0 + (sinks ? mt_exp2(sink - t0) : 0.0f), l1 = sum1 * f1 + (sinks ? mt_exp2(sink - t1) : 0.0f);
-                    w0 = l0 > 0.0f ? f0 / l0 : 0.0f;
-                    w1 = l1 > 0.0f ? -a.lambda * (f1 / l1) : 0.0f;
-                } else {
-                    const float t = fmaxf(fmaxf(ref, ref1), sink);
-                    const float f0 = ref == -INFINITY ? 0.0f : mt_exp2(ref - t), f1 = ref1 == -INFINITY ? 0.0f : mt_exp2(ref1 - t);
-                    const float l = sum * f0 + sum1 * f1 + (sinks ? mt_exp2(sink - t) : 0.0f);
-                    w0 = l > 0.0f ? f0 / l : 0.0f;
-                    w1 = l > 0.0f ? f1 / l : 0.0f;
-                }
+            if (__all_sync(0xffffffffu, ok && !sm.failed)) {
+                const float2 w = mt_join(a, h, ref, sum, sm.hand_ml[row][0], sm.hand_ml[row][1]);
+                const float w0 = w.x, w1 = w.y;
                 const bool two = a.maps == 2 || n_pages > 1;              // (else the second accumulator was never written)
                 auto columns = [&](int c, float (&v)[32]) {
                     uint32_t x[32], y[32];
@@ -383,6 +472,7 @@ mapped_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                 const __nv_bfloat16* gate = a.gate ? a.gate + (long long)(flat0 + min(row, count - 1)) * a.ldg : nullptr;
                 if (gate && !a.gate_each) times *= 1.0f / (1.0f + expf(-__bfloat162float(gate[h])));
                 __nv_bfloat16* dst = a.out + (long long)(flat0 + row) * a.ldo + (long long)h * a.vdim;
+                float odd = 0.0f;                        // NaN from the first value that is not finite on
                 for (int c = 0; c < a.vdim; c += 32) {
                     float v[32];
                     __syncwarp();
@@ -391,6 +481,8 @@ mapped_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                     for (int i = 0; i < 32; i += 8) {
                         if (!real || c + i >= a.vdim) break;
                         uint32_t word[4];
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) odd = fmaf(v[i + e], 0.0f, odd);
 #pragma unroll
                         for (int e = 0; e < 4; ++e) {
                             float y0 = v[i + 2 * e] * times, y1 = v[i + 2 * e + 1] * times;
@@ -404,6 +496,10 @@ mapped_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                         }
                         *reinterpret_cast<uint4*>(dst + c + i) = make_uint4(word[0], word[1], word[2], word[3]);
                     }
+                }
+                for (unsigned todo = __ballot_sync(0xffffffffu, isnan(odd)); todo; todo &= todo - 1) {
+                    const int r = quad * 32 + __ffs(todo) - 1;
+                    mt_row_alone(a, pages, page_lo, kept_pages, n_pages, h, g, flat0 + r, pos0 + r);
                 }
             }
         }
@@ -461,6 +557,7 @@ MU_EXPORT int mu_mapped_attention_tc(const void* q, long long ldq, int n_tokens,
     a.n_heads = n_heads, a.n_kv_heads = n_kv_heads, a.maps = maps, a.dim = dim, a.vdim = vdim, a.window = window, a.chunk = chunk;
     a.keep = keep, a.unit_rms = unit_rms, a.sink = sink, a.gate_each = gate_each, a.scale = scale, a.lambda = lambda;
     a.out_scale = out_scale, a.eps = eps, a.softcap = softcap, a.head_scale = head_scale, a.slopes = slopes, a.head_sink = head_sink;
+    a.q = (const __nv_bfloat16*)q, a.ldq = ldq, a.rows = (const __nv_bfloat16*)rows, a.row_width = width;
     a.gate = (const __nv_bfloat16*)gate, a.ldg = ldg, a.ldo = ldo, a.out = (__nv_bfloat16*)out, a.status = status;
     a.key_tiles = (kw + 63) / 64, a.val_boxes = (vdim + 63) / 64;
     a.key_step = kw, a.key_split = a.key_tiles;

@@ -113,6 +113,55 @@ def test_mapped_attention_on_tcgen05(c):
     assert float(worst[bad]) < 1.0, f"{float(worst[bad]):.2f} of the bound at token {bad} (sequence {tok_seq[bad]}, position {tok_pos[bad]})"
 
 
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("c", [CASES[i] for i in (0, 1, 3, 8, 9, 10, 11)], ids=lambda c: "-".join(f"{k}{v}" for k, v in c.items() if v))
+def test_values_that_are_not_finite_stay_with_the_queries_that_see_them(c, bad):
+    """One position's values, and whatever the last page holds behind the sequence's end, against the same rows with finite
+    values there: queries that do not see the position differ by no more than two results that are each rounded once."""
+    from math_utils_b200.csrc import ops
+    H, G, maps, dim, vdim, shared = (c[k] for k in ("H", "G", "maps", "dim", "vdim", "shared"))
+    n, new, at = 410, 405, 171                                     # the tiles begin inside a page
+    width, n_pages = G * (maps * dim + (0 if shared else vdim)), -(-n // 64)
+    table, rows = _ints([list(range(n_pages))[::-1]]), _rand((n_pages, 64, width), 2)
+    q = _rand((new, H * maps * dim), 3)
+    gate = _rand((new, H * (vdim if c["gate"] == "entry" else 1)), 4) if c["gate"] else None
+    slopes = 2.0 ** (-8.0 * (torch.arange(H, device="cuda") + 1).float() / H) if c["slopes"] else None
+    tiles, outs = _ints([(o, min(128, new - o)) for o in range(0, new, 128)]), []
+    for _ in range(2):
+        out = torch.zeros((new, H * vdim), device="cuda", dtype=torch.bfloat16)
+        ops.mapped_attention(q, rows, table, 64, _ints(range(n - new, n)), _ints([0] * new), H, G, maps, dim, vdim, dim ** -0.5,
+                             c["window"], out, lam=0.45 if maps == 2 else 0.0, out_scale=0.8, eps=1e-3, unit_rms=c["unit"],
+                             chunk=c["chunk"], keep=c["keep"], slopes=slopes, softcap=c["softcap"], sink=c["sink"], shared=shared,
+                             gate=gate, tiles_wide=tiles)
+        ops.check_status()
+        outs.append(out.double())
+        rows[n_pages - 1 - at // 64, at % 64, 0 if shared else G * maps * dim:] = bad
+        rows[0, n % 64:] = bad
+    p = torch.arange(n - new, n, device="cuda")
+    lo = p - p % c["chunk"] if c["chunk"] else p - c["window"] + 1 if c["window"] else 0 * p
+    sees = (at <= p) & ((at >= lo) | (at < c["keep"]))
+    assert sees.any() and not outs[1][sees].isfinite().all(1).any()
+    want, got = outs[0][~sees], outs[1][~sees]
+    bound = 2.0 ** -7 * want.abs() + 2.0 ** -8 * want.reshape(len(want), H, vdim).square().mean(-1).sqrt().repeat_interleave(vdim, 1) + 1e-6
+    assert torch.isfinite(got).all() and float(((got - want).abs() / bound).max()) < 1.0
+
+
+def test_expanded_values_that_are_not_finite_stay_with_the_queries_that_see_them():
+    from math_utils_b200.csrc import ops
+    H, dim, rot, vdim, n, at = 2, 64, 32, 48, 300, 130
+    rows, q = _rand((5, 64, H * (dim + vdim) + rot), 1), _rand((n, H * (dim + rot)), 2)
+    tiles, outs = _ints([(o, min(128, n - o)) for o in range(0, n, 128)]), []
+    for _ in range(2):
+        out = torch.zeros((n, H * vdim), device="cuda", dtype=torch.bfloat16)
+        ops.latent_prompt(q, rows, _ints([range(5)]), _ints(range(n)), _ints([0] * n), tiles, H, dim, rot, vdim, 0.1, out)
+        ops.check_status()
+        outs.append(out.double())
+        rows[at // 64, at % 64, H * dim: H * (dim + vdim)] = float("nan")
+    assert outs[1][at:].isnan().all() and torch.isfinite(outs[1][:at]).all()
+    want = outs[0][:at]
+    assert float(((outs[1][:at] - want).abs() / (2.0 ** -7 * want.abs() + 2.0 ** -8 * want.square().mean(1, keepdim=True).sqrt())).max()) < 1.0
+
+
 @pytest.mark.parametrize("H,dim,rot,vdim,rank,q_rank,layout,gate,sink", [(4, 64, 32, 64, 256, 96, "pairs", False, True),
                                                                          (2, 128, 64, 128, 64, 0, "half", True, False),
                                                                          (3, 64, 16, 48, 72, 0, "half", True, True)])
