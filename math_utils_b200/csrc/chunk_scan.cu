@@ -380,10 +380,38 @@ chunk_outputs_kernel(const __grid_constant__ ChunkArgs a) {
             cs_split(p1, ph[u][2], pl[u][2]);
             cs_split(p3, ph[u][3], pl[u][3]);
         }
+        // the last sixteen keys are this warp's own tokens: those after a token have the weight zero, which does not keep an
+        // infinite or NaN value out of a product
+        bool plain = true;
+        if (n + 2 >= key_tiles) {
+            float odd = 0.0f;                                   // NaN from the first value that is not finite on
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float* src = Vs + (8 * n + 2 * tig) * VP + half0 + 8 * j + gid;
-            cs_products(o[j], ph, pl, src[0], src[VP], src[8 * VP], src[9 * VP]);
+            for (int j = 0; j < 4; ++j) {
+                const float* src = Vs + (8 * n + 2 * tig) * VP + half0 + 8 * j + gid;
+                odd = fmaf(src[0], 0.0f, fmaf(src[VP], 0.0f, fmaf(src[8 * VP], 0.0f, fmaf(src[9 * VP], 0.0f, odd))));
+            }
+            plain = !__any_sync(0xffffffffu, isnan(odd));
+        }
+        if (plain) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float* src = Vs + (8 * n + 2 * tig) * VP + half0 + 8 * j + gid;
+                cs_products(o[j], ph, pl, src[0], src[VP], src[8 * VP], src[9 * VP]);
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {                      // key by key, seen keys alone
+                const int s = 8 * n + i, u = i >> 3, from = (lane & ~3) | ((i & 7) >> 1), f = 2 * (i & 1);
+                const float p = __uint_as_float(ph[u][f]) + __uint_as_float(pl[u][f]);
+                const float r = __uint_as_float(ph[u][f + 1]) + __uint_as_float(pl[u][f + 1]);
+                const float p0 = __shfl_sync(0xffffffffu, p, from), p1 = __shfl_sync(0xffffffffu, r, from);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float* src = Vs + s * VP + half0 + 8 * j + 2 * tig;
+                    if (s <= t0) o[j][0] = fmaf(p0, src[0], o[j][0]), o[j][1] = fmaf(p0, src[1], o[j][1]);
+                    if (s <= t1) o[j][2] = fmaf(p1, src[0], o[j][2]), o[j][3] = fmaf(p1, src[1], o[j][3]);
+                }
+            }
         }
     }
     const float d_skip = a.skip ? a.skip[h] : 0.0f;

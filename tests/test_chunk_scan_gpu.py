@@ -116,6 +116,34 @@ def test_state_space_scan_in_chunks(lens, H, P, N, G, dtype):
     _no_further_off(got["chunks"][1], got["tokens"][1], want_state)
 
 
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("at", [0, 7, 40, 63, 64, 149])
+@pytest.mark.parametrize("by_key", [False, True])
+def test_chunks_keep_values_that_are_not_finite_from_tokens_before_them(by_key, at, bad):
+    """One value entry of one token against the same step with a finite one: tokens before it, other entries and other heads
+    differ by the order of their sums alone (float32 sums of some hundred terms, by 2^-24 each)."""
+    ops = _ops()
+    lens, H, dk, dv = (130, 150), 2, 32, 40
+    tiles, tok_seq, seq_first, first = _step(lens)
+    T, slots, at, col = sum(lens), [0, 1], int(first[1]) + at, 35
+    u = _rand((T, H * (dv + 2 * dk)), 1)
+    gates, outs = torch.rand((T, H, 4), generator=torch.Generator(device="cuda").manual_seed(2), device="cuda"), []
+    for _ in range(2):
+        state, out = torch.zeros((2, H * dk * (dv + 1)), device="cuda"), torch.zeros((T, H * dv), device="cuda")
+        if by_key:
+            ops.ssd_scan_chunks(u, gates[..., 0].contiguous(), gates[0, :, 1].contiguous(), gates[0, :, 2].contiguous(),
+                                gates[0, :, 3].contiguous(), H, dv, dk, H, tiles, tok_seq, seq_first, _ints(slots), state, 0, out)
+        else:
+            v, q, k = u[:, :H * dv], u[:, H * dv:H * (dv + dk)], u[:, H * (dv + dk):]
+            ops.linear_scan_chunks(q, k, v, gates, H, dk, dv, 1.0, tiles, tok_seq, seq_first, _ints(slots), state, 0, out)
+        outs.append(out)
+        u[at, col] = bad
+    hit = torch.zeros((T, H * dv), dtype=torch.bool, device="cuda")
+    hit[at:, col] = True
+    assert not outs[1][hit].isfinite().any() and torch.isfinite(outs[1][~hit]).all()
+    assert float((outs[1] - outs[0])[~hit].abs().max() / outs[0].square().mean().sqrt()) < 1e-5
+
+
 @pytest.mark.parametrize("lens", [(800,), (1025, 1), (1000, 255, 3), (40, 1281)])
 @pytest.mark.parametrize("C,N,dtype", [(40, 16, torch.bfloat16), (17, 5, torch.float32), (24, 40, torch.float32), (16, 130, torch.bfloat16)])
 def test_selective_scan_in_segments(lens, C, N, dtype):
