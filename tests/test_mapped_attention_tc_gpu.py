@@ -70,6 +70,7 @@ def test_mapped_attention_on_tcgen05(c):
     head_sink = heads.float() - 0.5 if c["head_sink"] else None
     gate = _rand((T, H * (vdim if c["gate"] == "entry" else 1)), 4) if c["gate"] else None
     out = torch.zeros((T, H * vdim), device="cuda", dtype=torch.bfloat16)
+    assert ops.mapped_tc_ok(q, out, G, maps, dim, vdim, 64, shared)
     ops.mapped_attention(q, rows, _ints(table), 64, _ints(tok_pos), _ints(tok_seq), H, G, maps, dim, vdim, scale, c["window"], out,
                          lam=lam, out_scale=out_scale, eps=eps, unit_rms=c["unit"], chunk=c["chunk"], keep=c["keep"],
                          slopes=slopes, softcap=c["softcap"], sink=c["sink"], shared=shared, gate=gate, head_scale=head_scale,
@@ -162,49 +163,65 @@ def test_expanded_values_that_are_not_finite_stay_with_the_queries_that_see_them
     assert float(((outs[1][:at] - want).abs() / (2.0 ** -7 * want.abs() + 2.0 ** -8 * want.square().mean(1, keepdim=True).sqrt())).max()) < 1.0
 
 
-@pytest.mark.parametrize("H,dim,rot,vdim,rank,q_rank,layout,gate,sink", [(4, 64, 32, 64, 256, 96, "pairs", False, True),
-                                                                         (2, 128, 64, 128, 64, 0, "half", True, False),
-                                                                         (3, 64, 16, 48, 72, 0, "half", True, True)])
-def test_latent_prompts_over_expanded_rows(H, dim, rot, vdim, rank, q_rank, layout, gate, sink):
-    """A layer's prompt steps with keys and values expanded against the same layer in latent space: whole prompts, then steps
-    that go on from cached positions.  Both round a row's keys, values and sums to bfloat16 in different places: some three
-    roundings of 2^-9 of a value each side, held to 1.2 % of the output's rms, rms over rms."""
-    from math_utils_b200.cache import SequenceCache
+LATENTS = [(4, 64, 32, 64, 256, 96, "pairs", False, True), (2, 128, 64, 128, 64, 0, "half", True, False),
+           (3, 64, 16, 48, 72, 0, "half", True, True)]
+
+
+def _latent_part(H, dim, rot, vdim, rank, q_rank, layout, gate, sink):
+    """A layer whose prompt steps expand their rows whatever their size."""
     from math_utils_b200.config.base import PartSpec
-    from math_utils_b200.engine.batch import PinnedRing, StepEntry, build_context
     from math_utils_b200.engine.runtime import Runtime
     from math_utils_b200.parts.base import build_part
-    D = 192
     names = ["dkv", "dkv_norm", "uk", "uv", "out"] + (["dq", "dq_norm", "uq"] if q_rank else ["q"])
     names += ["gate"] * gate + ["sink"] * sink
-    params = dict(hidden_size=D, n_heads=H, dim=dim, rot_dim=rot, vdim=vdim, kv_rank=rank, q_rank=q_rank, gate=gate, sink=sink,
+    params = dict(hidden_size=192, n_heads=H, dim=dim, rot_dim=rot, vdim=vdim, kv_rank=rank, q_rank=q_rank, gate=gate, sink=sink,
                   softmax_scale=(dim + rot) ** -0.5, eps=1e-5, rot_layout=layout, exact_weights=True, rot={"base": 10000.0, "dims": rot})
     part = build_part("mixer", PartSpec("latent_attention", params, {n: n for n in names}))
-    runtime = Runtime.create("bfloat16", "cuda:0")
     tensors = {}
     for i, spec in enumerate(part.tensor_specs()):
         x = torch.randn(spec.shape, generator=torch.Generator(device="cuda").manual_seed(i), device="cuda")
         tensors[spec.name] = (x * spec.shape[-1] ** -0.5).to(torch.bfloat16) if spec.role == "matrix" else 1.0 + 0.1 * x
-    part.bind(tensors, runtime)
+    part.bind(tensors, Runtime.create("bfloat16", "cuda:0"))
     assert part.expand is not None
-    steps = [[70, 1, 200], [100, 130, 64], [3, 2, 190]]
-    expand, outs = part.expand, []
-    for way in (expand, None):
-        part.expand, found = way, []
-        cache = SequenceCache([part.cache_spec()], 4096, 4096, torch.bfloat16, runtime.device, n_slots=3)
-        slots, ring, work = [cache.acquire() for _ in range(3)], PinnedRing(), {}
+    part.EXPANDED_FLOP = 0.0
+    return part
+
+
+def _latent_steps(part, steps, monkeypatch, trace=None):
+    """The results of one step after another of three sequences, and how often each step expanded its rows."""
+    from math_utils_b200.cache import SequenceCache
+    from math_utils_b200.csrc import ops
+    from math_utils_b200.engine.batch import PinnedRing, StepEntry, build_context
+    took, found, check = [], [], ops._check
+    cache = SequenceCache([part.cache_spec()], 4096, 4096, torch.bfloat16, part.runtime.device, n_slots=3)
+    slots, ring, work = [cache.acquire() for _ in range(3)], PinnedRing(), {}
+    with monkeypatch.context() as m:
+        m.setattr(ops, "_check", lambda code, what, *a, **k: (took.append(str(what)), check(code, what, *a, **k))[1])
         for k, lens in enumerate(steps):
             entries = [StepEntry(s, [0] * n, ()) for s, n in zip(slots, lens)]
-            ctx = build_context(runtime, None, cache, entries, [cache.reserve(s, n) for s, n in zip(slots, lens)], ring, work)
-            h = _rand((sum(lens), D), 50 + k)
-            y = torch.zeros((sum(lens), D), device="cuda")
-            part.forward(h, y, ctx, cache.entry(0), True, accumulate=False)
+            ctx = build_context(part.runtime, None, cache, entries, [cache.reserve(s, n) for s, n in zip(slots, lens)], ring, work, trace)
+            y = torch.zeros((sum(lens), 192), device="cuda")
+            part.forward(_rand((sum(lens), 192), 50 + k), y, ctx, cache.entry(0), True, accumulate=False)
             for s, n in zip(slots, lens):
                 cache.commit(s, n)
             found.append(y)
-        runtime.ops.check_status()
-        outs.append(found)
-    for a, b in zip(*outs):
+            took.append("|")
+    ops.check_status()
+    return found, [(step.count("latent_rows"), step.count("latent_prompt(")) for step in " ".join(took).split("|")[:-1]]
+
+
+@pytest.mark.parametrize("H,dim,rot,vdim,rank,q_rank,layout,gate,sink", LATENTS)
+def test_latent_prompts_over_expanded_rows(H, dim, rot, vdim, rank, q_rank, layout, gate, sink, monkeypatch):
+    """A layer's prompt steps with keys and values expanded against the same layer in latent space: whole prompts, then steps
+    that go on from cached positions.  Both round a row's keys, values and sums to bfloat16 in different places: some three
+    roundings of 2^-9 of a value each side, held to 1.2 % of the output's rms, rms over rms."""
+    part = _latent_part(H, dim, rot, vdim, rank, q_rank, layout, gate, sink)
+    steps = [[70, 1, 200], [100, 130, 64], [3, 2, 190]]
+    expanded, runs = _latent_steps(part, steps, monkeypatch)
+    part.expand = None
+    latent, none = _latent_steps(part, steps, monkeypatch)
+    assert runs == [(1, 1)] * 3 and none == [(0, 0)] * 3
+    for a, b in zip(expanded, latent):
         assert torch.isfinite(a).all()
         off = (a - b).double().square().mean(1).sqrt() / b.double().square().mean().sqrt()
         assert float(off.max()) < 0.05 and float(off.square().mean().sqrt()) < 0.012
