@@ -132,9 +132,7 @@ _SIGNATURES = {
                     _c_int, _c_p, _c_p, _c_int],
     "mu_selective_scan_max_state": [],
     "mu_selective_scan_scratch": [_c_int] * 4,
-    "mu_selective_scan_segment": [],
-    "mu_selective_scan_least": [],
-    "mu_selective_scan_segments": [_c_int] * 3 + [_c_ll],
+    "mu_selective_scan_segments": [_c_int] * 4,
     "mu_selective_scan": [_c_p, _c_ll, _c_p, _c_ll, _c_p, _c_ll, _c_p, _c_ll, _c_int, _c_int, _c_p, _c_p, _c_int, _c_int, _c_int,
                           _c_p, _c_p, _c_p, _c_ll, _c_ll, _c_p, _c_ll, _c_int, _c_int, _c_p, _c_int, _c_p],
     "mu_ssd_scan": [_c_p, _c_int, _c_p, _c_ll, _c_int, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_p,
@@ -548,21 +546,13 @@ def qk_prepare(q: torch.Tensor, k: Optional[torch.Tensor], v: Optional[torch.Ten
 def mapped_tc_ok(q: torch.Tensor, out: torch.Tensor, n_kv_heads: int, maps: int, dim: int, vdim: int, page_tokens: int,
                  shared: bool = False) -> bool:
     """Whether ``mapped_attention`` takes the tcgen05 kernel for these queries (bfloat16 rows given wide tiles)."""
-    return (MAPPED_TC and q.dtype == torch.bfloat16 and q.stride(0) % 8 == 0 and q.stride(0) >= q.shape[1] and q.data_ptr() % 16 == 0
+    return (MAPPED_TC and q.dtype == torch.bfloat16 and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0
             and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0
             and _mapped_tc_fits(int(n_kv_heads), int(maps), int(dim), int(vdim), int(page_tokens), int(shared)))
 
 
 @functools.lru_cache(maxsize=None)
 def _mapped_tc_fits(*sizes) -> bool:
-def wide_tiles_pay(n_tiles: int, n_wide: int, n_heads: int, sms: int) -> bool:
-    """Whether a prompt step takes tiles of 128 queries on tcgen05 instead of tiles of 64 on ``mma.sync``.  A wide tile has an
-    SM to itself; while every one finds an SM it is the faster form from two tokens on (single layers on the device, 1 to 16
-    sequences of 2 to 1,000 tokens: 1.08 to 2.3 times).  Where they outnumber the SMs it wins if it halves the tiles (64 sequences of 65
-    tokens, 8 heads: 126.6 us against 100.3) and loses if no sequence has more than 64 tokens (64 of 17: 47.1 against 56.9)."""
-    return n_wide * n_heads <= sms or 2 * n_tiles >= 3 * n_wide
-
-
     return bool(library().mu_mapped_attention_tc_fits(*sizes))
 
 
@@ -592,7 +582,7 @@ def mapped_attention(q: torch.Tensor, rows: torch.Tensor, block_table: torch.Ten
     c * tanh(s / c) before anything is taken off it; ``shared``: the rows hold keys alone, which are the values too.
 
     ``tiles_wide`` (as ``tiles``, in runs of up to 128 tokens) lets the step take the tcgen05 kernel where it fits
-    (``mapped_tc_ok``) and pays (``wide_tiles_pay``); ``head_sink`` (float32, one per head; that kernel only): the sink's score, not scaled."""
+    (``mapped_tc_ok``); ``head_sink`` (float32, one per head; that kernel only): the sink's score, not scaled."""
     _need_cuda(q, rows, block_table, tok_pos, tok_seq, out, head_scale, gate, slopes)
     if slopes is not None and (slopes.dtype != torch.float32 or slopes.numel() != n_heads or not slopes.is_contiguous()):
         raise KernelError("mapped_attention: slopes are one contiguous float32 per head")
@@ -635,8 +625,6 @@ def mapped_attention(q: torch.Tensor, rows: torch.Tensor, block_table: torch.Ten
     if (tensor_cores and tiles_wide is not None and rows.dtype == torch.bfloat16
             and mapped_tc_ok(q, out, n_kv_heads, maps, dim, vdim, page_tokens, shared)
             and not (gate_each and (gate.stride(0) % 2 or gate.data_ptr() % 4))):
-            and (tiles is None or head_sink is not None
-                 or wide_tiles_pay(tiles.shape[0], tiles_wide.shape[0], n_heads, sm_count(q.device)))
         _need_cuda(tiles_wide, head_sink)
         _i32(tiles_wide, "tiles_wide")
         _check(library().mu_mapped_attention_tc(
@@ -761,20 +749,14 @@ def selective_scan_max_state() -> int:
 
 def selective_scan(x: torch.Tensor, z: torch.Tensor, dt: torch.Tensor, bc: torch.Tensor, b_at: int, c_at: int,
                    rates: torch.Tensor, skip: torch.Tensor, seq_first, seq_slots, state: torch.Tensor, state_offset: int,
-                   out: torch.Tensor, max_len: int = 0, workspace=None, lens=None) -> torch.Tensor:
+                   out: torch.Tensor, max_len: int = 0, workspace=None) -> torch.Tensor:
     """The recurrence S[c, n] = 2^(dt_c rates[c, n]) S[c, n] + dt_c x_c B_n, out_c = (sum_n S[c, n] C_n + skip_c x_c) silu(z_c)
     over the step's tokens of each sequence, from and to ``state[slot][state_offset:]`` (channels x N float32).  ``x``, ``z``
     and ``out`` [T, channels] in the compute dtype, ``dt`` float32; B and C are the columns of the float32 rows ``bc`` from
     ``b_at`` and ``c_at`` on, each followed by filling up to a multiple of four.  ``max_len``: the tokens that the longest
-    sequence brings, if the caller knows, and ``lens`` those of every one (host integers; None: all as long); few long
-    sequences then go in segments that work at once, which need room (``workspace`` as for ``ssd_scan_chunks``)."""
+    sequence brings, if the caller knows; few long sequences then go in segments that work at once, which need room
+    (``workspace`` as for ``ssd_scan_chunks``)."""
     _need_cuda(x, z, dt, bc, rates, skip, seq_first, seq_slots, state, out)
-@functools.lru_cache(maxsize=None)
-def _selective_sizes():
-    """(tokens of a segment, tokens of the longest sequence up to which nothing is cut)."""
-    return int(library().mu_selective_scan_segment()), int(library().mu_selective_scan_least())
-
-
     _i32(seq_first, "seq_first"); _i32(seq_slots, "seq_slots")
     T, inner = x.shape
     N = rates.shape[1]
@@ -790,10 +772,8 @@ def _selective_sizes():
         raise KernelError("selective_scan: step sizes, B and C, rates or state do not fit")
     lib, n_seqs = library(), seq_slots.numel()
     long_steps, segments, room = T > 4 * n_seqs, 1, None
-    if long_steps and max_len > _selective_sizes()[1]:
-        most = _selective_sizes()[0]
-        again = sum((n - 1) // most for n in lens if n) if lens is not None else n_seqs * ((max_len - 1) // most)
-        segments = lib.mu_selective_scan_segments(inner, N, int(max_len), again)
+    if long_steps and max_len > 512:                         # (two segments never pay)
+        segments = lib.mu_selective_scan_segments(n_seqs, inner, N, int(max_len))
     if segments > 1:
         lib.mu_selective_scan_scratch.restype = _c_ll
         room = _room(workspace, "selective_scan", x.device, int(lib.mu_selective_scan_scratch(n_seqs, segments, inner, N)))
@@ -1434,9 +1414,7 @@ def heads_gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, x_head_strid
             and x.stride(0) % 8 == 0 and x_head_stride % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
             and x.stride(1) == 1 and out.stride(1) == 1):
         fused = gate is not None and gate.dtype == torch.bfloat16 and gate.stride(1) == 1 and gate.shape == out.shape
-        rows, width = x.shape
-        if (2 * rows * heads * n * k >= HEADS_TC_FLOP and rows > 64 and k % 64 == 0
-                and x.stride(0) >= width >= (heads - 1) * x_head_stride + k):     # (rows that overlap have no tensor map)
+        if 2 * x.shape[0] * heads * n * k >= HEADS_TC_FLOP and x.shape[0] > 64 and k % 64 == 0 and x.shape[1] >= (heads - 1) * x_head_stride + k:
             _check(library().mu_heads_gemm_tc(_ptr(x), x.shape[1], x.stride(0), int(x_head_stride), _ptr(w), x.shape[0], heads,
                                               n, k, _ptr(out), out.stride(0), int(out_head_stride), _is_bf16(out),
                                               _ptr(gate) if fused else None, gate.stride(0) if fused else 0,
