@@ -551,6 +551,14 @@ def mapped_tc_ok(q: torch.Tensor, out: torch.Tensor, n_kv_heads: int, maps: int,
             and _mapped_tc_fits(int(n_kv_heads), int(maps), int(dim), int(vdim), int(page_tokens), int(shared)))
 
 
+def wide_tiles_pay(n_tiles: int, n_wide: int, n_heads: int, sms: int) -> bool:
+    """Whether a prompt step takes tiles of 128 queries on tcgen05 instead of tiles of 64 on ``mma.sync``.  A wide tile has an
+    SM to itself; while every one finds an SM it is the faster form from two tokens on (single layers on the device, 1 to 16
+    sequences of 2 to 1,000 tokens: 1.08 to 2.3 times).  Where they outnumber the SMs it wins if it halves the tiles (64 sequences of 65
+    tokens, 8 heads: 126.6 us against 100.3) and loses if no sequence has more than 64 tokens (64 of 17: 47.1 against 56.9)."""
+    return n_wide * n_heads <= sms or 2 * n_tiles >= 3 * n_wide
+
+
 @functools.lru_cache(maxsize=None)
 def _mapped_tc_fits(*sizes) -> bool:
     return bool(library().mu_mapped_attention_tc_fits(*sizes))
@@ -582,7 +590,7 @@ def mapped_attention(q: torch.Tensor, rows: torch.Tensor, block_table: torch.Ten
     c * tanh(s / c) before anything is taken off it; ``shared``: the rows hold keys alone, which are the values too.
 
     ``tiles_wide`` (as ``tiles``, in runs of up to 128 tokens) lets the step take the tcgen05 kernel where it fits
-    (``mapped_tc_ok``); ``head_sink`` (float32, one per head; that kernel only): the sink's score, not scaled."""
+    (``mapped_tc_ok``) and pays (``wide_tiles_pay``); ``head_sink`` (float32, one per head; that kernel only): the sink's score, not scaled."""
     _need_cuda(q, rows, block_table, tok_pos, tok_seq, out, head_scale, gate, slopes)
     if slopes is not None and (slopes.dtype != torch.float32 or slopes.numel() != n_heads or not slopes.is_contiguous()):
         raise KernelError("mapped_attention: slopes are one contiguous float32 per head")
@@ -623,6 +631,8 @@ def mapped_attention(q: torch.Tensor, rows: torch.Tensor, block_table: torch.Ten
     if head_sink is not None and (head_sink.dtype != torch.float32 or head_sink.numel() != n_heads or not head_sink.is_contiguous()):
         raise KernelError("mapped_attention: head_sink is one contiguous float32 per head")
     if (tensor_cores and tiles_wide is not None and rows.dtype == torch.bfloat16
+            and (tiles is None or head_sink is not None
+                 or wide_tiles_pay(tiles.shape[0], tiles_wide.shape[0], n_heads, sm_count(q.device)))
             and mapped_tc_ok(q, out, n_kv_heads, maps, dim, vdim, page_tokens, shared)
             and not (gate_each and (gate.stride(0) % 2 or gate.data_ptr() % 4))):
         _need_cuda(tiles_wide, head_sink)

@@ -114,6 +114,30 @@ def test_mapped_attention_on_tcgen05(c):
     assert float(worst[bad]) < 1.0, f"{float(worst[bad]):.2f} of the bound at token {bad} (sequence {tok_seq[bad]}, position {tok_pos[bad]})"
 
 
+# (sequences, tokens each): as many wide tiles as SMs, one sequence more, and as many of more than 64 tokens
+@pytest.mark.parametrize("seqs,n,wide", [(18, 17, True), (19, 17, False), (19, 65, True), (64, 64, False)])
+def test_short_sequences_keep_tiles_of_64(seqs, n, wide, monkeypatch):
+    """Which kernel a step of 8 heads takes on 148 SMs, by its launch; results as from the other, each rounded once."""
+    from math_utils_b200.csrc import ops
+    H, G, dim = 8, 2, 64
+    monkeypatch.setattr(ops, "sm_count", lambda device: 148)
+    took, check = [], ops._check
+    monkeypatch.setattr(ops, "_check", lambda code, what, *a, **k: (took.append(str(what)), check(code, what, *a, **k))[1])
+    pages = -(-n // 64)
+    rows, q = _rand((seqs * pages, 64, 2 * G * dim), 1), _rand((seqs * n, H * dim), 2)
+    table = _ints(np.arange(seqs * pages).reshape(seqs, pages))
+    tiles = {w: _ints([(s * n + o, min(w, n - o)) for s in range(seqs) for o in range(0, n, w)]) for w in (64, 128)}
+    pos, seq, outs = _ints(np.tile(np.arange(n), seqs)), _ints(np.repeat(np.arange(seqs), n)), []
+    for given in ({"tiles": tiles[64], "tiles_wide": tiles[128]}, {"tiles_wide" if not wide else "tiles": tiles[128 if not wide else 64]}):
+        out = torch.zeros((seqs * n, H * dim), device="cuda", dtype=torch.bfloat16)
+        ops.mapped_attention(q, rows, table, 64, pos, seq, H, G, 1, dim, dim, dim ** -0.5, 0, out, **given)
+        outs.append(out.double())
+    ops.check_status()
+    assert ["attention_tc" in t for t in took] == [wide, not wide]
+    bound = 2.0 ** -7 * outs[1].abs() + 2.0 ** -8 * outs[1].square().mean(1, keepdim=True).sqrt() + 1e-6
+    assert float(((outs[0] - outs[1]).abs() / bound).max()) < 1.0
+
+
 @pytest.mark.parametrize("bad", [float("nan"), float("inf")])
 @pytest.mark.parametrize("c", [CASES[i] for i in (0, 1, 3, 8, 9, 10, 11)], ids=lambda c: "-".join(f"{k}{v}" for k, v in c.items() if v))
 def test_values_that_are_not_finite_stay_with_the_queries_that_see_them(c, bad):
