@@ -546,7 +546,7 @@ def qk_prepare(q: torch.Tensor, k: Optional[torch.Tensor], v: Optional[torch.Ten
 def mapped_tc_ok(q: torch.Tensor, out: torch.Tensor, n_kv_heads: int, maps: int, dim: int, vdim: int, page_tokens: int,
                  shared: bool = False) -> bool:
     """Whether ``mapped_attention`` takes the tcgen05 kernel for these queries (bfloat16 rows given wide tiles)."""
-    return (MAPPED_TC and q.dtype == torch.bfloat16 and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0
+    return (MAPPED_TC and q.dtype == torch.bfloat16 and q.stride(0) % 8 == 0 and q.stride(0) >= q.shape[1] and q.data_ptr() % 16 == 0
             and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0
             and _mapped_tc_fits(int(n_kv_heads), int(maps), int(dim), int(vdim), int(page_tokens), int(shared)))
 

@@ -171,6 +171,20 @@ def test_values_that_are_not_finite_stay_with_the_queries_that_see_them(c, bad):
     assert torch.isfinite(got).all() and float(((got - want).abs() / bound).max()) < 1.0
 
 
+def test_one_query_row_for_all_tokens():
+    """Queries with a stride of zero have no tensor map: the other kernels take them, given wide tiles or not."""
+    from math_utils_b200.csrc import ops
+    n, H, dim = 130, 2, 64
+    rows, q, outs = _rand((3, 64, 2 * H * dim), 1), _rand((1, H * dim), 2), []
+    for x in (q.expand(n, H * dim), q.repeat(n, 1)):
+        out = torch.zeros((n, H * dim), device="cuda", dtype=torch.bfloat16)
+        ops.mapped_attention(x, rows, _ints([range(3)]), 64, _ints(range(n)), _ints([0] * n), H, H, 1, dim, dim, 0.1, 0, out,
+                             tiles=_ints([(0, 64), (64, 64), (128, 2)]), tiles_wide=_ints([(0, 128), (128, 2)]))
+        outs.append(out.double())
+    bound = 2.0 ** -7 * outs[1].abs() + 2.0 ** -8 * outs[1].square().mean(1, keepdim=True).sqrt()
+    assert float(((outs[0] - outs[1]).abs() / bound).max()) < 1.0
+
+
 def test_expanded_values_that_are_not_finite_stay_with_the_queries_that_see_them():
     from math_utils_b200.csrc import ops
     H, dim, rot, vdim, n, at = 2, 64, 32, 48, 300, 130
