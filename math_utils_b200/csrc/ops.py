@@ -1424,7 +1424,9 @@ def heads_gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, x_head_strid
             and x.stride(0) % 8 == 0 and x_head_stride % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
             and x.stride(1) == 1 and out.stride(1) == 1):
         fused = gate is not None and gate.dtype == torch.bfloat16 and gate.stride(1) == 1 and gate.shape == out.shape
-        if 2 * x.shape[0] * heads * n * k >= HEADS_TC_FLOP and x.shape[0] > 64 and k % 64 == 0 and x.shape[1] >= (heads - 1) * x_head_stride + k:
+        rows, width = x.shape
+        if (2 * rows * heads * n * k >= HEADS_TC_FLOP and rows > 64 and k % 64 == 0
+                and x.stride(0) >= width >= (heads - 1) * x_head_stride + k):     # (rows that overlap have no tensor map)
             _check(library().mu_heads_gemm_tc(_ptr(x), x.shape[1], x.stride(0), int(x_head_stride), _ptr(w), x.shape[0], heads,
                                               n, k, _ptr(out), out.stride(0), int(out_head_stride), _is_bf16(out),
                                               _ptr(gate) if fused else None, gate.stride(0) if fused else 0,

@@ -137,6 +137,19 @@ def test_products_per_head_see_their_own_slice_alone(n, k, lead, monkeypatch):
     assert torch.equal(outs[0][:, 0], outs[1][:, 0]) and torch.equal(outs[0][:, 2], outs[1][:, 2])
 
 
+def test_products_per_head_of_rows_that_overlap(monkeypatch):
+    """One row for all (a stride of zero), and rows that begin inside the row before: the kernel without tensor maps takes them."""
+    ops = _ops()
+    monkeypatch.setattr(ops, "HEADS_TC_FLOP", 0.0)
+    heads, n, k = 2, 64, 64
+    w, flat = _rand((heads, n, k), 2, torch.bfloat16, k ** -0.5), _rand((130 * 64 + heads * k,), 1, torch.bfloat16)
+    for x in (flat[:heads * k].expand(130, heads * k), flat.as_strided((130, heads * k), (64, 1))):
+        out = torch.zeros((130, heads * n), device="cuda")
+        ops.heads_gemm(x, w, out, k, n)
+        want = torch.einsum("thk,hnk->thn", x.double().reshape(130, heads, k), w.double()).reshape(130, -1)
+        assert float((out.double() - want).abs().max() / want.square().mean().sqrt()) < 1e-4
+
+
 # one block of 128 threads, of 1024, pairs beyond those it keeps in registers; identity experts; more experts than a warp
 @pytest.mark.parametrize("P,experts,real", [(1, 4, 4), (48, 72, 64), (256, 33, 33), (257, 5, 4), (12288, 64, 64), (20001, 70, 64)])
 @pytest.mark.parametrize("rows", [32, 128])
