@@ -67,10 +67,19 @@ class MatrixLstm(Mixer):
         self.chunked = runtime.dtype == torch.bfloat16 and runtime.ops.chunk_scan_ok(self.dim, self.vdim)
         self.i_bias, self.f_bias, self.norm_weight = t("i_bias"), t("f_bias"), t("norm")
 
-    # Tokens of the longest sequence from which on the chunked form pays: token by token a step takes as long as its longest
-    # sequence, in chunks two launches more (4 x 64 tokens: 58 us against 66, the host's time either way).
-    # 8 heads of 128 x 128: 2,000 tokens of one sequence 340 us token by token, 163 in chunks; 1 x 400 81 and 84, 4 x 500 147 both.
-    CHUNKED_TOKENS = 448
+    # Which form a prompt step takes goes by load: token by token it takes as long as its longest sequence while the blocks find
+    # room on the SMs, in chunks as long as all its tokens together, and two launches more.  Measured (the layer on the
+    # device, us, token by token and in chunks; heads of 128 x 128 unless said):
+    #   8 heads, 1 x 400 tokens 78 and 81, 1 x 512 91 and 80, 1 x 2,000 332 and 172, 4 x 512 143 and 146, 4 x 1,000 267 and 254,
+    #   6 x 512 191 and 209, 8 x 1,000 437 and 454, 16 x 512 419 and 448;  4 heads, 8 x 1,000 269 and 258, 16 x 512 237 and 249;
+    #   16 heads of 64 x 64, 4 x 512 144 and 125, 8 x 512 215 and 217, 8 x 2,000 763 and 757.
+    CHUNKED_TOKENS = 448             # of the longest sequence, at least
+    CHUNKED_LAUNCHES = 333           # tokens of it that the launches cost
+    CHUNKED_WORK = 1e6               # state entries moved over in the time that a token of it takes
+
+    def in_chunks(self, longest: int, tokens: int) -> bool:
+        return (longest >= self.CHUNKED_TOKENS
+                and (longest - self.CHUNKED_LAUNCHES) * self.CHUNKED_WORK >= self.n_heads * self.dim * self.vdim * tokens)
 
     def forward(self, h, residual, ctx, cache, owns_cache: bool, accumulate: bool = True) -> None:
         ops, T, H = self.runtime.ops, ctx.n_tokens, self.n_heads
@@ -84,7 +93,7 @@ class MatrixLstm(Mixer):
                       self.m_offset, gates)
         o = ctx.buffer("mlstm.o", (T, self.inner), torch.float32)
         read = ctx.buffer("mlstm.normalizer", (T, H), torch.float32)
-        if self.chunked and ctx.q_tiles is not None and ctx.max_q_len >= self.CHUNKED_TOKENS:
+        if self.chunked and ctx.q_tiles is not None and self.in_chunks(ctx.max_q_len, T):
             ops.linear_scan_chunks(q, k, v, gates, H, self.dim, self.vdim, self.dim ** -0.5, ctx.q_tiles, ctx.tok_seq,
                                    ctx.seq_first, ctx.seq_slots, cache.values, 0, o, norm_out=read, workspace=ctx.scratch)
         else:
