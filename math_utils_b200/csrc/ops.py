@@ -132,7 +132,9 @@ _SIGNATURES = {
                     _c_int, _c_p, _c_p, _c_int],
     "mu_selective_scan_max_state": [],
     "mu_selective_scan_scratch": [_c_int] * 4,
-    "mu_selective_scan_segments": [_c_int] * 4,
+    "mu_selective_scan_segment": [],
+    "mu_selective_scan_least": [],
+    "mu_selective_scan_segments": [_c_int] * 3 + [_c_ll],
     "mu_selective_scan": [_c_p, _c_ll, _c_p, _c_ll, _c_p, _c_ll, _c_p, _c_ll, _c_int, _c_int, _c_p, _c_p, _c_int, _c_int, _c_int,
                           _c_p, _c_p, _c_p, _c_ll, _c_ll, _c_p, _c_ll, _c_int, _c_int, _c_p, _c_int, _c_p],
     "mu_ssd_scan": [_c_p, _c_int, _c_p, _c_ll, _c_int, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_p,
@@ -753,19 +755,25 @@ def ssd_scan_chunks(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias, a_log, ski
     return out
 
 
+@functools.lru_cache(maxsize=None)
+def _selective_sizes():
+    """(tokens of a segment, tokens of the longest sequence up to which nothing is cut)."""
+    return int(library().mu_selective_scan_segment()), int(library().mu_selective_scan_least())
+
+
 def selective_scan_max_state() -> int:
     return int(library().mu_selective_scan_max_state())
 
 
 def selective_scan(x: torch.Tensor, z: torch.Tensor, dt: torch.Tensor, bc: torch.Tensor, b_at: int, c_at: int,
                    rates: torch.Tensor, skip: torch.Tensor, seq_first, seq_slots, state: torch.Tensor, state_offset: int,
-                   out: torch.Tensor, max_len: int = 0, workspace=None) -> torch.Tensor:
+                   out: torch.Tensor, max_len: int = 0, workspace=None, lens=None) -> torch.Tensor:
     """The recurrence S[c, n] = 2^(dt_c rates[c, n]) S[c, n] + dt_c x_c B_n, out_c = (sum_n S[c, n] C_n + skip_c x_c) silu(z_c)
     over the step's tokens of each sequence, from and to ``state[slot][state_offset:]`` (channels x N float32).  ``x``, ``z``
     and ``out`` [T, channels] in the compute dtype, ``dt`` float32; B and C are the columns of the float32 rows ``bc`` from
     ``b_at`` and ``c_at`` on, each followed by filling up to a multiple of four.  ``max_len``: the tokens that the longest
-    sequence brings, if the caller knows; few long sequences then go in segments that work at once, which need room
-    (``workspace`` as for ``ssd_scan_chunks``)."""
+    sequence brings, if the caller knows, and ``lens`` those of every one (host integers; None: all as long); few long
+    sequences then go in segments that work at once, which need room (``workspace`` as for ``ssd_scan_chunks``)."""
     _need_cuda(x, z, dt, bc, rates, skip, seq_first, seq_slots, state, out)
     _i32(seq_first, "seq_first"); _i32(seq_slots, "seq_slots")
     T, inner = x.shape
@@ -782,8 +790,10 @@ def selective_scan(x: torch.Tensor, z: torch.Tensor, dt: torch.Tensor, bc: torch
         raise KernelError("selective_scan: step sizes, B and C, rates or state do not fit")
     lib, n_seqs = library(), seq_slots.numel()
     long_steps, segments, room = T > 4 * n_seqs, 1, None
-    if long_steps and max_len > 512:                         # (two segments never pay)
-        segments = lib.mu_selective_scan_segments(n_seqs, inner, N, int(max_len))
+    if long_steps and max_len > _selective_sizes()[1]:
+        most = _selective_sizes()[0]
+        again = sum((n - 1) // most for n in lens if n) if lens is not None else n_seqs * ((max_len - 1) // most)
+        segments = lib.mu_selective_scan_segments(inner, N, int(max_len), again)
     if segments > 1:
         lib.mu_selective_scan_scratch.restype = _c_ll
         room = _room(workspace, "selective_scan", x.device, int(lib.mu_selective_scan_scratch(n_seqs, segments, inner, N)))

@@ -267,15 +267,21 @@ MU_EXPORT long long mu_selective_scan_scratch(int n_seqs, int segments, int inne
     return (long long)n_seqs * segments * inner * (((N + 1) & ~1) + 1);
 }
 
-// Segments of a long step's longest sequence, 1 where the scan goes whole.  They make the exponentials almost twice and pay
-// where the scan alone leaves the SMs with little to do for long.  The mixer around it, 2,048 channels: one sequence (fewer
-// blocks than SMs) of 900 tokens 126 us whole, 108 in segments, of 300 tokens 79 and 95; 2 x 900 tokens 150 and 155, up to
-// 1,000 tokens of 3 sequences 169 and 160; 4 x 500 tokens (3.5 blocks an SM) 134 and 154.
-MU_EXPORT int mu_selective_scan_segments(int n_seqs, int inner, int N, int max_len) {
+// Tokens of a segment, and of the longest sequence that the segments' second launch costs: up to so many nothing is cut.
+MU_EXPORT int mu_selective_scan_segment() { return mu::SS_SEGMENT; }
+MU_EXPORT int mu_selective_scan_least() { return 655; }
+
+// Segments of a long step's longest sequence, 1 where the scan goes whole; again: segments of all sequences but each one's last,
+// which are scanned twice.  Whole, a step takes as long as its longest sequence; in segments the SMs share the work evenly, and
+// every segment that a block scans again costs an SM as much as some 66 tokens of that sequence.  Measured (the mixer on the device, us,
+// whole and in segments, 275 steps): 2,048 channels, 1 x 800 tokens 116 and 118, 1 x 1,000 131 and 120, 2 x 1,000 150 and 150,
+// 2 x 1,500 219 and 192, 3 x 1,000 183 and 191, 3 x 2,000 340 and 320, 4 x 2,000 379 and 392, 1,000 + 83 + 900 155 and 149, 1,000 +
+// 500 + 2 x 250 172 and 147; 256 channels, 8 x 768 103 and 109, 8 x 1,000 120 and 113; 4,096 channels, 1 x 1,100 168 and 166,
+// 2 x 2,000 380 and 392.  By this rule no step of them is slower, all together take 0.4 % longer than each one's better form.
+MU_EXPORT int mu_selective_scan_segments(int inner, int N, int max_len, long long again) {
     const int lanes = N <= 8 ? 4 : N <= 16 ? 8 : N <= 32 ? 16 : 32;
-    const long long blocks = (long long)n_seqs * ((inner + mu::ss_channels(lanes) - 1) / mu::ss_channels(lanes));
-    const int sms = mu::sm_count();
-    if (blocks >= 3ll * sms || max_len < (blocks <= sms ? 640 : 960)) return 1;
+    const int blocks = (inner + mu::ss_channels(lanes) - 1) / mu::ss_channels(lanes), sms = mu::sm_count();
+    if (max_len <= mu_selective_scan_least() || (long long)(max_len - mu_selective_scan_least()) * sms < 66ll * blocks * again) return 1;
     return (max_len + mu::SS_SEGMENT - 1) / mu::SS_SEGMENT;
 }
 

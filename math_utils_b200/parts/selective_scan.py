@@ -88,7 +88,7 @@ class SelectiveScanMixer(Mixer):
         ops.low_rank(low, self.dt_up.dtype, ops.low_rank_part(self.dt_up, 0, dt, bias=self.dt_bias, fn="softplus"))
         y = ctx.buffer("selective.y", (T, C), dtype)
         ops.selective_scan(x, z, dt, low, self.b_at, self.c_at, self.rates, self.skip, ctx.seq_first, ctx.seq_slots,
-                           cache.values, self.tail_values, y, max_len=ctx.max_q_len, workspace=ctx.scratch)
+                           cache.values, self.tail_values, y, max_len=ctx.max_q_len, lens=ctx.q_lens, workspace=ctx.scratch)
         ctx.note("scan", y)
         self.out(y, residual=residual if accumulate else None, out=residual)
 

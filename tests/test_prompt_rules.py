@@ -16,3 +16,18 @@ def test_matrix_memory_in_chunks_by_load(heads, dim, lens, chunks):
     sizes = dict(hidden_size=512, n_heads=heads, dim=dim, vdim=dim, gate_cap=15.0, eps=1e-5)
     part = build_part("mixer", PartSpec("matrix_lstm", sizes, {}))
     assert part.in_chunks(max(lens), sum(lens)) == chunks
+
+
+# (channels, longest, segments scanned twice, whether cut) at 16 state entries a channel
+@pytest.mark.parametrize("inner,lens,cut", [
+    (2048, [800], False), (2048, [1000], True), (2048, [700], False), (2048, [1000] * 3, False), (2048, [2000] * 3, True),
+    (2048, [2000] * 4, False), (2048, [1000, 500, 250, 250], True), (2048, [1000, 83, 900], True), (256, [768] * 8, False),
+    (256, [1000] * 8, True), (512, [700], True), (4096, [2000] * 2, False), (1000, [800] * 2, False), (512, [655], False)])
+@pytest.mark.gpu
+def test_selective_scan_cut_by_load(inner, lens, cut):
+    from math_utils_b200.csrc import ops
+    if ops.sm_count("cuda:0") != 148:
+        pytest.skip("measured on 148 SMs")
+    tokens, least = ops._selective_sizes()
+    again = sum((n - 1) // tokens for n in lens)
+    assert (ops.library().mu_selective_scan_segments(inner, 16, max(lens), again) > 1) == cut
