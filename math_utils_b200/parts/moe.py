@@ -96,6 +96,9 @@ class RoutedExperts(FeedForward):
         self.gathered_pairs = -(-self.GATHERED_FLOP // (2 * weights))
         if 2 * weights * self.n_experts >= self.GATHERED_BYTES:                # (pairs meet as many experts at most)
             self.gathered_pairs = min(self.gathered_pairs, -(-self.GATHERED_BYTES // (2 * weights)))
+        items, sms = self.n_experts * -(-self.inner_size // 128), runtime.ops.sm_count(runtime.device)
+        if gated and sms < items < 1.5 * sms:                                  # (a tile an expert)
+            self.gathered_pairs = max(self.gathered_pairs, 96 * self.n_experts)
         self.shared_up = self.shared_down = self.shared_gate = None
         if self.shared_inner:
             from .linear import Linear
@@ -107,9 +110,12 @@ class RoutedExperts(FeedForward):
             if self.shared_gated:
                 self.shared_gate = tensors[name("shared_gate")].reshape(-1).contiguous()
 
-    # The gathered rows' product costs a launch more.  It pays from some 3 GFLOP on (16 experts of 1,024 x 704 x 3: 512 pairs
-    # 57 us either way, 4,000 pairs 122 us against 95) or with 400 MB of weights to read (48 pairs over 64 experts of 2,048 x
-    # 1,408 x 2: 136 us against 93; over 48 of 1,024 x 704 x 3: 71 against 78).
+    # The gathered rows' product costs a launch more, and a tile costs its weights whether it is full or not.  It pays from 3
+    # GFLOP on, or with 400 MB of weights to read (of 86 steps of either kind, eight sizes of experts, 2 to 6 choices, 1 to
+    # 1,000 tokens, two are slower by a hundredth and one by 4, the others up to 1.9 times faster; 16 experts of 1,024 x 704 x
+    # 3, 600 pairs: 62 us and 65, 900 pairs: 77 and 67; 64 of 2,048 x 1,408 x 2, 48 pairs: 112 and 71), but for gated experts
+    # whose tiles leave the second wave of items more than half empty: 48 of 768 x 512 x 3, 4 column blocks each, 1,320 pairs
+    # 65 us and 83, 3,000 pairs 86 and 96, 6,000 pairs 120 and 96.
     GATHERED_FLOP, GATHERED_BYTES = 3e9, 4e8
 
     fuses_output_norm = True           # forward(..., output_norm=): the norm of the result, added into the stream

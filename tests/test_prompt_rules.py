@@ -18,6 +18,26 @@ def test_matrix_memory_in_chunks_by_load(heads, dim, lens, chunks):
     assert part.in_chunks(max(lens), sum(lens)) == chunks
 
 
+@pytest.mark.parametrize("form,experts,width,inner,pairs,gathered", [
+    ("gated_silu", 48, 768, 512, 1320, False), ("gated_silu", 48, 768, 512, 3000, False), ("gated_silu", 48, 768, 512, 6000, True),
+    ("relu2", 48, 768, 512, 3000, True), ("gated_silu", 48, 1024, 704, 1800, True), ("gated_silu", 16, 512, 512, 3000, True),
+    ("relu2", 64, 2048, 1408, 48, True), ("gated_silu", 16, 1024, 704, 300, False)])
+def test_experts_rows_gathered_by_work(form, experts, width, inner, pairs, gathered):
+    import torch
+    names = {"router": "router", "up": "e{e}.up", "down": "e{e}.down", "gate": "e{e}.gate"}
+    sizes = dict(hidden_size=width, inner_size=inner, n_experts=experts, top=1, score="sigmoid", expert_form=form)
+    part = build_part("feed_forward", PartSpec("routed_experts", sizes, names))
+
+    class Runtime:
+        device, dtype = "cuda:0", torch.bfloat16
+
+        class ops:
+            moe_tile_rows, sm_count = staticmethod(lambda: 32), staticmethod(lambda device: 148)
+
+    part.bind({t.name: torch.empty(t.shape, dtype=torch.bfloat16, device="meta") for t in part.tensor_specs()}, Runtime)
+    assert (pairs >= part.gathered_pairs) == gathered
+
+
 # (channels, longest, segments scanned twice, whether cut) at 16 state entries a channel
 @pytest.mark.parametrize("inner,lens,cut", [
     (2048, [800], False), (2048, [1000], True), (2048, [700], False), (2048, [1000] * 3, False), (2048, [2000] * 3, True),
