@@ -305,7 +305,9 @@ latent_rows_kernel(const uint4* __restrict__ cache, const int* __restrict__ bloc
         int before = 0;
         for (int s0 = 0; s0 < n_seqs && before <= page; s0 += 32) {
             const int s = s0 + tid;
-            const int len = s < n_seqs ? tok_pos[seq_first[s + 1] - 1] + 1 : 0, mine = (len + 63) / 64;
+            // (one that brings no token attends to nothing)
+            const int end = s < n_seqs ? seq_first[s + 1] : 0, len = s < n_seqs && end > seq_first[s] ? tok_pos[end - 1] + 1 : 0;
+            const int mine = (len + 63) / 64;
             int upto = mine;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -381,7 +383,8 @@ MU_EXPORT int mu_latent_append(const void* dkv, long long ld, const float* norm_
 // For prompt steps whose keys and values are expanded (every position that the step's sequences hold, their pages one after
 // another, a sequence's on a page of its own): latents [n_pages * 64][kv_rank] receives the cached latents, rows
 // [n_pages * 64][width] the shared rotated part at column rot_at, both zeros past a sequence's end, and table [n_seqs]
-// [max_pages_out] the pages' numbers.  seq_first: the step's flat tokens per sequence, the last of each at its sequence's end.
+// [max_pages_out] the pages' numbers.  seq_first: the step's flat tokens per sequence, the last of each at its sequence's end; a sequence without tokens
+// of the step has no pages here.
 MU_EXPORT int mu_latent_rows(const void* cache, const int* block_table, int max_pages, const int* tok_pos, const int* seq_first,
                              int n_seqs, int n_pages, int kv_rank, int rot_dim, void* latents, void* rows, int width, int rot_at,
                              int* table, int max_pages_out, void* stream) {

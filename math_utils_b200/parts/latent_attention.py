@@ -173,7 +173,7 @@ class LatentAttention(Mixer):
             return False
         held = met = 0
         for start, n in zip(ctx.starts, ctx.q_lens):
-            held += start + n
+            held += start + n if n else 0
             met += n * (2 * start + n)                       # (twice the pairs of tokens and keys)
         return held <= self.EXPANDED_PER_TOKEN * ctx.n_tokens and met * each >= self.EXPANDED_FLOP
 
@@ -184,7 +184,7 @@ class LatentAttention(Mixer):
         ops.latent_append(views[self.at["dkv"]] if owns_cache else None, self.norm_weight, self.eps, self.freq_table,
                           self.magnitude, self.rot_dims, r, self.rot_dim, ctx.tok_pos, ctx.tok_seq, table, cache.page_tokens,
                           cache.pages, queries=rotated, pairs=self.rot_layout == "pairs")
-        pages = [-(-(start + n) // 64) for start, n in zip(ctx.starts, ctx.q_lens)]
+        pages = [-(-(start + n) // 64) if n else 0 for start, n in zip(ctx.starts, ctx.q_lens)]
         n_pages, both = sum(pages), H * (self.dim + self.vdim)
         latents = ctx.buffer("latent.held", (n_pages * 64, r), dt)
         rows = ctx.buffer("latent.rows", (n_pages, 64, both + self.rot_dim), dt)

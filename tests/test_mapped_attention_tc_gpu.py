@@ -263,3 +263,12 @@ def test_latent_prompts_over_expanded_rows(H, dim, rot, vdim, rank, q_rank, layo
         assert torch.isfinite(a).all()
         off = (a - b).double().square().mean(1).sqrt() / b.double().square().mean().sqrt()
         assert float(off.max()) < 0.05 and float(off.square().mean().sqrt()) < 0.012
+
+
+def test_latent_prompt_steps_with_sequences_that_bring_nothing(monkeypatch):
+    """Pages are counted for the sequences that attend: the same bits with a sequence without tokens before or between."""
+    part = _latent_part(*LATENTS[0])
+    want, _ = _latent_steps(part, [[70, 200, 0], [40, 100, 0]], monkeypatch)
+    for steps in ([[0, 70, 200], [0, 40, 100]], [[70, 0, 200], [40, 0, 100]]):
+        found, runs = _latent_steps(part, steps, monkeypatch)
+        assert runs == [(1, 1)] * 2 and all(torch.equal(a, b) for a, b in zip(found, want))
