@@ -722,10 +722,24 @@ def _room(workspace, name: str, device, numel: int) -> torch.Tensor:
     return workspace(name, numel) if workspace is not None else torch.empty(numel, dtype=torch.float32, device=device)
 
 
+# Bytes that a layer's prompt step may take beside its activations for a form that is faster but needs room (chunks' states,
+# segments' ends, expanded rows); a step that would need more takes the form without.  64k tokens of 8 heads of 128 x 128.
+STEP_ROOM = 1 << 29
+
+
 def _chunk_scratch(workspace, device, n_tokens: int, n_seqs: int, n_heads: int, dk: int, dv: int) -> torch.Tensor:
+    return _room(workspace, "chunk_scan", device, _chunk_floats(n_tokens, n_seqs, n_heads, dk, dv))
+
+
+def _chunk_floats(n_tokens: int, n_seqs: int, n_heads: int, dk: int, dv: int) -> int:
     lib = library()
     lib.mu_chunk_scan_scratch.restype = _c_ll
-    return _room(workspace, "chunk_scan", device, int(lib.mu_chunk_scan_scratch(n_tokens, n_seqs, n_heads, dk, dv)))
+    return int(lib.mu_chunk_scan_scratch(n_tokens, n_seqs, n_heads, dk, dv))
+
+
+def chunk_scan_room_ok(n_tokens: int, n_seqs: int, n_heads: int, dk: int, dv: int) -> bool:
+    """Whether a step of these sizes finds the room that ``linear_scan_chunks`` and ``ssd_scan_chunks`` need."""
+    return 4 * _chunk_floats(n_tokens, n_seqs, n_heads, dk, dv) <= STEP_ROOM
 
 
 def ssd_scan_chunks(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias, a_log, skip, n_heads: int, head_dim: int, n_state: int,
@@ -796,7 +810,11 @@ def selective_scan(x: torch.Tensor, z: torch.Tensor, dt: torch.Tensor, bc: torch
         segments = lib.mu_selective_scan_segments(inner, N, int(max_len), again)
     if segments > 1:
         lib.mu_selective_scan_scratch.restype = _c_ll
-        room = _room(workspace, "selective_scan", x.device, int(lib.mu_selective_scan_scratch(n_seqs, segments, inner, N)))
+        floats = int(lib.mu_selective_scan_scratch(n_seqs, segments, inner, N))
+        if 4 * floats <= STEP_ROOM:
+            room = _room(workspace, "selective_scan", x.device, floats)
+        else:
+            segments = 1
     _check(lib.mu_selective_scan(_ptr(x), x.stride(0), _ptr(z), z.stride(0), _ptr(dt), dt.stride(0), _ptr(bc), bc.stride(0),
                                        int(b_at), int(c_at), _ptr(rates), _ptr(skip), seq_slots.numel(), inner, N,
                                        _ptr(seq_first), _ptr(seq_slots), _ptr(state), state.stride(0), int(state_offset),

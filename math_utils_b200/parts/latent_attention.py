@@ -175,7 +175,9 @@ class LatentAttention(Mixer):
         for start, n in zip(ctx.starts, ctx.q_lens):
             held += start + n if n else 0
             met += n * (2 * start + n)                       # (twice the pairs of tokens and keys)
-        return held <= self.EXPANDED_PER_TOKEN * ctx.n_tokens and met * each >= self.EXPANDED_FLOP
+        row = self.n_heads * (self.dim + self.vdim) + self.kv_rank + self.rot_dim
+        return (held <= self.EXPANDED_PER_TOKEN * ctx.n_tokens and met * each >= self.EXPANDED_FLOP
+                and 2 * (held + 64 * ctx.n_seqs) * row <= self.runtime.ops.STEP_ROOM)
 
     def _prompt(self, q, views, gate, residual, ctx, cache, owns_cache, accumulate, table) -> None:
         ops, dt = self.runtime.ops, self.runtime.dtype

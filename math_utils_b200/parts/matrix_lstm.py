@@ -93,7 +93,8 @@ class MatrixLstm(Mixer):
                       self.m_offset, gates)
         o = ctx.buffer("mlstm.o", (T, self.inner), torch.float32)
         read = ctx.buffer("mlstm.normalizer", (T, H), torch.float32)
-        if self.chunked and ctx.q_tiles is not None and self.in_chunks(ctx.max_q_len, T):
+        if (self.chunked and ctx.q_tiles is not None and self.in_chunks(ctx.max_q_len, T)
+                and ops.chunk_scan_room_ok(T, ctx.n_seqs, H, self.dim, self.vdim)):
             ops.linear_scan_chunks(q, k, v, gates, H, self.dim, self.vdim, self.dim ** -0.5, ctx.q_tiles, ctx.tok_seq,
                                    ctx.seq_first, ctx.seq_slots, cache.values, 0, o, norm_out=read, workspace=ctx.scratch)
         else:

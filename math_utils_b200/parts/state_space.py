@@ -84,7 +84,8 @@ class StateSpaceMixer(Mixer):
                      ctx.is_decode, xbc)
         y = ctx.buffer("ssd.y", (T, inner), torch.float32)
         recurrence = (xbc, dt_raw, self.dt_bias, self.a_log, self.skip, self.n_heads, self.head_dim, self.state, self.groups)
-        if self.chunked and ctx.q_tiles is not None and ctx.max_q_len >= self.CHUNKED_TOKENS:
+        if (self.chunked and ctx.q_tiles is not None and ctx.max_q_len >= self.CHUNKED_TOKENS
+                and ops.chunk_scan_room_ok(T, ctx.n_seqs, self.n_heads, self.state, self.head_dim)):
             ops.ssd_scan_chunks(*recurrence, ctx.q_tiles, ctx.tok_seq, ctx.seq_first, ctx.seq_slots, cache.values,
                                 self.tail_values, y, workspace=ctx.scratch)
         else:

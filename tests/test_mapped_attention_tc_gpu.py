@@ -272,3 +272,9 @@ def test_latent_prompt_steps_with_sequences_that_bring_nothing(monkeypatch):
     for steps in ([[0, 70, 200], [0, 40, 100]], [[70, 0, 200], [40, 0, 100]]):
         found, runs = _latent_steps(part, steps, monkeypatch)
         assert runs == [(1, 1)] * 2 and all(torch.equal(a, b) for a, b in zip(found, want))
+
+
+def test_latent_prompt_steps_without_room_stay_in_latent_space(monkeypatch):
+    part = _latent_part(*LATENTS[0])
+    monkeypatch.setattr(part.runtime.ops, "STEP_ROOM", 2 * (200 + 64 * 3) * (4 * 128 + 256 + 32) - 1)
+    assert _latent_steps(part, [[70, 0, 129], [0, 0, 72]], monkeypatch)[1] == [(1, 1), (0, 0)]
