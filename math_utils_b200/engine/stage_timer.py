@@ -17,7 +17,7 @@ import torch
 STAGE_NAMES = OrderedDict([
     ("embed", "embedding"), ("ln1", "norm 1"), ("qkv", "q | k | v product"),
     ("proj", "queries | gate | latent product"), ("q_latent", "cache append, queries into latent space, rotation"),
-    ("mixed", "attention over latent rows"),
+    ("mixed", "attention over latent rows"), ("kv", "keys and values expanded from latent rows"),
     ("q", "q | k | v product, query/key norm, rotation, cache append"),
     ("scan", "state-space input product, convolution, scan"), ("attn", "attention / gated norm of the scan"),
     ("res1", "output projection"), ("ln2", "norm 2"), ("route", "router and grouping"), ("act", "feed-forward up"), ("res2", "feed-forward down"),

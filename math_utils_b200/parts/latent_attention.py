@@ -10,7 +10,8 @@ rotated key part (rot_dim values).  With k_h = U_h c and v_h = V_h c the score o
     (q_h^n . U_h c + q_h^r . k^r) * scale = ((U_h^T q_h^n) . c + q_h^r . k^r) * scale
 and the head's output V_h (sum_j p_j c_j), so the attention itself runs in latent space over the
 cached rows, the same rows for every head, and the two up-projections become products per head before
-and after it: keys and values are never expanded.  An output gate sigmoid(G h) multiplies the
+and after it: keys and values are not expanded, but in long prompt steps in bfloat16, where expanding them once a
+step is less work than meeting 2 kv_rank + rot_dim entries a key (``_expands``).  An output gate sigmoid(G h) multiplies the
 concatenated heads before the output projection.
 
 Switches for other designs, each with its constants: ``q_rank`` r_q > 0 sends the queries through a latent of
@@ -116,7 +117,7 @@ class LatentAttention(Mixer):
 
     def forward(self, h, residual, ctx, cache, owns_cache: bool, accumulate: bool = True) -> None:
         ops, dt = self.runtime.ops, self.runtime.dtype
-        T, H, r = ctx.n_tokens, self.n_heads, self.kv_rank
+        T, H = ctx.n_tokens, self.n_heads
         views = ctx.buffer("latent.proj", (T, sum(self.widths)), dt, columns=self.widths)
         proj = views[0]
         gate = views[self.at["gate"]] if self.has_gate else None
@@ -134,8 +135,20 @@ class LatentAttention(Mixer):
         if owns_cache and not self.own_kv:
             raise ConfigError("a latent-attention layer without a down-projection cannot own a cache")
         if self._expands(ctx, q, cache):
+            if ctx.trace is not None and getattr(ctx.trace, "wants_values", True):
+                self._mixed(q, views, ctx, cache, owns_cache, table)         # what the other form goes through, for the trace
+                owns_cache = False                                           # (its rows are written)
             self._prompt(q, views, gate, residual, ctx, cache, owns_cache, accumulate, table)
             return
+        mixed = self._mixed(q, views, ctx, cache, owns_cache, table)
+        heads = ctx.buffer("latent.heads", (T, H * self.vdim), dt)
+        ops.heads_gemm(mixed, self.v_up, heads, self.kv_rank, self.vdim, gate=gate)
+        ctx.note("attn", heads)
+        self.out(heads, residual=residual if accumulate else None, out=residual)
+
+    def _mixed(self, q, views, ctx, cache, owns_cache, table):
+        """Every head's sum of latents, [T, H * kv_rank], from attention over the cached rows."""
+        ops, T, H, r = self.runtime.ops, ctx.n_tokens, self.n_heads, self.kv_rank
         # queries in latent space, float32: [T, H, kv_rank | rot_dim]
         qa = ctx.buffer("latent.q", (T, H * self.row), torch.float32)
         # one launch: this step's cache rows (norm, rotation) and the rotated part of the queries
@@ -146,16 +159,13 @@ class LatentAttention(Mixer):
                               cache.page_tokens, cache.pages, queries=rotated, pairs=self.rot_layout == "pairs")
         ops.heads_gemm(q, self.q_up, qa, self.q_head, self.row)
         ctx.note("q_latent", qa)
-        mixed = ctx.buffer("latent.mixed", (T, H * r), dt)
+        mixed = ctx.buffer("latent.mixed", (T, H * r), self.runtime.dtype)
         n_splits, part_o, part_ml = self.splits(ctx)
         ops.latent_attention(qa, cache.pages, table, cache.page_tokens, ctx.tok_pos, ctx.tok_seq, H, r, self.scale,
                              mixed, n_splits, part_o, part_ml, tiles=ctx.q_tiles, single_tokens=ctx.is_decode,
                              sink=self.sink, two_term_weights=self.exact_weights)
         ctx.note("mixed", mixed)
-        heads = ctx.buffer("latent.heads", (T, H * self.vdim), dt)
-        ops.heads_gemm(mixed, self.v_up, heads, r, self.vdim, gate=gate)
-        ctx.note("attn", heads)
-        self.out(heads, residual=residual if accumulate else None, out=residual)
+        return mixed
 
     # A prompt step expands its sequences' positions where they are no more than this many times its own tokens: each costs
     # 2 r H (d + d_v) operations whoever sees it.
@@ -186,6 +196,7 @@ class LatentAttention(Mixer):
         ops.latent_append(views[self.at["dkv"]] if owns_cache else None, self.norm_weight, self.eps, self.freq_table,
                           self.magnitude, self.rot_dims, r, self.rot_dim, ctx.tok_pos, ctx.tok_seq, table, cache.page_tokens,
                           cache.pages, queries=rotated, pairs=self.rot_layout == "pairs")
+        ctx.note("q", q)
         pages = [-(-(start + n) // 64) if n else 0 for start, n in zip(ctx.starts, ctx.q_lens)]
         n_pages, both = sum(pages), H * (self.dim + self.vdim)
         latents = ctx.buffer("latent.held", (n_pages * 64, r), dt)
@@ -193,6 +204,7 @@ class LatentAttention(Mixer):
         page_list = ctx.buffer("latent.pages", (ctx.n_seqs, max(pages)), torch.int32)
         ops.latent_rows(cache.pages, table, ctx.tok_pos, ctx.seq_first, n_pages, r, latents, rows, both, page_list)
         self.expand(latents, out=rows.view(n_pages * 64, both + self.rot_dim)[:, :both])
+        ctx.note("kv", rows)
         heads = ctx.buffer("latent.heads", (T, H * self.vdim), dt)
         ops.latent_prompt(q, rows, page_list, ctx.tok_pos, ctx.tok_seq, ctx.q_tiles_wide, H, self.dim, self.rot_dim, self.vdim,
                           self.scale, heads, sink=self.sink, gate=gate)

@@ -274,6 +274,23 @@ def test_latent_prompt_steps_with_sequences_that_bring_nothing(monkeypatch):
         assert runs == [(1, 1)] * 2 and all(torch.equal(a, b) for a, b in zip(found, want))
 
 
+def test_latent_prompt_steps_tell_a_trace_what_both_forms_go_through(monkeypatch):
+    part, steps, names = _latent_part(*LATENTS[1]), [[70, 1, 200]], []
+    plain, runs = _latent_steps(part, steps, monkeypatch)
+    traced, also = _latent_steps(part, steps, monkeypatch, lambda name, tensor: names.append(name))
+    assert names == ["proj", "q_latent", "mixed", "q", "kv", "attn"] and torch.equal(plain[0], traced[0]) and runs == also == [(1, 1)]
+
+    class Times:
+        wants_values = False
+
+        def __call__(self, name, tensor):
+            names.append(name)
+
+    names.clear()
+    _latent_steps(part, steps, monkeypatch, Times())
+    assert names == ["proj", "q", "kv", "attn"]
+
+
 def test_latent_prompt_steps_without_room_stay_in_latent_space(monkeypatch):
     part = _latent_part(*LATENTS[0])
     monkeypatch.setattr(part.runtime.ops, "STEP_ROOM", 2 * (200 + 64 * 3) * (4 * 128 + 256 + 32) - 1)
