@@ -58,7 +58,7 @@ __global__ void rotary_kernel(const TI* __restrict__ x, long long ldx, int x_hea
 // With q (and qa): the same block also rotates the token's queries (every head's rot_dim entries at q + h *
 // q_head_stride) into qa + h * qa_head_stride as float32, so that a step needs one launch for both.  With dkv
 // null only the queries are rotated (a layer that reads another layer's cache).
-constexpr int LA_TURNS = 768;     // rotated pairs at most (a cached row has 1,536 values at most)
+constexpr int LA_TURNS = 768;     // rotated pairs whose angles a block keeps (a cached row has 1,536 values at most)
 
 template <typename T, typename TQ>
 __global__ void latent_append_kernel(const T* __restrict__ dkv, long long ld, const float* __restrict__ norm_w, float eps,
@@ -73,13 +73,14 @@ __global__ void latent_append_kernel(const T* __restrict__ dkv, long long ld, co
     pdl_wait();
     const int t = blockIdx.x;
     const int p = tok_pos[t];
-    // the angles of a token are the same for every head: made once
+    // the angles of a token are the same for every head: made once (queries alone may have more of them)
     __shared__ float2 turns[LA_TURNS];
-    for (int e = threadIdx.x; e < rot_dims / 2; e += blockDim.x) {
+    auto turn = [&](int e) {
         float sn, cs;
         sincosf((float)p * freqs[e], &sn, &cs);
-        turns[e] = make_float2(sn * mag, cs * mag);
-    }
+        return make_float2(sn * mag, cs * mag);
+    };
+    for (int e = threadIdx.x; e < min(rot_dims / 2, LA_TURNS); e += blockDim.x) turns[e] = turn(e);
     __syncthreads();
     if (q) {
         const int half = rot_dims / 2, per_head = rot_dim - half;
@@ -90,7 +91,8 @@ __global__ void latent_append_kernel(const T* __restrict__ dkv, long long ld, co
             const T* s = src + (long long)h * q_head_stride;
             TQ* d = dst + (long long)h * qa_head_stride;
             if (e < half) {
-                const float sn = turns[e].x, cs = turns[e].y;
+                const float2 w = e < LA_TURNS ? turns[e] : turn(e);
+                const float sn = w.x, cs = w.y;
                 const int lo = pairs ? 2 * e : e, hi = pairs ? 2 * e + 1 : e + half;
                 const float u = to_float(s[lo]), v = to_float(s[hi]);
                 d[lo] = from_float<TQ>(u * cs - v * sn);
@@ -117,7 +119,8 @@ __global__ void latent_append_kernel(const T* __restrict__ dkv, long long ld, co
     dst += kv_rank;
     for (int e = threadIdx.x; e < rot_dim - half; e += blockDim.x) {
         if (e < half) {
-            const float sn = turns[e].x, cs = turns[e].y;
+            const float2 w = e < LA_TURNS ? turns[e] : turn(e);
+            const float sn = w.x, cs = w.y;
             const int lo = pairs ? 2 * e : e, hi = pairs ? 2 * e + 1 : e + half;
             const float u = to_float(src[lo]), v = to_float(src[hi]);
             dst[lo] = from_float<T>(u * cs - v * sn);
@@ -366,7 +369,6 @@ MU_EXPORT int mu_latent_append(const void* dkv, long long ld, const float* norm_
         (dkv && (!norm_w || !tok_seq || !block_table || !rows || page_tokens <= 0)) || (q && (!qa || n_heads <= 0)) ||
         (qa_bf16 && !is_bf16))
         return MU_ERR_BAD_ARGUMENT;
-    if (rot_dims / 2 > mu::LA_TURNS) return MU_ERR_UNSUPPORTED_SIZE;
     cudaStream_t s = (cudaStream_t)stream;
     const dim3 grid(n_tokens), block(kv_rank >= 512 ? 256 : 128);
     typedef __nv_bfloat16 bf;

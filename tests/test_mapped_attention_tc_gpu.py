@@ -295,3 +295,19 @@ def test_latent_prompt_steps_without_room_stay_in_latent_space(monkeypatch):
     part = _latent_part(*LATENTS[0])
     monkeypatch.setattr(part.runtime.ops, "STEP_ROOM", 2 * (200 + 64 * 3) * (4 * 128 + 256 + 32) - 1)
     assert _latent_steps(part, [[70, 0, 129], [0, 0, 72]], monkeypatch)[1] == [(1, 1), (0, 0)]
+
+
+def test_queries_rotate_more_pairs_than_a_block_keeps_angles_of():
+    """Queries alone (no cache row is written) of any rotated size, as the angles in float32 turn them."""
+    from math_utils_b200.csrc import ops
+    T, H, rot = 5, 2, 1604
+    q, qa = _rand((T, H * rot), 1).float(), torch.zeros((T, H * rot), device="cuda")
+    freqs = 10000.0 ** (-torch.arange(rot // 2, device="cuda").float() * 2 / rot)
+    rows = torch.zeros((1, 64, 8 + rot), device="cuda")
+    ops.latent_append(None, None, 0.0, freqs, 1.0, rot, 8, rot, _ints(range(T)), _ints([0] * T), _ints([[0]]), 64, rows,
+                      queries=(q, rot, qa, rot, H))
+    angle = torch.arange(T, device="cuda")[:, None].float() * freqs
+    cos, sin = (f(angle.double())[:, None] for f in (torch.cos, torch.sin))
+    lo, hi = q.double().reshape(T, H, 2, rot // 2).unbind(2)
+    want = torch.stack([lo * cos - hi * sin, hi * cos + lo * sin], 2).reshape(T, -1)
+    assert float((qa.double() - want).abs().max()) < 1e-5
