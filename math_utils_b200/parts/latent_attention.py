@@ -111,7 +111,9 @@ class LatentAttention(Mixer):
         self.expand = None
         if runtime.dtype == torch.bfloat16 and not self.window and runtime.ops.latent_prompt_ok(self.dim, self.rot_dim,
                                                                                                 self.vdim, self.kv_rank):
-            self.expand = Linear(torch.cat([t("uk"), t("uv")], dim=0).contiguous(), None, runtime)
+            both = torch.cat([t("uk"), t("uv")], dim=0).contiguous()
+            self.expand = Linear(both, None, runtime)
+            self.v_up = both[H * self.dim:].view(H, self.vdim, self.kv_rank)        # (held once)
         # (one entry at least, so that the kernels always get a table)
         self.freq_table = torch.tensor(self.freqs or [0.0], dtype=torch.float64).to(torch.float32).to(runtime.device)
 

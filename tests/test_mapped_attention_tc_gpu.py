@@ -297,6 +297,12 @@ def test_latent_prompt_steps_without_room_stay_in_latent_space(monkeypatch):
     assert _latent_steps(part, [[70, 0, 129], [0, 0, 72]], monkeypatch)[1] == [(1, 1), (0, 0)]
 
 
+def test_latent_layers_hold_their_value_projection_once():
+    part = _latent_part(*LATENTS[2])
+    H, dim = part.n_heads, part.dim
+    assert part.v_up.data_ptr() == part.expand.weight[H * dim:].data_ptr() and part.v_up.is_contiguous()
+
+
 def test_queries_rotate_more_pairs_than_a_block_keeps_angles_of():
     """Queries alone (no cache row is written) of any rotated size, as the angles in float32 turn them."""
     from math_utils_b200.csrc import ops
