@@ -180,6 +180,31 @@ def test_whole_prompt_and_every_layer(folders, name, dtype):
     check_logits(run_whole(model, cache, toks), want, dtype, f"pelenex {name} whole prompt, no trace")
 
 
+def test_prompts_with_gathered_rows_and_recurrences_in_chunks(folders, monkeypatch):
+    """The forms that only larger steps take, taken by small ones: the experts' rows gathered into tiles of 128 slots, the
+    matrix memories chunk by chunk in the step's own workspace."""
+    from math_utils_b200.csrc import ops
+    from math_utils_b200.parts.matrix_lstm import MatrixLstm
+    from math_utils_b200.parts.moe import RoutedExperts
+    monkeypatch.setattr(MatrixLstm, "in_chunks", lambda self, longest, tokens: True)
+    monkeypatch.setattr(RoutedExperts, "GATHERED_FLOP", 0)
+    model = DecoderModel.from_dir(folders["c", "bfloat16"], dtype="bfloat16")
+    cache = model.new_cache(max_tokens=64 * 24, n_slots=8)
+    took, check = [], ops._check
+    monkeypatch.setattr(ops, "_check", lambda code, what, *a, **k: (took.append(str(what)), check(code, what, *a, **k))[1])
+    toks = tokens_for("c", 150)
+    want = plain_logits("c", "bfloat16", toks)
+    check_logits(run_whole(model, cache, toks), want, "bfloat16", "pelenex c whole prompt, chunks and gathered rows")
+    count = lambda name: sum(name in t for t in took)
+    n_lstm, n_moe = (sum(f(layer) for layer in CFG_C["layers"]) for f in (lambda x: x["type"] == "mlstm", lambda x: x["mlp"]["kind"] == "moe"))
+    assert count("linear_scan_chunks") == n_lstm and count("moe_gemm_tc") == 2 * n_moe and ("chunk_scan", torch.float32) in model._workspace
+    slot, rows = cache.acquire(), []
+    for a, b in ((0, 70), (70, 71), (71, 150)):                   # states that one form leaves and the other goes on from
+        rows.append(model.step(cache, [StepEntry(slot, toks[a:b], list(range(b - a)))]).float().cpu().numpy())
+    cache.release(slot)
+    check_logits(np.concatenate(rows), want, "bfloat16", "pelenex c in portions, chunks and gathered rows")
+
+
 @pytest.mark.parametrize("name,dtype", CASES)
 def test_prompt_then_token_by_token(folders, name, dtype):
     model, cache = engine(folders, name, dtype)

@@ -157,6 +157,20 @@ def test_whole_prompt_and_every_layer(folders, name, dtype):
     check_logits(run_whole(model, cache, toks), want, dtype, f"tokolorn {name} whole prompt, no trace")
 
 
+@pytest.mark.parametrize("name,dtype", [("a", "float32"), ("c", "bfloat16")])
+def test_long_prompt_with_selective_scans_in_segments(folders, name, dtype, monkeypatch):
+    """A prompt long enough for its selective scans to be cut, in the step's own workspace; then from where the cut scan ended."""
+    from math_utils_b200.csrc import ops
+    model, cache = engine(folders, name, dtype)
+    cuts, check = [], ops._check
+    monkeypatch.setattr(ops, "_check", lambda code, what, launches=1: (cuts.append((str(what), launches)), check(code, what, launches))[1])
+    toks = tokens_for(name, 720, seed=9)
+    got = run_tail_one_by_one(model, cache, toks, tail=4)
+    check_logits(got, plain_logits(name, toks), dtype, f"tokolorn {name} long prompt")
+    scans = [n for what, n in cuts if "selective_scan(" in what]
+    assert scans.count(2) > 0 and set(scans[:scans.count(2)]) == {2} and ("selective_scan", torch.float32) in model._workspace
+
+
 @pytest.mark.parametrize("name,dtype", CASES)
 def test_prompt_then_token_by_token(folders, name, dtype):
     model, cache = engine(folders, name, dtype)
