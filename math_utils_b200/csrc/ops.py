@@ -611,62 +611,53 @@ def mapped_attention(q: torch.Tensor, rows: torch.Tensor, block_table: torch.Ten
               _ptr(slopes), int(keep), float(softcap), int(gate_each), int(shared))
     for t, name in ((tok_pos, "tok_pos"), (tok_seq, "tok_seq"), (block_table, "block_table")):
         _i32(t, name)
-    if (q.dtype != rows.dtype or out.dtype != rows.dtype or q.stride(1) != 1 or out.stride(1) != 1
-            or not rows.is_contiguous() or rows.shape[2] != n_kv_heads * (maps * dim + (0 if shared else vdim))
-            or q.shape[1] != n_heads * maps * dim or out.shape[1] != n_heads * vdim):
+    # (the tensors' sizes and places once: a prompt step of few tokens waits for this function)
+    (n_tokens, q_width), (ldq, q_step), (ldo, out_step), dtype = q.shape, q.stride(), out.stride(), rows.dtype
+    n_pages, _, row_width = rows.shape
+    if (q.dtype != dtype or out.dtype != dtype or q_step != 1 or out_step != 1
+            or not rows.is_contiguous() or row_width != n_kv_heads * (maps * dim + (0 if shared else vdim))
+            or q_width != n_heads * maps * dim or out.shape[1] != n_heads * vdim):
         raise KernelError("mapped_attention: queries, rows and output do not fit the sizes given")
-    if single_tokens and library().mu_mapped_decode_fits(int(n_heads), int(n_kv_heads), int(maps), int(dim), int(vdim),
-                                                         int(page_tokens), _is_bf16(rows)):
-        lib = library()
+    lib, bf16, pq, po = library(), _is_bf16(rows), q.data_ptr(), out.data_ptr()
+    held = (rows.data_ptr(), block_table.data_ptr(), block_table.shape[1], int(page_tokens), tok_pos.data_ptr(), tok_seq.data_ptr())
+    sizes = (int(n_heads), int(n_kv_heads), int(maps), int(dim), int(vdim))
+    numbers = (float(scale), int(window), float(lam), float(out_scale), float(eps), int(unit_rms))
+    if single_tokens and lib.mu_mapped_decode_fits(*sizes, int(page_tokens), bf16):
         lib.mu_mapped_decode_scratch.restype = _c_ll
-        need = int(lib.mu_mapped_decode_scratch(q.shape[0], int(n_heads), int(maps), int(vdim)))
+        need = int(lib.mu_mapped_decode_scratch(n_tokens, sizes[0], sizes[2], sizes[4]))
         room = scratch("mapped_decode", q.device, need, torch.float32)
-        _check(lib.mu_mapped_attention_decode(
-            _ptr(q), q.stride(0), _ptr(rows), _ptr(block_table), block_table.shape[1], int(page_tokens), _ptr(tok_pos),
-            _ptr(tok_seq), q.shape[0], int(n_heads), int(n_kv_heads), int(maps), int(dim), int(vdim), float(scale),
-            int(window), float(lam), float(out_scale), float(eps), int(unit_rms), _ptr(room), _ptr(out), out.stride(0),
-            _is_bf16(rows), _stream(), *extras),
-            ("mapped_attention_decode(heads={}/{}, maps={}, dim={}, vdim={})", n_heads, n_kv_heads, maps, dim, vdim), launches=2)
+        _check(lib.mu_mapped_attention_decode(pq, ldq, *held, n_tokens, *sizes, *numbers, _ptr(room), po, ldo, bf16, _stream(),
+                                              *extras),
+               ("mapped_attention_decode(heads={}/{}, maps={}, dim={}, vdim={})", *sizes), launches=2)
         return out
     if tensor_cores is None:
         tensor_cores = MAPPED_TC
     if head_sink is not None and (head_sink.dtype != torch.float32 or head_sink.numel() != n_heads or not head_sink.is_contiguous()):
         raise KernelError("mapped_attention: head_sink is one contiguous float32 per head")
-    if (tensor_cores and tiles_wide is not None and rows.dtype == torch.bfloat16
-            and (tiles is None or head_sink is not None
-                 or wide_tiles_pay(tiles.shape[0], tiles_wide.shape[0], n_heads, sm_count(q.device)))
-            and mapped_tc_ok(q, out, n_kv_heads, maps, dim, vdim, page_tokens, shared)
-            and not (gate_each and (gate.stride(0) % 2 or gate.data_ptr() % 4))):
-        _need_cuda(tiles_wide, head_sink)
-        _i32(tiles_wide, "tiles_wide")
-        _check(library().mu_mapped_attention_tc(
-            _ptr(q), q.stride(0), q.shape[0], _ptr(rows), rows.shape[0], _ptr(block_table), block_table.shape[1],
-            int(page_tokens), _ptr(tok_pos), _ptr(tok_seq), _ptr(tiles_wide), tiles_wide.shape[0], int(n_heads), int(n_kv_heads),
-            int(maps), int(dim), int(vdim), float(scale), int(window), float(lam), float(out_scale), float(eps), int(unit_rms),
-            _ptr(out), out.stride(0), status_word(q.device).data_ptr(), _stream(), *extras, _ptr(head_sink), 0),
-            ("mapped_attention_tc(heads={}/{}, maps={}, dim={}, vdim={})", n_heads, n_kv_heads, maps, dim, vdim))
-        return out
+    aligned = (tensor_cores and bf16 and ldq % 8 == 0 and pq % 16 == 0
+               and not (gate_each and (gate.stride(0) % 2 or gate.data_ptr() % 4)))
+    if aligned and tiles_wide is not None and ldq >= q_width and ldo % 8 == 0 and po % 16 == 0:
+        n_wide = tiles_wide.shape[0]
+        if ((tiles is None or head_sink is not None or wide_tiles_pay(tiles.shape[0], n_wide, n_heads, sm_count(q.device)))
+                and MAPPED_TC and _mapped_tc_fits(*sizes[1:], int(page_tokens), int(shared))):
+            _need_cuda(tiles_wide, head_sink)
+            _i32(tiles_wide, "tiles_wide")
+            _check(lib.mu_mapped_attention_tc(pq, ldq, n_tokens, held[0], n_pages, *held[1:], tiles_wide.data_ptr(), n_wide, *sizes,
+                                              *numbers, po, ldo, status_word(q.device).data_ptr(), _stream(), *extras,
+                                              _ptr(head_sink), 0),
+                   ("mapped_attention_tc(heads={}/{}, maps={}, dim={}, vdim={})", *sizes))
+            return out
     if head_sink is not None:
         raise KernelError("mapped_attention: sinks with a score per head need the tcgen05 kernel")
-    if (tensor_cores and tiles is not None and rows.dtype == torch.bfloat16 and q.stride(0) % 8 == 0
-            and out.stride(0) % 2 == 0 and q.data_ptr() % 16 == 0 and out.data_ptr() % 4 == 0
-            and not (gate_each and (gate.stride(0) % 2 or gate.data_ptr() % 4))
-            and library().mu_mapped_attention_mma_fits(int(n_kv_heads), int(maps), int(dim), int(vdim), int(page_tokens),
-                                                       int(shared))):
+    if (aligned and tiles is not None and ldo % 2 == 0 and po % 4 == 0
+            and lib.mu_mapped_attention_mma_fits(*sizes[1:], int(page_tokens), int(shared))):
         _need_cuda(tiles)
         _i32(tiles, "tiles")
-        _check(library().mu_mapped_attention_mma(
-            _ptr(q), q.stride(0), _ptr(rows), _ptr(block_table), block_table.shape[1], int(page_tokens), _ptr(tok_pos),
-            _ptr(tok_seq), _ptr(tiles), tiles.shape[0], int(n_heads), int(n_kv_heads), int(maps), int(dim), int(vdim),
-            float(scale), int(window), float(lam), float(out_scale), float(eps), int(unit_rms), _ptr(out), out.stride(0),
-            _stream(), *extras), ("mapped_attention_mma(heads={}/{}, maps={}, dim={}, vdim={})", n_heads, n_kv_heads, maps, dim, vdim))
+        _check(lib.mu_mapped_attention_mma(pq, ldq, *held, tiles.data_ptr(), tiles.shape[0], *sizes, *numbers, po, ldo, _stream(),
+                                           *extras), ("mapped_attention_mma(heads={}/{}, maps={}, dim={}, vdim={})", *sizes))
         return out
-    _check(library().mu_mapped_attention(_ptr(q), q.stride(0), _ptr(rows), _ptr(block_table), block_table.shape[1],
-                                         int(page_tokens), _ptr(tok_pos), _ptr(tok_seq), q.shape[0], int(n_heads),
-                                         int(n_kv_heads), int(maps), int(dim), int(vdim), float(scale), int(window),
-                                         float(lam), float(out_scale), float(eps), int(unit_rms), _ptr(out),
-                                         out.stride(0), _is_bf16(rows), _stream(), *extras),
-           ("mapped_attention(heads={}/{}, maps={}, dim={}, vdim={})", n_heads, n_kv_heads, maps, dim, vdim))
+    _check(lib.mu_mapped_attention(pq, ldq, *held, n_tokens, *sizes, *numbers, po, ldo, bf16, _stream(), *extras),
+           ("mapped_attention(heads={}/{}, maps={}, dim={}, vdim={})", *sizes))
     return out
 
 
@@ -1188,7 +1179,7 @@ def latent_append(dkv: Optional[torch.Tensor], norm_weight: Optional[torch.Tenso
     if queries is not None:
         q, qs, qa, qas, heads = queries
         _need_cuda(q, qa)
-        if q.dtype != rows.dtype or qa.dtype not in (torch.float32, rows.dtype) or q.stride(1) != 1 or qa.stride(1) != 1:
+        if q.dtype != rows.dtype or (qa.dtype != torch.float32 and qa.dtype != q.dtype) or q.stride(1) != 1 or qa.stride(1) != 1:
             raise KernelError("latent_append: queries in the cache's dtype, rotated queries as float32 or likewise")
     elif dkv is None:
         raise KernelError("latent_append: nothing to do")
@@ -1448,25 +1439,20 @@ def heads_gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, x_head_strid
     launch runs, as a launch of its own otherwise."""
     _need_cuda(x, w, out, gate)
     heads, n, k = w.shape
+    (rows, width), (ldx, x_step), (ldo, out_step), px, pw = x.shape, x.stride(), out.stride(), x.data_ptr(), w.data_ptr()
     if (LATENT_TC and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and w.is_contiguous() and k % 8 == 0
-            and x.stride(0) % 8 == 0 and x_head_stride % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
-            and x.stride(1) == 1 and out.stride(1) == 1):
+            and ldx % 8 == 0 and x_head_stride % 8 == 0 and px % 16 == 0 and pw % 16 == 0 and x_step == 1 and out_step == 1):
         fused = gate is not None and gate.dtype == torch.bfloat16 and gate.stride(1) == 1 and gate.shape == out.shape
-        rows, width = x.shape
-        if (2 * rows * heads * n * k >= HEADS_TC_FLOP and rows > 64 and k % 64 == 0
-                and x.stride(0) >= width >= (heads - 1) * x_head_stride + k):     # (rows that overlap have no tensor map)
-            _check(library().mu_heads_gemm_tc(_ptr(x), x.shape[1], x.stride(0), int(x_head_stride), _ptr(w), x.shape[0], heads,
-                                              n, k, _ptr(out), out.stride(0), int(out_head_stride), _is_bf16(out),
-                                              _ptr(gate) if fused else None, gate.stride(0) if fused else 0,
-                                              status_word(x.device).data_ptr(), _stream()),
+        gated = (gate.data_ptr(), gate.stride(0)) if fused else (None, 0)
+        if (rows > 64 and 2 * rows * heads * n * k >= HEADS_TC_FLOP and k % 64 == 0
+                and ldx >= width >= (heads - 1) * x_head_stride + k):             # (rows that overlap have no tensor map)
+            _check(library().mu_heads_gemm_tc(px, width, ldx, int(x_head_stride), pw, rows, heads, n, k, out.data_ptr(), ldo,
+                                              int(out_head_stride), _is_bf16(out), *gated, status_word(x.device).data_ptr(), _stream()),
                    ("heads_gemm_tc(heads={}, n={}, k={})", heads, n, k))
-            if gate is not None and not fused:
-                sigmoid_gate(out, gate)
-            return out
-        _check(library().mu_heads_gemm(_ptr(x), x.stride(0), int(x_head_stride), _ptr(w), w.stride(0), w.stride(1),
-                                       x.shape[0], heads, n, k, _ptr(out), out.stride(0), int(out_head_stride),
-                                       _is_bf16(out), _ptr(gate) if fused else None, gate.stride(0) if fused else 0,
-                                       _stream()), ("heads_gemm(heads={}, n={}, k={})", heads, n, k))
+        else:
+            _check(library().mu_heads_gemm(px, ldx, int(x_head_stride), pw, n * k, k, rows, heads, n, k, out.data_ptr(), ldo,
+                                           int(out_head_stride), _is_bf16(out), *gated, _stream()),
+                   ("heads_gemm(heads={}, n={}, k={})", heads, n, k))
         if gate is not None and not fused:
             sigmoid_gate(out, gate)
         return out

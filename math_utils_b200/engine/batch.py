@@ -10,6 +10,7 @@ copy from pinned memory.
 """
 from __future__ import annotations
 
+import functools
 from dataclasses import dataclass, field
 from typing import List, Optional, Sequence
 
@@ -103,6 +104,17 @@ class StepContext:
     @property
     def is_decode(self) -> bool:
         return self.max_q_len == 1
+
+    @functools.cached_property
+    def prompt_load(self):
+        """(positions that the step's sequences hold after it, twice the pairs of a token and a position it sees); sequences
+        that bring no token hold none."""
+        held = met = 0
+        for start, n in zip(self.starts, self.q_lens):
+            if n:
+                held += start + n
+                met += n * (2 * start + n)
+        return held, met
 
     def buffer(self, name: str, shape, dtype, columns=None):
         """An activation buffer of this shape that lives from step to step and is

@@ -177,19 +177,14 @@ class LatentAttention(Mixer):
     EXPANDED_FLOP = 2.5e9
 
     def _expands(self, ctx, q, cache) -> bool:
-        each = self.n_heads * (2 * self.kv_rank + self.rot_dim)
-        if self.expand is None or ctx.is_decode or 2 * ctx.n_tokens * ctx.max_kv_len * each < self.EXPANDED_FLOP:
+        T = ctx.n_tokens
+        if T <= 64 or self.expand is None or ctx.is_decode or ctx.q_tiles_wide is None:
             return False
-        if (ctx.q_tiles_wide is None or ctx.n_tokens <= 64 or cache.page_tokens != 64 or q.stride(0) % 8
-                or q.data_ptr() % 16):
-            return False
-        held = met = 0
-        for start, n in zip(ctx.starts, ctx.q_lens):
-            held += start + n if n else 0
-            met += n * (2 * start + n)                       # (twice the pairs of tokens and keys)
-        row = self.n_heads * (self.dim + self.vdim) + self.kv_rank + self.rot_dim
-        return (held <= self.EXPANDED_PER_TOKEN * ctx.n_tokens and met * each >= self.EXPANDED_FLOP
-                and 2 * (held + 64 * ctx.n_seqs) * row <= self.runtime.ops.STEP_ROOM)
+        held, met = ctx.prompt_load
+        H, r, rot = self.n_heads, self.kv_rank, self.rot_dim
+        return (met * H * (2 * r + rot) >= self.EXPANDED_FLOP and held <= self.EXPANDED_PER_TOKEN * T
+                and 2 * (held + 64 * ctx.n_seqs) * (H * (self.dim + self.vdim) + r + rot) <= self.runtime.ops.STEP_ROOM
+                and cache.page_tokens == 64 and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0)
 
     def _prompt(self, q, views, gate, residual, ctx, cache, owns_cache, accumulate, table) -> None:
         ops, dt = self.runtime.ops, self.runtime.dtype

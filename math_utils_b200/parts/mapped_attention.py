@@ -183,11 +183,12 @@ class MappedAttention(Mixer):
                        pairs=self.rot_layout == "pairs", shared=self.shared_rows and owns_cache)
         ctx.note("q", q)
         heads = ctx.buffer("mapped.heads", (T, self.n_heads * self.vdim), dt)
+        single = ctx.is_decode
         ops.mapped_attention(q, cache.pages, table, cache.page_tokens, ctx.tok_pos, ctx.tok_seq, self.n_heads,
                              self.n_kv_heads, self.maps, self.dim, self.vdim, self.scale, self.window, heads,
                              lam=self.lam, out_scale=self.out_scale, eps=self.eps, unit_rms=self.maps == 2,
-                             tiles=None if ctx.is_decode else ctx.q_tiles, single_tokens=ctx.is_decode,
-                             tiles_wide=None if ctx.is_decode else ctx.q_tiles_wide,
+                             tiles=None if single else ctx.q_tiles, single_tokens=single,
+                             tiles_wide=None if single else ctx.q_tiles_wide,
                              gate=gate, chunk=self.chunk, slopes=self.slope_table, keep=self.keep,
                              sink=self.sink, softcap=self.softcap, shared=self.shared_rows)
         ctx.note("attn", heads)

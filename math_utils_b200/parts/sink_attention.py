@@ -113,10 +113,11 @@ class SinkAttention(Mixer):
                           ctx.tok_pos, ctx.tok_seq, table, cache.page_tokens, cache.pages, first, mode, self.mix)
         ctx.note("q", q)
         heads = ctx.buffer("sink_attention.heads", (T, self.n_heads * self.vdim), dt)
+        single = ctx.is_decode
         ops.mapped_attention(q, cache.pages, table, cache.page_tokens, ctx.tok_pos, ctx.tok_seq, self.n_heads,
                              self.n_kv_heads, 1, self.dim, self.vdim, self.scale, self.window, heads,
-                             tiles=None if ctx.is_decode else ctx.q_tiles, single_tokens=ctx.is_decode,
-                             tiles_wide=None if ctx.is_decode else ctx.q_tiles_wide,
+                             tiles=None if single else ctx.q_tiles, single_tokens=single,
+                             tiles_wide=None if single else ctx.q_tiles_wide,
                              head_scale=self.head_scales, sink=self.sink, gate=gate)
         ctx.note("attn", heads)
         self.out(heads, residual=residual if accumulate else None, out=residual)
