@@ -107,12 +107,18 @@ __device__ __forceinline__ float2 mt_join(const MtArgs& a, int h, float ref0, fl
 
 // One query's result over exactly the keys that it sees, by a warp: for rows that came out infinite or NaN.  A weight of
 // zero does not keep an infinite or NaN value out of a product, and a tile's rows meet all pages of the tile: those with later
-// tokens, and what lies in the last page behind the sequence's end.  Finite rows pay one multiply-add a value for the check.
+// tokens, and what lies in the last page behind the sequence's end.  Finite rows pay one multiply-add a pair of values for the check.
 // A row whose scores hold a NaN is NaN throughout and stops there.
-__device__ __noinline__ void mt_row_alone(const MtArgs& a, const int* pages, int page_lo, int kept_pages, int n_pages, int h, int g,
-                                          int flat, int pos) {
+// (Everything is worked out anew from the tile and the row, so that nothing is kept in registers for it.)
+__device__ __noinline__ void mt_row_alone(const MtArgs& a, int row) {
     constexpr float LOG2E = 1.4426950408889634f;
     const int lane = threadIdx.x & 31, kw = a.maps * a.dim;
+    const int tile = blockIdx.x / a.n_heads, h = blockIdx.x % a.n_heads, g = h / (a.n_heads / a.n_kv_heads);
+    const int flat0 = a.tiles[2 * tile], flat = flat0 + row, pos0 = a.tok_pos[flat0], pos = pos0 + row;
+    const int last = (pos0 + min(a.tiles[2 * tile + 1], MT_Q) - 1) / MT_K;
+    const int page_lo = (a.chunk > 0 ? pos0 - pos0 % a.chunk : a.window > 0 ? max(0, pos0 - a.window + 1) : 0) / MT_K;
+    const int kept_pages = min((a.keep + MT_K - 1) / MT_K, page_lo), n_pages = kept_pages + last - page_lo + 1;
+    const int* pages = a.block_table + (long long)a.tok_seq[flat0] * a.max_pages;
     const int lo = a.chunk > 0 ? pos - pos % a.chunk : a.window > 0 ? pos - a.window + 1 : 0;
     const float scale = a.head_scale ? a.scale * a.head_scale[h] : a.scale;
     const float inv_cap = a.softcap > 0.0f ? 1.0f / a.softcap : 0.0f, slope = a.slopes ? a.slopes[h] * LOG2E : 0.0f;
@@ -472,7 +478,8 @@ mapped_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                 const __nv_bfloat16* gate = a.gate ? a.gate + (long long)(flat0 + min(row, count - 1)) * a.ldg : nullptr;
                 if (gate && !a.gate_each) times *= 1.0f / (1.0f + expf(-__bfloat162float(gate[h])));
                 __nv_bfloat16* dst = a.out + (long long)(flat0 + row) * a.ldo + (long long)h * a.vdim;
-                float odd = 0.0f;                        // NaN from the first value that is not finite on
+                const __nv_bfloat162 zero = __floats2bfloat162_rn(0.0f, 0.0f);
+                __nv_bfloat162 odd[4] = {zero, zero, zero, zero};          // NaN from the first value that is not finite on
                 for (int c = 0; c < a.vdim; c += 32) {
                     float v[32];
                     __syncwarp();
@@ -482,8 +489,6 @@ mapped_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                         if (!real || c + i >= a.vdim) break;
                         uint32_t word[4];
 #pragma unroll
-                        for (int e = 0; e < 8; ++e) odd = fmaf(v[i + e], 0.0f, odd);
-#pragma unroll
                         for (int e = 0; e < 4; ++e) {
                             float y0 = v[i + 2 * e] * times, y1 = v[i + 2 * e + 1] * times;
                             if (a.gate_each) {
@@ -492,14 +497,15 @@ mapped_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                                 y1 = __fdividef(y1, 1.0f + __expf(-__high2float(z)));
                             }
                             const __nv_bfloat162 b = __floats2bfloat162_rn(y0, y1);
+                            odd[e] = __hfma2(b, zero, odd[e]);
                             word[e] = *reinterpret_cast<const uint32_t*>(&b);
                         }
                         *reinterpret_cast<uint4*>(dst + c + i) = make_uint4(word[0], word[1], word[2], word[3]);
                     }
                 }
-                for (unsigned todo = __ballot_sync(0xffffffffu, isnan(odd)); todo; todo &= todo - 1) {
-                    const int r = quad * 32 + __ffs(todo) - 1;
-                    mt_row_alone(a, pages, page_lo, kept_pages, n_pages, h, g, flat0 + r, pos0 + r);
+                const float2 some = __bfloat1622float2(__hadd2(__hadd2(odd[0], odd[1]), __hadd2(odd[2], odd[3])));
+                for (unsigned todo = __ballot_sync(0xffffffffu, isnan(some.x + some.y)); todo; todo &= todo - 1) {
+                    mt_row_alone(a, ((int)threadIdx.x >> 5 & 3) * 32 + __ffs(todo) - 1);
                 }
             }
         }
