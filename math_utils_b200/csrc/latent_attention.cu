@@ -58,9 +58,10 @@ __global__ void rotary_kernel(const TI* __restrict__ x, long long ldx, int x_hea
 // With q (and qa): the same block also rotates the token's queries (every head's rot_dim entries at q + h *
 // q_head_stride) into qa + h * qa_head_stride as float32, so that a step needs one launch for both.  With dkv
 // null only the queries are rotated (a layer that reads another layer's cache).
-constexpr int LA_TURNS = 768;     // rotated pairs whose angles a block keeps (a cached row has 1,536 values at most)
+constexpr int LA_TURNS = 768;     // rotated pairs whose angles a block can keep (a cached row has 1,536 values at most)
 
-template <typename T, typename TQ>
+// KEPT: a token's angles, the same for every head, are made once and kept in shared memory; queries alone may have more of them.
+template <typename T, typename TQ, bool KEPT>
 __global__ void latent_append_kernel(const T* __restrict__ dkv, long long ld, const float* __restrict__ norm_w, float eps,
                                      const float* __restrict__ freqs, float mag, int rot_dims, int kv_rank, int rot_dim,
                                      const int* __restrict__ tok_pos, const int* __restrict__ tok_seq,
@@ -73,15 +74,16 @@ __global__ void latent_append_kernel(const T* __restrict__ dkv, long long ld, co
     pdl_wait();
     const int t = blockIdx.x;
     const int p = tok_pos[t];
-    // the angles of a token are the same for every head: made once (queries alone may have more of them)
-    __shared__ float2 turns[LA_TURNS];
+    __shared__ float2 turns[KEPT ? LA_TURNS : 1];
     auto turn = [&](int e) {
         float sn, cs;
         sincosf((float)p * freqs[e], &sn, &cs);
         return make_float2(sn * mag, cs * mag);
     };
-    for (int e = threadIdx.x; e < min(rot_dims / 2, LA_TURNS); e += blockDim.x) turns[e] = turn(e);
-    __syncthreads();
+    if (KEPT) {
+        for (int e = threadIdx.x; e < rot_dims / 2; e += blockDim.x) turns[e] = turn(e);
+        __syncthreads();
+    }
     if (q) {
         const int half = rot_dims / 2, per_head = rot_dim - half;
         const T* src = q + (long long)t * ldq;
@@ -91,7 +93,7 @@ __global__ void latent_append_kernel(const T* __restrict__ dkv, long long ld, co
             const T* s = src + (long long)h * q_head_stride;
             TQ* d = dst + (long long)h * qa_head_stride;
             if (e < half) {
-                const float2 w = e < LA_TURNS ? turns[e] : turn(e);
+                const float2 w = KEPT ? turns[e] : turn(e);
                 const float sn = w.x, cs = w.y;
                 const int lo = pairs ? 2 * e : e, hi = pairs ? 2 * e + 1 : e + half;
                 const float u = to_float(s[lo]), v = to_float(s[hi]);
@@ -119,7 +121,7 @@ __global__ void latent_append_kernel(const T* __restrict__ dkv, long long ld, co
     dst += kv_rank;
     for (int e = threadIdx.x; e < rot_dim - half; e += blockDim.x) {
         if (e < half) {
-            const float2 w = e < LA_TURNS ? turns[e] : turn(e);
+            const float2 w = KEPT ? turns[e] : turn(e);
             const float sn = w.x, cs = w.y;
             const int lo = pairs ? 2 * e : e, hi = pairs ? 2 * e + 1 : e + half;
             const float u = to_float(src[lo]), v = to_float(src[hi]);
@@ -371,9 +373,10 @@ MU_EXPORT int mu_latent_append(const void* dkv, long long ld, const float* norm_
         return MU_ERR_BAD_ARGUMENT;
     cudaStream_t s = (cudaStream_t)stream;
     const dim3 grid(n_tokens), block(kv_rank >= 512 ? 256 : 128);
+    const bool kept = rot_dims / 2 <= mu::LA_TURNS;
     typedef __nv_bfloat16 bf;
 #define MU_APPEND(T, TQ)                                                                                                \
-    return mu::launch_pdl(mu::latent_append_kernel<T, TQ>, grid, block, 0, s, 1, (const T*)dkv, ld, norm_w, eps, freqs, mag, \
+    return mu::launch_pdl(kept ? mu::latent_append_kernel<T, TQ, true> : mu::latent_append_kernel<T, TQ, false>, grid, block, 0, s, 1, (const T*)dkv, ld, norm_w, eps, freqs, mag, \
                           rot_dims, kv_rank, rot_dim, tok_pos, tok_seq, block_table, max_pages, page_tokens, (T*)rows,   \
                           (const T*)q, ldq, q_head_stride, (TQ*)qa, ldqa, qa_head_stride, n_heads, pairs)
     if (is_bf16 && qa_bf16) MU_APPEND(bf, bf);
