@@ -11,8 +11,9 @@
 // That is the first kernel, which takes any type, stride and size.  The second (gemm_f32_tile) takes float32 operands whose
 // rows are whole 16-byte pieces, which is every product of the 32-bit path.  Its sums are four, over the k of every fourth
 // run of eight, added in order at the end: as independent of the rest of the step, and no less exact.  It is bound by the
-// FMA pipes (2 m n k / 73 TFLOP/s) and next by shared-memory reads, of which a small thread tile needs too many, while the
-// large tile that needs few leaves a step of some hundred tokens with two warps an SM.  So a thread owns TM x 8 outputs
+// FMA pipes (2 m n k / 73 TFLOP/s) and next by how few warps share a scheduler: a small thread tile needs too many
+// shared-memory reads, and the large one that needs few leaves two (80 rows) to four of them, which issue in 45 to 59 % of the
+// cycles and wait for fixed latencies and the pipe otherwise, not for shared memory (50 to 66 % busy).  So a thread owns TM x 8 outputs
 // (pairs of columns, fma.rn.f32x2: two FMAs an instruction, each rounded as its scalar form), and four groups of warps
 // share every staged tile, each taking a quarter of its k.  Operands lie k-major in shared memory; the next 32 of k are on
 // their way from global memory meanwhile.  Measured (B200, microseconds; the first kernel's in brackets): 777 x 3072 x 768 120
