@@ -88,11 +88,41 @@ moe_route_kernel(const T* __restrict__ h, long long ldh, const float* __restrict
             }
         }
     };
-    // NE router rows a pass: a staged row's piece, read from shared memory once, serves them all (with one row a pass the
-    // kernel waits for those reads: four multiply-adds each)
-    constexpr int NE = TOK >= 4 ? 2 : 1, AHEAD = TOK == 8 ? 1 : TOK == 4 ? 4 : 8;
-    for (int e0 = warp; e0 < rows; e0 += NE * ROUTE_WARPS) {
+    // One router row: the lane's part of every token's sum.
+    auto sum_row = [&](const float* w, float (&z)[TOK]) {
         if (wide) {
+            const float4* w4 = reinterpret_cast<const float4*>(w);
+            const float4* h4 = reinterpret_cast<const float4*>(hrow);
+            const int n4 = hidden / 4;
+            float z0[TOK], z1[TOK], z2[TOK], z3[TOK];                        // a lane's sum in four parts, then in order
+#pragma unroll
+            for (int i = 0; i < TOK; ++i) z0[i] = z1[i] = z2[i] = z3[i] = 0.0f;
+#pragma unroll 8
+            for (int d = lane; d < n4; d += 32) {                            // (unrolled: the row's loads go out together)
+                const float4 b = w4[d];
+#pragma unroll
+                for (int i = 0; i < TOK; ++i) {
+                    const float4 a = h4[i * n4 + d];
+                    z0[i] += a.x * b.x; z1[i] += a.y * b.y; z2[i] += a.z * b.z; z3[i] += a.w * b.w;
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < TOK; ++i) z[i] = (z0[i] + z1[i]) + (z2[i] + z3[i]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < TOK; ++i) z[i] = 0.0f;
+            for (int d = lane; d < hidden; d += 32) {
+                const float b = w[d];
+#pragma unroll
+                for (int i = 0; i < TOK; ++i) z[i] += hrow[i * hidden + d] * b;
+            }
+        }
+    };
+    // Four and more tokens: two router rows a pass; a staged row's piece, read from shared memory once, serves both (with one
+    // row a pass the kernel waits for those reads: four multiply-adds each).  Fewer tokens wait for the rows themselves.
+    constexpr int NE = TOK >= 4 ? 2 : 1, AHEAD = TOK == 8 ? 1 : 4;
+    for (int e0 = warp; e0 < rows; e0 += NE * ROUTE_WARPS) {
+        if (NE > 1 && wide) {
             const float4* w4[NE];
 #pragma unroll
             for (int n = 0; n < NE; ++n) w4[n] = reinterpret_cast<const float4*>(row_of(min(e0 + n * ROUTE_WARPS, rows - 1)));
@@ -128,16 +158,9 @@ moe_route_kernel(const T* __restrict__ h, long long ldh, const float* __restrict
 #pragma unroll
             for (int n = 0; n < NE; ++n) {
                 const int e = e0 + n * ROUTE_WARPS;
-                if (e >= rows) break;
-                const float* w = row_of(e);
+                if (n > 0 && e >= rows) break;
                 float z[TOK];
-#pragma unroll
-                for (int i = 0; i < TOK; ++i) z[i] = 0.0f;
-                for (int d = lane; d < hidden; d += 32) {
-                    const float b = w[d];
-#pragma unroll
-                    for (int i = 0; i < TOK; ++i) z[i] += hrow[i * hidden + d] * b;
-                }
+                sum_row(row_of(e), z);
                 put(e, z);
             }
         }
