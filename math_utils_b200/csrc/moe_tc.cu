@@ -101,7 +101,7 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                     mbar_expect_tx(&sm.full[s], subs * SUB_BYTES);
 #pragma unroll
                     for (int u = 0; u < KSUB; ++u) {
-                        if (u >= subs) break;
+                        if (u > 0 && u >= subs) break;
                         const int x = (kb * KSUB + u) * TC_BK;
                         tma_load_2d(sm.a[s][u], &map_a, ax + x, w.row0, &sm.full[s]);
                         tma_load_2d(sm.b[s][u], &map_w1, x, wy, &sm.full[s]);
@@ -143,12 +143,13 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                     const uint64_t b_stage = b_desc0 + (uint64_t)((uint32_t)s * (KSUB * B_SUB));
                     const int subs = sub_tiles(kb);
 #pragma unroll
-                    for (int u = 0; u < KSUB; ++u)
+                    for (int u = 0; u < KSUB; ++u) {
+                        if (u > 0 && u >= subs) break;
 #pragma unroll
                         for (int kk = 0; kk < TC_BK / 16; ++kk)
-                            if (u < subs)
-                                umma_bf16(tmem_d, a_stage + (uint64_t)(u * A_SUB + 2 * kk), b_stage + (uint64_t)(u * B_SUB + 2 * kk),
-                                          idesc, (kb > 0 || u > 0 || kk > 0) ? 1u : 0u);
+                            umma_bf16(tmem_d, a_stage + (uint64_t)(u * A_SUB + 2 * kk), b_stage + (uint64_t)(u * B_SUB + 2 * kk),
+                                      idesc, (kb > 0 || u > 0 || kk > 0) ? 1u : 0u);
+                    }
                     umma_commit(&sm.empty[s]);
                 }
                 if (ok) umma_commit(&sm.acc_full[buf]);
