@@ -83,28 +83,35 @@ __device__ __forceinline__ void cs_mma(float (&d)[4], const uint32_t (&a)[4], ui
 // average over mantissas (2^-24 (1 - 1/2) / ln 2).
 constexpr float CS_CUT = 4.3e-8f;
 
-// d += the product over two steps of 8 (a: their two-term fragments; b: slots tig, tig + 4 of each).  The products of large
-// terms and the small ones go into sums of their own, which join d by an ordinary addition: the tensor cores cut a running
-// sum off where an addition rounds it.  What the cut takes on average is put back with the small sum.  (Measured against float64
-// over the layers' sizes, one sum for all six and nothing put back: 1.87e-7 of the output, 8 heads of 128 x 128, and 1.03e-7, 16
-// heads of 64 x 128 by key; so 1.55e-7 and 0.88e-7 in 3 % more time; token by token 1.64e-7 and 0.77e-7.  The product of
-// the two small terms, and a third sum, would bring 1.42e-7 and 0.83e-7 in 10 % more time.)
+// x as two TF32 terms that are together longer than x by that share.
+__device__ __forceinline__ void cs_split_more(float x, uint32_t& hi, uint32_t& lo) {
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hi) : "f"(x));
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lo) : "f"(fmaf(x, CS_CUT, x - __uint_as_float(hi))));
+}
+
+// d += the product over two steps of 8 (a: their two-term fragments; b: slots tig, tig + 4 of each).  Six products go into
+// a sum of their own, the small ones first, which joins d by an ordinary addition: the tensor cores cut a running sum off
+// where an addition rounds it, and what the cut takes on average the right operand brings along.  Measured against float64
+// over the layers' sizes (of the outputs): 8 heads of 128 x 128 1.47e-7, token by token in float32 1.64e-7, without
+// the share 1.87e-7; 16 heads of 64 x 128 by key 0.85e-7, 0.77e-7 and 1.03e-7; the states 1.0e-7, 1.5e-7 and 1.2e-7.  (A second
+// sum for the products of the large terms: 1.55e-7 and 0.88e-7; the product of the two small terms as well: 1.42e-7 and
+// 0.83e-7 in 6 % more time.)
 __device__ __forceinline__ void cs_products(float (&d)[4], const uint32_t (&ah)[2][4], const uint32_t (&al)[2][4], float b0,
                                             float b1, float b2, float b3) {
     uint32_t h0, l0, h1, l1, h2, l2, h3, l3;
-    cs_split(b0, h0, l0);
-    cs_split(b1, h1, l1);
-    cs_split(b2, h2, l2);
-    cs_split(b3, h3, l3);
-    float t[4] = {}, u[4] = {};
+    cs_split_more(b0, h0, l0);
+    cs_split_more(b1, h1, l1);
+    cs_split_more(b2, h2, l2);
+    cs_split_more(b3, h3, l3);
+    float t[4] = {};
     cs_mma(t, al[0], h0, h1);
     cs_mma(t, ah[0], l0, l1);
     cs_mma(t, al[1], h2, h3);
     cs_mma(t, ah[1], l2, l3);
-    cs_mma(u, ah[0], h0, h1);
-    cs_mma(u, ah[1], h2, h3);
+    cs_mma(t, ah[0], h0, h1);
+    cs_mma(t, ah[1], h2, h3);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) d[i] += u[i] + fmaf(u[i], CS_CUT, t[i]);
+    for (int i = 0; i < 4; ++i) d[i] += t[i];
 }
 
 // Rows flat0 .. flat0 + count - 1 of `src` (row stride ld), `width` floats of each, to [64][pitch]; zeros for the rows past
@@ -314,6 +321,15 @@ chunk_outputs_kernel(const __grid_constant__ ChunkArgs a) {
     const int lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
     const bool norm = a.norm_sums != nullptr && col0 == 0 && half0 == 0;
     if (warp * 16 >= count || half0 >= cols) return;
+    // The last sixteen keys of a warp are its own tokens: those after a token have the weight zero, which does not keep an
+    // infinite or NaN value out of a product.  With such a value among them they are added key by key.
+    float odd = 0.0f;                                          // NaN from the first value that is not finite on
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float4 x = *reinterpret_cast<const float4*>(Vs + (warp * 16 + 4 * i + (lane >> 3)) * VP + half0 + 4 * (lane & 7));
+        odd = fmaf(x.x, 0.0f, fmaf(x.y, 0.0f, fmaf(x.z, 0.0f, fmaf(x.w, 0.0f, odd))));
+    }
+    const bool plain = !__any_sync(0xffffffffu, isnan(odd));
     const int t0 = warp * 16 + gid, t1 = t0 + 8;               // this thread's two tokens
     const float* q0 = a.q + (long long)(flat0 + min(t0, count - 1)) * a.ld + key_at + 4 * tig;
     const float* q1 = a.q + (long long)(flat0 + min(t1, count - 1)) * a.ld + key_at + 4 * tig;
@@ -387,19 +403,7 @@ chunk_outputs_kernel(const __grid_constant__ ChunkArgs a) {
             cs_split(p1, ph[u][2], pl[u][2]);
             cs_split(p3, ph[u][3], pl[u][3]);
         }
-        // the last sixteen keys are this warp's own tokens: those after a token have the weight zero, which does not keep an
-        // infinite or NaN value out of a product
-        bool plain = true;
-        if (n + 2 >= key_tiles) {
-            float odd = 0.0f;                                   // NaN from the first value that is not finite on
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float* src = Vs + (8 * n + 2 * tig) * VP + half0 + 8 * j + gid;
-                odd = fmaf(src[0], 0.0f, fmaf(src[VP], 0.0f, fmaf(src[8 * VP], 0.0f, fmaf(src[9 * VP], 0.0f, odd))));
-            }
-            plain = !__any_sync(0xffffffffu, isnan(odd));
-        }
-        if (plain) {
+        if (plain || n + 2 < key_tiles) {
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const float* src = Vs + (8 * n + 2 * tig) * VP + half0 + 8 * j + gid;
