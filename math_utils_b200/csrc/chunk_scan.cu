@@ -18,10 +18,11 @@
 // and added to the running sum by ordinary additions (cs_products).  L is summed
 // in float64 and kept as two floats, since exp(L_t - L_s) of neighbours takes the difference of two large numbers.
 //
-// What bounds it: the latency of staging a chunk and of its dependent products; the token-by-token forms are bound by the
-// chain of 1,024 tokens a sequence.  Measured (B200, 2 x 1,024 tokens): 16 heads of 128 x 64 by key 319 -> 26 + 19 + 64 us
-// (the state-space layer 365 -> 139 us), 8 heads of 128 x 128 with normalizer over 2,018 tokens 185 -> ~95 us (the matrix
-// memory's layer 265 -> 168 us); one sequence of some 300 tokens gains half.
+// What bounds it: dependent products of three warps a scheduler, which issue in half of the cycles and wait for fixed latencies
+// and the pipe otherwise; the token-by-token forms are bound by the chain of 1,024 tokens a sequence.  Measured (B200,
+// 2 x 1,024 tokens): 16 heads of 128 x 64 by key 319 -> 28 + 8 + 64 us (the state-space layer 365 -> 145 us), 8 heads of 128 x
+// 128 with normalizer over 2,018 tokens 185 -> 26 + 8 + 64 us (the matrix memory's layer 265 -> 171 us); one sequence of some 300
+// tokens gains half, wide batches of the matrix memory nothing (matrix_lstm.py has the rule).
 #include "common.cuh"
 
 #include <math.h>

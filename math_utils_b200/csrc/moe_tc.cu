@@ -19,7 +19,8 @@
 // Measured (B200): 64 experts of 2,048 x 1,408 x 3, 12,288 pairs, first product 586 -> 213 us, second 357 -> 147 us (143 GFLOP
 // in 213 us, 670 TFLOP/s, with a quarter of the tiles' rows empty; the weights alone take 113 and 56 us), the gather ~20 us,
 // the whole feed-forward 1,002 -> 502 us; 48 pairs over those experts with two matrices each 136 -> 93 us.  mma.sync with 64
-// rows a block gave the first figures; per head, 2,048 rows x 16 heads: 440 -> 416 us for the attention layer around both.
+// rows a block gave the first figures.  Per head, 16 heads, 2,048 rows, the launch alone: 512 x 128 36 -> 25 us, 128 x 512 26 -> 9;
+// at 300 rows 8.3 -> 8.5 and 14.5 -> 6.0.
 #include "gemm_tc_kernel.cuh"
 
 #include <math.h>

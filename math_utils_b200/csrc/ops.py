@@ -1425,8 +1425,9 @@ def moe_gemm(x: torch.Tensor, pair_of: Optional[torch.Tensor], top: int, w1: tor
     return out
 
 
-# Per-head products of at least so much work go to the tcgen05 kernel: 4 heads of 256 x 32, 256 rows, twice a layer: 81 us with
-# `mma.sync`, 87 so (the host's time); 16 heads of 512 x 128, 2,048 rows (4.3 GFLOP): 440 us and 416.
+# Per-head products of at least so much work go to the tcgen05 kernel: 16 heads of 512 x 128, 2,048 rows (4.3 GFLOP) 36 us with
+# `mma.sync`, 25 so, of 128 x 512 26 and 9; smaller ones go either way (300 rows 8.3 and 8.5, 14.5 and 6.0; 4 heads of 256 x 64, 2,048
+# rows 6.7 and 8.0) and cost the host the launch's tensor maps (4 heads of 256 x 32, 256 rows, the layer around two: 81 us and 87).
 HEADS_TC_FLOP = 1e9
 
 
