@@ -119,6 +119,11 @@ __device__ __forceinline__ float2x pair_fma(float2x a, float2x b, float2x c) {
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
     return r;
 }
+__device__ __forceinline__ float2x pair_add(float2x a, float2x b) {
+    float2x r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
 __device__ __forceinline__ float2x pair_mul(float2x a, float2x b) {
     float2x r;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));

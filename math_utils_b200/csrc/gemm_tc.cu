@@ -80,6 +80,30 @@ bool tensor_map_out(CUtensorMap* map, const void* base, long long rows, int cols
     return true;
 }
 
+// A [rows, cols] float32 matrix with `ld` elements between rows, cut into boxes of box_rows x 32 with the 128-byte swizzle.
+bool tensor_map_f32(CUtensorMap* map, const void* base, long long rows, int cols, long long ld, int box_rows) {
+    const MapKey key = {base, rows, cols, box_rows, ld, 3};
+    const size_t h = ((uintptr_t)base >> 8) * 0x9E3779B97F4A7C15ull + (size_t)rows * 29 + (size_t)cols * 127 + box_rows;
+    MapSlot& slot = map_cache[(h >> 20) & 511];
+    std::lock_guard<std::mutex> lock(map_mutex);
+    if (slot.used && slot.key == key) { *map = slot.map; return true; }
+    EncodeTiledFn fn = encode_tiled();
+    if (!fn) return false;
+    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)ld * sizeof(float)};
+    const cuuint32_t box[2] = {32, (cuuint32_t)box_rows};
+    const cuuint32_t elem[2] = {1, 1};
+    if (fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box, elem,
+           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return false;
+    slot.key = key; slot.map = *map; slot.used = true;
+    return true;
+}
+
+struct F32SplitRoom { float* parts; long long bytes; int* tickets; int n_tickets; };
+F32SplitRoom split_room() { return {g_split.parts, g_split.parts_bytes, g_split.tickets, g_split.n_tickets}; }
+
 // A [rows, cols] bfloat16 matrix with `ld` elements between rows, cut into boxes of box_rows x 64.
 static bool make_map_uncached(CUtensorMap* map, const void* base, long long rows, int cols, long long ld, int box_rows) {
     EncodeTiledFn fn = encode_tiled();

@@ -63,6 +63,8 @@ _SIGNATURES = {
     "mu_gemm_tc_split_workspace": [_c_p, _c_ll, _c_p, _c_int],
     "mu_gemm_tc": [_c_p, _c_p, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_ll, _c_ll, _c_ll, _c_ll,
                    _c_int, _c_int, _c_int, _c_int, _c_p, _c_p],
+    "mu_gemm_f32_tc": [_c_p, _c_p, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_ll, _c_ll, _c_ll, _c_ll,
+                       _c_int, _c_int, _c_int, _c_p, _c_p],
     "mu_gemm_rows": [_c_p, _c_p, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_ll, _c_ll, _c_ll, _c_ll,
                      _c_int, _c_int, _c_int, _c_p, _c_p],
     "mu_kv_append": [_c_p, _c_ll, _c_p, _c_ll, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int,
@@ -1566,6 +1568,21 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = N
     return out
 
 
+def gemm_f32_tc(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
+                act: Optional[str] = None, residual: Optional[torch.Tensor] = None,
+                out: Optional[torch.Tensor] = None, tile: int = 0, cut: int = -1) -> torch.Tensor:
+    """The 32-bit product on tensor cores (three TF32 products a pair, float32 sums): float32 operands whose rows are whole
+    16-byte pieces.  ``tile`` (columns of a tile) and ``cut`` (1: a block a run of k) change no bit of the result."""
+    if a.dtype != torch.float32 or w.dtype != torch.float32 or (out is not None and out.dtype != torch.float32):
+        raise KernelError("gemm_f32_tc takes float32")
+    m, n, k, out = _gemm_args(a, w, bias, residual, out, torch.float32)
+    _check(library().mu_gemm_f32_tc(
+        _ptr(a), _ptr(w), _ptr(bias), _ptr(residual), _ptr(out), m, n, k, a.stride(0), w.stride(0), out.stride(0),
+        residual.stride(0) if residual is not None else 0, ACT_CODES[act], int(tile), int(cut), _ptr(status_word(a.device)),
+        _stream()), ("gemm_f32_tc({}x{}x{})", m, n, k))
+    return out
+
+
 _status = {}
 
 
@@ -2087,11 +2104,18 @@ def prompt_layer(args: PromptLayerArgs) -> None:
 
 
 # -------------------------------------------------------------------- dispatch
+# float32 products over at least this much of k run on tensor cores: there their error against float64 is the smaller (2-norm,
+# normal values: k = 128 1.09e-7 against 1.11e-7 of the multiply-adds, 192 1.13 and 1.32, 768 1.37 and 2.52, 3072 1.43 and
+# 4.98), and they are no slower (1 x 64 x 512 11.8 us and 13.8, 8 x 3072 x 768 14.7 and 19, 2000 x 768 x 192 12 and 25).
+F32_TC_K = 192
+
+
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None,
            act: Optional[str] = None, residual: Optional[torch.Tensor] = None,
            out: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
     """act(x @ weight^T + bias) + residual through the kernel that fits the
-    dtype and the shape.  float32 operands always take the CUDA-core kernel.
+    dtype and the shape.  float32 operands take the three-term tensor-core product from 192 of k on and the CUDA-core
+    kernel below (by k alone, so that a row's bits do not depend on the rows beside it).
     ``x`` may be a ``NormedInput``: with few rows and bfloat16 weights the norm is
     made inside the product kernel, otherwise it is computed first."""
     if isinstance(x, NormedInput) and weight.dtype == torch.bfloat16 and _rows_kernel(x.n_rows, *weight.shape):
@@ -2157,6 +2181,11 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
         _check(lib.mu_gemm_tc(pa, pw, pb, pr, out.data_ptr(), m, n, k, lda, ldw, out.stride(0), ldr, code,
                               _is_bf16(out), 0, -1, status_word(x.device).data_ptr(), _stream()),
                ("gemm_tc({}x{}x{})", m, n, k))
+    elif (dtype == torch.float32 and out.dtype == torch.float32 and k >= F32_TC_K and k % 4 == 0 and lda % 4 == 0
+          and ldw % 4 == 0 and pa % 16 == 0 and pw % 16 == 0
+          and (x.device in _status or not torch.cuda.is_current_stream_capturing())):   # (its workspace is made outside captures)
+        _check(lib.mu_gemm_f32_tc(pa, pw, pb, pr, out.data_ptr(), m, n, k, lda, ldw, out.stride(0), ldr, code, 0, -1,
+                                  status_word(x.device).data_ptr(), _stream()), ("gemm_f32_tc({}x{}x{})", m, n, k))
     else:
         _check(lib.mu_gemm_simt(pa, pw, pb, pr, out.data_ptr(), m, n, k, lda, ldw, out.stride(0), ldr, code,
                                 _is_bf16(x), _is_bf16(out), _stream()), ("gemm_simt({}x{}x{})", m, n, k))

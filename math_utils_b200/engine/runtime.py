@@ -15,8 +15,9 @@ _ops = None            # the kernel module, imported when first asked for
 class Runtime:
     """``dtype`` is the compute dtype: bfloat16 (the serving path: bfloat16
     weights, activations and cache, float32 accumulation, norms, softmax and
-    residual stream) or float32 (everything in true 32-bit, CUDA-core products
-    only)."""
+    residual stream) or float32 (everything in true 32-bit: products by float32
+    multiply-adds or, over a long k, of three terms on tensor cores with no
+    larger an error)."""
     dtype: torch.dtype
     device: torch.device
 

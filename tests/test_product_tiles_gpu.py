@@ -39,6 +39,47 @@ def test_float32_tiles(m, n, k):
     assert torch.equal(ops.linear(a[m // 2:m // 2 + 1], w, bias), ops.linear(a, w, bias)[m // 2:m // 2 + 1])
 
 
+# one row, rows and columns at and past the ends of warps and tiles, k at the rule's line, past a step, at, past and far past a
+# run of 768
+@pytest.mark.parametrize("m,n,k", [(1, 1, 192), (33, 31, 196), (129, 161, 260), (300, 97, 768), (64, 65, 772), (200, 320, 2308)])
+def test_float32_tensor_tiles(m, n, k):
+    """Operands of 22 bits, sums in float32: within 1e-5 of the rms like the multiply-adds, and no further off in the 2-norm
+    (10 % for the luck of few values); the tile's width, the cut and the rows beside it change no bit."""
+    ops = _ops()
+    a, w = _rand((m, k + 4), 1)[:, :k], _rand((n, k), 2, scale=k ** -0.5)
+    bias, res = _rand((n,), 3), _rand((m, n), 4)
+    plain = a.double() @ w.double().T
+    want = torch.relu(plain + bias.double()) ** 2 + res.double()
+    x = res.clone()
+    ops.linear(a, w, bias, act="relu2", residual=x, out=x)
+    assert float((x.double() - want).abs().max() / want.square().mean().sqrt()) < 1e-5
+    full = ops.linear(a, w)
+    error, before = ((f.double() - plain).norm() for f in (full, ops.gemm_simt(a, w)))
+    assert m * n < 100 or float(error) <= 1.1 * float(before)
+    odd = torch.zeros((m, n + 3), device="cuda")
+    ops.linear(a, w, out=odd[:, 1:n + 1])
+    assert torch.equal(odd[:, 1:n + 1], full) and not odd[:, 0].any() and not odd[:, n + 1:].any()
+    assert torch.equal(ops.linear(a[m // 2:m // 2 + 1], w), full[m // 2:m // 2 + 1])
+    for tile in (32, 64, 96, 128, 160):
+        for cut in (0, 1):
+            assert torch.equal(ops.gemm_f32_tc(a, w, tile=tile, cut=cut), full), (tile, cut)
+    ops.check_status()
+
+
+def test_float32_tensor_tiles_pass_on_what_is_not_finite():
+    """An infinite, NaN or largest value gives what multiply-adds give, in whole and in cut products."""
+    ops = _ops()
+    a, w = _rand((150, 800), 1), _rand((70, 800), 2)
+    a[3, 5], a[70, 100], a[149, 0], w[7, 3], w[9, 9] = float("inf"), float("nan"), 3.4e38, -float("inf"), 1e30
+    want = ops.gemm_simt(a, w)
+    for cut in (0, 1):
+        got = ops.gemm_f32_tc(a, w, cut=cut)
+        known = torch.isfinite(want)
+        assert torch.equal(torch.nan_to_num(got[~known], nan=7.0), torch.nan_to_num(want[~known], nan=7.0))
+        assert torch.equal(torch.isfinite(got), known) and torch.allclose(got[known], want[known], rtol=1e-4, atol=1e-3)
+    ops.check_status()
+
+
 # tiles of 128 slots: an expert without rows, with one, with exactly a tile and one more; few and many experts; columns and
 # k past a box; identity experts (no slots) and weights on the input
 @pytest.mark.parametrize("form,experts,identity,top,tokens,D,F", [
