@@ -67,7 +67,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                             int* status) {
     extern __shared__ unsigned char pt_raw[];
     PtSmem& sm = *reinterpret_cast<PtSmem*>(((uintptr_t)pt_raw + 1023) & ~(uintptr_t)1023);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int item = blockIdx.x;
     const int tile = item / n_heads, h = item % n_heads, kvh = h / (n_heads / n_kv_heads);
     constexpr uint32_t TMEM_COLS = 512;              // scores of group g at 64 g; its P V buffers at 128 + 128 g + {0, 64}
@@ -162,7 +162,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         }
     } else if (warp == 1) {
         // S = Q K^T of every page into the score buffer of the page's softmax group
-        if (lane == 0) {
+        {
+            const bool one = elect_one();
             constexpr uint32_t idesc = idesc_bf16(PT_Q, PT_K);
             const uint32_t q_addr = smem_u32(sm.q);
             ok = mbar_wait_poll(&sm.q_full, 0);
@@ -174,20 +175,22 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t k_addr = smem_u32(sm.k[s]);
+                if (!one) continue;
 #pragma unroll
                 for (int k = 0; k < PT_D / 16; ++k)
                     umma_bf16(tmem_base + 64 * g, smem_desc_sw128(q_addr + k * 32), smem_desc_sw128(k_addr + k * 32), idesc,
                               k > 0 ? 1u : 0u);
                 umma_commit(&sm.s_full[g]);
             }
-            if (!ok) {
+            if (!ok && one) {
                 atomicExch(status, 6);
                 sm.failed = 1;
             }
         }
     } else if (warp == 2) {
         // O_page = P V of every page into one of the two P V buffers of the page's group
-        if (lane == 0) {
+        {
+            const bool one = elect_one();
             constexpr uint32_t idesc = idesc_bf16(PT_Q, PT_D);
             for (int j = 0; j < n_pages && ok; ++j) {
                 const int g = j & 1, u = j >> 1, b = u & 1, s = j % PT_VSTAGES;
@@ -199,13 +202,14 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t p_addr = smem_u32(sm.p[g][b]), v_addr = smem_u32(sm.v[s]);
+                if (!one) continue;
 #pragma unroll
                 for (int k = 0; k < PT_K / 16; ++k)
                     umma_bf16(tmem_base + 128 + 128 * g + 64 * b, smem_desc_sw128(p_addr + k * 32),
                               smem_desc_sw128(v_addr + k * 32), idesc, k > 0 ? 1u : 0u);
                 umma_commit(&sm.pv_full[g][b]);
             }
-            if (!ok) {
+            if (!ok && one) {
                 atomicExch(status, 6);
                 sm.failed = 1;
             }

@@ -45,13 +45,6 @@ F32SplitRoom split_room();                               // (gemm_tc.cu)
 __host__ __device__ constexpr uint32_t idesc_tf32(int m, int n) {
     return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
-// One lane of a warp whose lanes are together (an issuing warp that stays together spends fewer cycles on a product than a
-// lone lane: 8 x 3072 x 768 17.1 us against 20.3).
-__device__ __forceinline__ bool elect_one() {
-    uint32_t e;
-    asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\tselp.b32 %0, 1, 0, e;\n\t}" : "=r"(e));
-    return e != 0;
-}
 __device__ __forceinline__ void umma_tf32_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
                                              uint32_t accumulate) {
     asm volatile(

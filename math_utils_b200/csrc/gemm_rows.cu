@@ -89,7 +89,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     __shared__ uint32_t tmem_slot;
     __shared__ float bias_s[GR_BM];
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int rank = splits > 1 ? (int)cluster_rank() : 0;
     const int tile = blockIdx.x / splits;
     const int n0 = tile * GR_BM;
@@ -153,7 +153,8 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {
+            const bool one = elect_one();
             constexpr uint32_t idesc = idesc_bf16(GR_BM, NB);
             for (int i = 0; i < my_kb && ok; ++i) {
                 const int s = i % stages;
@@ -162,14 +163,15 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t w_addr = smem_u32(w_smem + (size_t)s * GR_W_BYTES);
                 const uint32_t a_addr = smem_u32(a_smem + (size_t)s * A_BYTES);
+                if (!one) continue;
 #pragma unroll
                 for (int k = 0; k < GR_BK / 16; ++k)      // the weights are the instruction's 128-row operand
                     umma_bf16(tmem_acc, smem_desc_sw128(w_addr + k * 32), smem_desc_sw128(a_addr + k * 32), idesc,
                               (i > 0 || k > 0) ? 1u : 0u);
                 umma_commit(&empty[s]);
             }
-            if (ok) umma_commit(&acc_full);
-            else atomicExch(status, 2);
+            if (ok && one) umma_commit(&acc_full);
+            if (!ok && one) atomicExch(status, 2);
         }
     } else {
         // epilogue warps: warp w may read tensor-memory lanes 32 * (w % 4) .. + 31; a lane is an output column

@@ -58,7 +58,7 @@ bool tensor_map_bf16(CUtensorMap* map, const void* base, long long rows, int col
 }
 
 // An output matrix [rows, cols] of bfloat16 or float32 with `ld` elements between rows, cut into boxes of
-// 32 x 32 that lie row after row in shared memory (no swizzle): what the epilogue's bulk stores write.
+// 32 x 32 that lie row after row in shared memory, their 16-byte pieces swizzled over a row: what the epilogue's bulk stores write.
 bool tensor_map_out(CUtensorMap* map, const void* base, long long rows, int cols, long long ld, int is_bf16) {
     const MapKey key = {base, rows, cols, 32, ld, is_bf16 ? 1 : 2};
     const size_t h = ((uintptr_t)base >> 8) * 0x9E3779B97F4A7C15ull + (size_t)rows * 37 + (size_t)cols * 113 + key.kind;
@@ -73,7 +73,7 @@ bool tensor_map_out(CUtensorMap* map, const void* base, long long rows, int cols
     const cuuint32_t box[2] = {32, 32};
     const cuuint32_t elem[2] = {1, 1};
     if (fn(map, is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims,
-           strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+           strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, is_bf16 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return false;
     slot.key = key; slot.map = *map; slot.used = true;

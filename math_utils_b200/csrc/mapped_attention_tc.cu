@@ -201,7 +201,7 @@ mapped_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
     unsigned char* sk = sp + 4 * 2 * MT_BOX;                               // [stages] pages of keys
     unsigned char* sv = sk + a.stages * key_bytes;                         // [stages] pages of values
     MtBars& sm = *reinterpret_cast<MtBars*>(sv + a.stages * val_bytes);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int tile = blockIdx.x / a.n_heads, h = blockIdx.x % a.n_heads, g = h / (a.n_heads / a.n_kv_heads);
     const int kw = a.maps * a.dim, stages = a.stages;
     constexpr uint32_t TMEM_COLS = 512;              // scores of stream i at 64 i, its output at 128 + 128 i
@@ -288,7 +288,8 @@ mapped_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                 mbar_wait(&sm.v_full[j % stages], (uint32_t)((j / stages) & 1));
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {
+            const bool one = elect_one();
             constexpr uint32_t idesc = idesc_bf16(MT_Q, MT_K);
             const uint64_t q_desc = smem_desc_sw128(smem_u32(sq)), k_desc = smem_desc_sw128(smem_u32(sk));
             ok = mbar_wait_poll(&sm.q_full, 0);
@@ -300,6 +301,7 @@ mapped_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                     ok = mbar_wait_poll(&sm.s_free[i], (uint32_t)((u & 1) ^ 1));
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    if (!one) continue;
                     for (int kk = 0; kk < a.dim / 16; ++kk) {
                         const int col = m * a.dim + 16 * kk, t = col >> 6, in = (col & 63) >> 3;      // box, 16-byte piece in its rows
                         umma_bf16(tmem_base + 64 * i, q_desc + (uint64_t)(t * (2 * MT_BOX / 16) + in),
@@ -307,15 +309,16 @@ mapped_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                     }
                     umma_commit(&sm.s_full[i]);
                 }
-                if (ok) umma_commit(&sm.k_empty[s]);         // the keys are free once these products have read them
+                if (ok && one) umma_commit(&sm.k_empty[s]);         // the keys are free once these products have read them
             }
-            if (!ok) {
+            if (!ok && one) {
                 atomicExch(a.status, 6);
                 sm.failed = 1;
             }
         }
     } else if (warp == 2) {
-        if (lane == 0) {
+        {
+            const bool one = elect_one();
             const uint32_t idesc = idesc_bf16(MT_Q, a.vdim) | (1u << 16);                     // the right operand is MN-major
             const uint64_t p_desc = smem_desc_sw128(smem_u32(sp)), v_desc = mt_desc_mn(smem_u32(sv));
             for (int j = 0; j < n_pages && ok; ++j) {
@@ -326,6 +329,7 @@ mapped_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                     ok = mbar_wait_poll(&sm.p_full[i], (uint32_t)(u & 1));
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    if (!one) continue;
 #pragma unroll
                     for (int term = 0; term < 2; ++term)
 #pragma unroll
@@ -335,9 +339,9 @@ mapped_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                                       u > 0 || term > 0 || kk > 0 ? 1u : 0u);
                     umma_commit(&sm.pv_done[i]);
                 }
-                if (ok) umma_commit(&sm.v_empty[s]);
+                if (ok && one) umma_commit(&sm.v_empty[s]);
             }
-            if (!ok) {
+            if (!ok && one) {
                 atomicExch(a.status, 6);
                 sm.failed = 1;
             }

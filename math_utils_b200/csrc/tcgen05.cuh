@@ -108,6 +108,12 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t desc_a, uint
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
 }
+// One lane of a warp whose lanes are together: the issuing warps wait with all lanes and issue with this one.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\tselp.b32 %0, 1, 0, e;\n\t}" : "=r"(e));
+    return e != 0;
+}
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
                  ::"r"(smem_u32(bar)) : "memory");
@@ -146,7 +152,7 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 // 128-byte swizzle (gemm_tc.cu; descriptors are cached by address and shape).  False if the driver refuses.
 bool tensor_map_bf16(CUtensorMap* map, const void* base, long long rows, int cols, long long ld, int box_rows);
 
-// An output matrix [rows, cols] of bfloat16 or float32, cut into boxes of 32 x 32 without swizzle, for the
+// An output matrix [rows, cols] of bfloat16 or float32, cut into boxes of 32 x 32 (rows swizzled), for the
 // bulk stores (and bulk additions) of an epilogue.  The base must be 16-byte aligned and rows 16 bytes apart
 // or a multiple.  False if the driver refuses.
 bool tensor_map_out(CUtensorMap* map, const void* base, long long rows, int cols, long long ld, int is_bf16);
