@@ -14,6 +14,11 @@ int launch_tc_split(int bn, const void* A, const void* W, const float* bias, con
                     int N, int K, long long lda, long long ldw, long long ldc, long long ldr, int act, int out_bf16,
                     int* status, int splits, cudaStream_t s);
 
+// tiles of 256 rows by pairs of SMs (gemm_pair.cu); bn: 128, 192 or 256
+int launch_gemm_pair(int bn, const void* A, const void* W, const float* bias, const float* residual, void* C, int M, int N, int K,
+                     long long lda, long long ldw, long long ldc, long long ldr, int act, int out_bf16, int* status,
+                     cudaStream_t s);
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -134,8 +139,8 @@ MU_EXPORT int mu_gemm_tc_split_workspace(void* parts, long long parts_bytes, int
 // bfloat16 A [M, K] (lda) and W [N, K] (ldw): K, lda, ldw multiples of 8, bases 16-byte aligned.
 // C bfloat16 or float32 (ldc); residual float32 (ldr), may be C itself.  `status` is a device word
 // that stays 0 unless a wait inside the kernel ran out (1 producer, 2 tensor-core issuer, 3 epilogue).
-// tile: width of the tiles of C (64, 128 or 256; 0: chosen here).  splits: parts that K is cut into
-// (-1: chosen here; 0 or 1: never cut; n: n parts wherever K allows).
+// tile: width of the tiles of C (64, 128 or 256; -128, -192 or -256: of a pair of SMs, never cut; 0: chosen here).
+// splits: parts that K is cut into (-1: chosen here; 0 or 1: never cut; n: n parts wherever K allows).
 MU_EXPORT int mu_gemm_tc(const void* A, const void* W, const float* bias, const float* residual, void* C,
                          int M, int N, int K, long long lda, long long ldw, long long ldc, long long ldr,
                          int act, int out_bf16, int tile, int want_splits, int* status, void* stream) {
@@ -146,29 +151,40 @@ MU_EXPORT int mu_gemm_tc(const void* A, const void* W, const float* bias, const 
     if (lda < K || ldw < K || ldc < N || (residual && ldr < N)) return MU_ERR_BAD_ARGUMENT;
     if ((M + mu::TC_BM - 1) / mu::TC_BM > 65535) return MU_ERR_UNSUPPORTED_SIZE;
     cudaStream_t s = (cudaStream_t)stream;
-    // Tile width: wider tiles do more products per byte loaded, but the tiles must also fill whole
-    // rounds of the SMs; take the width with the best (fill of the last round) x (worth of the width).
     const int sms = mu::sm_count();
     if (sms <= 0) return MU_ERR_LAUNCH;
-    if (tile != 0 && tile != 64 && tile != 128 && tile != 256) return MU_ERR_BAD_ARGUMENT;
+    if (tile != 0 && tile != 64 && tile != 128 && tile != 256 && tile != -128 && tile != -192 && tile != -256)
+        return MU_ERR_BAD_ARGUMENT;
     const long long m_tiles = (M + mu::TC_BM - 1) / mu::TC_BM;
-    int best_bn = 64;
-    double best = -1.0;
-    const int widths[3] = {64, 128, 256};
-    const double worth[3] = {0.6, 0.85, 1.0};
-    for (int i = 0; i < 3; ++i) {
-        if (widths[i] > 64 && N <= widths[i] / 2) continue;
-        const long long tiles = m_tiles * ((N + widths[i] - 1) / widths[i]);
-        const long long rounds = (tiles + sms - 1) / sms;
-        const double score = (double)tiles / (double)(rounds * sms) * worth[i];
-        if (score > best) { best = score; best_bn = widths[i]; }
+    // Tile width, and one SM or a pair a tile: by what the SM that ends last has to do, in microseconds.  A launch costs `fixed` (to
+    // the first product and from the last one to the end), a tile 64 of k `step` each or its epilogue, whichever is longer
+    // (float32 1.3 of bfloat16's).  The figures are fitted to 28 sizes from 130 x 1,024 x 64 to 8,192^3, both output types: what
+    // they choose is 0.2 % from the best width on average.  Pairs pay for large tiles, which they feed with fewer bytes, and in
+    // their launch: 2,048 x 1,344 x 2,048 14.8 -> 13.1 us, 2,048 x 1,600 x 6,400 41 -> 31, 4,096^3 116 -> 102 (1,347 TFLOP/s).
+    const struct { int tile; double fixed, step, epilogue; } forms[6] = {
+        {64, 2.8, 0.155, 1.15}, {128, 3.1, 0.21, 2.0}, {256, 4.5, 0.315, 2.8},
+        {-128, 5.0, 0.225, 1.7}, {-192, 4.85, 0.26, 2.3}, {-256, 5.7, 0.28, 3.2}};
+    int best_bn = 64, best_pair = 0;
+    double best = -1.0, best_of_pairs = -1.0;
+    for (int i = 0; i < 6; ++i) {
+        const int bn = forms[i].tile < 0 ? -forms[i].tile : forms[i].tile;
+        const long long rows = forms[i].tile < 0 ? 2 * mu::TC_BM : mu::TC_BM, units = forms[i].tile < 0 ? sms / 2 : sms;
+        if ((bn > 64 && N <= bn / 2) || units == 0) continue;
+        const long long tiles = (M + rows - 1) / rows * ((N + bn - 1) / bn), rounds = (tiles + units - 1) / units;
+        const double products = (K + 63) / 64 * forms[i].step, end = forms[i].epilogue * (out_bf16 ? 1.0 : 1.3);
+        const double cost = forms[i].fixed + rounds * (products > end ? products : end);
+        if (forms[i].tile > 0 ? best < 0.0 || cost < best : best_of_pairs < 0.0 || cost < best_of_pairs) {
+            if (forms[i].tile > 0) best = cost, best_bn = bn;
+            else best_of_pairs = cost, best_pair = bn;
+        }
     }
 #define MU_TC(BN, ST, KS)                                                                                       \
     (out_bf16 ? mu::launch_tc<BN, ST, KS, __nv_bfloat16, false>(A, W, bias, residual, (__nv_bfloat16*)C, M, N, K, \
                                                                 lda, ldw, ldc, ldr, act, status, 1, s)           \
               : mu::launch_tc<BN, ST, KS, float, false>(A, W, bias, residual, (float*)C, M, N, K, lda, ldw, ldc,   \
                                                         ldr, act, status, 1, s))
-    if (tile) best_bn = tile;
+    if (tile > 0) best_bn = tile;
+    if (tile < 0) best_pair = -tile;
     // Few tiles and a long K can be cut along K so that (tiles x parts) fill the SMs.  Handing the parts over
     // (stores, a fence, a ticket, the sum) costs some microseconds, as much as a dozen 64-deep stages of
     // products, so the rule here cuts a K of 2,048 or more into parts of six stages or more.
@@ -189,6 +205,8 @@ MU_EXPORT int mu_gemm_tc(const void* A, const void* W, const float* bias, const 
             tiles * splits * (long long)(mu::TC_BM * best_bn * sizeof(float)) > mu::g_split.parts_bytes)
             splits = 1;
     }
+    if (tile < 0 || (tile == 0 && splits == 1 && want_splits < 0 && best_pair && best_of_pairs < best))
+        return mu::launch_gemm_pair(best_pair, A, W, bias, residual, C, M, N, K, lda, ldw, ldc, ldr, act, out_bf16, status, s);
     if (splits > 1)
         return mu::launch_tc_split(best_bn, A, W, bias, residual, C, M, N, K, lda, ldw, ldc, ldr, act, out_bf16, status,
                                    splits, s);

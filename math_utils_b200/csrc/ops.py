@@ -1651,7 +1651,7 @@ def gemm_tc(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = Non
             out: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None,
             tile: int = 0, splits: int = -1) -> torch.Tensor:
     """The product on the tcgen05 tensor cores (TMA loads, accumulator in tensor memory).
-    ``tile``: width of the output tiles (64, 128, 256; 0: the library chooses); ``splits``: parts that k
+    ``tile``: width of the output tiles (64, 128, 256; -128, -192, -256: by pairs of SMs; 0: the library chooses); ``splits``: parts that k
     is cut into (-1: the library chooses; 0 or 1: none)."""
     m, n, k, out = _gemm_args(a, w, bias, residual, out, out_dtype or a.dtype)
     _check(library().mu_gemm_tc(

@@ -39,6 +39,29 @@ def test_float32_tiles(m, n, k):
     assert torch.equal(ops.linear(a[m // 2:m // 2 + 1], w, bias), ops.linear(a, w, bias)[m // 2:m // 2 + 1])
 
 
+# a pair's tile of 256 rows: none, one and all of the second block's rows, one row more; columns at and past a tile's and a
+# block's half; k of less than a stage, of a stage and more than the ring holds
+@pytest.mark.parametrize("m,n,k", [(1, 8, 8), (128, 130, 64), (129, 256, 72), (256, 97, 200), (257, 520, 1000), (700, 391, 520)])
+@pytest.mark.parametrize("tile", [-128, -192, -256])
+def test_products_by_pairs_of_sms(m, n, k, tile):
+    """The one-SM product's bits: the same products in the same order.  Bulk stores, stores by row (rows that are no whole
+    16-byte pieces), a residual in place and beside."""
+    ops = _ops()
+    dt = torch.bfloat16
+    a, w, bias, res = _rand((m, k), 1, dt), _rand((n, k), 2, dt, k ** -0.5), _rand((n,), 3), _rand((m, n), 4)
+    for kwargs in ({"act": "gelu_new"}, {"residual": res, "out_dtype": torch.float32, "act": "relu2"}):
+        want, got = (ops.gemm_tc(a, w, bias, tile=t, splits=0, **kwargs) for t in (64, tile))
+        assert torch.equal(got, want)
+    plain = a.double() @ w.double().T + bias.double()
+    x, odd = res.clone(), torch.zeros((m, n + 3), dtype=torch.float32, device="cuda")
+    ops.gemm_tc(a, w, bias, residual=x, out=x, tile=tile)
+    ops.gemm_tc(a, w, bias, out=odd[:, 1:n + 1], tile=tile)
+    assert float((x.double() - plain - res.double()).abs().max()) < 1e-5 * max(1.0, float(plain.abs().max()))
+    assert float((odd[:, 1:n + 1].double() - plain).abs().max()) < 1e-5 * max(1.0, float(plain.abs().max()))
+    assert not odd[:, 0].any() and not odd[:, n + 1:].any()
+    ops.check_status()
+
+
 # one row, rows and columns at and past the ends of warps and tiles, k at the rule's line, past a step, at, past and far past a
 # run of 768
 @pytest.mark.parametrize("m,n,k", [(1, 1, 192), (33, 31, 196), (129, 161, 260), (300, 97, 768), (64, 65, 772), (200, 320, 2308)])
