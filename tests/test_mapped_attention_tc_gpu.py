@@ -317,3 +317,38 @@ def test_queries_rotate_more_pairs_than_a_block_keeps_angles_of():
     lo, hi = q.double().reshape(T, H, 2, rot // 2).unbind(2)
     want = torch.stack([lo * cos - hi * sin, hi * cos + lo * sin], 2).reshape(T, -1)
     assert float((qa.double() - want).abs().max()) < 1e-5
+
+
+# pieces of eight entries: one a slice, lanes without a piece (24, 40, 96, 200), all of a warp's; no rotation, a part of the slice
+# and all of it, by halves and by pairs (6: within a piece); with and without norms; more slices than a block takes at once
+@pytest.mark.parametrize("heads,kv_heads,maps,dim,vdim,rot,pairs,normed", [
+    (3, 1, 1, 8, 8, 0, False, True), (4, 2, 2, 24, 16, 16, False, True), (5, 1, 1, 40, 24, 6, True, False),
+    (16, 4, 2, 64, 128, 32, False, True), (8, 8, 1, 96, 96, 96, False, True), (4, 2, 1, 128, 64, 128, True, True),
+    (2, 1, 1, 200, 40, 16, False, False), (9, 3, 1, 256, 128, 32, True, True)])
+def test_preparation_by_pieces_is_the_general_one(heads, kv_heads, maps, dim, vdim, rot, pairs, normed):
+    """Against the form for any alignment (rows one entry off): float32 in between, so a result differs by the last bit of a
+    bfloat16 (2^-7 of its size at most) where a sum of another order rounds the other way, and rarely."""
+    from math_utils_b200.csrc import ops
+    rng = np.random.default_rng(dim)
+    T, qw, kw, vw = 70, heads * maps * dim, kv_heads * maps * dim, kv_heads * vdim
+    width = qw + kw + vw
+    x = torch.as_tensor(rng.normal(0, 2, (T, width)), dtype=torch.float32).cuda().bfloat16()
+    weights = [torch.as_tensor(rng.normal(1, 0.2, dim), dtype=torch.float32).cuda() if normed else None for _ in range(2)]
+    freqs = torch.as_tensor(300.0 ** -np.linspace(0, 1, max(rot // 2, 1)), dtype=torch.float32).cuda()
+    ints = lambda a: torch.as_tensor(np.asarray(a), dtype=torch.int32).cuda()
+    pos, table = ints(np.arange(T) + 30), ints([[2, 0]])
+    got = []
+    for off in (0, 1):
+        proj = torch.zeros((T, width + 8 if off == 0 else width + 9), dtype=torch.bfloat16, device="cuda")
+        proj[:, off:off + width] = x
+        rows = torch.zeros((3, 64, kw + vw), dtype=torch.bfloat16, device="cuda")
+        q, k, v = proj[:, off:off + qw], proj[:, off + qw:off + qw + kw], proj[:, off + qw + kw:off + width]
+        ops.qk_prepare(q, k, v, *weights, freqs, 1.25, rot, 1e-3, heads, kv_heads, maps, dim, vdim, pos, ints([0] * T), table, 64,
+                       rows, pairs=pairs)
+        assert not proj[:, :off].any() and not proj[:, off + width:].any()
+        got.append((q.float().clone(), rows.float()))
+    for a, b in zip(*got):
+        assert ((a - b).abs() <= b.abs() * 2.0 ** -7).all() and float((a != b).float().mean()) < 0.01
+    untouched = torch.ones(3, 64, dtype=torch.bool)
+    untouched[2, 30:] = untouched[0, :36] = False
+    assert not got[0][1][untouched.cuda()].any()
