@@ -11,15 +11,15 @@
 // 128 rows of A begin at its first slot; what follows an expert's last slot belongs to the next one (or lies past the
 // matrix and is zero), is multiplied along and never stored: a row of the accumulator depends on its own row of A alone.
 // The rows are gathered by a launch of their own, which costs what reading and writing them once costs and lets TMA fetch
-// whole boxes.  Consecutive work items are different tiles of one column block, so an expert's tiles, which read the same
-// weights, run side by side and the weights cross from memory once.
+// whole boxes.  The items' order (tiles_first) keeps an expert's tiles close together, so the weights cross from
+// memory once.
 //
-// What bounds it: with few rows an expert the weights' bytes (nothing is computed for the rows a tile lacks that takes
-// longer than fetching its weights); with hundreds, the operands' way from the L2, 48 KB for every 128 x 256 x 64 step.
-// Measured (B200): 64 experts of 2,048 x 1,408 x 3, 12,288 pairs, first product 586 -> 213 us, second 357 -> 147 us (143 GFLOP
-// in 213 us, 670 TFLOP/s, with a quarter of the tiles' rows empty; the weights alone take 113 and 56 us), the gather ~20 us,
-// the whole feed-forward 1,002 -> 502 us; 48 pairs over those experts with two matrices each 136 -> 93 us.  mma.sync with 64
-// rows a block gave the first figures.  Per head, 16 heads, 2,048 rows, the launch alone: 512 x 128 36 -> 25 us, 128 x 512 26 -> 9;
+// What bounds it: the weights' bytes, and with hundreds of rows an expert their products beside them, a quarter of the tiles'
+// rows empty.  Measured (B200): 64 experts of 2,048 x 1,408 x 3, 12,288 pairs, both products: mma.sync with 64 rows a block
+// 943 us; tiles of 128 slots 338, tile by tile 297 (the weights alone take 113 + 56 us); the gather ~10 us; 48 pairs over those
+// experts with two matrices each, the whole feed-forward 136 -> 93 us.  Tiles of 256 slots by pairs of SMs (cta_group::2)
+// took 263 us with equal experts, but where routing loads them unequally their emptier tiles cost what the feeding saves
+// (the whole feed-forward 447 us against 436).  Per head, 16 heads, 2,048 rows, the launch alone: 512 x 128 36 -> 25 us, 128 x 512 26 -> 9;
 // at 300 rows 8.3 -> 8.5 and 14.5 -> 6.0.
 #include "gemm_tc_kernel.cuh"
 
@@ -34,12 +34,12 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                   const __grid_constant__ CUtensorMap map_w2, const int* __restrict__ tile_info,
                   const int* __restrict__ n_tiles, const int* __restrict__ pair_of, const float* __restrict__ row_weight,
                   int n, int k, TC* __restrict__ out, long long ldo, int act, int* status, int n_rows, int n_groups,
-                  int x_group_offset, long long out_group_offset, const __nv_bfloat16* __restrict__ gate, long long ldg) {
+                  int x_group_offset, long long out_group_offset, const __nv_bfloat16* __restrict__ gate, long long ldg, int tile_first) {
     constexpr int BN = 128 * NB, STAGES = NB == 2 ? 4 : 3, KSUB = NB == 2 ? 1 : 2, OUT_COLS = GATED ? 128 : BN;
     typedef TcSmem<BN, STAGES, KSUB> Smem;
     extern __shared__ unsigned char tc_raw[];
     Smem& sm = *reinterpret_cast<Smem*>(((uintptr_t)tc_raw + 1023) & ~(uintptr_t)1023);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     // (a sub-tile that would begin past k is neither fetched nor multiplied: by head there lies the gap after the slice, or the
     // next head's slice, and zeros of the weights do not make a product with an infinity or a NaN zero)
     const int num_kb = (k + KSUB * TC_BK - 1) / (KSUB * TC_BK);
@@ -73,14 +73,15 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     const int items = tiles * n_blocks * (by_head ? n_groups : 1);
     struct Item { int group, row0, rows, n0; };
     auto item_at = [&](int item) {
-        const int tile = item % tiles, rest = item / tiles;
         Item w;
         if (by_head) {
+            const int tile = item % tiles, rest = item / tiles;
             w.group = rest / n_blocks, w.row0 = tile * TC_BM, w.rows = min(TC_BM, n_rows - w.row0);
             w.n0 = rest % n_blocks * OUT_COLS;
         } else {
-            w.group = tile_info[3 * tile], w.row0 = tile_info[3 * tile + 1], w.rows = tile_info[3 * tile + 2];
-            w.n0 = rest * OUT_COLS;
+            const int* info = tile_info + 3 * (tile_first ? item / n_blocks : item % tiles);
+            w.group = info[0], w.row0 = info[1], w.rows = info[2];
+            w.n0 = (tile_first ? item % n_blocks : item / tiles) * OUT_COLS;
         }
         return w;
     };
@@ -122,7 +123,8 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {
+            const bool one = elect_one();
             constexpr uint32_t idesc = idesc_bf16(TC_BM, BN);
             const uint64_t a_desc0 = smem_desc_sw128(smem_u32(sm.a[0][0]));
             const uint64_t b_desc0 = smem_desc_sw128(smem_u32(sm.b[0][0]));
@@ -143,6 +145,7 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                     const uint64_t a_stage = a_desc0 + (uint64_t)((uint32_t)s * (KSUB * A_SUB));
                     const uint64_t b_stage = b_desc0 + (uint64_t)((uint32_t)s * (KSUB * B_SUB));
                     const int subs = sub_tiles(kb);
+                    if (!one) continue;
 #pragma unroll
                     for (int u = 0; u < KSUB; ++u) {
                         if (u > 0 && u >= subs) break;
@@ -153,9 +156,9 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                     }
                     umma_commit(&sm.empty[s]);
                 }
-                if (ok) umma_commit(&sm.acc_full[buf]);
+                if (ok && one) umma_commit(&sm.acc_full[buf]);
             }
-            if (!ok) atomicExch(status, 2);
+            if (!ok && one) atomicExch(status, 2);
         }
     } else {
         const int quad = warp & 3, half = (warp - 2) / 4;       // 32 rows and half of the columns a warp, as in gemm_tc
@@ -230,6 +233,15 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
 }
 
+// The order of the items.  One column block after another for all tiles reads every expert's tiles side by side, and the rows once
+// a column block; once these no longer stay in the L2 beside the weights that pass through it they come from memory each time,
+// and the items go tile by tile, all its column blocks together (an expert's tiles still follow one another).  64 experts
+// of 2,048 x 1,408 x 3, pairs and their rows' megabytes, microseconds of the first product by column blocks and by tiles:
+// 1,024 (4) 132 and 131, 4,096 (17) 138 and 131, 6,144 (25) 146 and 136, 12,288 (50) 220 and 191; of two matrices 68 and 70,
+// 72 and 76, 82 and 72, 128 and 109.
+constexpr long long GROUPED_ROWS_KEPT = 17000000;
+inline bool tiles_first(long long rows, int k) { return rows * k * 2 > GROUPED_ROWS_KEPT; }
+
 template <int NB, bool GATED, typename TC>
 static int launch_grouped(const void* x, long long x_rows, int x_cols, long long ldx, const void* w1, const void* w2,
                           long long w_rows, long long ldw, const int* tile_info, const int* n_tiles, const int* pair_of,
@@ -250,7 +262,7 @@ static int launch_grouped(const void* x, long long x_rows, int x_cols, long long
     if (sms <= 0) return MU_ERR_LAUNCH;
     const dim3 grid((unsigned)(most_items < sms ? most_items : sms));
     return launch_pdl(kernel, grid, dim3(TC_THREADS), smem, s, 1, a, b1, b2, tile_info, n_tiles, pair_of, row_weight, n, k, out,
-                      ldo, act, status, n_rows, n_groups, x_group_offset, out_group_offset, (const __nv_bfloat16*)gate, ldg);
+                      ldo, act, status, n_rows, n_groups, x_group_offset, out_group_offset, (const __nv_bfloat16*)gate, ldg, (int)tiles_first(x_rows, k));
 }
 
 // A warp a pair: its token's row to the pair's slot, sixteen bytes a lane at a time.
