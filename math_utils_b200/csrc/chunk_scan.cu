@@ -20,8 +20,8 @@
 //
 // What bounds it: dependent products of three warps a scheduler, which issue in half of the cycles and wait for fixed latencies
 // and the pipe otherwise; the token-by-token forms are bound by the chain of 1,024 tokens a sequence.  Measured (B200,
-// 2 x 1,024 tokens): 16 heads of 128 x 64 by key 319 -> 28 + 8 + 64 us (the state-space layer 365 -> 145 us), 8 heads of 128 x
-// 128 with normalizer over 2,018 tokens 185 -> 26 + 8 + 64 us (the matrix memory's layer 265 -> 171 us); one sequence of some 300
+// 2 x 1,024 tokens): the state-space layer of 16 heads of 128 x 64 by key 365 us token by token, 123 in chunks, the matrix memory's
+// of 8 heads of 128 x 128 with normalizer over 2,018 tokens 265 and 146; one sequence of some 300
 // tokens gains half, wide batches of the matrix memory nothing (matrix_lstm.py has the rule).
 #include "common.cuh"
 
@@ -30,6 +30,7 @@
 namespace mu {
 
 constexpr int CS_TOK = 64, CS_COLS = 64, CS_THREADS = 256;
+constexpr int CS_PP = CS_TOK + 8;                             // a row of the weights in shared memory: 8 banks apart
 
 // Where a chunk's part of the scratch lies (as lightning_prompt.cu): no two chunks of a step share a place.
 __device__ __forceinline__ long long cs_place(int flat0, int s, int first) { return first / CS_TOK + s + (flat0 - first) / CS_TOK; }
@@ -69,9 +70,13 @@ __device__ __forceinline__ void cs_copy8(float* dst, const float* src, bool ther
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
                  "r"(there ? 8 : 0) : "memory");
 }
+// x rounded to TF32 (to nearest, ties away from zero) as two integer operations: the conversion instruction gives the same bits at
+// a fraction of their rate (with the rest's conversion as it was: state space 140 -> 132 us, matrix memory 161 -> 153).  A NaN
+// of all ones comes out as zero; what that leaves of it is NaN, which the instruction keeps.
+__device__ __forceinline__ uint32_t cs_tf32(float x) { return (__float_as_uint(x) + 0x1000u) & 0xffffe000u; }
 // x as two TF32 terms: the rounded value, and what the rounding left.
 __device__ __forceinline__ void cs_split(float x, uint32_t& hi, uint32_t& lo) {
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hi) : "f"(x));
+    hi = cs_tf32(x);
     asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lo) : "f"(x - __uint_as_float(hi)));
 }
 __device__ __forceinline__ void cs_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
@@ -86,7 +91,7 @@ constexpr float CS_CUT = 4.3e-8f;
 
 // x as two TF32 terms that are together longer than x by that share.
 __device__ __forceinline__ void cs_split_more(float x, uint32_t& hi, uint32_t& lo) {
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hi) : "f"(x));
+    hi = cs_tf32(x);
     asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lo) : "f"(fmaf(x, CS_CUT, x - __uint_as_float(hi))));
 }
 
@@ -280,7 +285,10 @@ chunk_states_kernel(const __grid_constant__ ChunkArgs a) {
     *kept = S;
 }
 
-// A block takes a chunk, a head and 64 value columns; a warp 16 tokens and 32 of the columns.  Along dk the lanes take
+// A block takes a chunk, a head and 64 value columns; a warp 16 tokens and 32 of the columns.  The two warps of the same tokens
+// make the weights of half of their keys each and find the rest in shared memory (each made all of them before: state space
+// 132 -> 123 us, matrix memory 153 -> 146).
+// Along dk the lanes take
 // their entries four at a time (lane tig's k slots of two steps of 8 are entries 4 tig .. 4 tig + 3 of 16), so queries come
 // as 16-byte loads from global memory and keys and states by value as 16-byte loads from shared memory.
 template <bool BY_KEY, typename TD>
@@ -292,7 +300,8 @@ chunk_outputs_kernel(const __grid_constant__ ChunkArgs a) {
     const int kp = (a.dk + 31) / 32 * 32 + 16;
     float* Ks = cs_sm;                                         // [64 tokens][kp]
     float* Vs = Ks + CS_TOK * kp;                              // [64 tokens][VP]
-    float* Ss = Vs + CS_TOK * VP;                              // [64 columns][kp], or by key [dk][SP]
+    float* Ps = Vs + CS_TOK * VP;                              // [64 tokens][PP] weights of the keys
+    float* Ss = Ps + CS_TOK * CS_PP;                           // [64 columns][kp], or by key [dk][SP]
     pdl_trigger();
     pdl_wait();
     const int flat0 = a.tiles[2 * blockIdx.x], count = min(a.tiles[2 * blockIdx.x + 1], CS_TOK), h = blockIdx.y;
@@ -321,7 +330,7 @@ chunk_outputs_kernel(const __grid_constant__ ChunkArgs a) {
     const int warp = (threadIdx.x >> 5) & 3, half0 = (threadIdx.x >> 7) * 32;
     const int lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
     const bool norm = a.norm_sums != nullptr && col0 == 0 && half0 == 0;
-    if (warp * 16 >= count || half0 >= cols) return;
+    const bool mine = warp * 16 < count;
     // The last sixteen keys of a warp are its own tokens: those after a token have the weight zero, which does not keep an
     // infinite or NaN value out of a product.  With such a value among them they are added key by key.
     float odd = 0.0f;                                          // NaN from the first value that is not finite on
@@ -335,11 +344,12 @@ chunk_outputs_kernel(const __grid_constant__ ChunkArgs a) {
     const float* q0 = a.q + (long long)(flat0 + min(t0, count - 1)) * a.ld + key_at + 4 * tig;
     const float* q1 = a.q + (long long)(flat0 + min(t1, count - 1)) * a.ld + key_at + 4 * tig;
     const float* nrow = norm ? a.norm_sums + at * dk + 4 * tig : q0;
-    const int key_tiles = 2 * (warp + 1);                      // runs of 8 keys that this warp's tokens see
-    float o[4][4] = {}, w[CS_TOK / 8][4] = {}, den0 = 0.0f, den1 = 0.0f;
+    const int key_tiles = 2 * (warp + 1), own_tiles = warp + 1;         // runs of 8 keys that these tokens see, and this warp's
+    const int own0 = half0 ? 8 * own_tiles : 0;                // the first of its keys
+    float o[4][4] = {}, w[CS_TOK / 16][4] = {}, den0 = 0.0f, den1 = 0.0f;
     float4 x0 = *reinterpret_cast<const float4*>(q0), x1 = *reinterpret_cast<const float4*>(q1);
     float4 nv = *reinterpret_cast<const float4*>(nrow);
-    for (int k0 = 0; k0 < dk; k0 += 16) {
+    for (int k0 = 0; mine && k0 < dk; k0 += 16) {
         const float4 c0 = x0, c1 = x1, cn = nv;
         const int next = k0 + 16 < dk ? k0 + 16 : k0;
         x0 = *reinterpret_cast<const float4*>(q0 + next);
@@ -370,9 +380,9 @@ chunk_outputs_kernel(const __grid_constant__ ChunkArgs a) {
             cs_products(o[j], ah, al, f.x, f.y, f.z, f.w);
         }
 #pragma unroll
-        for (int j = 0; j < CS_TOK / 8; ++j) {
-            if (j >= key_tiles) break;
-            const float4 f = *reinterpret_cast<const float4*>(Ks + (8 * j + gid) * kp + k0 + 4 * tig);
+        for (int j = 0; j < CS_TOK / 16; ++j) {
+            if (j >= own_tiles) break;
+            const float4 f = *reinterpret_cast<const float4*>(Ks + (own0 + 8 * j + gid) * kp + k0 + 4 * tig);
             cs_products(w[j], ah, al, f.x, f.y, f.z, f.w);
         }
     }
@@ -384,6 +394,22 @@ chunk_outputs_kernel(const __grid_constant__ ChunkArgs a) {
         o[j][2] *= f1, o[j][3] *= f1;
     }
     den0 *= f0, den1 *= f1;
+    if (mine) {
+#pragma unroll
+        for (int j = 0; j < CS_TOK / 16; ++j) {
+            if (j >= own_tiles) break;
+            const int s0 = own0 + 8 * j + 2 * tig, s1 = s0 + 1;
+            const float (&x)[4] = w[j];
+            const float p0 = s0 <= t0 ? x[0] * (expf((h0 - l_hi[s0]) + (e0 - l_lo[s0])) * b[s0]) : 0.0f;
+            const float p1 = s1 <= t0 ? x[1] * (expf((h0 - l_hi[s1]) + (e0 - l_lo[s1])) * b[s1]) : 0.0f;
+            const float p2 = s0 <= t1 ? x[2] * (expf((h1 - l_hi[s0]) + (e1 - l_lo[s0])) * b[s0]) : 0.0f;
+            const float p3 = s1 <= t1 ? x[3] * (expf((h1 - l_hi[s1]) + (e1 - l_lo[s1])) * b[s1]) : 0.0f;
+            *reinterpret_cast<float2*>(Ps + t0 * CS_PP + s0) = make_float2(p0, p1);
+            *reinterpret_cast<float2*>(Ps + t1 * CS_PP + s0) = make_float2(p2, p3);
+        }
+    }
+    __syncthreads();
+    if (!mine || half0 >= cols) return;
 #pragma unroll
     for (int n = 0; n < CS_TOK / 8; n += 2) {
         if (n >= key_tiles) break;
@@ -391,18 +417,14 @@ chunk_outputs_kernel(const __grid_constant__ ChunkArgs a) {
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
             // a pair of keys a lane: its slots of this step are keys 2 tig and 2 tig + 1 of the eight
-            const int s0 = 8 * (n + u) + 2 * tig, s1 = s0 + 1;
-            const float (&x)[4] = w[n + u];
-            const float p0 = s0 <= t0 ? x[0] * (expf((h0 - l_hi[s0]) + (e0 - l_lo[s0])) * b[s0]) : 0.0f;
-            const float p1 = s1 <= t0 ? x[1] * (expf((h0 - l_hi[s1]) + (e0 - l_lo[s1])) * b[s1]) : 0.0f;
-            const float p2 = s0 <= t1 ? x[2] * (expf((h1 - l_hi[s0]) + (e1 - l_lo[s0])) * b[s0]) : 0.0f;
-            const float p3 = s1 <= t1 ? x[3] * (expf((h1 - l_hi[s1]) + (e1 - l_lo[s1])) * b[s1]) : 0.0f;
-            den0 += p0 + p1;
-            den1 += p2 + p3;
-            cs_split(p0, ph[u][0], pl[u][0]);
-            cs_split(p2, ph[u][1], pl[u][1]);
-            cs_split(p1, ph[u][2], pl[u][2]);
-            cs_split(p3, ph[u][3], pl[u][3]);
+            const float2 pa = *reinterpret_cast<const float2*>(Ps + t0 * CS_PP + 8 * (n + u) + 2 * tig);
+            const float2 pb = *reinterpret_cast<const float2*>(Ps + t1 * CS_PP + 8 * (n + u) + 2 * tig);
+            den0 += pa.x + pa.y;
+            den1 += pb.x + pb.y;
+            cs_split(pa.x, ph[u][0], pl[u][0]);
+            cs_split(pb.x, ph[u][1], pl[u][1]);
+            cs_split(pa.y, ph[u][2], pl[u][2]);
+            cs_split(pb.y, ph[u][3], pl[u][3]);
         }
         if (plain || n + 2 < key_tiles) {
 #pragma unroll
@@ -458,11 +480,11 @@ static int launch_chunks(const ChunkArgs& a, int n_tiles, int n_seqs, cudaStream
     const int M = BY_KEY ? a.dk : a.dv, N = BY_KEY ? a.dv : a.dk;
     const size_t smem1 = sizeof(float) * CS_TOK * ((M + 31) / 32 * 32 + 8 + (N + 63) / 64 * 64 + 8);
     const int kp = (a.dk + 31) / 32 * 32 + 16;
-    const size_t smem3 = sizeof(float) * (CS_TOK * kp + CS_TOK * (CS_COLS + 4) + (BY_KEY ? a.dk * (CS_COLS + 2) : CS_COLS * kp));
+    const size_t smem3 = sizeof(float) * (CS_TOK * kp + CS_TOK * (CS_COLS + 4) + CS_TOK * CS_PP + (BY_KEY ? a.dk * (CS_COLS + 2) : CS_COLS * kp));
     auto k1 = chunk_sums_kernel<BY_KEY, TD>;
     auto k3 = chunk_outputs_kernel<BY_KEY, TD>;
-    if (!allow_shared((const void*)k1, 140 * 1024) || !allow_shared((const void*)k3, 100 * 1024) || smem1 > 140 * 1024 ||
-        smem3 > 100 * 1024)
+    if (!allow_shared((const void*)k1, 140 * 1024) || !allow_shared((const void*)k3, 112 * 1024) || smem1 > 140 * 1024 ||
+        smem3 > 112 * 1024)
         return MU_ERR_LAUNCH;
     prefer_shared_memory((const void*)k1);
     prefer_shared_memory((const void*)k3);
