@@ -263,3 +263,18 @@ def test_router_of_several_tokens_a_block(tokens, hidden, experts, gate):
     for t in (0, 7, tokens - 1):
         e1, w1, g1 = route(h[t:t + 1])
         assert torch.equal(e1[0], expert[t]) and torch.equal(w1[0], weight[t]) and (not gate or torch.equal(g1[0], out[t]))
+
+
+# clusters of eight blocks, of four and single blocks a token at their lines (half the SMs, all of them); lanes with a piece more
+@pytest.mark.parametrize("tokens", [1, 74, 75, 148, 149])
+def test_router_of_few_tokens_by_clusters(tokens):
+    """The bits of the form for many tokens."""
+    ops = _ops()
+    h, router = _rand((600, 520), 1, torch.bfloat16), _rand((70, 520), 2, scale=520 ** -0.5)
+
+    def route(x):
+        expert, weight = torch.zeros(x.shape[0] * 4, dtype=torch.int32, device="cuda"), torch.zeros(x.shape[0] * 4, device="cuda")
+        ops.moe_route(x, router, None, 4, 1.0, expert, weight)
+        return expert, weight
+
+    assert all(torch.equal(few, many[:tokens * 4]) for few, many in zip(route(h[:tokens]), route(h)))
