@@ -17,29 +17,35 @@
 // to arrival: a step of 32 took 0.42 us (32 columns), 0.67 (96), 0.80 (128) and 1.0 (160) whatever of the splitting,
 // the products or the sums was left out alone, so two teams of eight warps split every other step.  Measured (B200,
 // microseconds; the multiply-adds in brackets): 777 x 3072 x 768 30 (121), 777 x 768 x 3072 40 (129), 2048 x 4096 x 4096 412
-// (1,700; 167 TFLOP/s), 8 x 3072 x 768 15 (19), 8 x 768 x 3072 17 (66).
+// (1,700; 167 TFLOP/s), 8 x 3072 x 768 14 (19), 8 x 768 x 3072 12.5 (66).
 //
-// A tile's sum is, for every run of GROUP of k, the sum of its steps in order, and then the runs' sums in order.  A product of
-// few tiles is cut into those runs (CUT: parts to the library's workspace, the last block of a tile adds them in order), so
-// a row's result is the same bits whatever the cut, the tile's width and the rest of the step are.
+// A tile's sum is, for every run of k, the sum of its steps in order, and then the runs' sums in order; how long a run is
+// follows from k alone.  A product of few tiles is cut into those runs (CUT): a cluster of blocks has a tile, each block
+// a run, and every block adds the runs of its share of the columns, in order, as they lie in the other blocks' shared memory.  So
+// a row's result is the same bits whatever the cut, the tile's width and the rest of the step are, and no launch keeps
+// anything in device memory that another one, on another stream, could meet.
 //
 // A value that is infinite, or NaN, or rounds to infinity in 11 bits, has parts that make NaN where float32 gives
 // an infinity; so a sum that comes out not finite is made once more by multiply-adds, by the lane that stores it.
 #include "tcgen05.cuh"
 
+#include <atomic>
+
 namespace mu {
 
 constexpr int FC_BM = 128, FC_BK = 32, FC_WORKERS = 16, FC_THREADS = 64 + 32 * FC_WORKERS;
-constexpr int FC_GROUP = 24;                             // steps of 32 whose sums are one run
+constexpr int FC_RUN = 24, FC_RUNS = 8;                  // a run's steps of 32, if k has no more than that many runs
+// Steps of a run: runs of one length, as few as FC_RUN allows (a cluster has eight blocks).
+inline int fc_group(int steps) {
+    const int runs = (steps + FC_RUN - 1) / FC_RUN;
+    return (steps + (runs < FC_RUNS ? runs : FC_RUNS) - 1) / (runs < FC_RUNS ? runs : FC_RUNS);
+}
 constexpr int FC_TEAM = FC_WORKERS / 2;                  // two teams of warps split every other step
 // What tensor cores cut off of an accumulator's four large additions is 2^-23 of it on average; it is given back.
 constexpr float FC_GIVE_BACK = 1.0f + 1.1920929e-7f;
 constexpr int FC_PITCH = 9;                              // floats a row of an epilogue patch (32 rows x 8 columns)
 
 bool tensor_map_f32(CUtensorMap* map, const void* base, long long rows, int cols, long long ld, int box_rows);
-
-struct F32SplitRoom { float* parts; long long bytes; int* tickets; int n_tickets; };
-F32SplitRoom split_room();                               // (gemm_tc.cu)
 
 // Instruction descriptor of kind::tf32: float32 accumulator, TF32 operands (2 at bits 7 and 10), both K-major.
 __host__ __device__ constexpr uint32_t idesc_tf32(int m, int n) {
@@ -81,9 +87,7 @@ struct FcSmem {
     float patch[FC_WORKERS][fc_room<BN>(RUNS)];          // a warp's patch, and before that (RUNS) its sum of the runs so far
     uint64_t full[STAGES], split[STAGES], empty[STAGES]; // loaded; split into parts; read by the products
     uint64_t acc_full[2], acc_empty[2];
-    uint64_t part_stored, part_decided;
     uint32_t tmem_base;
-    int part_last;
 };
 
 // The sum once more by multiply-adds in the order of k.
@@ -99,9 +103,7 @@ struct FcArgs {
     int M, N, K;
     long long lda, ldw, ldc, ldr;
     int* status;
-    int cut;                                             // parts of a tile (CUT), else 1
-    float* parts;
-    int* tickets;
+    int group, runs;                                     // steps of a run, runs of k
 };
 
 template <int ACT> __device__ __forceinline__ float fc_act(float x) {
@@ -140,7 +142,16 @@ __device__ __forceinline__ void fc_finish(const FcArgs& g, const float* sum, flo
     }
 }
 
-// RUNS: a block sums several runs of a tile.  CUT: a block's item is one run of a tile.
+__device__ __forceinline__ void fc_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float4 fc_load_remote(uint32_t addr) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+
+// RUNS: a block sums several runs of a tile.  CUT: a cluster's blocks (along y) have a run of one tile each.
 template <int BN, int STAGES, bool RUNS, bool CUT>
 __global__ void __launch_bounds__(FC_THREADS, 1)
 gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const FcArgs g, int act) {
@@ -150,12 +161,10 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     constexpr uint32_t TMEM_COLS = COLS <= 128 ? 128 : COLS <= 256 ? 256 : 512;
     static_assert(COLS <= 512 && BN % 32 == 0, "tensor memory");
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-    const int steps = (g.K + FC_BK - 1) / FC_BK, cut = CUT ? g.cut : 1;
+    const int steps = (g.K + FC_BK - 1) / FC_BK;
     const int m_tiles = (g.M + FC_BM - 1) / FC_BM, n_tiles = (g.N + BN - 1) / BN;
-    const int items = m_tiles * n_tiles * cut;
-    // steps of an item: its run, or all
-    auto first_step = [&](int item) { return CUT ? item % cut * FC_GROUP : 0; };
-    auto last_step = [&](int item) { return CUT ? min(steps, (item % cut + 1) * FC_GROUP) : steps; };
+    const int tiles = m_tiles * n_tiles;
+    const int begin = CUT ? (int)blockIdx.y * g.group : 0, end = CUT ? min(steps, begin + g.group) : steps;      // this block's steps
     bool ok = true;
 
     if (threadIdx.x == 0) {
@@ -163,8 +172,6 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         tma_prefetch_map(&map_w);
         for (int s = 0; s < STAGES; ++s) { mbar_init(&sm.full[s], 1); mbar_init(&sm.split[s], FC_TEAM); mbar_init(&sm.empty[s], 1); }
         for (int b = 0; b < 2; ++b) { mbar_init(&sm.acc_full[b], 1); mbar_init(&sm.acc_empty[b], FC_WORKERS); }
-        mbar_init(&sm.part_stored, FC_WORKERS);
-        mbar_init(&sm.part_decided, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -182,9 +189,9 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     if (warp == 0) {
         if (lane == 0) {
             int it = 0, issued = 0;
-            for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
-                const int tile = item / cut, m0 = tile % m_tiles * FC_BM, n0 = tile / m_tiles * BN;
-                for (int st = first_step(item); st < last_step(item); ++st, ++it) {
+            for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+                const int m0 = tile % m_tiles * FC_BM, n0 = tile / m_tiles * BN;
+                for (int st = begin; st < end; ++st, ++it) {
                     const int s = it % STAGES;
                     ok = mbar_wait(&sm.empty[s], (uint32_t)((it / STAGES & 1) ^ 1));
                     if (!ok) break;
@@ -205,9 +212,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         const bool one = elect_one();
         const uint64_t hi0 = smem_desc_sw128(smem_u32(sm.w_hi[0])), lo0 = smem_desc_sw128(smem_u32(sm.w_lo[0]));
         int it = 0;
-        for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
-            const int end = last_step(item);
-            for (int st = first_step(item); st < end; ++st, ++it) {
+        for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+            for (int st = begin; st < end; ++st, ++it) {
                 const int s = it % STAGES, buf = it & 1;
                 ok = mbar_wait(&sm.split[s], (uint32_t)(it / STAGES & 1)) &&
                      mbar_wait(&sm.acc_empty[buf], (uint32_t)((it >> 1 & 1) ^ 1));
@@ -233,8 +239,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         const uint32_t lanes = tmem + ((uint32_t)(quad * 32) << 16);
         const bool rows_here = g.M > quad * 32;          // a single row of tiles may leave whole warps without rows
         float* patch = sm.patch[warp - 2];
-        int total = 0;
-        for (int item = blockIdx.x; item < items; item += gridDim.x) total += last_step(item) - first_step(item);
+        const int total = ((int)blockIdx.x < tiles ? (tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0) * (end - begin);
         auto split = [&](int it) {                       // this warp's share of a step: 32 rows x 16 of k of A, an eighth of W
             const int s = it % STAGES;
             if (!mbar_wait(&sm.full[s], (uint32_t)(it / STAGES & 1))) return false;
@@ -282,13 +287,13 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             return true;
         };
         const int team = part >> 1;
-        int it = 0, local = 0;
+        int it = 0;
         if (total > 0 && team == 0) ok = split(0);
-        for (int item = blockIdx.x; item < items && ok; item += gridDim.x, ++local) {
+        for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
             float2x sum[CW / 2];
 #pragma unroll
             for (int i = 0; i < CW / 2; ++i) sum[i] = 0ull;
-            const int begin = first_step(item), end = last_step(item);
+            int run_end = begin + g.group;
             for (int st = begin; st < end; ++st, ++it) {
                 if (it + 1 < total && team == ((it + 1) & 1)) ok = split(it + 1);
                 const int buf = it & 1;
@@ -308,17 +313,18 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&sm.acc_empty[buf]);
-                if (RUNS && (st + 1) % FC_GROUP == 0 && st + 1 != end) {         // a run is complete: onto those before it
+                if (RUNS && st + 1 == run_end && st + 1 != end) {                // a run is complete: onto those before it
                     float2x* at = reinterpret_cast<float2x*>(patch) + lane;
 #pragma unroll
                     for (int i = 0; i < CW / 2; ++i) {
-                        at[32 * i] = st + 1 == FC_GROUP ? sum[i] : pair_add(at[32 * i], sum[i]);
+                        at[32 * i] = run_end == g.group ? sum[i] : pair_add(at[32 * i], sum[i]);
                         sum[i] = 0ull;
                     }
+                    run_end += g.group;
                 }
             }
             if (!ok) break;
-            if (RUNS && steps > FC_GROUP) {
+            if (RUNS && g.runs > 1) {
                 const float2x* at = reinterpret_cast<const float2x*>(patch) + lane;
 #pragma unroll
                 for (int i = 0; i < CW / 2; ++i) sum[i] = pair_add(at[32 * i], sum[i]);
@@ -330,53 +336,14 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 out[2 * i] = two.x;
                 out[2 * i + 1] = two.y;
             }
-            const int tile = item / cut, m0 = tile % m_tiles * FC_BM, n0 = tile / m_tiles * BN;
-            const int row0 = m0 + quad * 32, col0 = n0 + part * CW;
+            const int row0 = tile % m_tiles * FC_BM + quad * 32, col0 = tile / m_tiles * BN + part * CW;
             if constexpr (CUT) {
-                // (a part lies as its warps hold it: four columns of 32 rows side by side, warp after warp)
-                constexpr long long PART4 = FC_BM * BN / 4;
-                float4* tile_parts = reinterpret_cast<float4*>(g.parts) + tile * cut * PART4 + (warp - 2) * (CW / 4) * 32 + lane;
-                const bool mine = row0 < g.M && col0 < g.N;
-                if (mine) {
-                    float4* to = tile_parts + (item - tile * cut) * PART4;
+                // The run's sums to where the operands lay (every product has read them): four columns of 32 rows side by side,
+                // warp after warp.
+                float4* mine = reinterpret_cast<float4*>(sm.a[0]) + (warp - 2) * (CW / 4) * 32 + lane;
 #pragma unroll
-                    for (int j = 0; j < CW / 4; ++j)
-                        __stcg(to + 32 * j, make_float4(out[4 * j], out[4 * j + 1], out[4 * j + 2], out[4 * j + 3]));
-                }
-                __threadfence();                         // the part is out before the ticket is drawn
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&sm.part_stored);
-                if (warp == 2) {
-                    const bool stored = mbar_wait(&sm.part_stored, (uint32_t)(local & 1));
-                    if (lane == 0) {
-                        int last = 0;
-                        if (stored) {
-                            last = atomicAdd(&g.tickets[tile], 1) == cut - 1;
-                            if (last) g.tickets[tile] = 0;           // as the next launch expects it
-                            __threadfence();
-                        }
-                        sm.part_last = last;
-                        mbar_arrive(&sm.part_decided);
-                    }
-                    __syncwarp();
-                    if (!stored) ok = false;
-                }
-                if (!mbar_wait(&sm.part_decided, (uint32_t)(local & 1))) ok = false;
-                if (!ok) break;
-                if (!sm.part_last || !mine) continue;
-                __threadfence();
-                for (int p = 0; p < cut; ++p) {
-                    float4 more[CW / 4];
-#pragma unroll
-                    for (int j = 0; j < CW / 4; ++j) more[j] = __ldcg(tile_parts + p * PART4 + 32 * j);
-#pragma unroll
-                    for (int j = 0; j < CW / 4; ++j) {
-                        out[4 * j] = p ? out[4 * j] + more[j].x : more[j].x;
-                        out[4 * j + 1] = p ? out[4 * j + 1] + more[j].y : more[j].y;
-                        out[4 * j + 2] = p ? out[4 * j + 2] + more[j].z : more[j].z;
-                        out[4 * j + 3] = p ? out[4 * j + 3] + more[j].w : more[j].w;
-                    }
-                }
+                for (int j = 0; j < CW / 4; ++j) mine[32 * j] = make_float4(out[4 * j], out[4 * j + 1], out[4 * j + 2], out[4 * j + 3]);
+                continue;                                // (a block has one tile)
             }
             if (row0 < g.M && col0 < g.N) {
                 if (act == ACT_GELU_NEW) fc_finish<ACT_GELU_NEW, CW>(g, out, patch, lane, row0, col0);
@@ -386,6 +353,37 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             }
         }
         if (!ok && lane == 0) atomicExch(g.status, 3);
+    }
+    if constexpr (CUT) {
+        static_assert(sizeof(sm.a) + sizeof(sm.w_hi) + sizeof(sm.w_lo) >= FC_BM * BN * sizeof(float), "room for a run's sums");
+        ok = __all_sync(0xffffffffu, ok);
+        fc_cluster_sync();                               // every run's sums are in its block's shared memory
+        if (warp >= 2 && ok) {
+            // Eight columns of 32 rows at a time, dealt out to the cluster's blocks and their warps.
+            constexpr int EIGHTS = CW / 8;
+            const int m0 = (int)blockIdx.x % m_tiles * FC_BM, n0 = (int)blockIdx.x / m_tiles * BN;
+            for (int p = (int)blockIdx.y + (warp - 2) * g.runs; p < FC_WORKERS * EIGHTS; p += FC_WORKERS * g.runs) {
+                const int owner = p / EIGHTS, row0 = m0 + ((owner + 2) & 3) * 32, col0 = n0 + (owner >> 2) * CW + p % EIGHTS * 8;
+                if (row0 >= g.M || col0 >= g.N) continue;
+                const uint32_t at = smem_u32(reinterpret_cast<const float4*>(sm.a[0]) + 2 * p * 32 + lane);
+                float out[8];
+                for (int r = 0; r < g.runs; ++r) {
+                    uint32_t there;
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(at), "r"(r));
+                    const float4 x = fc_load_remote(there), y = fc_load_remote(there + 32 * sizeof(float4));
+                    const float more[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) out[j] = r ? out[j] + more[j] : more[j];
+                }
+                float* patch = sm.patch[warp - 2];
+                if (act == ACT_GELU_NEW) fc_finish<ACT_GELU_NEW, 8>(g, out, patch, lane, row0, col0);
+                else if (act == ACT_GELU_ERF) fc_finish<ACT_GELU_ERF, 8>(g, out, patch, lane, row0, col0);
+                else if (act == ACT_RELU2) fc_finish<ACT_RELU2, 8>(g, out, patch, lane, row0, col0);
+                else fc_finish<0, 8>(g, out, patch, lane, row0, col0);
+            }
+        }
+        __syncwarp();
+        fc_cluster_sync();                               // no block leaves while another reads its sums
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -401,15 +399,43 @@ int launch_f32_tc(const FcArgs& g, int act, int sms, cudaStream_t s) {
     const size_t smem = sizeof(FcSmem<BN, STAGES, RUNS>) + 1024;
     if (!allow_shared(reinterpret_cast<const void*>(kernel), smem)) return MU_ERR_LAUNCH;
     prefer_shared_memory(reinterpret_cast<const void*>(kernel));
-    const long long items = (long long)((g.M + FC_BM - 1) / FC_BM) * ((g.N + BN - 1) / BN) * (CUT ? g.cut : 1);
-    return launch_pdl(kernel, dim3((unsigned)(items < sms ? items : sms)), dim3(FC_THREADS), smem, s, 1, map_a, map_w, g, act);
+    const long long tiles = (long long)((g.M + FC_BM - 1) / FC_BM) * ((g.N + BN - 1) / BN);
+    const dim3 grid((unsigned)(CUT || tiles < sms ? tiles : sms), CUT ? g.runs : 1);
+    return launch_pdl(kernel, grid, dim3(FC_THREADS), smem, s, CUT ? g.runs : 1, map_a, map_w, g, act);
+}
+
+// Tiles that are worked on at once if each is cut into `runs`: clusters that the device takes at a time (asked for once).
+template <int BN, int STAGES>
+int fc_clusters(int runs) {
+    static std::atomic<int> known[FC_RUNS + 1];
+    int n = known[runs].load(std::memory_order_relaxed);
+    if (n != 0) return n;
+    auto kernel = gemm_f32_tc_kernel<BN, STAGES, false, true>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1, runs);
+    cfg.blockDim = dim3(FC_THREADS);
+    cfg.dynamicSmemBytes = sizeof(FcSmem<BN, STAGES, false>) + 1024;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = (unsigned)runs;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (!allow_shared(reinterpret_cast<const void*>(kernel), cfg.dynamicSmemBytes) ||
+        cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n <= 0) {
+        cudaGetLastError();
+        n = -1;                                          // (never cut)
+    }
+    known[runs].store(n, std::memory_order_relaxed);
+    return n;
 }
 
 }  // namespace mu
 
 // float32 A [M, K] (lda), W [N, K] (ldw): K, lda, ldw multiples of 4, bases 16-byte aligned.  C float32 (ldc); residual
 // float32 (ldr), may be C itself.  `status`: as mu_gemm_tc's.  tile: width of the tiles (0: chosen here); cut: 0 never, 1
-// wherever K has several runs and the workspace has room, -1 chosen here.  Neither changes a bit of the result.
+// wherever K has several runs, -1 chosen here.  Neither changes a bit of the result.
 MU_EXPORT int mu_gemm_f32_tc(const void* A, const void* W, const float* bias, const float* residual, void* C, int M, int N,
                              int K, long long lda, long long ldw, long long ldc, long long ldr, int act, int tile, int cut,
                              int* status, void* stream) {
@@ -422,10 +448,13 @@ MU_EXPORT int mu_gemm_f32_tc(const void* A, const void* W, const float* bias, co
     if (sms <= 0) return MU_ERR_LAUNCH;
     const long long m_tiles = (M + mu::FC_BM - 1) / mu::FC_BM;
     if (m_tiles * ((N + 31) / 32) > (1LL << 30)) return MU_ERR_UNSUPPORTED_SIZE;
-    const int steps = (K + mu::FC_BK - 1) / mu::FC_BK, runs = (steps + mu::FC_GROUP - 1) / mu::FC_GROUP;
-    const mu::F32SplitRoom room = mu::split_room();
+    const int steps = (K + mu::FC_BK - 1) / mu::FC_BK, group = mu::fc_group(steps), runs = (steps + group - 1) / group;
+    const mu::FcArgs g = {(const float*)A, (const float*)W, bias, residual, (float*)C, M, N, K, lda, ldw, ldc, ldr, status,
+                          group, runs};
+    cudaStream_t s = (cudaStream_t)stream;
+#define MU_FC_ALL(DO) DO(32, 7, 6) DO(64, 6, 5) DO(96, 5, 4) DO(128, 4, 3) DO(160, 3, 3)
     // The width, and whether to cut, by what the SM that ends last has to do, in microseconds: a step took 0.42 (32 columns), 0.67
-    // (96), 0.80 (128) and 1.0 (160), handing the parts over 4.
+    // (96), 0.80 (128) and 1.0 (160), handing the sums over 4.
     int best = 0, best_cut = 0;
     double best_cost = 0.0;
     const int widths[5] = {32, 64, 96, 128, 160};
@@ -434,33 +463,30 @@ MU_EXPORT int mu_gemm_f32_tc(const void* A, const void* W, const float* bias, co
         if (tile ? bn != tile : bn > 32 && bn - 32 >= N) continue;
         const long long tiles = m_tiles * ((N + bn - 1) / bn);
         for (int c = 0; c < 2; ++c) {
-            if (c == 1 && (cut == 0 || runs == 1 || !room.parts || tiles > room.n_tickets ||
-                           tiles * runs * (long long)(mu::FC_BM * bn * sizeof(float)) > room.bytes)) continue;
+            if (c == 1 && (cut == 0 || runs == 1)) continue;
             if (c == 0 && runs > 1 && bn == 160) continue;           // (no registers for both sums)
-            const long long items = tiles * (c ? runs : 1), rounds = (items + sms - 1) / sms;
-            double cost = rounds * ((c ? mu::FC_GROUP : steps) * (0.28 + 0.0045 * bn) + 1.0 + 0.01 * bn) + (c ? 4.0 : 0.0);
+            long long at_once = sms;
+            if (c == 1) {
+#define MU_FC_CLUSTERS(BN, ST, ST_RUNS) if (bn == BN) at_once = mu::fc_clusters<BN, ST>(runs);
+                MU_FC_ALL(MU_FC_CLUSTERS)
+#undef MU_FC_CLUSTERS
+                if (at_once <= 0) continue;
+            }
+            const long long rounds = (tiles + at_once - 1) / at_once;
+            double cost = rounds * ((c ? group : steps) * (0.28 + 0.0045 * bn) + 1.0 + 0.01 * bn) + (c ? 4.0 : 0.0);
             if (c == 1 && cut == 1) cost *= 1e-6;
             if (best == 0 || cost < best_cost) best = bn, best_cut = c, best_cost = cost;
         }
     }
     if (best == 0) best = tile == 160 ? 128 : tile, best_cut = 0;
-    const mu::FcArgs g = {(const float*)A, (const float*)W, bias, residual, (float*)C, M, N, K, lda, ldw, ldc, ldr, status,
-                          best_cut ? runs : 1, room.parts, room.tickets};
-    cudaStream_t s = (cudaStream_t)stream;
 #define MU_FC(BN, ST, ST_RUNS)                                                                                         \
-    case BN:                                                                                                           \
-        return best_cut ? mu::launch_f32_tc<BN, ST, false, true>(g, act, sms, s)                                       \
-               : runs == 1 ? mu::launch_f32_tc<BN, ST, false, false>(g, act, sms, s)                                   \
-                           : mu::launch_f32_tc<BN, ST_RUNS, true, false>(g, act, sms, s)
-    switch (best) {
-        MU_FC(32, 7, 6);
-        MU_FC(64, 6, 5);
-        MU_FC(96, 5, 4);
-        MU_FC(128, 4, 3);
-        case 160:
-            return best_cut ? mu::launch_f32_tc<160, 3, false, true>(g, act, sms, s)
-                            : mu::launch_f32_tc<160, 3, false, false>(g, act, sms, s);
+    if (best == BN) {                                                                                                  \
+        if (best_cut) return mu::launch_f32_tc<BN, ST, false, true>(g, act, sms, s);                                   \
+        if (runs == 1) return mu::launch_f32_tc<BN, ST, false, false>(g, act, sms, s);                                 \
+        if constexpr (BN < 160) return mu::launch_f32_tc<BN, ST_RUNS, true, false>(g, act, sms, s);                    \
     }
+    MU_FC_ALL(MU_FC)
 #undef MU_FC
+#undef MU_FC_ALL
     return MU_ERR_BAD_ARGUMENT;
 }

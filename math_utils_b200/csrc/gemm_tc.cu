@@ -106,9 +106,6 @@ bool tensor_map_f32(CUtensorMap* map, const void* base, long long rows, int cols
     return true;
 }
 
-struct F32SplitRoom { float* parts; long long bytes; int* tickets; int n_tickets; };
-F32SplitRoom split_room() { return {g_split.parts, g_split.parts_bytes, g_split.tickets, g_split.n_tickets}; }
-
 // A [rows, cols] bfloat16 matrix with `ld` elements between rows, cut into boxes of box_rows x 64.
 static bool make_map_uncached(CUtensorMap* map, const void* base, long long rows, int cols, long long ld, int box_rows) {
     EncodeTiledFn fn = encode_tiled();
