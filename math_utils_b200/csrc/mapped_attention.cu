@@ -175,7 +175,8 @@ qk_prepare_pieces_kernel(__nv_bfloat16* __restrict__ q, long long ldq, const __n
             x[2 * j] = f.x, x[2 * j + 1] = f.y;
         }
         if (base + slots < n) raw = load(item + slots);
-        const float* weight = is_q ? q_weight : k_weight;
+        // (with or without a weight for all lanes: given keys, the two weights come together, else slices past the end are queries)
+        const float* weight = is_q || !k ? q_weight : k_weight;
         if (weight) {
             float ss = 0.0f;
 #pragma unroll

@@ -352,3 +352,38 @@ def test_preparation_by_pieces_is_the_general_one(heads, kv_heads, maps, dim, vd
     untouched = torch.ones(3, 64, dtype=torch.bool)
     untouched[2, 30:] = untouched[0, :36] = False
     assert not got[0][1][untouched.cuda()].any()
+
+
+# a layer that reads another layer's rows prepares its queries alone: slices that leave lanes of a warp without one, and that fill it
+@pytest.mark.parametrize("heads,maps,dim", [(6, 1, 64), (3, 1, 128), (3, 2, 64), (1, 1, 8), (5, 1, 96), (16, 2, 64)])
+@pytest.mark.parametrize("rot,pairs", [(0, False), (16, False), (6, True)])
+def test_queries_alone_by_pieces(heads, maps, dim, rot, pairs):
+    """The general form's values (rows one entry off), as above, and the float64 ones."""
+    from math_utils_b200.csrc import ops
+    rng = np.random.default_rng(heads * dim)
+    T, width = 37, heads * maps * dim
+    rot = rot if dim >= 16 or pairs else 0
+    x = torch.as_tensor(rng.normal(0, 2, (T, width)), dtype=torch.float32).cuda().bfloat16()
+    weight = torch.as_tensor(rng.normal(1, 0.2, dim), dtype=torch.float32).cuda()
+    freqs = torch.as_tensor(300.0 ** -np.linspace(0, 1, max(rot // 2, 1)), dtype=torch.float32).cuda()
+    pos = torch.arange(T, dtype=torch.int32, device="cuda") + 30
+    got = []
+    for off in (0, 1):
+        proj = torch.zeros((T, width + 8 if off == 0 else width + 9), dtype=torch.bfloat16, device="cuda")
+        proj[:, off:off + width] = x
+        ops.qk_prepare(proj[:, off:off + width], None, None, weight, None, freqs, 1.25, rot, 1e-3, heads, 1, maps, dim, dim, pos, None,
+                       None, 64, None, pairs=pairs)
+        assert not proj[:, :off].any() and not proj[:, off + width:].any()
+        got.append(proj[:, off:off + width].float())
+    a, b = got
+    assert ((a - b).abs() <= b.abs() * 2.0 ** -7).all() and float((a != b).float().mean()) < 0.01
+    y = x.double().reshape(T, heads * maps, dim)
+    y = y / (y.square().mean(-1, keepdim=True) + 1e-3).sqrt() * weight.double()
+    if rot:
+        angle = (pos[:, None].float() * freqs).double()[:, None]
+        cos, sin = angle.cos() * 1.25, angle.sin() * 1.25
+        lo, hi = (y[..., 0:rot:2], y[..., 1:rot:2]) if pairs else (y[..., :rot // 2], y[..., rot // 2:rot])
+        turned = torch.stack([lo * cos - hi * sin, hi * cos + lo * sin], -1 if pairs else -2).reshape(T, -1, rot)
+        y = torch.cat([turned, y[..., rot:]], -1)
+    # half a bfloat16's last bit, and float32 angles, norms and turns in front of it
+    assert ((a.double() - y.reshape(T, -1)).abs() <= y.reshape(T, -1).abs() * 2.0 ** -8 + 1e-4).all()
