@@ -118,7 +118,7 @@ qk_prepare_kernel(TE* __restrict__ q, long long ldq, const TE* __restrict__ k, l
 // The same for bfloat16 slices whose pieces of eight entries are 16-byte aligned: LANES lanes a slice, a piece a lane, so the
 // norm's sum takes log2(LANES) exchanges and a rotation's partner is a lane's own piece (pairs) or a whole piece of another lane
 // (rotated halves of whole pieces).  A block takes a token: its angles are made once, while the first pieces are on their
-// way.  A warp a slice, two-byte loads and blocks of four slices, each with the angles again (the form above, for other
+// way.  With few tokens of more slices than a block holds the slices are shared by blocks while all of these find room at once.  A warp a slice, two-byte loads and blocks of four slices, each with the angles again (the form above, for other
 // alignments), took 20 us where this takes 7, for 2,048 tokens of 20 slices of 64 and 256 values: the layer of two score
 // maps 75 -> 63 us.  What is left is the launch and a token's chain of loads, angles and exchanges; its bytes take 1.6 us.
 template <int LANES>
@@ -143,7 +143,8 @@ qk_prepare_pieces_kernel(__nv_bfloat16* __restrict__ q, long long ldq, const __n
             raw = *reinterpret_cast<const uint4*>((item < n_q ? q_row + (long long)item * dim : k_row + (long long)(item - n_q) * dim) + d0);
         return raw;
     };
-    uint4 raw = load(slot);
+    const int begin = blockIdx.y * slots, step = gridDim.y * slots;             // (this block's share of the token's slices)
+    uint4 raw = load(begin + slot);
     __nv_bfloat16* row = nullptr;
     if (k) {
         const long long page = block_table[(long long)tok_seq[t] * max_pages + pos / page_tokens];
@@ -156,7 +157,7 @@ qk_prepare_pieces_kernel(__nv_bfloat16* __restrict__ q, long long ldq, const __n
         staged[half + i] = sn * magnitude;
     }
     __syncthreads();
-    if (v) {
+    if (v && blockIdx.y == 0) {
         const uint4* src = reinterpret_cast<const uint4*>(v + (long long)t * ldv);
         uint4* dst = reinterpret_cast<uint4*>(row + (long long)n_kv_heads * maps * dim);
         for (int i = threadIdx.x; i < n_kv_heads * vdim / 8; i += blockDim.x) dst[i] = src[i];
@@ -164,7 +165,7 @@ qk_prepare_pieces_kernel(__nv_bfloat16* __restrict__ q, long long ldq, const __n
     // what this lane's piece is rotated with, the same for every slice
     const bool first = d0 < half, turned = d0 < rot_dims;
     const int partner = (threadIdx.x & 31) - sub + (pairs || !turned ? sub : first ? sub + half / 8 : sub - half / 8);
-    for (int base = 0; base < n; base += slots) {           // (whole warps stay together: slices past the end are zeros)
+    for (int base = begin; base < n; base += step) {        // (whole warps stay together: slices past the end are zeros)
         const int item = base + slot;
         const bool is_q = item < n_q, live = item < n && d0 < dim;
         const __nv_bfloat162* in = reinterpret_cast<const __nv_bfloat162*>(&raw);
@@ -174,7 +175,7 @@ qk_prepare_pieces_kernel(__nv_bfloat16* __restrict__ q, long long ldq, const __n
             const float2 f = __bfloat1622float2(in[j]);
             x[2 * j] = f.x, x[2 * j + 1] = f.y;
         }
-        if (base + slots < n) raw = load(item + slots);
+        if (base + step < n) raw = load(item + step);
         // (with or without a weight for all lanes: given keys, the two weights come together, else slices past the end are queries)
         const float* weight = is_q || !k ? q_weight : k_weight;
         if (weight) {
@@ -710,8 +711,13 @@ MU_EXPORT int mu_qk_prepare(void* q, long long ldq, const void* k, long long ldk
     if (pieces) {
         const int lanes = dim <= 64 ? 8 : dim <= 128 ? 16 : 32;
         const int wanted = (items * lanes + 31) / 32 * 32, block = wanted < 256 ? wanted : 256;
+        // Passes that a block alone would make over a token's slices, and blocks of 256 that the device holds for each token.  72
+        // slices of 256, 1, 64 and 300 tokens: 3.3, 6.7 and 17 us by parts, 11, 11 and 31 by one block a token (6.5, 7.7 and 19 in the
+        // general form); of 128: 2.9, 4.7 and 7.6, before 6.0, 6.6 and 12.
+        const long long passes = (items + block / lanes - 1) / (block / lanes), held = 8LL * mu::sm_count() / n_tokens;
+        const int parts = (int)(held < 1 ? 1 : held < passes ? held : passes);
 #define MU_PIECES(LANES)                                                                                                \
-    return mu::launch_pdl(mu::qk_prepare_pieces_kernel<LANES>, dim3(n_tokens), dim3(block), rot_dims * sizeof(float), s, 1, \
+    return mu::launch_pdl(mu::qk_prepare_pieces_kernel<LANES>, dim3(n_tokens, parts), dim3(block), rot_dims * sizeof(float), s, 1, \
                           (bf*)q, ldq, (const bf*)k, ldk, (const bf*)v, ldv, q_weight, k_weight, freqs, magnitude, rot_dims, eps, \
                           n_heads, n_kv_heads, maps, dim, vdim, tok_pos, tok_seq, block_table, max_pages, page_tokens, (bf*)rows, \
                           pairs, shared)
