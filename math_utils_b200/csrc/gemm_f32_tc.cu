@@ -1,23 +1,29 @@
 // C[M, N] = act(A[M, K] . W[N, K]^T + bias) (+ residual), float32 in and out, on the 5th-generation tensor cores: the 32-bit
 // path's products over a long K.
 //
-// Every operand is two TF32 numbers, hi = x rounded to 11 bits and lo = x - hi rounded to 11 bits (together 22 to 23 bits of
-// x's 24), and a product three: lo hi + hi lo + hi hi.  What tensor cores lose of a sum is not in the operands but in the
-// accumulator, which they cut off instead of rounding it; so an accumulator only ever holds 32 of k (twelve products, the
-// small ones first), and warps add it to the tile's float32 sums in registers, rounded.  Error against float64 (2-norm, normal
-// values; float32 multiply-adds, gemm_simt.cu, in brackets): k = 192 1.13e-7 (1.32e-7), 768 1.37e-7 (2.52e-7), 3072 1.43e-7
-// (4.98e-7); all values positive: 4.6e-8 (6.6e-8), 7.6e-8 (1.11e-7), 5.7e-8 (2.08e-7).
+// Every operand is three bfloat16 numbers that are together exactly it (8 bits each of its 24, each rounded from what those
+// before left), and a product eight: all but lo lo, which is 2^-36 of it at most.  What is left to lose is in the accumulators, which
+// tensor cores cut off instead of rounding.  So the large products, hi hi (16 bits each), have an accumulator of their own that
+// holds 32 of k (two instructions) and is added to the tile's float32 sums in registers, rounded; the seven others, 2^-8 and
+// less of these, run on in a second one and are added at the end of a run of k (below), where what they were cut by is nothing.
+// A product that float32 holds is exact, and so are sums of whole numbers up to 2^24; entries below 2^-109 lose their last bits
+// (bfloat16 has none below 2^-133).
+// Error against float64, rms over the outputs of |error| / (|a| . |w|) (float32 multiply-adds, gemm_simt.cu, in brackets): normal
+// values k = 384 5.8e-9 (1.45e-8), 768 4.9e-9 (1.42e-8), 3072 3.2e-9 (1.41e-8); positive ones 768 6.1e-8 (1.11e-7), 3072 6.3e-8
+// (2.11e-7); rows of 1, 4, 16 and 64 values, k = 768, 2.53e-8 (2.53e-8), 2.40e-8 (2.95e-8), 1.49e-8 (2.21e-8), 9.7e-9 (1.66e-8);
+// log-normal factors of sigma 2 and any sign 4.2e-8 (9.9e-8).  Further off than multiply-adds only where both rows are
+// positive and a few terms carry the sum (log-normal factors of sigma 2, none negative: k = 384 1.34 times, 512 1.22, 768 1.10, from
+// 1536 on less over whole rows), and by 8 % where k has eight runs and a row two positive values in each.
 //
 // A block per SM walks over tiles of 128 x BN.  Warp 0 issues the TMA loads of 32 of k (128 rows of A, BN of W, 128-byte
-// swizzle).  Sixteen warps split them: A's parts go to tensor memory (a row a lane), W's hi part back to where it came from and
-// its lo part beside it, which keeps the swizzle.  Warp 1 issues the products with A from tensor memory and W from shared
-// memory into one of two accumulators; the sixteen warps meanwhile add the other to their sums (32 rows x BN / 4 columns a
-// warp).  With A's operands in shared memory as well a step would move 252 KB through it instead of 172 (BN = 160), at 128
-// bytes a cycle more than its products take; as it is both take about as long.  What is left is the warps' chain from load
-// to arrival: a step of 32 took 0.42 us (32 columns), 0.67 (96), 0.80 (128) and 1.0 (160) whatever of the splitting,
-// the products or the sums was left out alone, so two teams of eight warps split every other step.  Measured (B200,
-// microseconds; the multiply-adds in brackets): 777 x 3072 x 768 30 (121), 777 x 768 x 3072 40 (129), 2048 x 4096 x 4096 412
-// (1,700; 167 TFLOP/s), 8 x 3072 x 768 14 (19), 8 x 768 x 3072 12.5 (66).
+// swizzle).  Sixteen warps split them: A's parts go to tensor memory (a row a lane), W's hi and mid parts back to where the row
+// came from and its lo parts beside it.  Warp 1 issues the products with A from tensor memory and W from shared memory; the
+// sixteen warps add what is complete to their sums (32 rows x BN / 4 columns a warp).  A step of 32 of k and 128 columns takes
+// 0.79 us: its products 1,024 cycles, its shared memory 1,190 (fill, split, and W's parts eight times), and the warps' chain from
+// load to arrival, which two teams of eight that take every other step, two steps ahead, hide for the most part (one step
+// ahead: 0.92).  Others: 0.48 us (32 columns), 0.56 (64), 0.71 (96), 1.04 (160).  Measured (B200, microseconds; the multiply-adds in
+// brackets): 777 x 3072 x 768 37 (121), 777 x 768 x 768 15.4 (34), 777 x 768 x 3072 44 (129), 2048 x 4096 x 4096 475 (1,700; 145
+// TFLOP/s), 8 x 3072 x 768 11.6 (17.5), 8 x 768 x 3072 14 (66).
 //
 // A tile's sum is, for every run of k, the sum of its steps in order, and then the runs' sums in order; how long a run is
 // follows from k alone.  A product of few tiles is cut into those runs (CUT): a cluster of blocks has a tile, each block
@@ -25,7 +31,7 @@
 // a row's result is the same bits whatever the cut, the tile's width and the rest of the step are, and no launch keeps
 // anything in device memory that another one, on another stream, could meet.
 //
-// A value that is infinite, or NaN, or rounds to infinity in 11 bits, has parts that make NaN where float32 gives
+// A value that is infinite, or NaN, or rounds to infinity in 8 bits, has parts that make NaN where float32 gives
 // an infinity; so a sum that comes out not finite is made once more by multiply-adds, by the lane that stores it.
 #include "tcgen05.cuh"
 
@@ -34,29 +40,30 @@
 namespace mu {
 
 constexpr int FC_BM = 128, FC_BK = 32, FC_WORKERS = 16, FC_THREADS = 64 + 32 * FC_WORKERS;
-constexpr int FC_RUN = 24, FC_RUNS = 8;                  // a run's steps of 32, if k has no more than that many runs
-// Steps of a run: runs of one length, as few as FC_RUN allows (a cluster has eight blocks).
+// k in runs of one length: two, more where they would be longer than FC_RUN steps of 32, up to the eight blocks of a cluster.  One
+// sum over all of k rounds at its full size at every step, and rows of 32 to 256 positive values (k = 768) came out up to
+// 1.28 times as far off as by multiply-adds, which keep four sums; two runs 0.88 times.  768 of k are some 20 us of a block (128
+// columns), against 3 for a cluster's start and handing over, and every run more is a rounding more of sums of few values.
+constexpr int FC_RUN = 24, FC_RUNS = 8;
 inline int fc_group(int steps) {
-    const int runs = (steps + FC_RUN - 1) / FC_RUN;
-    return (steps + (runs < FC_RUNS ? runs : FC_RUNS) - 1) / (runs < FC_RUNS ? runs : FC_RUNS);
+    const int most = (steps + FC_RUN - 1) / FC_RUN, runs = most < 2 ? 2 : most < FC_RUNS ? most : FC_RUNS;
+    return (steps + runs - 1) / runs;
 }
 constexpr int FC_TEAM = FC_WORKERS / 2;                  // two teams of warps split every other step
-// What tensor cores cut off of an accumulator's four large additions is 2^-23 of it on average; it is given back.
-constexpr float FC_GIVE_BACK = 1.0f + 1.1920929e-7f;
 constexpr int FC_PITCH = 9;                              // floats a row of an epilogue patch (32 rows x 8 columns)
 
 bool tensor_map_f32(CUtensorMap* map, const void* base, long long rows, int cols, long long ld, int box_rows);
 
-// Instruction descriptor of kind::tf32: float32 accumulator, TF32 operands (2 at bits 7 and 10), both K-major.
-__host__ __device__ constexpr uint32_t idesc_tf32(int m, int n) {
-    return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+// K-major operand in rows of 64 bytes with the 64-byte swizzle, groups of 8 rows 512 bytes apart (mode 4; the rest as smem_desc_sw128).
+__device__ __forceinline__ uint64_t fc_desc_sw64(uint32_t smem_addr) {
+    return (uint64_t)((smem_addr & 0x3FFFF) >> 4) | (uint64_t)1 << 16 | (uint64_t)(512 >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)4 << 61;
 }
-__device__ __forceinline__ void umma_tf32_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
+__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
                                              uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
         ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
 }
 __device__ __forceinline__ void tmem_ld_x8_nowait(uint32_t taddr, uint32_t* r) {
@@ -69,24 +76,27 @@ __device__ __forceinline__ void tmem_st_x8(uint32_t taddr, const uint32_t (&r)[8
                  ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
                  : "memory");
 }
-// x to 11 bits, ties away from zero (a NaN may lose its mark here: its other part, x - hi, keeps it).
-__device__ __forceinline__ uint32_t tf32_bits(float x) { return (__float_as_uint(x) + 0x1000u) & 0xffffe000u; }
-__device__ __forceinline__ void tf32_parts(float x, uint32_t& hi, uint32_t& lo) {
-    hi = tf32_bits(x);
-    lo = __float_as_uint(x - __uint_as_float(hi));       // (exact; the tensor cores read its first 11 bits)
+// Two values as three pairs of bfloat16 (the first in the low half), each rounded from what those before it left: exactly the
+// values, down to 2^-109 (where the third falls below bfloat16's range).
+__device__ __forceinline__ void fc_parts(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(hi) : "f"(y), "f"(x));
+    x -= __uint_as_float(hi << 16), y -= __uint_as_float(hi & 0xffff0000u);
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(mid) : "f"(y), "f"(x));
+    x -= __uint_as_float(mid << 16), y -= __uint_as_float(mid & 0xffff0000u);
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(y), "f"(x));
 }
 __device__ __forceinline__ bool is_finite_bits(float v) { return (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u; }
 
-template <int BN> constexpr int fc_room(bool runs) { return runs && BN * 8 > 32 * FC_PITCH ? BN * 8 : 32 * FC_PITCH; }
+template <int BN> constexpr int fc_room(bool cut) { return !cut && BN * 8 > 32 * FC_PITCH ? BN * 8 : 32 * FC_PITCH; }
 
-template <int BN, int STAGES, bool RUNS>
+template <int BN, int STAGES, bool CUT>
 struct FcSmem {
     float a[STAGES][FC_BM * FC_BK];                      // rows of 128 bytes, 128-byte swizzle, each tile 1024-byte aligned
-    float w_hi[STAGES][BN * FC_BK];                      // W as it came, then its hi parts
-    float w_lo[STAGES][BN * FC_BK];
-    float patch[FC_WORKERS][fc_room<BN>(RUNS)];          // a warp's patch, and before that (RUNS) its sum of the runs so far
+    float w[STAGES][BN * FC_BK];                         // W as it came, then a row's hi parts and its mid parts, 64 bytes each
+    __nv_bfloat16 w_lo[STAGES][BN * FC_BK];              // rows of 64 bytes, 64-byte swizzle
+    float patch[FC_WORKERS][fc_room<BN>(CUT)];           // a warp's patch, and before that (uncut) its sum of the runs so far
     uint64_t full[STAGES], split[STAGES], empty[STAGES]; // loaded; split into parts; read by the products
-    uint64_t acc_full[2], acc_empty[2];
+    uint64_t acc_full, acc_empty, small_empty[2];
     uint32_t tmem_base;
 };
 
@@ -151,14 +161,16 @@ __device__ __forceinline__ float4 fc_load_remote(uint32_t addr) {
     return v;
 }
 
-// RUNS: a block sums several runs of a tile.  CUT: a cluster's blocks (along y) have a run of one tile each.
-template <int BN, int STAGES, bool RUNS, bool CUT>
+// CUT: a cluster's blocks (along y) have a run of one tile each; otherwise a block sums all runs of its tiles.
+template <int BN, int STAGES, bool CUT>
 __global__ void __launch_bounds__(FC_THREADS, 1)
 gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const FcArgs g, int act) {
     extern __shared__ unsigned char fc_raw[];
-    FcSmem<BN, STAGES, RUNS>& sm = *reinterpret_cast<FcSmem<BN, STAGES, RUNS>*>(((uintptr_t)fc_raw + 1023) & ~(uintptr_t)1023);
-    constexpr int CW = BN / 4, COL_A = 2 * BN, COLS = COL_A + 64 * STAGES;
-    constexpr uint32_t TMEM_COLS = COLS <= 128 ? 128 : COLS <= 256 ? 256 : 512;
+    FcSmem<BN, STAGES, CUT>& sm = *reinterpret_cast<FcSmem<BN, STAGES, CUT>*>(((uintptr_t)fc_raw + 1023) & ~(uintptr_t)1023);
+    // tensor memory: sums of the large products, of the small ones (SMALL buffers), A's parts of AHEAD + 1 steps
+    constexpr int CW = BN / 4, AHEAD = 2, SMALL = BN <= 96 ? 2 : 1, COL_SMALL = BN;
+    constexpr int COL_A = COL_SMALL + SMALL * BN, COLS = COL_A + (AHEAD + 1) * 48;
+    constexpr uint32_t TMEM_COLS = COLS <= 256 ? 256 : 512;
     static_assert(COLS <= 512 && BN % 32 == 0, "tensor memory");
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int steps = (g.K + FC_BK - 1) / FC_BK;
@@ -171,7 +183,9 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         tma_prefetch_map(&map_a);
         tma_prefetch_map(&map_w);
         for (int s = 0; s < STAGES; ++s) { mbar_init(&sm.full[s], 1); mbar_init(&sm.split[s], FC_TEAM); mbar_init(&sm.empty[s], 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(&sm.acc_full[b], 1); mbar_init(&sm.acc_empty[b], FC_WORKERS); }
+        mbar_init(&sm.acc_full, 1);
+        mbar_init(&sm.acc_empty, FC_WORKERS);
+        for (int b = 0; b < 2; ++b) mbar_init(&sm.small_empty[b], FC_WORKERS);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -197,7 +211,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                     if (!ok) break;
                     mbar_expect_tx(&sm.full[s], (FC_BM + BN) * FC_BK * sizeof(float));
                     tma_load_2d(sm.a[s], &map_a, st * FC_BK, m0, &sm.full[s]);
-                    tma_load_2d(sm.w_hi[s], &map_w, st * FC_BK, n0, &sm.full[s]);
+                    tma_load_2d(sm.w[s], &map_w, st * FC_BK, n0, &sm.full[s]);
                     issued = it + 1;
                 }
             }
@@ -208,76 +222,102 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             }
         }
     } else if (warp == 1) {
-        constexpr uint32_t idesc = idesc_tf32(FC_BM, BN), STAGE16 = BN * FC_BK * sizeof(float) / 16;
+        constexpr uint32_t idesc = idesc_bf16(FC_BM, BN), W_STAGE = BN * FC_BK * sizeof(float) / 16, LO_STAGE = W_STAGE / 2;
         const bool one = elect_one();
-        const uint64_t hi0 = smem_desc_sw128(smem_u32(sm.w_hi[0])), lo0 = smem_desc_sw128(smem_u32(sm.w_lo[0]));
-        int it = 0;
+        const uint64_t w0 = smem_desc_sw128(smem_u32(sm.w[0])), lo0 = fc_desc_sw64(smem_u32(sm.w_lo[0]));
+        int it = 0, run = -1;
         for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+            int run_at = begin;                          // the step that begins a run
             for (int st = begin; st < end; ++st, ++it) {
-                const int s = it % STAGES, buf = it & 1;
-                ok = mbar_wait(&sm.split[s], (uint32_t)(it / STAGES & 1)) &&
-                     mbar_wait(&sm.acc_empty[buf], (uint32_t)((it >> 1 & 1) ^ 1));
+                const int s = it % STAGES;
+                const bool first = st == run_at;
+                if (first) run_at += g.group, ++run;
+                const int small = run % SMALL;
+                ok = mbar_wait(&sm.split[s], (uint32_t)(it / STAGES & 1));
+                if (ok && first) ok = mbar_wait(&sm.small_empty[small], (uint32_t)((run / SMALL & 1) ^ 1));
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t d = tmem + (uint32_t)(buf * BN), a_hi = tmem + (uint32_t)(COL_A + 64 * s), a_lo = a_hi + 32;
-                const uint64_t w_hi = hi0 + (uint64_t)(s * STAGE16), w_lo = lo0 + (uint64_t)(s * STAGE16);
-                if (!one) continue;
+                const uint32_t a_hi = tmem + (uint32_t)(COL_A + 48 * (it % (AHEAD + 1))), a_mid = a_hi + 16, a_lo = a_hi + 32;
+                const uint64_t w_hi = w0 + (uint64_t)(s * W_STAGE), w_mid = w_hi + 4, w_lo = lo0 + (uint64_t)(s * LO_STAGE);
+                if (one) {
+                    const uint32_t d = tmem + (uint32_t)(COL_SMALL + small * BN);
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {            // 8 of k: 8 columns, 32 bytes
-                    umma_tf32_ts(d, a_lo + 8 * k, w_hi + 2 * k, idesc, k > 0);
-                    umma_tf32_ts(d, a_hi + 8 * k, w_lo + 2 * k, idesc, 1);
+                    for (int k = 0; k < 2; ++k) {        // 16 of k: 8 columns, 32 bytes
+                        umma_bf16_ts(d, a_lo + 8 * k, w_mid + 2 * k, idesc, k > 0 || !first);
+                        umma_bf16_ts(d, a_mid + 8 * k, w_lo + 2 * k, idesc, 1);
+                        umma_bf16_ts(d, a_lo + 8 * k, w_hi + 2 * k, idesc, 1);
+                        umma_bf16_ts(d, a_hi + 8 * k, w_lo + 2 * k, idesc, 1);
+                        umma_bf16_ts(d, a_mid + 8 * k, w_mid + 2 * k, idesc, 1);
+                        umma_bf16_ts(d, a_mid + 8 * k, w_hi + 2 * k, idesc, 1);
+                        umma_bf16_ts(d, a_hi + 8 * k, w_mid + 2 * k, idesc, 1);
+                    }
                 }
+                __syncwarp();
+                ok = mbar_wait(&sm.acc_empty, (uint32_t)((it & 1) ^ 1));
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (one) {
 #pragma unroll
-                for (int k = 0; k < 4; ++k) umma_tf32_ts(d, a_hi + 8 * k, w_hi + 2 * k, idesc, 1);
-                umma_commit(&sm.empty[s]);
-                umma_commit(&sm.acc_full[buf]);
+                    for (int k = 0; k < 2; ++k) umma_bf16_ts(tmem, a_hi + 8 * k, w_hi + 2 * k, idesc, k > 0);
+                    umma_commit(&sm.empty[s]);
+                    umma_commit(&sm.acc_full);
+                }
+                __syncwarp();
             }
         }
         if (!ok && lane == 0) atomicExch(g.status, 2);
     } else {
-        const int quad = warp & 3, part = (warp - 2) >> 2, tid = threadIdx.x - 64;
+        const int quad = warp & 3, part = (warp - 2) >> 2;
         const uint32_t lanes = tmem + ((uint32_t)(quad * 32) << 16);
         const bool rows_here = g.M > quad * 32;          // a single row of tiles may leave whole warps without rows
         float* patch = sm.patch[warp - 2];
         const int total = ((int)blockIdx.x < tiles ? (tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0) * (end - begin);
-        auto split = [&](int it) {                       // this warp's share of a step: 32 rows x 16 of k of A, an eighth of W
+        // This warp's share of a step's parts: 32 rows x 16 of k of A, and rows of W, eight at a time.  Lanes take eight of k of a
+        // row; those that touch shared memory together are of rows r and r ^ 5, whose pieces lie in other banks both as they
+        // came and as the parts lie (hi | mid).
+        auto split = [&](int it) {
             const int s = it % STAGES;
             if (!mbar_wait(&sm.full[s], (uint32_t)(it / STAGES & 1))) return false;
-            constexpr int THREADS = 32 * FC_TEAM, PIECES = (BN * 8 + THREADS - 1) / THREADS, QUARTERS = 4;
-            constexpr bool EVEN = BN * 8 % THREADS == 0;
-            const int row = quad * 32 + lane, at = tid & (THREADS - 1), k4 = (part & 1) * QUARTERS;
-            float4 x[QUARTERS], w[PIECES];               // all are asked for before any is split
+            constexpr int EIGHTS = BN / 8, PIECES = (EIGHTS + FC_TEAM - 1) / FC_TEAM;
+            constexpr bool EVEN = EIGHTS % FC_TEAM == 0;
+            const int row = quad * 32 + lane, k4 = (part & 1) * 4, eight0 = (warp - 2) & (FC_TEAM - 1);
+            const int r8 = lane >> 3 ^ (lane & 4 ? 5 : 0), j8 = lane & 3;
+            float4 x[4], w[PIECES][2];                   // all are asked for before any is split
 #pragma unroll
-            for (int j = 0; j < QUARTERS; ++j)
+            for (int j = 0; j < 4; ++j)
                 x[j] = *reinterpret_cast<const float4*>(sm.a[s] + row * FC_BK + (((k4 + j) ^ (row & 7)) << 2));
-            float4* w_at = reinterpret_cast<float4*>(sm.w_hi[s]) + at;
-            uint4* lo_at = reinterpret_cast<uint4*>(sm.w_lo[s]) + at;
-#pragma unroll
-            for (int i = 0; i < PIECES; ++i)
-                if (EVEN || at + i * THREADS < BN * 8) w[i] = w_at[i * THREADS];
-            if (rows_here) {
-#pragma unroll
-                for (int h = 0; h < QUARTERS / 2; ++h) {
-                    uint32_t hi[8], lo[8];
-#pragma unroll
-                    for (int j = 0; j < 2; ++j) {
-                        const float4 v = x[2 * h + j];
-                        tf32_parts(v.x, hi[4 * j], lo[4 * j]); tf32_parts(v.y, hi[4 * j + 1], lo[4 * j + 1]);
-                        tf32_parts(v.z, hi[4 * j + 2], lo[4 * j + 2]); tf32_parts(v.w, hi[4 * j + 3], lo[4 * j + 3]);
-                    }
-                    tmem_st_x8(lanes + (uint32_t)(COL_A + 64 * s + 4 * k4 + 8 * h), hi);
-                    tmem_st_x8(lanes + (uint32_t)(COL_A + 64 * s + 32 + 4 * k4 + 8 * h), lo);
-                }
-            }
 #pragma unroll
             for (int i = 0; i < PIECES; ++i) {
-                if (EVEN || at + i * THREADS < BN * 8) {
-                    uint4 hi, lo;
-                    tf32_parts(w[i].x, hi.x, lo.x); tf32_parts(w[i].y, hi.y, lo.y);
-                    tf32_parts(w[i].z, hi.z, lo.z); tf32_parts(w[i].w, hi.w, lo.w);
-                    *reinterpret_cast<uint4*>(w_at + i * THREADS) = hi;
-                    lo_at[i * THREADS] = lo;
+                if (!EVEN && eight0 + i * FC_TEAM >= EIGHTS) continue;
+                const float4* from = reinterpret_cast<const float4*>(sm.w[s]) + (8 * (eight0 + i * FC_TEAM) + r8) * 8;
+                w[i][0] = from[(2 * j8) ^ r8], w[i][1] = from[(2 * j8 + 1) ^ r8];
+            }
+            if (rows_here) {
+                uint32_t hi[8], mid[8], lo[8];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    fc_parts(x[j].x, x[j].y, hi[2 * j], mid[2 * j], lo[2 * j]);
+                    fc_parts(x[j].z, x[j].w, hi[2 * j + 1], mid[2 * j + 1], lo[2 * j + 1]);
                 }
+                const uint32_t at = lanes + (uint32_t)(COL_A + 48 * (it % (AHEAD + 1)) + 2 * k4);
+                tmem_st_x8(at, hi);
+                tmem_st_x8(at + 16, mid);
+                tmem_st_x8(at + 32, lo);
+            }
+            __syncwarp();                                // a row's lanes have read it
+#pragma unroll
+            for (int i = 0; i < PIECES; ++i) {
+                if (!EVEN && eight0 + i * FC_TEAM >= EIGHTS) continue;
+                const int wrow = 8 * (eight0 + i * FC_TEAM) + r8;
+                uint4 hi, mid, lo;
+                fc_parts(w[i][0].x, w[i][0].y, hi.x, mid.x, lo.x);
+                fc_parts(w[i][0].z, w[i][0].w, hi.y, mid.y, lo.y);
+                fc_parts(w[i][1].x, w[i][1].y, hi.z, mid.z, lo.z);
+                fc_parts(w[i][1].z, w[i][1].w, hi.w, mid.w, lo.w);
+                uint4* to = reinterpret_cast<uint4*>(sm.w[s]) + wrow * 8;
+                to[j8 ^ r8] = hi;
+                to[(4 + j8) ^ r8] = mid;
+                reinterpret_cast<uint4*>(sm.w_lo[s])[wrow * 4 + (j8 ^ (r8 >> 1 & 3))] = lo;
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -287,33 +327,40 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             return true;
         };
         const int team = part >> 1;
-        int it = 0;
-        if (total > 0 && team == 0) ok = split(0);
+        int it = 0, run = 0;
+        if (team < total) ok = split(team);
         for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
             float2x sum[CW / 2];
 #pragma unroll
             for (int i = 0; i < CW / 2; ++i) sum[i] = 0ull;
             int run_end = begin + g.group;
             for (int st = begin; st < end; ++st, ++it) {
-                if (it + 1 < total && team == ((it + 1) & 1)) ok = split(it + 1);
-                const int buf = it & 1;
-                ok = ok && mbar_wait(&sm.acc_full[buf], (uint32_t)(it >> 1 & 1));
+                if (it + AHEAD < total && team == (it & 1)) ok = split(it + AHEAD);
+                ok = ok && mbar_wait(&sm.acc_full, (uint32_t)(it & 1));
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (rows_here) {
+                auto add = [&](uint32_t column) {        // an accumulator's columns of this warp onto the sums
+                    if (!rows_here) return;
                     uint32_t r[CW];
 #pragma unroll
-                    for (int c = 0; c < CW; c += 8) tmem_ld_x8_nowait(lanes + (uint32_t)(buf * BN + part * CW + c), r + c);
+                    for (int c = 0; c < CW; c += 8) tmem_ld_x8_nowait(lanes + column + (uint32_t)(part * CW + c), r + c);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
                     for (int i = 0; i < CW / 2; ++i)
-                        sum[i] = pair_fma(pair_of_floats(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])),
-                                          pair_of_floats(FC_GIVE_BACK, FC_GIVE_BACK), sum[i]);
-                }
+                        sum[i] = pair_add(sum[i], pair_of_floats(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])));
+                };
+                add(0u);
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&sm.acc_empty[buf]);
-                if (RUNS && st + 1 == run_end && st + 1 != end) {                // a run is complete: onto those before it
+                if (lane == 0) mbar_arrive(&sm.acc_empty);
+                if (st + 1 == run_end || st + 1 == end) {                        // a run is complete: its small products
+                    add((uint32_t)(COL_SMALL + run % SMALL * BN));
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&sm.small_empty[run % SMALL]);
+                    ++run;
+                }
+                if (!CUT && st + 1 == run_end && st + 1 != end) {                // onto the runs before it
                     float2x* at = reinterpret_cast<float2x*>(patch) + lane;
 #pragma unroll
                     for (int i = 0; i < CW / 2; ++i) {
@@ -324,7 +371,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 }
             }
             if (!ok) break;
-            if (RUNS && g.runs > 1) {
+            if (!CUT && g.runs > 1) {
                 const float2x* at = reinterpret_cast<const float2x*>(patch) + lane;
 #pragma unroll
                 for (int i = 0; i < CW / 2; ++i) sum[i] = pair_add(at[32 * i], sum[i]);
@@ -355,7 +402,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         if (!ok && lane == 0) atomicExch(g.status, 3);
     }
     if constexpr (CUT) {
-        static_assert(sizeof(sm.a) + sizeof(sm.w_hi) + sizeof(sm.w_lo) >= FC_BM * BN * sizeof(float), "room for a run's sums");
+        static_assert(sizeof(sm.a) + sizeof(sm.w) + sizeof(sm.w_lo) >= FC_BM * BN * sizeof(float), "room for a run's sums");
         ok = __all_sync(0xffffffffu, ok);
         fc_cluster_sync();                               // every run's sums are in its block's shared memory
         if (warp >= 2 && ok) {
@@ -391,12 +438,12 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
 }
 
-template <int BN, int STAGES, bool RUNS, bool CUT>
+template <int BN, int STAGES, bool CUT>
 int launch_f32_tc(const FcArgs& g, int act, int sms, cudaStream_t s) {
     CUtensorMap map_a, map_w;
     if (!tensor_map_f32(&map_a, g.A, g.M, g.K, g.lda, FC_BM) || !tensor_map_f32(&map_w, g.W, g.N, g.K, g.ldw, BN)) return MU_ERR_LAUNCH;
-    auto kernel = gemm_f32_tc_kernel<BN, STAGES, RUNS, CUT>;
-    const size_t smem = sizeof(FcSmem<BN, STAGES, RUNS>) + 1024;
+    auto kernel = gemm_f32_tc_kernel<BN, STAGES, CUT>;
+    const size_t smem = sizeof(FcSmem<BN, STAGES, CUT>) + 1024;
     if (!allow_shared(reinterpret_cast<const void*>(kernel), smem)) return MU_ERR_LAUNCH;
     prefer_shared_memory(reinterpret_cast<const void*>(kernel));
     const long long tiles = (long long)((g.M + FC_BM - 1) / FC_BM) * ((g.N + BN - 1) / BN);
@@ -410,11 +457,11 @@ int fc_clusters(int runs) {
     static std::atomic<int> known[FC_RUNS + 1];
     int n = known[runs].load(std::memory_order_relaxed);
     if (n != 0) return n;
-    auto kernel = gemm_f32_tc_kernel<BN, STAGES, false, true>;
+    auto kernel = gemm_f32_tc_kernel<BN, STAGES, true>;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(1, runs);
     cfg.blockDim = dim3(FC_THREADS);
-    cfg.dynamicSmemBytes = sizeof(FcSmem<BN, STAGES, false>) + 1024;
+    cfg.dynamicSmemBytes = sizeof(FcSmem<BN, STAGES, true>) + 1024;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 1;
@@ -452,39 +499,39 @@ MU_EXPORT int mu_gemm_f32_tc(const void* A, const void* W, const float* bias, co
     const mu::FcArgs g = {(const float*)A, (const float*)W, bias, residual, (float*)C, M, N, K, lda, ldw, ldc, ldr, status,
                           group, runs};
     cudaStream_t s = (cudaStream_t)stream;
-#define MU_FC_ALL(DO) DO(32, 7, 6) DO(64, 6, 5) DO(96, 5, 4) DO(128, 4, 3) DO(160, 3, 3)
-    // The width, and whether to cut, by what the SM that ends last has to do, in microseconds: a step took 0.42 (32 columns), 0.67
-    // (96), 0.80 (128) and 1.0 (160), handing the sums over 4.
+    // (columns of a tile, stages of the ring if it is cut and if not)
+#define MU_FC_ALL(DO) DO(32, 8, 8) DO(64, 7, 6) DO(96, 6, 5) DO(128, 5, 4) DO(160, 4, 3)
+    // The width, and whether to cut, by what the SM that ends last has to do, in microseconds: a step and a tile's end as below, a
+    // launch 3, a further round of clusters 2.5 (fitted to one to three rounds of 192 to 768 of k; a cut tile's end, spread over its
+    // cluster, is 0.6 of it; uncut tiles of 160 have three stages for three steps).  777 x 3,072 x 768 takes 37 us of 160, uncut,
+    // and 48 of the next best form, 777 x 768 x 768 15.4 of 96, cut, and 20, 8 x 3,072 x 768 11.5 of 64, cut, and 16.
     int best = 0, best_cut = 0;
     double best_cost = 0.0;
-    const int widths[5] = {32, 64, 96, 128, 160};
+    const struct { int width; double step, step_cut, end; } forms[5] = {
+        {32, 0.50, 0.48, 1.4}, {64, 0.63, 0.56, 2.6}, {96, 0.75, 0.71, 4.2}, {128, 0.86, 0.79, 4.4}, {160, 1.20, 1.04, 7.3}};
     for (int i = 0; i < 5; ++i) {
-        const int bn = widths[i];
+        const int bn = forms[i].width;
         if (tile ? bn != tile : bn > 32 && bn - 32 >= N) continue;
         const long long tiles = m_tiles * ((N + bn - 1) / bn);
         for (int c = 0; c < 2; ++c) {
             if (c == 1 && (cut == 0 || runs == 1)) continue;
-            if (c == 0 && runs > 1 && bn == 160) continue;           // (no registers for both sums)
             long long at_once = sms;
             if (c == 1) {
-#define MU_FC_CLUSTERS(BN, ST, ST_RUNS) if (bn == BN) at_once = mu::fc_clusters<BN, ST>(runs);
+#define MU_FC_CLUSTERS(BN, ST_CUT, ST) if (bn == BN) at_once = mu::fc_clusters<BN, ST_CUT>(runs);
                 MU_FC_ALL(MU_FC_CLUSTERS)
 #undef MU_FC_CLUSTERS
                 if (at_once <= 0) continue;
             }
-            const long long rounds = (tiles + at_once - 1) / at_once;
-            double cost = rounds * ((c ? group : steps) * (0.28 + 0.0045 * bn) + 1.0 + 0.01 * bn) + (c ? 4.0 : 0.0);
+            const double rounds = (double)((tiles + at_once - 1) / at_once);
+            double cost = c ? rounds * (group * forms[i].step_cut + 0.6 * forms[i].end + 2.5) + 0.5
+                            : rounds * (steps * forms[i].step + forms[i].end) + 3.0;
             if (c == 1 && cut == 1) cost *= 1e-6;
             if (best == 0 || cost < best_cost) best = bn, best_cut = c, best_cost = cost;
         }
     }
-    if (best == 0) best = tile == 160 ? 128 : tile, best_cut = 0;
-#define MU_FC(BN, ST, ST_RUNS)                                                                                         \
-    if (best == BN) {                                                                                                  \
-        if (best_cut) return mu::launch_f32_tc<BN, ST, false, true>(g, act, sms, s);                                   \
-        if (runs == 1) return mu::launch_f32_tc<BN, ST, false, false>(g, act, sms, s);                                 \
-        if constexpr (BN < 160) return mu::launch_f32_tc<BN, ST_RUNS, true, false>(g, act, sms, s);                    \
-    }
+#define MU_FC(BN, ST_CUT, ST)                                                                                          \
+    if (best == BN)                                                                                                    \
+        return best_cut ? mu::launch_f32_tc<BN, ST_CUT, true>(g, act, sms, s) : mu::launch_f32_tc<BN, ST, false>(g, act, sms, s);
     MU_FC_ALL(MU_FC)
 #undef MU_FC
 #undef MU_FC_ALL

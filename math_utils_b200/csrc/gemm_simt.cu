@@ -1,7 +1,7 @@
 // C[M, N] = act(A[M, K] . W[N, K]^T + bias[N]) (+ residual[M, N]) on CUDA cores.
 //
 // This is the 32-bit matrix product of the library in float32 multiply-adds (for
-// short k and any shape; over a longer k gemm_f32_tc.cu has it) and also the
+// short k and any shape; from 384 of k on gemm_f32_tc.cu has it) and also the
 // any-shape fallback of the bfloat16 path.  Every output element is one
 // running sum over k = 0..K-1 in order, whatever M is and wherever the row
 // lies in the batch, so a row's result does not depend on what else is in the
@@ -9,7 +9,7 @@
 // (include/ai/LocalModel.hpp:1052-1126; include/ai/Kernels.hpp:184-207, 315-430).
 //
 // That is the first kernel, which takes any type, stride and size.  The second (gemm_f32_tile) takes float32 operands whose
-// rows are whole 16-byte pieces: the 32-bit path's products up to k = 188.  Its sums are four, over the k of every fourth
+// rows are whole 16-byte pieces: the 32-bit path's products up to k = 380.  Its sums are four, over the k of every fourth
 // run of eight, added in order at the end: as independent of the rest of the step, and no less exact.  It is bound by the
 // FMA pipes (2 m n k / 73 TFLOP/s) and next by how few warps share a scheduler: a small thread tile needs too many
 // shared-memory reads, and the large one that needs few leaves two (80 rows) to four of them, which issue in 45 to 59 % of the

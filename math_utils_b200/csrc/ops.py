@@ -1571,8 +1571,8 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = N
 def gemm_f32_tc(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
                 act: Optional[str] = None, residual: Optional[torch.Tensor] = None,
                 out: Optional[torch.Tensor] = None, tile: int = 0, cut: int = -1) -> torch.Tensor:
-    """The 32-bit product on tensor cores (three TF32 products a pair, float32 sums): float32 operands whose rows are whole
-    16-byte pieces.  ``tile`` (columns of a tile) and ``cut`` (1: a block a run of k) change no bit of the result."""
+    """The 32-bit product on tensor cores (operands as three bfloat16 numbers that are together exactly them, eight products a
+    pair, float32 sums): float32 operands whose rows are whole 16-byte pieces.  ``tile`` (columns of a tile) and ``cut`` (1: a block a run of k) change no bit of the result."""
     if a.dtype != torch.float32 or w.dtype != torch.float32 or (out is not None and out.dtype != torch.float32):
         raise KernelError("gemm_f32_tc takes float32")
     m, n, k, out = _gemm_args(a, w, bias, residual, out, torch.float32)
@@ -2104,18 +2104,21 @@ def prompt_layer(args: PromptLayerArgs) -> None:
 
 
 # -------------------------------------------------------------------- dispatch
-# float32 products over at least this much of k run on tensor cores: there their error against float64 is the smaller (2-norm,
-# normal values: k = 128 1.09e-7 against 1.11e-7 of the multiply-adds, 192 1.13 and 1.32, 768 1.37 and 2.52, 3072 1.43 and
-# 4.98), and they are no slower (1 x 64 x 512 11.8 us and 13.8, 8 x 3072 x 768 14.7 and 19, 2000 x 768 x 192 12 and 25).
-F32_TC_K = 192
+# float32 products over at least this much of k run on tensor cores: with a smaller error against float64 for all but rows of
+# positive values of which a few carry the sum (gemm_f32_tc.cu).  Of 1 to 777 rows and 4 to 50,257 columns, microseconds against
+# multiply-adds: k = 192 is slower in half of the sizes (1 x 4,096 6.9 and 5.7, 1 x 50,257 29 and 22), 256 with many columns
+# (8 x 4,096 7.7 and 7.1, 8 x 50,257 34 and 28), 384 with 50,257 columns and up to 16 rows (44 and 39 to 41), 512 and more nowhere
+# (1 x 768 x 768 9.0 and 17, 8 x 4,096 x 2,048 20 and 43, 777 x 4,096 x 768 54 and 137).
+F32_TC_K = 384
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None,
            act: Optional[str] = None, residual: Optional[torch.Tensor] = None,
            out: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
     """act(x @ weight^T + bias) + residual through the kernel that fits the
-    dtype and the shape.  float32 operands take the three-term tensor-core product from 192 of k on and the CUDA-core
-    kernel below (by k alone, so that a row's bits do not depend on the rows beside it).
+    dtype and the shape.  float32 operands whose rows are whole 16-byte pieces take the three-term tensor-core product from
+    384 of k on, and the CUDA-core kernel below (by k alone, so that a row's bits do not depend on the rows beside it); rows
+    that lie otherwise take that kernel's form for any alignment, as ever with sums of another order.
     ``x`` may be a ``NormedInput``: with few rows and bfloat16 weights the norm is
     made inside the product kernel, otherwise it is computed first."""
     if isinstance(x, NormedInput) and weight.dtype == torch.bfloat16 and _rows_kernel(x.n_rows, *weight.shape):

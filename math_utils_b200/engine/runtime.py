@@ -16,8 +16,9 @@ class Runtime:
     """``dtype`` is the compute dtype: bfloat16 (the serving path: bfloat16
     weights, activations and cache, float32 accumulation, norms, softmax and
     residual stream) or float32 (everything in true 32-bit: products by float32
-    multiply-adds or, over a long k, of three terms on tensor cores with no
-    larger an error)."""
+    multiply-adds or, over a long k, on tensor cores from operands cut into
+    three bfloat16 numbers that are together exactly them, with an error no
+    larger than the multiply-adds')."""
     dtype: torch.dtype
     device: torch.device
 

@@ -2,7 +2,8 @@
 
 ``y = act(x @ W^T + b) (+ residual)`` with ``W`` kept ``[out, in]``.  Which
 kernel runs is decided here from the compute dtype and the number of rows:
-float32 always takes the CUDA-core kernel (the true 32-bit path); bfloat16
+float32 takes the CUDA-core kernel or, over a long k, the tensor-core one that
+holds whole float32 operands (the true 32-bit path); bfloat16
 takes the tensor-core kernels where the shape allows them and the CUDA-core
 kernel otherwise.  The reference's counterpart is ``Weight`` + ``apply``
 (include/ai/LocalModel.hpp:989-1126).
