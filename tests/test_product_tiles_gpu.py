@@ -131,6 +131,7 @@ def test_float32_tensor_tiles_pass_on_what_is_not_finite():
     ops = _ops()
     a, w = _rand((150, 800), 1), _rand((70, 800), 2)
     a[3, 5], a[70, 100], a[149, 0], w[7, 3], w[9, 9] = float("inf"), float("nan"), 3.4e38, -float("inf"), 1e30
+    a[90, 799], a[91, 798], a[91, 2] = float("nan"), -float("inf"), float("inf")           # (found at the end; two infinities)
     want = ops.gemm_simt(a, w)
     for cut in (0, 1):
         got = ops.gemm_f32_tc(a, w, cut=cut)
