@@ -121,6 +121,13 @@ static bool make_map_uncached(CUtensorMap* map, const void* base, long long rows
 
 }  // namespace mu
 
+// The status word of the current device, zero at first: a variable of the library, so that it is there without an allocation,
+// inside a capture too.
+static __device__ int status_of_device;
+MU_EXPORT int mu_status_word(void** address) {
+    return cudaGetSymbolAddress(address, status_of_device) == cudaSuccess ? MU_OK : MU_ERR_LAUNCH;
+}
+
 // Gives the product kernel room for products that are cut along K (few tiles of C, long K): `parts` takes
 // the partial tiles (float32, 16-byte aligned), `tickets` n_tickets counters that are zero now and are left
 // zero by every launch.  Without it, or where it is too small, such products run uncut.

@@ -60,6 +60,7 @@ _SIGNATURES = {
                      _c_int, _c_int, _c_int, _c_p],
     "mu_gemm_skinny": [_c_p, _c_p, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_ll, _c_ll, _c_ll, _c_ll,
                        _c_int, _c_int, _c_p],
+    "mu_status_word": [_c_p],
     "mu_gemm_tc_split_workspace": [_c_p, _c_ll, _c_p, _c_int],
     "mu_gemm_tc": [_c_p, _c_p, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_ll, _c_ll, _c_ll, _c_ll,
                    _c_int, _c_int, _c_int, _c_int, _c_p, _c_p],
@@ -1583,16 +1584,31 @@ def gemm_f32_tc(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] =
     return out
 
 
-_status = {}
+_status = {}           # by device name; by the device itself once the room for cut products is there too
+
+
+class _LibraryWord:
+    """A 32-bit word of the library's own device memory, for ``torch.as_tensor``."""
+    def __init__(self, address: int):
+        self.__cuda_array_interface__ = {"shape": (1,), "typestr": "<i4", "data": (address, False), "version": 2}
 
 
 def status_word(device) -> torch.Tensor:
     """A device word that kernels with bounded waits write to when a wait runs
-    out (it stays 0 otherwise); ``check_status`` reads it."""
+    out (it stays 0 otherwise); ``check_status`` reads it.  It needs no
+    allocation: a first call inside a capture gets the word that every other does."""
     word = _status.get(device)
     if word is None:
-        word = _status[device] = _status[str(device)] = torch.zeros(1, dtype=torch.int32, device=device)
-        _split_workspace(device)
+        device = torch.device(device)
+        word = _status.get(str(device))
+        if word is None:
+            address = ctypes.c_void_p()
+            with torch.cuda.device(device):
+                _check(library().mu_status_word(ctypes.byref(address)), "status_word", launches=0)
+                word = _status[str(device)] = torch.as_tensor(_LibraryWord(address.value), device=device)
+        if not torch.cuda.is_current_stream_capturing():
+            _split_workspace(device)
+            _status[device] = word
     return word
 
 
@@ -1608,7 +1624,8 @@ def _split_workspace(device) -> None:
     """Room for tensor-core products that are cut along k (few output tiles,
     long k: a batch of 33 to 128 single tokens): partial tiles for one tile per
     SM at the widest tile, and a ticket per tile.  Set once per device, at the
-    first use of a kernel with a status word, hence never inside a capture."""
+    first use of a kernel with a status word outside a capture (until then such
+    products run uncut)."""
     parts = scratch("gemm_tc_parts", device, sm_count(device) * 128 * 256, torch.float32)
     tickets = zeroed_workspace("gemm_tc_tickets", device, 4 * 1024)
     _check(library().mu_gemm_tc_split_workspace(parts.data_ptr(), parts.numel() * 4, tickets.data_ptr(),
@@ -2185,8 +2202,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
                               _is_bf16(out), 0, -1, status_word(x.device).data_ptr(), _stream()),
                ("gemm_tc({}x{}x{})", m, n, k))
     elif (dtype == torch.float32 and out.dtype == torch.float32 and k >= F32_TC_K and k % 4 == 0 and lda % 4 == 0
-          and ldw % 4 == 0 and pa % 16 == 0 and pw % 16 == 0
-          and (x.device in _status or not torch.cuda.is_current_stream_capturing())):   # (its workspace is made outside captures)
+          and ldw % 4 == 0 and pa % 16 == 0 and pw % 16 == 0):
         _check(lib.mu_gemm_f32_tc(pa, pw, pb, pr, out.data_ptr(), m, n, k, lda, ldw, out.stride(0), ldr, code, 0, -1,
                                   status_word(x.device).data_ptr(), _stream()), ("gemm_f32_tc({}x{}x{})", m, n, k))
     else:

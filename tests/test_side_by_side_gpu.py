@@ -1,5 +1,9 @@
 """32-bit products at work on two streams at once: launches share nothing in device memory, so the results have the bits of
 the same launches one after the other."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
@@ -108,3 +112,36 @@ def test_float32_steps_with_members_side_by_side(monkeypatch):
             alone, beside = steps(0, replayed), steps(32, replayed)
             assert all(torch.equal(a, b) for a, b in zip(alone, beside)), (n, replayed)
     ops.check_status()
+
+
+def test_first_product_of_a_process_inside_a_capture():
+    """A float32 product is the same kernel whatever the process has run before: recorded as its first launch, then eager."""
+    code = """
+import torch
+from math_utils_b200.csrc import ops
+g = torch.Generator(device="cuda").manual_seed(1)
+a, w = torch.randn((40, 768), generator=g, device="cuda"), torch.randn((300, 768), generator=g, device="cuda")
+out = torch.zeros((40, 300), device="cuda")
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    ops.linear(a, w, out=out)
+for _ in range(3):
+    out.zero_()
+    graph.replay()
+    eager = ops.linear(a, w)
+    assert torch.equal(out, eager) and torch.equal(eager, ops.gemm_f32_tc(a, w))
+x, y = a.bfloat16().repeat(4, 1), w.bfloat16()
+assert torch.equal(ops.linear(x, y), ops.gemm_tc(x, y))
+word = ops.status_word(a.device)
+assert word.data_ptr() == ops.status_word("cuda:0").data_ptr() and int(word) == 0
+word.fill_(2)
+try:
+    ops.check_status()
+    raise SystemExit("no error for a wait that ran out")
+except ops.KernelError as e:
+    assert "tensor cores" in str(e)
+ops.check_status()
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    proc = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
+    assert proc.returncode == 0, proc.stdout + proc.stderr
