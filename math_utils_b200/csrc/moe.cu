@@ -538,7 +538,7 @@ MU_EXPORT int mu_moe_route(const void* h, long long ldh, int h_bf16, const float
 #define MU_ROUTE(T, TOK, WARPS, NE, SHARED, GRID, CLUSTER)                                                             \
     do {                                                                                                               \
         auto kernel = mu::moe_route_kernel<T, TOK, WARPS, NE, SHARED>;                                                 \
-        if (!mu::allow_shared(reinterpret_cast<const void*>(kernel), TOK > 1 ? mu::ROUTE_SMEM : 0)) return MU_ERR_LAUNCH; \
+        if (!mu::allow_shared(reinterpret_cast<const void*>(kernel), (TOK > 1 ? mu::ROUTE_SMEM : 48 * 1024) + 16)) return MU_ERR_LAUNCH; \
         return mu::launch_pdl(kernel, GRID, dim3(WARPS * 32), room(TOK), s, CLUSTER, (const T*)h, ldh, router, correction, \
                               n_tokens, hidden, n_experts, top, scale, softmax, renormalize, expert_of, weight_of, renorm_eps, \
                               gate_w, gate_out);                                                                       \
@@ -553,12 +553,15 @@ MU_EXPORT int mu_moe_route(const void* h, long long ldh, int h_bf16, const float
     // token the router came out of the L2 once per token), as many as there is room for
     const int sms = mu::sm_count();
     if (sms <= 0) return MU_ERR_LAUNCH;
-    if (n_tokens >= 4 * sms) {
+    // widths: what one token in 48 KB as float32, or two of many in ROUTE_SMEM, leave room for (16 bytes more where a row's end is
+    // rounded up), whatever the rows' type
+    const bool many = n_tokens >= 4 * sms;
+    if (many ? limit(2) > mu::ROUTE_SMEM : limit(1) > 48 * 1024) return MU_ERR_UNSUPPORTED_SIZE;
+    if (many) {
         if (room(7) <= mu::ROUTE_SMEM) MU_ROUTE_MANY(7, 16, 2);
         if (room(4) <= mu::ROUTE_SMEM) MU_ROUTE_MANY(4, 16, 2);
-        if (room(2) <= mu::ROUTE_SMEM) MU_ROUTE_MANY(2, 16, 1);
+        MU_ROUTE_MANY(2, 16, 1);
     }
-    if (limit(1) > 48 * 1024) return MU_ERR_UNSUPPORTED_SIZE;     // (one token takes no more than 48 KB, as it always did)
     // few tokens: a block each, or a cluster of blocks that share the experts while these blocks find an SM
     const int rows = n_experts + (gate_w ? 1 : 0);
     const int shares = rows <= 16 ? 1 : n_tokens <= sms / 2 ? 8 : n_tokens <= sms ? 4 : 1;

@@ -316,3 +316,24 @@ def test_router_of_few_tokens_by_clusters(tokens):
         return expert, weight
 
     assert all(torch.equal(few, many[:tokens * 4]) for few, many in zip(route(h[:tokens]), route(h)))
+
+
+# the widest rows: one token's 12,288 values with the scores of its experts twice, two of many tokens 25,600; rows that end off a
+# 16-byte boundary
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("tokens,experts,hidden", [(1, 7, 12274), (20, 24, 12240), (592, 7, 12786), (592, 24, 12752)])
+def test_router_takes_the_widths_it_took(tokens, experts, hidden, dtype):
+    ops = _ops()
+
+    def route(width):
+        h, router = _rand((tokens, width), 1, dtype), _rand((experts, width), 2, scale=width ** -0.5)
+        expert, weight = torch.zeros(tokens * 2, dtype=torch.int32, device="cuda"), torch.zeros(tokens * 2, device="cuda")
+        ops.moe_route(h, router, None, 2, 1.0, expert, weight)
+        top = torch.topk(h.double() @ router.double().T, 2)
+        # (float32 logits: a pair closer than their error may fall either way)
+        sure = (top.values[:, 0] - top.values[:, 1]) > 1e-3
+        assert torch.equal(expert.view(tokens, 2)[sure, 0].long(), top.indices[sure, 0])
+
+    route(hidden)
+    with pytest.raises(ops.KernelError):
+        route(hidden + 2)
