@@ -276,9 +276,10 @@ def test_grouping_of_pairs(P, experts, real, rows):
     assert n == len(want) and [tuple(t) for t in info[:n]] == want
 
 
-# eight, four and two tokens a block (what the staged rows leave room for), a block's tokens cut off, an odd number of rows
-@pytest.mark.parametrize("tokens,hidden,experts,gate", [(601, 256, 64, True), (700, 2048, 17, False), (650, 4096, 16, True),
-                                                        (593, 6200, 5, True)])
+# seven, eight (1,100 are two rounds of seven), four and two tokens a block (what the staged rows leave room for), a block's tokens
+# cut off, an odd number of rows
+@pytest.mark.parametrize("tokens,hidden,experts,gate", [(601, 256, 64, True), (1100, 260, 65, True), (700, 2048, 17, False), (650, 4096, 16, True),
+                                                        (593, 6200, 5, True), (600, 8200, 5, True), (595, 12600, 9, False)])
 def test_router_of_several_tokens_a_block(tokens, hidden, experts, gate):
     """Each logit a float32 sum of `hidden` terms in 128 parts: scores within 1e-5; and the bits that a token alone gives."""
     ops = _ops()
