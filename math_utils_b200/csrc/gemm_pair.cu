@@ -3,9 +3,9 @@
 //
 // What bounds the one-SM product at these sizes is the bytes an SM takes in from the L2 (16 KB of A and BN x 128 bytes of W for
 // 64 of k).  In a pair every SM loads its own rows of A and HALF of W's rows, and tcgen05.mma.cta_group::2, which the first
-// block issues, reads both halves: 32 KB for 128 x 256 x 64 instead of 48.  Once that is fed its products run near the
-// instruction's rate (128 cycles for 256 x 256 x 16) in either form; a pair's launch costs about 1 us more, so small products
-// stay with one SM (the rule, with both sides: gemm_tc.cu).
+// block issues, reads both halves: 32 KB for 128 x 256 x 64 instead of 48.  4,096 x 4,096 x 2,048
+// in one launch of each: tensor pipe active in 81 % of the SMs' cycles, by single SMs in 74.  A pair's launch costs about 1 us
+// more, so small products stay with one SM (the rule, with both sides: gemm_tc.cu).
 //
 // Roles in each block: warp 0 loads its share of every stage; both blocks' copies count on the FIRST block's "full" barrier.  Warp
 // 1 allocates tensor memory (all 128 lanes of both SMs, two accumulators of BN columns); the first block's warp 1 issues

@@ -1,4 +1,4 @@
-// Pieces of the products by pairs of SMs (clusters of two blocks, tcgen05 with cta_group::2): gemm_pair.cu, moe_tc.cu.
+// Pieces of the products by pairs of SMs (clusters of two blocks, tcgen05 with cta_group::2): gemm_pair.cu.
 #pragma once
 #include "gemm_tc_kernel.cuh"
 

@@ -162,8 +162,9 @@ MU_EXPORT int mu_gemm_tc(const void* A, const void* W, const float* bias, const 
     const long long m_tiles = (M + mu::TC_BM - 1) / mu::TC_BM;
     // Tile width, and one SM or a pair a tile: by what the SM that ends last has to do, in microseconds.  A launch costs `fixed` (to
     // the first product and from the last one to the end), a tile 64 of k `step` each or its epilogue, whichever is longer
-    // (float32 1.3 of bfloat16's).  The figures are fitted to 28 sizes from 130 x 1,024 x 64 to 8,192^3, both output types: what
-    // they choose is 0.2 % from the best width on average.  Pairs pay for large tiles, which they feed with fewer bytes, and in
+    // (float32 1.3 of bfloat16's).  The figures are fitted to 28 sizes from 130 x 1,024 x 64 to 8,192^3, both output types.  Of 84
+    // other sizes (1,000 to 16,384 rows, and 30 drawn ones) and both types what they choose is 0.5 % from the best form on average
+    // and 10 % at most (16,384 x 768 x 768, float32).  Pairs pay for large tiles, which they feed with fewer bytes, and in
     // their launch: 2,048 x 1,344 x 2,048 14.8 -> 13.1 us, 2,048 x 1,600 x 6,400 41 -> 31, 4,096^3 116 -> 102 (1,347 TFLOP/s).
     const struct { int tile; double fixed, step, epilogue; } forms[6] = {
         {64, 2.8, 0.155, 1.15}, {128, 3.1, 0.21, 2.0}, {256, 4.5, 0.315, 2.8},

@@ -14,9 +14,10 @@
 // whole boxes.  The items' order (tiles_first) keeps an expert's tiles close together, so the weights cross from
 // memory once.
 //
-// What bounds it: the weights' bytes, and with hundreds of rows an expert their products beside them, a quarter of the tiles'
-// rows empty.  Measured (B200): 64 experts of 2,048 x 1,408 x 3, 12,288 pairs, both products: mma.sync with 64 rows a block
-// 943 us; tiles of 128 slots 338, tile by tile 297 (the weights alone take 113 + 56 us); the gather ~10 us; 48 pairs over those
+// What bounds it: with few rows an expert the weights' bytes; with hundreds the operands' way from the L2, 48 KB for every 128 x
+// 256 x 64 step, some 11 TB/s, a quarter of the tiles' rows empty.  Measured (B200): 64 experts of 2,048 x 1,408 x 3, 12,288
+// pairs, the same number for every expert, both products: mma.sync with 64 rows a block 943 us; tiles of 128 slots 338 (220 + 119),
+// tile by tile 297 (190 + 106; the weights' bytes alone take 113 + 56); the gather ~10 us; 48 pairs over those
 // experts with two matrices each, the whole feed-forward 136 -> 93 us.  Tiles of 256 slots by pairs of SMs (cta_group::2)
 // took 263 us with equal experts, but where routing loads them unequally their emptier tiles cost what the feeding saves
 // (the whole feed-forward 447 us against 436).  Per head, 16 heads, 2,048 rows, the launch alone: 512 x 128 36 -> 25 us, 128 x 512 26 -> 9;
@@ -238,7 +239,8 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 // and the items go tile by tile, all its column blocks together (an expert's tiles still follow one another).  64 experts
 // of 2,048 x 1,408 x 3, pairs and their rows' megabytes, microseconds of the first product by column blocks and by tiles:
 // 1,024 (4) 132 and 131, 4,096 (17) 138 and 131, 6,144 (25) 146 and 136, 12,288 (50) 220 and 191; of two matrices 68 and 70,
-// 72 and 76, 82 and 72, 128 and 109.
+// 72 and 76, 82 and 72, 128 and 109.  The line, an eighth of the L2, lies between the two middle ones; seven other shapes (8 to 48
+// experts of 768 to 4,096 x 512 to 4,096, rows of 4 to 98 MB) in two forms took 0.99 to 1.19 times less than by column blocks.
 constexpr long long GROUPED_ROWS_KEPT = 17000000;
 inline bool tiles_first(long long rows, int k) { return rows * k * 2 > GROUPED_ROWS_KEPT; }
 
