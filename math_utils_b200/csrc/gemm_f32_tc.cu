@@ -22,7 +22,8 @@
 // 0.79 us, some 1,500 cycles: its products need 1,024, its bytes through shared memory 1,190 at 128 a cycle (fill, split, W's
 // parts eight times), its instructions about half; none is the bound alone (tensor pipe active in 36 to 46 % of a whole launch's
 // cycles, issue in 46 to 52 %).  The warps' chain from load to arrival lies over them: two teams of eight split every other step,
-// two steps ahead (one step ahead: 0.92).  Others: 0.48 us (32 columns), 0.56 (64), 0.71 (96), 1.04 (160).  Measured (B200, microseconds; the multiply-adds in
+// two steps ahead (one step ahead: 0.92).  Eighteen warps leave 96 registers each: uncut tiles of 128 columns spill 128 bytes, of 64
+// 36 and of 160 20, cut ones of the same steps, whose ends take eight columns a warp at a time, 4 bytes at most.  Others: 0.48 us (32 columns), 0.56 (64), 0.71 (96), 1.04 (160).  Measured (B200, microseconds; the multiply-adds in
 // brackets): 777 x 3072 x 768 37 (121), 777 x 768 x 768 15.4 (34), 777 x 768 x 3072 44 (129), 2048 x 4096 x 4096 475 (1,700; 145
 // TFLOP/s), 8 x 3072 x 768 11.6 (17.5), 8 x 768 x 3072 14 (66).
 //
